@@ -428,7 +428,7 @@ int xb_get_counters(xb_engine* e, xb_counters* out);
 
 /* Kernel-level test hook: y[T,N] (fp32) = x[T,K] * w[N,K]^T on device buffers.
  * use_tensor_cores = 1 runs the tcgen05 kernel the engine uses (force_splits > 0 pins the
- * K split count; round_bf16 rounds like nn.Linear), 0 runs the CUDA-core checker kernel.
+ * K split count, above 128 rows the number, from 1, of the tile variant; round_bf16 rounds like nn.Linear), 0 runs the CUDA-core checker kernel.
  * scratch: device fp32, at least 16*T*N elements. */
 int xb_debug_linear(const void* x, const void* w, int T, int N, int K, float* y, float* scratch,
                     int use_tensor_cores, int force_splits, int round_bf16, void* stream);

@@ -3,6 +3,7 @@
 #include "../../include/xb200.h"
 #include "xb_common.cuh"
 #include "xb_gemm.cuh"
+#include "xb_wide.cuh"
 #include "xb_loader.cuh"
 #include "xb_kernels.cuh"
 #include "xb_attn_mma.cuh"
@@ -764,7 +765,8 @@ static int get_plan(xb_engine* e, int site, int layer, const bf16* x, long long 
     GemmPlan p;
     // (a decode Linear is one block per SM; SMs set aside with xb_reserve_sms stay free for a resident communication kernel)
     const int sms = (T <= 128 && e->reserved_sms > 0 && e->reserved_sms < e->num_sms) ? e->num_sms - e->reserved_sms : e->num_sms;
-    XB_TRY(xb_gemm_plan(&p, x, ldx, w, 1, T, N, K, out, ld_out, bias, round_bf16, sms, 0));
+    const int col_unit = site == SITE_QKV && e->d.rope_kind == XB_ROPE_HALF_SPLIT ? e->d.head_dim : 32;
+    XB_TRY(xb_gemm_plan(&p, x, ldx, w, 1, T, N, K, out, ld_out, bias, round_bf16, sms, 0, col_unit));
     if (p.args.mode == XB_GEMM_WIDE && site == SITE_QKV) {
       // prefill: bias + RoPE + q store + paged-KV append happen in the GEMM epilogue
       const xb_model_desc& d = e->d;

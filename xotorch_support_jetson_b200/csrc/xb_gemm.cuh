@@ -121,7 +121,7 @@ struct GemmCfg {
 };
 
 
-// ---- WIDE epilogues: one thread = one token row `t`, TMEM chunks of 16 consecutive columns ----
+// ---- pieces of the WIDE epilogues (xb_wide.cuh) ----
 __device__ __forceinline__ void epi_store16(bf16* dst, const float* x) {
   uint4 p0, p1;
   p0.x = f2_to_bf2(x[0], x[1]);   p0.y = f2_to_bf2(x[2], x[3]);
@@ -130,15 +130,6 @@ __device__ __forceinline__ void epi_store16(bf16* dst, const float* x) {
   p1.z = f2_to_bf2(x[12], x[13]); p1.w = f2_to_bf2(x[14], x[15]);
   reinterpret_cast<uint4*>(dst)[0] = p0;
   reinterpret_cast<uint4*>(dst)[1] = p1;
-}
-// nn.Linear rounding point: bf16(acc + bias)
-__device__ __forceinline__ void epi_linear16(const GemmArgs& g, const uint32_t* v, int n0, float* x) {
-#pragma unroll
-  for (int j = 0; j < 16; ++j) {
-    float a = __uint_as_float(v[j]);
-    if (g.bias != nullptr) a += bf2f(g.bias[n0 + j]);
-    x[j] = rbf(a);
-  }
 }
 // where 16 elements [e, e+16) of fused-QKV head `head` of token row t go: q buffer or the paged cache
 __device__ __forceinline__ bf16* epi_qkv_dst(const GemmArgs& g, int t, int pos, int head, int e) {
@@ -152,94 +143,8 @@ __device__ __forceinline__ bf16* epi_qkv_dst(const GemmArgs& g, int t, int pos, 
   return pool + (((long long)page * KV + kvh) * g.page_tokens + off) * hd + e;
 }
 
-template <int BN>
-__device__ __forceinline__ void epi_wide_qkv(const GemmArgs& g, uint32_t t_addr, int t, int tb) {
-  const int hd = g.head_dim, half = hd >> 1, H = g.n_heads, KV = g.n_kv_heads;
-  const bool row_ok = t < g.a_rows;
-  const int pos = row_ok ? g.tok_pos[t] : 0;
-  const float* rope_row = g.rope + (long long)pos * half * 2;
-  if (g.rope_kind == 0) {
-    // interleaved pairs (2i, 2i+1): both members sit in one 16-column chunk
-#pragma unroll 1
-    for (int c = 0; c < BN; c += 16) {
-      uint32_t v[16];
-      tmem_ld16(t_addr + c, v);
-      tmem_ld_wait();
-      const int n0 = tb * BN + c;
-      if (!row_ok || n0 >= g.b_rows) continue;
-      const int head = n0 / hd, e = n0 % hd;
-      float x[16];
-      epi_linear16(g, v, n0, x);
-      if (head < H + KV) {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const float2 cs = *reinterpret_cast<const float2*>(rope_row + (e / 2 + j) * 2);
-          const float a = x[2 * j], b = x[2 * j + 1];
-          x[2 * j] = __fsub_rn(__fmul_rn(a, cs.x), __fmul_rn(b, cs.y));
-          x[2 * j + 1] = __fadd_rn(__fmul_rn(b, cs.x), __fmul_rn(a, cs.y));
-        }
-      }
-      epi_store16(epi_qkv_dst(g, t, pos, head, e), x);
-    }
-  } else {
-    // half-split pairs (i, i + hd/2): take the two chunks of a head together
-#pragma unroll 1
-    for (int hb = 0; hb < BN; hb += hd) {
-#pragma unroll 1
-      for (int c = 0; c < half; c += 16) {
-        uint32_t vl[16], vh[16];
-        tmem_ld16(t_addr + hb + c, vl);
-        tmem_ld16(t_addr + hb + half + c, vh);
-        tmem_ld_wait();
-        const int n0 = tb * BN + hb + c;
-        if (!row_ok || n0 >= g.b_rows) continue;
-        const int head = n0 / hd;
-        float lo[16], hi[16];
-        epi_linear16(g, vl, n0, lo);
-        epi_linear16(g, vh, n0 + half, hi);
-        if (head < H + KV) {
-#pragma unroll
-          for (int j = 0; j < 16; ++j) {
-            const float2 cs = *reinterpret_cast<const float2*>(rope_row + (c + j) * 2);
-            const float cc = rbf(cs.x), ss = rbf(cs.y);
-            const float a = lo[j], b = hi[j];
-            lo[j] = __fadd_rn(rbf(__fmul_rn(a, cc)), rbf(__fmul_rn(-b, ss)));
-            hi[j] = __fadd_rn(rbf(__fmul_rn(b, cc)), rbf(__fmul_rn(a, ss)));
-          }
-        }
-        bf16* dst = epi_qkv_dst(g, t, pos, head, c);
-        epi_store16(dst, lo);
-        epi_store16(dst + half, hi);
-      }
-    }
-  }
-}
-
-// gate/up rows are interleaved in blocks of 16 features: columns [32b, 32b+16) = gate of features
-// [16b, 16b+16), columns [32b+16, 32b+32) = up of the same features.  act = bf16(bf16(silu(g)) * u).
-template <int BN>
-__device__ __forceinline__ void epi_wide_silu(const GemmArgs& g, uint32_t t_addr, int t, int tb) {
-  bf16* out = reinterpret_cast<bf16*>(g.out);
-#pragma unroll 1
-  for (int c = 0; c < BN; c += 32) {
-    uint32_t vg[16], vu[16];
-    tmem_ld16(t_addr + c, vg);
-    tmem_ld16(t_addr + c + 16, vu);
-    tmem_ld_wait();
-    const int n0 = tb * BN + c;
-    if (t >= g.a_rows || n0 >= g.b_rows) continue;
-    float x[16];
-#pragma unroll
-    for (int j = 0; j < 16; ++j) {
-      const float gg = rbf(__uint_as_float(vg[j])), uu = rbf(__uint_as_float(vu[j]));
-      x[j] = rbf(gg / (1.0f + expf(-gg))) * uu;
-    }
-    epi_store16(out + (long long)t * g.ld_out + (n0 >> 1), x);
-  }
-}
-
 template <int BN, int STAGES>
-__global__ void __launch_bounds__(192, 1)
+__global__ void __launch_bounds__(224, 1)
 xb_gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                        const __grid_constant__ CUtensorMap tmC, GemmArgs g) {
   using Cfg = GemmCfg<BN, STAGES>;
@@ -265,7 +170,7 @@ xb_gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
   if (warp == 1) {
     if (lane == 0) {
       for (int i = 0; i < STAGES; ++i) {
-        mbar_init(&full_bar[i], 1);
+        mbar_init(&full_bar[i], 2);   // one arrival (with its byte count) per producer
         mbar_init(&empty_bar[i], 1);
       }
       for (int i = 0; i < 2; ++i) {
@@ -287,81 +192,49 @@ xb_gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
   walk.init(g);
   GemmUnit wu;
 
+  // Roles are entered by elect.sync and weights and activations have a producer thread each: under `lane == 0` one thread
+  // needed 0.35 us to issue a k-block, as long as HBM takes to deliver its 16 KB to every SM, so no gap was ever made up.
+  // llama-3.2-1b, one sequence: 929 -> 795 us a step; four 8B layers: one sequence 450 -> 390, 32 sequences 835 -> 786.
   if (warp == 0) {
-    // ===================== TMA producer =====================
-    if (lane == 0) {
-      int stage = 0;
+    // ===================== TMA producer of the weights =====================
+    // They never depend on the preceding kernel: their boxes go out at once, as far as the ring reaches.
+    if (elect_one()) {
+      int stage = 0, issued = 0;
       uint32_t phase = 0;
-      bool waited = false;
-      int pre = 0;   // stages whose weight box was issued ahead of the dependency wait
       while (walk.next(g, wu)) {
-        const int ta = wu.ta, tb = wu.tb, kb0 = wu.kb0, kb1 = wu.kb1;
-        if (!waited) {
-          // first unit: weight boxes of up to STAGES k-blocks go out before the upstream grid is done
-          const int npre = (kb1 - kb0) < STAGES ? (kb1 - kb0) : STAGES;
-          for (int i = 0; i < npre; ++i) {
-            mbar_expect_tx(&full_bar[i], Cfg::A_BYTES + Cfg::B_BYTES);
-            int c0, c1;
-            if (g.mode == XB_GEMM_SKINNY) {
-              gemm_w_coord(g, ta, kb0 + i, c0, c1);
-              tma_load_2d(sA + i * Cfg::A_BYTES, &tmA, &full_bar[i], c0, c1);
-            } else {
-#pragma unroll
-              for (int j = 0; j < BN / 128; ++j) {
-                if (g.w_tiled) {
-                  gemm_w_coord(g, tb * (BN / 128) + j, kb0 + i, c0, c1);
-                  tma_load_2d(sB + i * Cfg::B_BYTES + j * Cfg::A_BYTES, &tmB, &full_bar[i], c0, c1);
-                } else if (j == 0) {
-                  tma_load_2d(sB + i * Cfg::B_BYTES, &tmB, &full_bar[i], (kb0 + i) * 64, tb * BN);
-                }
-              }
-            }
-          }
-          XB_TS(g, 1);
-          pdl_wait();
-          XB_TS(g, 2);
-          waited = true;
-          pre = npre;
-        }
-        for (int kb = kb0; kb < kb1; ++kb) {
-          const bool w_issued = pre > 0;
-          if (!w_issued) {
-            mbar_wait(&empty_bar[stage], phase ^ 1);
-            mbar_expect_tx(&full_bar[stage], Cfg::A_BYTES + Cfg::B_BYTES);
-          } else {
-            --pre;
-          }
+        for (int kb = wu.kb0; kb < wu.kb1; ++kb) {
+          mbar_wait(&empty_bar[stage], phase ^ 1);
+          mbar_expect_tx(&full_bar[stage], Cfg::A_BYTES);
           int c0, c1;
-          if (g.mode == XB_GEMM_SKINNY) {
-            if (!w_issued) {
-              gemm_w_coord(g, ta, kb, c0, c1);
-              tma_load_2d(sA + stage * Cfg::A_BYTES, &tmA, &full_bar[stage], c0, c1);
-            }
-            tma_load_2d(sB + stage * Cfg::B_BYTES, &tmB, &full_bar[stage], kb * 64, tb * BN);
-          } else {
-            tma_load_2d(sA + stage * Cfg::A_BYTES, &tmA, &full_bar[stage], kb * 64, ta * 128);
-            if (!w_issued) {
-#pragma unroll
-              for (int j = 0; j < BN / 128; ++j) {
-                if (g.w_tiled) {
-                  gemm_w_coord(g, tb * (BN / 128) + j, kb, c0, c1);
-                  tma_load_2d(sB + stage * Cfg::B_BYTES + j * Cfg::A_BYTES, &tmB, &full_bar[stage], c0, c1);
-                } else if (j == 0) {
-                  tma_load_2d(sB + stage * Cfg::B_BYTES, &tmB, &full_bar[stage], kb * 64, tb * BN);
-                }
-              }
-            }
-          }
+          gemm_w_coord(g, wu.ta, kb, c0, c1);
+          tma_load_2d(sA + stage * Cfg::A_BYTES, &tmA, &full_bar[stage], c0, c1);
+          if (++issued == STAGES) XB_TS(g, 1);
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
       }
       XB_TS(g, 9);
-      if (!waited) pdl_wait();
+    }
+  } else if (warp == 6) {
+    // ===================== TMA producer of the activations =====================
+    if (elect_one()) {
+      int stage = 0;
+      uint32_t phase = 0;
+      pdl_wait();
+      XB_TS(g, 2);
+      while (walk.next(g, wu)) {
+        for (int kb = wu.kb0; kb < wu.kb1; ++kb) {
+          mbar_wait(&empty_bar[stage], phase ^ 1);
+          mbar_expect_tx(&full_bar[stage], Cfg::B_BYTES);
+          tma_load_2d(sB + stage * Cfg::B_BYTES, &tmB, &full_bar[stage], kb * 64, wu.tb * BN);
+          if (++stage == STAGES) { stage = 0; phase ^= 1; }
+        }
+      }
     }
   } else if (warp == 1) {
-    // ===================== MMA issuer (one thread) =====================
-    if (lane == 0) {
+    // ===================== MMA issuer (one elected thread) =====================
+    if (elect_one()) {
       constexpr uint32_t idesc = umma_idesc_bf16(BN);
+      const uint64_t desc_a0 = umma_desc_sw128(smem_u32(sA)), desc_b0 = umma_desc_sw128(smem_u32(sB));
       int stage = 0, acc = 0;
       uint32_t phase = 0, acc_phase = 0;
       bool first_mma = true;
@@ -375,13 +248,10 @@ xb_gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
           if (first_mma) { XB_TS(g, 3); first_mma = false; }
           if (kb + 1 == kb1) XB_TS(g, 10);
           tc_fence_after();
-          const uint32_t a_addr = smem_u32(sA + stage * Cfg::A_BYTES);
-          const uint32_t b_addr = smem_u32(sB + stage * Cfg::B_BYTES);
+          const uint64_t da = desc_a0 + (uint64_t)(stage * (Cfg::A_BYTES >> 4)), db = desc_b0 + (uint64_t)(stage * (Cfg::B_BYTES >> 4));
 #pragma unroll
-          for (int k = 0; k < 4; ++k) {               // 4 x (K = 16) per 64-wide k-block
-            tc_mma_bf16(d_tmem, umma_desc_sw128(a_addr + k * 32), umma_desc_sw128(b_addr + k * 32), idesc,
-                        (kb > kb0 || k > 0) ? 1u : 0u);
-          }
+          for (int k = 0; k < 4; ++k)                 // 4 x (K = 16) per 64-wide k-block
+            tc_mma_bf16(d_tmem, da + k * 2, db + k * 2, idesc, (kb > kb0 || k > 0) ? 1u : 0u);
           tc_commit(&empty_bar[stage]);               // frees the smem slot when the MMAs retire
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
@@ -410,12 +280,12 @@ xb_gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
       const uint32_t t_addr = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(acc * BN);
       const int arow = ta * 128 + row_in_tile;
       bool last_unit = false;
-      if (BN <= 128 && g.mode == XB_GEMM_SKINNY && g.bulk_epi && g.out2 == nullptr) {
+      if (g.bulk_epi && g.out2 == nullptr) {
         UnitWalker peek = walk;
         GemmUnit nu;
         last_unit = !peek.next(g, nu);
       }
-      if (BN <= 128 && last_unit) {
+      if (last_unit) {
         // The block's LAST unit is pure tail: nothing overlaps its epilogue (earlier units drain while the next
         // unit's MMAs run).  Measured on B200 with per-block timestamps (profiles/gemm_timeline.py): the per-token
         // strided fp32 stores of the general path take 2.4 us per unit at 32 token rows -- more than the whole gap
@@ -449,56 +319,23 @@ xb_gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
           asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");   // shared memory may be released at exit
           XB_TS(g, 14);
         }
-      } else if (BN == 256 && g.mode == XB_GEMM_WIDE && g.epi == XB_EPI_QKV) {
-        epi_wide_qkv<BN>(g, t_addr, arow, tb);
-      } else if (BN == 256 && g.mode == XB_GEMM_WIDE && g.epi == XB_EPI_SILU) {
-        epi_wide_silu<BN>(g, t_addr, arow, tb);
       } else
 #pragma unroll 1
       for (int c = 0; c < BN; c += 16) {
         uint32_t v[16];
         tmem_ld16(t_addr + c, v);
         tmem_ld_wait();
-        if (g.mode == XB_GEMM_SKINNY) {
-          // arow = output feature n, column = token t; lanes write consecutive n (coalesced)
-          float* out = reinterpret_cast<float*>(g.out);
-          if (arow < g.a_rows) {
+        // arow = output feature n, column = token t; lanes write consecutive n (coalesced)
+        float* out = reinterpret_cast<float*>(g.out);
+        if (arow < g.a_rows) {
 #pragma unroll
-            for (int j = 0; j < 16; ++j) {
-              const int t = tb * BN + c + j;
-              if (t < g.b_rows) {
-                float x = __uint_as_float(v[j]);
-                if (g.round_bf16) x = rbf(x);
-                out[((long long)s * g.b_rows + t) * g.ld_out + arow] = x;
-                if (g.out2 != nullptr) g.out2[((long long)s * g.b_rows + t) * g.ld_out + arow] = x;
-              }
-            }
-          }
-        } else {
-          // arow = token t, columns = 16 consecutive features
-          bf16* out = reinterpret_cast<bf16*>(g.out);
-          const int n0 = tb * BN + c;
-          if (arow < g.a_rows && n0 < g.b_rows) {
-            float x[16];
-#pragma unroll
-            for (int j = 0; j < 16; ++j) x[j] = __uint_as_float(v[j]);
-            if (g.bias != nullptr) {
-#pragma unroll
-              for (int j = 0; j < 16; ++j)
-                if (n0 + j < g.b_rows) x[j] += bf2f(g.bias[n0 + j]);
-            }
-            bf16* dst = out + (long long)arow * g.ld_out + n0;
-            if (n0 + 16 <= g.b_rows && ((reinterpret_cast<uintptr_t>(dst) & 15) == 0)) {
-              uint4 p0, p1;
-              p0.x = f2_to_bf2(x[0], x[1]);   p0.y = f2_to_bf2(x[2], x[3]);
-              p0.z = f2_to_bf2(x[4], x[5]);   p0.w = f2_to_bf2(x[6], x[7]);
-              p1.x = f2_to_bf2(x[8], x[9]);   p1.y = f2_to_bf2(x[10], x[11]);
-              p1.z = f2_to_bf2(x[12], x[13]); p1.w = f2_to_bf2(x[14], x[15]);
-              reinterpret_cast<uint4*>(dst)[0] = p0;
-              reinterpret_cast<uint4*>(dst)[1] = p1;
-            } else {
-              for (int j = 0; j < 16; ++j)
-                if (n0 + j < g.b_rows) dst[j] = f2bf(x[j]);
+          for (int j = 0; j < 16; ++j) {
+            const int t = tb * BN + c + j;
+            if (t < g.b_rows) {
+              float x = __uint_as_float(v[j]);
+              if (g.round_bf16) x = rbf(x);
+              out[((long long)s * g.b_rows + t) * g.ld_out + arow] = x;
+              if (g.out2 != nullptr) g.out2[((long long)s * g.b_rows + t) * g.ld_out + arow] = x;
             }
           }
         }
@@ -634,7 +471,7 @@ static int xb_gemm_launch_t(const CUtensorMap& tmA, const CUtensorMap& tmB, cons
   }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid, 1, 1);
-  cfg.blockDim = dim3(192, 1, 1);
+  cfg.blockDim = dim3(224, 1, 1);
   cfg.dynamicSmemBytes = Cfg::SMEM_BYTES;
   cfg.stream = st;
   cudaLaunchAttribute attr[1];
@@ -654,8 +491,14 @@ struct GemmPlan {
   SplitInfo split;   // how a consumer sums the fp32 partial planes (SKINNY)
   int bn;
   int grid;
-  int stages;        // SKINNY: depth of the smem pipeline (xb_skinny_stages)
+  int stages;        // SKINNY: depth of the smem pipeline (xb_skinny_stages); WIDE: 0
+  int wide;          // WIDE: index of the kernel variant (xb_wide.cuh)
 };
+
+// more than 128 rows (xb_wide.cuh)
+static int xb_wide_plan(GemmPlan* p, const bf16* x, long long ldx, const bf16* w, int w_tiled, int T, int N, int K, int col_unit, int num_sms,
+                        int force_variant);
+static int xb_wide_run(const GemmPlan& p, cudaStream_t st, int pdl);
 
 // Depth of the shared-memory pipeline of the skinny (decode) Linear by token-column width.  Every stage is a 16 KB box
 // of weights plus the token tile; the stages a block can fill before the upstream grid is done are what keeps HBM
@@ -682,9 +525,9 @@ static int xb_skinny_stages(int bn) {
 static int xb_pick_bn_skinny(int T) { return T <= 16 ? 16 : T <= 32 ? 32 : T <= 64 ? 64 : 128; }
 
 // y[T,N] = x[T,K] W[N,K]^T.  T <= 128 -> SKINNY (fp32 partials [splits][T][N] into `out`);
-// otherwise WIDE (bf16 [T, ld_out] into `out`).
+// otherwise WIDE (bf16 [T, ld_out] into `out`; col_unit: columns a tile may not cut, force_splits > 0: that variant).
 static int xb_gemm_plan(GemmPlan* p, const bf16* x, long long ldx, const bf16* w, int w_tiled, int T, int N, int K,
-                        void* out, long long ld_out, const bf16* bias, int round_bf16, int num_sms, int force_splits) {
+                        void* out, long long ld_out, const bf16* bias, int round_bf16, int num_sms, int force_splits, int col_unit = 32) {
   XB_CHECK(K % 8 == 0, "K=%d must be a multiple of 8", K);
   GemmArgs& g = p->args;
   g.k_blocks = (K + 63) / 64;
@@ -725,56 +568,41 @@ static int xb_gemm_plan(GemmPlan* p, const bf16* x, long long ldx, const bf16* w
     XB_TRY(xb_make_tmap(&p->tmB, x, T, K, ldx, bn));
     p->tmC = p->tmA;
   } else {
-    p->bn = 256;
     g.mode = XB_GEMM_WIDE;
-    g.a_tiles = (T + 127) / 128;
-    g.b_tiles = (N + 255) / 256;
-    g.a_rows = T;
-    g.b_rows = N;
     g.splits = 1;
     g.sk_q = 0;
     g.sk_items = 0;
-    XB_TRY(xb_make_tmap(&p->tmA, x, T, K, ldx, 128));
-    if (w_tiled) XB_TRY(xb_make_tmap(&p->tmB, w, w_tiles * g.k_blocks * 128, 64, 64, 128));
-    else XB_TRY(xb_make_tmap(&p->tmB, w, N, K, K, 256));
+    p->stages = 0;
+    p->split = SplitInfo{g.k_blocks, 0, 1};
+    return xb_wide_plan(p, x, ldx, w, w_tiled, T, N, K, col_unit, num_sms, force_splits);
   }
   // one block per SM: under programmatic dependent launch the NEXT kernel's block co-resides
   // and prefetches its first weight stages while this one drains
-  if (g.mode == XB_GEMM_SKINNY && g.sk_q > 0) {
+  if (g.sk_q > 0) {
     p->grid = (g.sk_items + g.sk_q - 1) / g.sk_q;
   } else {
     const int units = g.a_tiles * g.b_tiles * g.splits;
     p->grid = units < num_sms ? units : num_sms;
   }
-  if (g.mode == XB_GEMM_SKINNY) {
-    // last-unit epilogue through a TMA store: 16-byte aligned base and row pitch (XB_BULK_EPI=0: per-token stores only)
-    const char* bv = getenv("XB_BULK_EPI");
-    if (!(bv != nullptr && bv[0] == '0') && ld_out % 4 == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0) {
-      XB_TRY(xb_make_tmap_f32(&p->tmC, out, (long long)g.splits * T, N, ld_out, T));
-      g.bulk_epi = 1;
-    }
-  } else {
-    p->tmC = p->tmA;
+  // last-unit epilogue through a TMA store: 16-byte aligned base and row pitch (XB_BULK_EPI=0: per-token stores only)
+  const char* bv = getenv("XB_BULK_EPI");
+  if (!(bv != nullptr && bv[0] == '0') && ld_out % 4 == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0) {
+    XB_TRY(xb_make_tmap_f32(&p->tmC, out, (long long)g.splits * T, N, ld_out, T));
+    g.bulk_epi = 1;
   }
-  p->stages = g.mode == XB_GEMM_SKINNY ? xb_skinny_stages(p->bn) : 0;
+  p->stages = xb_skinny_stages(p->bn);
   p->split.k_blocks = g.k_blocks;
-  p->split.q = g.mode == XB_GEMM_SKINNY ? g.sk_q : 0;
-  p->split.splits = g.mode == XB_GEMM_SKINNY ? g.splits : 1;
+  p->split.q = g.sk_q;
+  p->split.splits = g.splits;
   return 0;
 }
 
 static int xb_gemm_run(const GemmPlan& p, cudaStream_t st, int pdl) {
-  if (p.stages > 0) {
+  if (p.stages == 0) return xb_wide_run(p, st, pdl);
 #define XB_STAGE_CASE(BN_, N_) if (p.bn == BN_ && p.stages == N_) return xb_gemm_launch_t<BN_, N_>(p.tmA, p.tmB, p.tmC, p.args, p.grid, st, pdl);
-    XB_STAGE_CASE(16, 7) XB_STAGE_CASE(32, 6) XB_STAGE_CASE(64, 8) XB_STAGE_CASE(128, 6)          // defaults
-    XB_STAGE_CASE(16, 5) XB_STAGE_CASE(32, 5) XB_STAGE_CASE(64, 4) XB_STAGE_CASE(128, 7)          // A/B (XB_GEMM_STAGES)
-    XB_STAGE_CASE(32, 7) XB_STAGE_CASE(32, 8)
+  XB_STAGE_CASE(16, 7) XB_STAGE_CASE(32, 6) XB_STAGE_CASE(64, 8) XB_STAGE_CASE(128, 6)          // defaults
+  XB_STAGE_CASE(16, 5) XB_STAGE_CASE(32, 5) XB_STAGE_CASE(64, 4) XB_STAGE_CASE(128, 7)          // A/B (XB_GEMM_STAGES)
+  XB_STAGE_CASE(32, 7) XB_STAGE_CASE(32, 8)
 #undef XB_STAGE_CASE
-    return xb_fail(1, "no skinny Linear instantiated for %d token columns with %d stages", p.bn, p.stages);
-  }
-  switch (p.bn) {
-    case 128: return xb_gemm_launch_t<128, 6>(p.tmA, p.tmB, p.tmC, p.args, p.grid, st, pdl);
-    case 256: return xb_gemm_launch_t<256, 4>(p.tmA, p.tmB, p.tmC, p.args, p.grid, st, pdl);
-  }
-  return xb_fail(1, "unsupported BN %d", p.bn);
+  return xb_fail(1, "no skinny Linear instantiated for %d token columns with %d stages", p.bn, p.stages);
 }

@@ -1,0 +1,528 @@
+// Linear of more than 128 token rows: y[T,N] (bf16) = x[T,K] W[N,K]^T with the fused prompt epilogues.
+//
+//   D[128 tokens x BN features] (fp32, TMEM) += A[128 x 64] (x, smem) * B[BN x 64]^T (W, smem)
+//
+// Same pipeline as the decode Linear (xb_gemm.cuh): one thread feeds each operand by TMA, one issues tcgen05.mma, four warps
+// drain TMEM, persistent over tiles with two accumulators.  What varies is how the tiles cover the chip:
+//   CG = 2  a pair of CTAs works on one 256 x BN tile (cta_group::2): each stages its own 128 token rows and HALF of the
+//           weight rows, 32 KB instead of 48 KB a k-block at BN = 256.
+//   S > 1   S CTAs of a cluster share one tile, each a part of K; the fp32 partial tiles meet through distributed shared
+//           memory, every CTA reduces its share of the columns in rank order (same bits every time) and stores it.
+#pragma once
+#include "xb_gemm.cuh"
+
+template <int BN, int CG, int S>
+struct WideCfg {
+  static constexpr int BROWS = BN / CG;                       // weight rows this CTA stages
+  static constexpr int BOX = BROWS % 128 == 0 ? 128 : 64;     // rows of one TMA box (divides 128: a box stays in its weight tile)
+  static constexpr int A_BYTES = 128 * 64 * 2;
+  static constexpr int B_BYTES = BROWS * 64 * 2;
+  static constexpr int KS = BN <= 128 ? 2 : 1;                // k-blocks of one stage: narrow tiles halve the barrier round trips a k-block
+  static constexpr int STAGES_RAW = (216 * 1024) / (KS * (A_BYTES + B_BYTES));
+  static constexpr int STAGES = STAGES_RAW > 8 ? 8 : STAGES_RAW;
+  static constexpr int ACC_STAGES = S > 1 ? 1 : 2;
+  static constexpr int TM_RAW = ACC_STAGES * BN;
+  static constexpr int TM_COLS = TM_RAW <= 128 ? 128 : TM_RAW <= 256 ? 256 : 512;
+  static constexpr int ACC_COLS = TM_COLS / ACC_STAGES;
+  static constexpr int PAIRS = BN / 32;                       // column pairs (two chunks of 16) of a tile
+  static constexpr int RING_BYTES = STAGES * KS * (A_BYTES + B_BYTES);
+  static constexpr int SMEM_BYTES = RING_BYTES + 1024 + 256;
+  static_assert(BROWS % BOX == 0 && PAIRS % S == 0 && (S - 1) * (BN / S) * 128 * 4 <= RING_BYTES, "tile");
+};
+
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync_aligned() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// shared::cluster address of this CTA's shared address `a` in CTA `rank` of the cluster
+__device__ __forceinline__ uint32_t cluster_map(uint32_t a, uint32_t rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+// TMA load into this CTA whose bytes are counted by a barrier of the CTA pair (`bar`: shared::cluster address)
+__device__ __forceinline__ void tma_load_2d_pair(void* dst, const CUtensorMap* m, uint32_t bar, int c0, int c1) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+      ::"r"(smem_u32(dst)), "l"(m), "r"(bar), "r"(c0), "r"(c1)
+      : "memory");
+}
+template <int CG>
+__device__ __forceinline__ void wide_tmem_alloc(uint32_t* dst_smem, uint32_t cols) {
+  if (CG == 1) {
+    tmem_alloc(dst_smem, cols);
+  } else {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(dst_smem)), "r"(cols) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+  }
+}
+template <int CG>
+__device__ __forceinline__ void wide_tmem_dealloc(uint32_t taddr, uint32_t cols) {
+  if (CG == 1) tmem_dealloc(taddr, cols);
+  else asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(cols) : "memory");
+}
+// completion of the MMAs issued so far arrives at `bar`, for a pair at the same barrier of both CTAs
+template <int CG>
+__device__ __forceinline__ void wide_commit(uint64_t* bar) {
+  if (CG == 1) {
+    tc_commit(bar);
+  } else {
+    const uint16_t both = 3;
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+                 ::"r"(smem_u32(bar)), "h"(both) : "memory");
+  }
+}
+template <int CG>
+__device__ __forceinline__ void wide_mma(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+  if (CG == 1) {
+    tc_mma_bf16(tmem_d, desc_a, desc_b, idesc, accumulate);
+  } else {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
+        : "memory");
+  }
+}
+
+// ---- epilogues: one thread = one token row, two chunks of 16 columns at a time ----
+// The chunks of pair p: neighbours (gate beside up, interleaved rotation), or for the half-split rotation the two chunks
+// whose entries turn together, half a head apart.
+__device__ __forceinline__ void wide_pair_cols(const GemmArgs& g, int p, int& c0, int& c1) {
+  if (g.epi == XB_EPI_QKV && g.rope_kind != 0) {
+    const int per = g.head_dim >> 5, head = p / per, j = p - head * per;
+    c0 = head * g.head_dim + j * 16;
+    c1 = c0 + (g.head_dim >> 1);
+  } else {
+    c0 = p * 32;
+    c1 = c0 + 16;
+  }
+}
+__device__ __forceinline__ void wide_bias_round(const GemmArgs& g, int n0, float* x) {
+#pragma unroll
+  for (int j = 0; j < 16; ++j) {   // nn.Linear rounding point: bf16(acc + bias)
+    float a = x[j];
+    if (g.bias != nullptr) a += bf2f(g.bias[n0 + j]);
+    x[j] = rbf(a);
+  }
+}
+__device__ __forceinline__ void wide_store_plain(const GemmArgs& g, int t, int n0, float* x) {
+  if (n0 >= g.b_rows) return;
+  bf16* dst = reinterpret_cast<bf16*>(g.out) + (long long)t * g.ld_out + n0;
+  if (g.bias != nullptr) {
+#pragma unroll
+    for (int j = 0; j < 16; ++j)
+      if (n0 + j < g.b_rows) x[j] += bf2f(g.bias[n0 + j]);
+  }
+  if (n0 + 16 <= g.b_rows && (reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
+    epi_store16(dst, x);
+  } else {
+#pragma unroll
+    for (int j = 0; j < 16; ++j)
+      if (n0 + j < g.b_rows) dst[j] = f2bf(x[j]);
+  }
+}
+// x0 / x1: fp32 sums of the columns n0.. and n1.. of token row t
+__device__ __forceinline__ void wide_emit(const GemmArgs& g, int t, int pos, int n0, int n1, float* x0, float* x1) {
+  if (t >= g.a_rows) return;
+  if (g.epi == XB_EPI_SILU) {
+    // gate/up rows are interleaved in blocks of 16 features: act = bf16(bf16(silu(gate)) * up)
+    if (n0 >= g.b_rows) return;
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      const float gg = rbf(x0[j]), uu = rbf(x1[j]);
+      x0[j] = rbf(gg / (1.0f + expf(-gg))) * uu;
+    }
+    epi_store16(reinterpret_cast<bf16*>(g.out) + (long long)t * g.ld_out + (n0 >> 1), x0);
+  } else if (g.epi == XB_EPI_QKV) {
+    if (n0 >= g.b_rows) return;
+    const int hd = g.head_dim, half = hd >> 1, turned = g.n_heads + g.n_kv_heads;
+    const float* rope_row = g.rope + (long long)pos * half * 2;
+    wide_bias_round(g, n0, x0);
+    if (n1 < g.b_rows) wide_bias_round(g, n1, x1);
+    const int h0 = n0 / hd, e0 = n0 - h0 * hd;
+    if (g.rope_kind != 0) {
+      if (h0 < turned) {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+          const float2 cs = *reinterpret_cast<const float2*>(rope_row + (e0 + j) * 2);
+          const float cc = rbf(cs.x), ss = rbf(cs.y);
+          const float a = x0[j], b = x1[j];
+          x0[j] = __fadd_rn(rbf(__fmul_rn(a, cc)), rbf(__fmul_rn(-b, ss)));
+          x1[j] = __fadd_rn(rbf(__fmul_rn(b, cc)), rbf(__fmul_rn(a, ss)));
+        }
+      }
+      bf16* dst = epi_qkv_dst(g, t, pos, h0, e0);
+      epi_store16(dst, x0);
+      epi_store16(dst + half, x1);
+    } else {
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        float* x = c == 0 ? x0 : x1;
+        const int n = c == 0 ? n0 : n1;
+        if (n >= g.b_rows) break;
+        const int head = n / hd, e = n - head * hd;
+        if (head < turned) {
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            const float2 cs = *reinterpret_cast<const float2*>(rope_row + (e / 2 + j) * 2);
+            const float a = x[2 * j], b = x[2 * j + 1];
+            x[2 * j] = __fsub_rn(__fmul_rn(a, cs.x), __fmul_rn(b, cs.y));
+            x[2 * j + 1] = __fadd_rn(__fmul_rn(b, cs.x), __fmul_rn(a, cs.y));
+          }
+        }
+        epi_store16(epi_qkv_dst(g, t, pos, head, e), x);
+      }
+    }
+  } else {
+    wide_store_plain(g, t, n0, x0);
+    wide_store_plain(g, t, n1, x1);
+  }
+}
+
+// Roles are entered by elect.sync, not by lane == 0, and the two operands have a producer thread each: one thread doing
+// everything under `lane == 0` spent 0.35 us a k-block whatever the tile (a 128 x 64 tile took as long as 128 x 256), most of
+// it issuing.  4096^3, CUDA events: 256x256 pair 103 -> 94 us, 128x256 107 -> 103, 128x128 166 -> 116, 128x64 306 -> 202.
+template <int BN, int CG, int S>
+__global__ void __launch_bounds__(224, 1)
+xb_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, GemmArgs g) {
+  using Cfg = WideCfg<BN, CG, S>;
+  constexpr int STAGES = Cfg::STAGES, KS = Cfg::KS;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* sA = smem;
+  uint8_t* sB = smem + STAGES * KS * Cfg::A_BYTES;
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + Cfg::RING_BYTES);
+  uint64_t* empty_bar = full_bar + STAGES;
+  uint64_t* tfull_bar = empty_bar + STAGES;
+  uint64_t* tempty_bar = tfull_bar + 2;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty_bar + 2);
+
+  const int warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
+  const uint32_t rank = CG * S > 1 ? cluster_rank() : 0;
+  const int a_units = (g.a_tiles + CG - 1) / CG;
+  const int n_units = a_units * g.b_tiles;
+  const int u0 = blockIdx.x / (CG * S), u_step = S > 1 ? n_units : gridDim.x / CG;
+  const int kb0 = S > 1 ? (int)(((long long)rank * g.k_blocks) / S) : 0;
+  const int kb1 = S > 1 ? (int)(((long long)(rank + 1) * g.k_blocks) / S) : g.k_blocks;
+
+  if (warp == 0 && lane == 0) {
+    tma_prefetch_desc(&tmA);
+    tma_prefetch_desc(&tmB);
+  }
+  if (warp == 1) {
+    if (lane == 0) {
+      for (int i = 0; i < STAGES; ++i) {
+        mbar_init(&full_bar[i], 2);   // one arrival (with its byte count) per producer
+        mbar_init(&empty_bar[i], 1);
+      }
+      for (int i = 0; i < 2; ++i) {
+        mbar_init(&tfull_bar[i], 1);
+        mbar_init(&tempty_bar[i], 4 * CG);
+      }
+      fence_mbar_init();
+    }
+    __syncwarp();
+    wide_tmem_alloc<CG>(tmem_slot, Cfg::TM_COLS);
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (CG * S > 1) cluster_sync_aligned();   // barriers of the peers are ready too
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+  pdl_launch_dependents();
+
+  if (warp == 0 || warp == 6) {
+    // ===================== TMA producers: warp 0 weights, warp 6 activations =====================
+    if (elect_one()) {
+      int stage = 0;
+      uint32_t phase = 0;
+      const uint32_t pair_bar = CG == 2 ? cluster_map(smem_u32(full_bar), 0) : 0;   // a pair counts the bytes of both CTAs at the first one's barriers
+      auto expect = [&](uint32_t bytes) {
+        if (CG == 1) mbar_expect_tx(&full_bar[stage], bytes);
+        else if (rank == 0) mbar_expect_tx(&full_bar[stage], 2 * bytes);
+      };
+      auto load = [&](void* dst, const CUtensorMap* m, int c0, int c1) {
+        if (CG == 1) tma_load_2d(dst, m, &full_bar[stage], c0, c1);
+        else tma_load_2d_pair(dst, m, pair_bar + stage * 8, c0, c1);
+      };
+      if (warp == 6) pdl_wait();   // weights never depend on the preceding kernel: their boxes go out at once
+      for (int u = u0; u < n_units; u += u_step) {
+        const int ta = (u % a_units) * CG + (CG == 2 ? (int)rank : 0), tb = u / a_units;
+        for (int kb = kb0; kb < kb1; kb += KS) {
+          const int nk = KS == 1 || kb + 1 == kb1 ? 1 : KS;
+          mbar_wait(&empty_bar[stage], phase ^ 1);
+          if (warp == 6) {
+            expect(nk * Cfg::A_BYTES);
+#pragma unroll
+            for (int q = 0; q < KS; ++q)
+              if (q < nk) load(sA + (stage * KS + q) * Cfg::A_BYTES, &tmA, (kb + q) * 64, ta * 128);
+          } else {
+            expect(nk * Cfg::B_BYTES);
+#pragma unroll
+            for (int q = 0; q < KS; ++q) {
+              if (q >= nk) break;
+#pragma unroll
+              for (int j = 0; j < Cfg::BROWS / Cfg::BOX; ++j) {
+                const int n = tb * BN + (CG == 2 ? (int)rank * Cfg::BROWS : 0) + j * Cfg::BOX;
+                uint8_t* dst = sB + (stage * KS + q) * Cfg::B_BYTES + j * Cfg::BOX * 128;
+                if (g.w_tiled) load(dst, &tmB, 0, ((n >> 7) * g.k_blocks + kb + q) * 128 + (n & 127));
+                else load(dst, &tmB, (kb + q) * 64, n);
+              }
+            }
+          }
+          if (++stage == STAGES) { stage = 0; phase ^= 1; }
+        }
+      }
+      pdl_wait();
+    }
+  } else if (warp == 1) {
+    // ===================== MMA issuer (one elected thread, of a pair: of its first CTA) =====================
+    if ((CG == 1 || rank == 0) && elect_one()) {
+      constexpr uint32_t idesc = (umma_idesc_bf16(BN) & ~(0x1fu << 24)) | ((uint32_t)(128 * CG >> 4) << 24);
+      int stage = 0, acc = 0;
+      uint32_t phase = 0, acc_phase = 0;
+      const uint64_t desc_a0 = umma_desc_sw128(smem_u32(sA)), desc_b0 = umma_desc_sw128(smem_u32(sB));
+      for (int u = u0; u < n_units; u += u_step) {
+        mbar_wait(&tempty_bar[acc], acc_phase ^ 1);   // epilogue has drained this accumulator
+        tc_fence_after();
+        const uint32_t d_tmem = tmem_base + (uint32_t)(acc * Cfg::ACC_COLS);
+        for (int kb = kb0; kb < kb1; kb += KS) {
+          mbar_wait(&full_bar[stage], phase);
+          tc_fence_after();
+#pragma unroll
+          for (int q = 0; q < KS; ++q) {
+            if (q > 0 && kb + q >= kb1) break;
+            const uint64_t da = desc_a0 + (uint64_t)((stage * KS + q) * (Cfg::A_BYTES >> 4));
+            const uint64_t db = desc_b0 + (uint64_t)((stage * KS + q) * (Cfg::B_BYTES >> 4));
+#pragma unroll
+            for (int k = 0; k < 4; ++k)               // 4 x (K = 16) per 64-wide k-block
+              wide_mma<CG>(d_tmem, da + k * 2, db + k * 2, idesc, (kb > kb0 || q > 0 || k > 0) ? 1u : 0u);
+          }
+          wide_commit<CG>(&empty_bar[stage]);
+          if (++stage == STAGES) { stage = 0; phase ^= 1; }
+        }
+        wide_commit<CG>(&tfull_bar[acc]);
+        if (++acc == Cfg::ACC_STAGES) { acc = 0; acc_phase ^= 1; }
+      }
+    }
+  } else {
+    // ===================== epilogue warps 2..5 =====================
+    const int quad = warp & 3;
+    const int row_in_tile = quad * 32 + lane;
+    const uint32_t lane_base = tmem_base + ((uint32_t)(quad * 32) << 16);
+    pdl_wait();                                       // `out` may still be read by the upstream grid
+    if (S == 1) {
+      int acc = 0;
+      uint32_t acc_phase = 0;
+      for (int u = u0; u < n_units; u += u_step) {
+        const int ta = (u % a_units) * CG + (CG == 2 ? (int)rank : 0), tb = u / a_units;
+        const int t = ta * 128 + row_in_tile;
+        const int pos = g.epi == XB_EPI_QKV && t < g.a_rows ? g.tok_pos[t] : 0;
+        mbar_wait(&tfull_bar[acc], acc_phase);
+        tc_fence_after();
+        const uint32_t t_addr = lane_base + (uint32_t)(acc * Cfg::ACC_COLS);
+#pragma unroll 1
+        for (int p = 0; p < Cfg::PAIRS; ++p) {
+          int c0, c1;
+          wide_pair_cols(g, p, c0, c1);
+          uint32_t v0[16], v1[16];
+          tmem_ld16(t_addr + c0, v0);
+          tmem_ld16(t_addr + c1, v1);
+          tmem_ld_wait();
+          wide_emit(g, t, pos, tb * BN + c0, tb * BN + c1, reinterpret_cast<float*>(v0), reinterpret_cast<float*>(v1));
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) {
+          if (CG == 1) mbar_arrive(&tempty_bar[acc]);
+          else mbar_arrive_cluster(cluster_map(smem_u32(&tempty_bar[acc]), 0));
+        }
+        if (++acc == Cfg::ACC_STAGES) { acc = 0; acc_phase ^= 1; }
+      }
+    } else {
+      mbar_wait(&tfull_bar[0], 0);                    // all MMAs of this CTA have retired: its ring is free for the exchange
+      tc_fence_after();
+    }
+  }
+  __syncwarp();
+  if (S > 1) {
+    constexpr int OWN = Cfg::PAIRS / S;               // pairs this CTA finishes
+    cluster_sync_aligned();                           // every CTA's ring is free
+    float* xch = reinterpret_cast<float*>(smem);      // [S - 1 senders][OWN pairs][32 columns][128 rows]
+    const int quad = warp & 3, row_in_tile = quad * 32 + lane;
+    const uint32_t lane_base = tmem_base + ((uint32_t)(quad * 32) << 16);
+    if (warp >= 2 && warp < 6) {
+#pragma unroll 1
+      for (int d = 0; d < S; ++d) {
+        if (d == (int)rank) continue;
+        const uint32_t dst = cluster_map(smem_u32(xch), d) + (uint32_t)(((int)rank < d ? rank : rank - 1) * OWN * 32 * 128 + row_in_tile) * 4;
+#pragma unroll 1
+        for (int p = 0; p < OWN; ++p) {
+          int c0, c1;
+          wide_pair_cols(g, d * OWN + p, c0, c1);
+          uint32_t v0[16], v1[16];
+          tmem_ld16(lane_base + c0, v0);
+          tmem_ld16(lane_base + c1, v1);
+          tmem_ld_wait();
+#pragma unroll
+          for (int j = 0; j < 16; ++j) {
+            asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(dst + (uint32_t)((p * 32 + j) * 128) * 4), "r"(v0[j]) : "memory");
+            asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(dst + (uint32_t)((p * 32 + 16 + j) * 128) * 4), "r"(v1[j]) : "memory");
+          }
+        }
+      }
+    }
+    __syncwarp();
+    cluster_sync_aligned();                           // the partial columns of the peers have arrived
+    if (warp >= 2 && warp < 6) {
+      const int ta = u0 % a_units, tb = u0 / a_units;
+      const int t = ta * 128 + row_in_tile;
+      const int pos = g.epi == XB_EPI_QKV && t < g.a_rows ? g.tok_pos[t] : 0;
+#pragma unroll 1
+      for (int p = 0; p < OWN; ++p) {
+        int c0, c1;
+        wide_pair_cols(g, (int)rank * OWN + p, c0, c1);
+        uint32_t v0[16], v1[16];
+        tmem_ld16(lane_base + c0, v0);
+        tmem_ld16(lane_base + c1, v1);
+        tmem_ld_wait();
+        float x0[16], x1[16];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) x0[j] = x1[j] = 0.f;
+#pragma unroll
+        for (int s = 0; s < S; ++s) {                 // rank order: the same sums every time
+          if (s == (int)rank) {
+#pragma unroll
+            for (int j = 0; j < 16; ++j) { x0[j] += __uint_as_float(v0[j]); x1[j] += __uint_as_float(v1[j]); }
+          } else {
+            const float* src = xch + (size_t)((s < (int)rank ? s : s - 1) * OWN + p) * 32 * 128 + row_in_tile;
+#pragma unroll
+            for (int j = 0; j < 16; ++j) { x0[j] += src[j * 128]; x1[j] += src[(16 + j) * 128]; }
+          }
+        }
+        wide_emit(g, t, pos, tb * BN + c0, tb * BN + c1, x0, x1);
+      }
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (CG == 2) cluster_sync_aligned();                // no CTA of a pair leaves while the other still uses its memory
+  if (warp == 1) {
+    tc_fence_after();
+    wide_tmem_dealloc<CG>(tmem_base, Cfg::TM_COLS);
+  }
+}
+
+// ----------------------------------------------------------------------------- host side
+struct WideVariant {
+  int bn, cg, split;
+  int (*run)(const CUtensorMap&, const CUtensorMap&, const GemmArgs&, int grid, cudaStream_t, int pdl);
+};
+
+template <int BN, int CG, int S>
+static int xb_wide_launch_t(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmArgs& g, int grid, cudaStream_t st, int pdl) {
+  using Cfg = WideCfg<BN, CG, S>;
+  {
+    static bool done[XB_MAX_DEVICES] = {false};
+    int dev = 0;
+    XB_CUDA(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= XB_MAX_DEVICES || !done[dev]) {
+      XB_CUDA(cudaFuncSetAttribute(xb_wide_kernel<BN, CG, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES));
+      if (dev >= 0 && dev < XB_MAX_DEVICES) done[dev] = true;
+    }
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid, 1, 1);
+  cfg.blockDim = dim3(224, 1, 1);
+  cfg.dynamicSmemBytes = Cfg::SMEM_BYTES;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[2];
+  int na = 0;
+  if (pdl) {
+    attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[na].val.programmaticStreamSerializationAllowed = 1;
+    ++na;
+  }
+  if (CG * S > 1) {
+    attr[na].id = cudaLaunchAttributeClusterDimension;
+    attr[na].val.clusterDim.x = CG * S;
+    attr[na].val.clusterDim.y = 1;
+    attr[na].val.clusterDim.z = 1;
+    ++na;
+  }
+  cfg.attrs = attr;
+  cfg.numAttrs = na;
+  XB_CUDA(cudaLaunchKernelEx(&cfg, xb_wide_kernel<BN, CG, S>, tmA, tmB, g));
+  return 0;
+}
+
+#define XB_WIDE_VARIANT(BN, CG, S) {BN, CG, S, xb_wide_launch_t<BN, CG, S>}
+static const WideVariant g_wide_variants[] = {
+  XB_WIDE_VARIANT(256, 2, 1), XB_WIDE_VARIANT(256, 1, 1), XB_WIDE_VARIANT(192, 1, 1), XB_WIDE_VARIANT(128, 1, 1),
+  XB_WIDE_VARIANT(256, 1, 2), XB_WIDE_VARIANT(192, 1, 2), XB_WIDE_VARIANT(128, 1, 2), XB_WIDE_VARIANT(128, 1, 4),
+};
+#undef XB_WIDE_VARIANT
+enum { XB_WIDE_VARIANTS = sizeof(g_wide_variants) / sizeof(g_wide_variants[0]) };
+
+// The variant with the least estimated time: waves x (k-blocks of a CTA x time of one) + epilogue, exchange and launch.
+// The times (us) are fitted to a sweep of T = 192 .. 4096 over the Linears of the registered models (K 2048 .. 18944, N 2048 ..
+// 37888): the rule's choice is on average within 1 % of the best variant.  What the variants are for, us cold, old 128 x 256
+// tiling -> choice: T 192, 2048 x 8192: 54.8 -> 18.9 (K in four); T 373, 3072 x 8192: 57 -> 28 (K in two); T 733, 4096 x 14336:
+// 96 -> 87 (192 columns); T 4096, 28672 x 4096: 664 -> 644 (pairs).
+// col_unit: columns that have to stay together in a tile (a head where the rotation pairs its halves).
+static int xb_pick_wide(int T, int N, int K, int col_unit, int num_sms) {
+  int best = 1;
+  double best_t = 1e30;
+  const int a_tiles = (T + 127) / 128, k_blocks = (K + 63) / 64;
+  for (int i = 0; i < XB_WIDE_VARIANTS; ++i) {
+    const WideVariant& v = g_wide_variants[i];
+    if (v.bn % col_unit != 0 || k_blocks < 4 * v.split) continue;
+    const long long units = (long long)((a_tiles + v.cg - 1) / v.cg) * ((N + v.bn - 1) / v.bn);
+    const int slots = v.split == 4 ? (num_sms - 4) / 4 : num_sms / (v.cg * v.split);   // clusters of four leave some SMs idle
+    const long long waves = (units + slots - 1) / slots;
+    const double kb = v.cg == 2 ? 0.36 : v.bn == 256 ? 0.40 : v.bn == 192 ? 0.31 : 0.26;
+    const double epi = v.bn * 0.02;
+    const double t = (double)waves * k_blocks / v.split * kb + (v.split > 1 ? 0.6 * epi + 1.7 + 5.0 * (double)(waves - 1) : epi);
+    if (t < best_t) { best_t = t; best = i; }
+  }
+  return best;
+}
+
+static int xb_wide_plan(GemmPlan* p, const bf16* x, long long ldx, const bf16* w, int w_tiled, int T, int N, int K, int col_unit, int num_sms,
+                        int force_variant) {
+  const int vi = force_variant > 0 ? force_variant - 1 : xb_pick_wide(T, N, K, col_unit, num_sms);
+  XB_CHECK(vi < XB_WIDE_VARIANTS, "wide Linear variant %d of %d", vi + 1, (int)XB_WIDE_VARIANTS);
+  const WideVariant& v = g_wide_variants[vi];
+  GemmArgs& g = p->args;
+  XB_CHECK(g.k_blocks >= v.split, "K=%d is too short for %d parts", K, v.split);
+  p->wide = vi;
+  p->bn = v.bn;
+  g.a_tiles = (T + 127) / 128;
+  g.b_tiles = (N + v.bn - 1) / v.bn;
+  g.a_rows = T;
+  g.b_rows = N;
+  const int units = (g.a_tiles + v.cg - 1) / v.cg * g.b_tiles;
+  if (v.split > 1) p->grid = units * v.split;
+  else p->grid = (units < num_sms / v.cg ? units : num_sms / v.cg) * v.cg;
+  const int box = (v.bn / v.cg) % 128 == 0 ? 128 : 64;
+  const long long w_tiles = (N + 127) / 128;
+  XB_TRY(xb_make_tmap(&p->tmA, x, T, K, ldx, 128));
+  if (w_tiled) XB_TRY(xb_make_tmap(&p->tmB, w, w_tiles * g.k_blocks * 128, 64, 64, box));
+  else XB_TRY(xb_make_tmap(&p->tmB, w, N, K, K, box));
+  p->tmC = p->tmA;
+  return 0;
+}
+
+static int xb_wide_run(const GemmPlan& p, cudaStream_t st, int pdl) {
+  return g_wide_variants[p.wide].run(p.tmA, p.tmB, p.args, p.grid, st, pdl);
+}

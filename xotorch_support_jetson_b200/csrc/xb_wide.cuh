@@ -479,6 +479,8 @@ enum { XB_WIDE_VARIANTS = sizeof(g_wide_variants) / sizeof(g_wide_variants[0]) }
 // 37888): the rule's choice is on average within 1 % of the best variant.  What the variants are for, us cold, old 128 x 256
 // tiling -> choice: T 192, 2048 x 8192: 54.8 -> 18.9 (K in four); T 373, 3072 x 8192: 57 -> 28 (K in two); T 733, 4096 x 14336:
 // 96 -> 87 (192 columns); T 4096, 28672 x 4096: 664 -> 644 (pairs).
+// K goes in parts up to 512 rows only: above, that is best for a few shapes (by 18 % at most, 1024 x 2048 x 8192), and without it
+// a long prompt and its portions sum alike.
 // col_unit: columns that have to stay together in a tile (a head where the rotation pairs its halves).
 static int xb_pick_wide(int T, int N, int K, int col_unit, int num_sms) {
   int best = 1;
@@ -486,7 +488,7 @@ static int xb_pick_wide(int T, int N, int K, int col_unit, int num_sms) {
   const int a_tiles = (T + 127) / 128, k_blocks = (K + 63) / 64;
   for (int i = 0; i < XB_WIDE_VARIANTS; ++i) {
     const WideVariant& v = g_wide_variants[i];
-    if (v.bn % col_unit != 0 || k_blocks < 4 * v.split) continue;
+    if (v.bn % col_unit != 0 || k_blocks < 4 * v.split || (v.split > 1 && T > 512)) continue;
     const long long units = (long long)((a_tiles + v.cg - 1) / v.cg) * ((N + v.bn - 1) / v.bn);
     const int slots = v.split == 4 ? (num_sms - 4) / 4 : num_sms / (v.cg * v.split);   // clusters of four leave some SMs idle
     const long long waves = (units + slots - 1) / slots;

@@ -4,6 +4,7 @@
 #include "xb_common.cuh"
 #include "xb_gemm.cuh"
 #include "xb_wide.cuh"
+#include "xb_linear_f32.cuh"
 #include "xb_loader.cuh"
 #include "xb_kernels.cuh"
 #include "xb_attn_mma.cuh"

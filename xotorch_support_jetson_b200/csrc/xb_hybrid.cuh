@@ -115,12 +115,15 @@ struct HyModel {
   int use_tc = 1;            // XB_HY_TC=0: every Linear through the plain kernels (A/B)
   size_t cap_P = 0, cap_m = 0, cap_head = 0;   // bytes of the Linear output buffers
   std::map<std::tuple<const void*, const void*, const void*, int>, GemmPlan> plans;
+  bf16* pieces = nullptr;    // float32 mode: the rows of a Linear's input as three planes of bf16 pieces [3][pieces_rows][K]
+  int pieces_rows = 0;
+  std::map<std::tuple<const void*, const void*, const void*, int, int, int>, F32Plan> f32_plans;
 };
 
 static int* hy_rows_buffer(xb_engine* e) { return e->hy->d_rows; }
 static int hy_max_rows(xb_engine* e) { return e->hy->d.max_logit_rows > e->hy->d.max_seqs ? e->hy->d.max_logit_rows : e->hy->d.max_seqs; }
 
-static void hy_drop_plans(xb_engine* e) { e->hy->plans.clear(); }
+static void hy_drop_plans(xb_engine* e) { e->hy->plans.clear(); e->hy->f32_plans.clear(); }
 
 static int hy_alloc(HyModel* hy, void** p, size_t bytes) {
   XB_TRY(dmalloc(p, bytes));
@@ -846,6 +849,11 @@ static int hy_create(xb_engine* e, const xb_hybrid_desc& d, const xb_hybrid_laye
   XB_TRY(hy_alloc(hy, &hy->a1, Tm * hy->maxK * as));
   XB_TRY(hy_alloc(hy, &hy->a2, Tm * hy->maxK * as));
   XB_TRY(hy_alloc(hy, &hy->head_in, R * D * as));
+  if (d.compute_fp32) {
+    const size_t most = Tm > R ? Tm : R;
+    hy->pieces_rows = most < XB_F32_ROWS ? (int)most : XB_F32_ROWS;
+    XB_TRY(hy_alloc_t(hy, &hy->pieces, 3 * (size_t)hy->pieces_rows * hy->maxK));
+  }
   if (d.block == XB_BLOCK_PARALLEL || d.block == XB_BLOCK_PRENORM) XB_TRY(hy_alloc(hy, &hy->ah, Tm * D * as));
   {
     // the first layer that blends values leaves them for the others, whose value rows must have the same width
@@ -956,6 +964,7 @@ static int hy_finalize(xb_engine* e) {
   if (hy->finalized) return 0;
   hy->finalized = true;
   hy->plans.clear();
+  hy->f32_plans.clear();
   if (hy->d.compute_fp32 || !hy->use_tc || hy_n_missing(hy) > 0) return 0;
   const size_t D = hy->d.dim;
   auto retile = [&](bf16** dst, const bf16* src, size_t rows, size_t K) -> int {
@@ -1145,6 +1154,32 @@ static bool hy_tc_linear(xb_engine* e, const void* x, long long ldx, const bf16*
   return true;
 }
 
+// The float32 mode on the tensor cores (xb_linear_f32.cuh); input widths off its grid take the plain kernels.
+static bool hy_f32_linear_takes(const xb_engine* e, const bf16* w, int K) {
+  return e->hy->use_tc && e->hy->pieces != nullptr && (size_t)K <= e->hy->maxK && xb_f32_takes(w, K);
+}
+static int hy_f32_linear(xb_engine* e, const float* x, long long ldx, const bf16* w, const float* bias, int T, int N, int K, float* out, cudaStream_t st,
+                         LinOut* y) {
+  HyModel* hy = e->hy;
+  for (int t0 = 0; t0 < T; t0 += hy->pieces_rows) {
+    const int rows = T - t0 < hy->pieces_rows ? T - t0 : hy->pieces_rows;
+    float* yo = out + (long long)t0 * N;
+    const auto key = std::make_tuple((const void*)w, (const void*)bias, (const void*)yo, rows, N, K);
+    auto it = hy->f32_plans.find(key);
+    if (it == hy->f32_plans.end()) {
+      F32Plan p;
+      XB_TRY(xb_f32_plan(&p, hy->pieces, hy->pieces_rows, w, bias, yo, N, rows, N, K, e->num_sms));
+      it = hy->f32_plans.emplace(key, p).first;
+    }
+    XB_TRY(hy_launch(e, xb_f32_pieces_kernel, dim3((unsigned)(((long long)rows * (K / 8) + 255) / 256)), dim3(256), 0, st, x + (long long)t0 * ldx, ldx,
+                     hy->pieces, (long long)hy->pieces_rows * K, rows, K));
+    XB_TRY(xb_f32_run(it->second, st, e->use_pdl && hy->pdl_now));
+    LAUNCH_COUNT(e);
+  }
+  *y = hy_plain(out, N);
+  return 0;
+}
+
 // y[T, N] = x[T, K] w^T + bias into `out` (`cap` bytes).  wt: the weight's tile-major copy or nullptr.
 template <typename AT>
 static int hy_linear(xb_engine* e, const void* x, long long ldx, const bf16* w, const bf16* wt, const float* bias, int T, int N, int K,
@@ -1154,6 +1189,7 @@ static int hy_linear(xb_engine* e, const void* x, long long ldx, const bf16* w, 
     if (hy_tc_linear(e, x, ldx, wt, bias, T, N, K, out, cap, st, y, &rc)) return rc;
   }
   const AT* xa = reinterpret_cast<const AT*>(x);
+  if (std::is_same<AT, float>::value && hy_f32_linear_takes(e, w, K)) return hy_f32_linear(e, (const float*)x, ldx, w, bias, T, N, K, out, st, y);
   if (T <= HY_SMALL_T)
     XB_TRY(hy_launch(e, hy_linear_small_kernel<AT>, dim3((N + 7) / 8), dim3(256), 0, st, xa, ldx, w, bias, out, (long long)N, T, N, K));
   else

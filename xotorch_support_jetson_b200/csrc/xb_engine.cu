@@ -1545,7 +1545,25 @@ extern "C" int xb_sample(xb_engine* e, const float* logits, int n, float temp, i
   XB_CUDA(cudaSetDevice(e->device));
   cudaStream_t st = (cudaStream_t)stream;
   if (temp <= 0.f) {
-    xb_argmax_kernel<1024><<<n, 1024, 0, st>>>(logits, e->d.vocab, tokens_out);
+    constexpr int CL = 8;
+    const int V = e->d.vocab;
+    // eight blocks a row up to two waves of clusters; more rows, or rows of a few thousand numbers, fill the chip a block each
+    if (V >= 4096 && n <= 2 * e->num_sms / CL) {
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(n * CL);
+      cfg.blockDim = dim3(512);
+      cfg.stream = st;
+      cudaLaunchAttribute attr[1];
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = CL;
+      attr[0].val.clusterDim.y = 1;
+      attr[0].val.clusterDim.z = 1;
+      cfg.attrs = attr;
+      cfg.numAttrs = 1;
+      XB_CUDA(cudaLaunchKernelEx(&cfg, xb_argmax_cluster_kernel<512, CL>, logits, V, (((V + CL - 1) / CL) + 3) & ~3, (int*)tokens_out));
+    } else {
+      xb_argmax_kernel<1024><<<n, 1024, 0, st>>>(logits, V, tokens_out);
+    }
   } else {
     // a cluster of 4 blocks per row keeps the row in shared memory (xb_sample_cluster.cuh); rows too long
     // for 4 x 200 KB, or XB_SAMPLE_CLUSTER=0, take the one-block-per-row kernel

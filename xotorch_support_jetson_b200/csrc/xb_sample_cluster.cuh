@@ -24,6 +24,111 @@ struct SampleXchg {
   int pad;
 };
 
+// Top-k of up to XB_TOPK_FAST: the row is dealt into buckets (what eight lanes, or a warp, have read); the k-th largest bucket
+// maximum has k elements at or above it, so the elements from there on contain the kept set -- about k + k^2 / (2 buckets) of
+// 128256, 41 for k = 35.  Only these candidates are looked at again: pivot, softmax, nucleus and draw run over them in the first
+// block of the cluster.  Bound by reading the row and by four cluster barriers: 32 x 128256 logits, top-k 35, 26.6 -> 19.9 us a call (what the host needs to enqueue it),
+// top-k 35 + top-p 0.9 45 -> 35, against four radix passes over every element.  Rows with more candidates than fit (many ties), or with a NaN, and larger k
+// take the radix passes.
+#define XB_TOPK_FAST 256
+#define XB_TOPK_CAND 512    // candidates a block can hold
+struct SampleCand {
+  float bucket[128];        // this block's bucket maxima
+  float v[XB_TOPK_CAND];
+  int i[XB_TOPK_CAND];
+  int n;                    // > XB_TOPK_CAND: take the radix passes
+};
+
+// the first block's last steps over n candidates (v, i in shared memory, any order): the chosen index, in every thread
+template <int NT>
+__device__ int sample_candidates(const float* v, const int* idx, int n, int top_k, float top_p, const float* __restrict__ q_row, unsigned long long seed,
+                                 int rowi, float* sorted_e, float* cum, float* s_f, int* s_i) {
+  const int tid = threadIdx.x;
+  if (tid == 0) { s_f[0] = -INFINITY; s_f[1] = -INFINITY; }
+  __syncthreads();
+  // rank of every candidate by (value down, index up): a fixed order whatever order they arrived in
+  float my_v[2];
+  int my_i[2], my_r[2], gt[2], ge[2];
+#pragma unroll
+  for (int c = 0; c < 2; ++c) {
+    const int a = tid + c * NT;
+    my_r[c] = gt[c] = ge[c] = 0;
+    if (a < n) {
+      my_v[c] = v[a]; my_i[c] = idx[a];
+      for (int b = 0; b < n; ++b) {
+        const float o = v[b];
+        gt[c] += o > my_v[c];
+        ge[c] += o >= my_v[c];
+        my_r[c] += o > my_v[c] || (o == my_v[c] && idx[b] < my_i[c]);
+      }
+      if (my_r[c] == 0) s_f[1] = my_v[c];                       // largest value
+      if (gt[c] < top_k && ge[c] >= top_k) s_f[0] = my_v[c];    // k-th largest value (every thread that writes has the same)
+    }
+  }
+  __syncthreads();
+  const float pivot = s_f[0], mxv = s_f[1];
+#pragma unroll
+  for (int c = 0; c < 2; ++c)
+    if (tid + c * NT < n) sorted_e[my_r[c]] = my_v[c] >= pivot ? expf(my_v[c] - mxv) : 0.f;
+  __syncthreads();
+  if (tid < 32) {               // running sums in rank order, a fixed tree
+    float base = 0.f;
+    for (int a = 0; a < n; a += 32) {
+      float x = a + tid < n ? sorted_e[a + tid] : 0.f;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const float y = __shfl_up_sync(0xffffffffu, x, o);
+        if (tid >= o) x += y;
+      }
+      x += base;
+      if (a + tid < n) cum[a + tid] = x;
+      base = __shfl_sync(0xffffffffu, x, 31);
+    }
+    if (tid == 0) { s_f[2] = base; s_f[3] = 0.f; }
+  }
+  __syncthreads();
+  const float sum = s_f[2];
+  if (top_p > 0.f && top_p < 1.f) {   // smallest probability of the shortest head that reaches top_p, equal ones with it
+    for (int a = tid; a < n; a += NT)
+      if (cum[a] >= top_p * sum && (a == 0 || cum[a - 1] < top_p * sum)) s_f[3] = sorted_e[a];
+    __syncthreads();
+  }
+  const float p_cut = s_f[3];
+  float best = -INFINITY;
+  int bi = 0x7fffffff;
+#pragma unroll
+  for (int c = 0; c < 2; ++c) {
+    if (tid + c * NT >= n || my_v[c] < pivot) continue;
+    const float e = expf(my_v[c] - mxv);
+    if (e < p_cut) continue;
+    float qv;
+    if (q_row != nullptr) {
+      qv = q_row[my_i[c]];
+    } else {
+      const uint32_t r = mix32(seed * 0x9E3779B97F4A7C15ULL + ((unsigned long long)rowi << 32) + (unsigned)my_i[c]);
+      const float u = ((float)(r & 0xffffff) + 0.5f) * (1.0f / 16777216.0f);
+      qv = -logf(u);
+    }
+    const float sc = (e / sum) / qv;
+    if (sc > best || (sc == best && my_i[c] < bi)) { best = sc; bi = my_i[c]; }
+  }
+  auto better = [](float a, int ai, float b, int bj) { return a > b || (a == b && ai < bj); };
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const float ov = __shfl_xor_sync(0xffffffffu, best, o);
+    const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
+    if (better(ov, oi, best, bi)) { best = ov; bi = oi; }
+  }
+  __syncthreads();
+  if ((tid & 31) == 0) { s_f[4 + (tid >> 5)] = best; s_i[tid >> 5] = bi; }
+  __syncthreads();
+  best = s_f[4];
+  bi = s_i[0];
+  for (int w = 1; w < NT / 32; ++w)
+    if (better(s_f[4 + w], s_i[w], best, bi)) { best = s_f[4 + w]; bi = s_i[w]; }
+  return bi;
+}
+
 template <int NT, int CL>
 __global__ void __launch_bounds__(NT) xb_sample_cluster_kernel(const float* __restrict__ logits, int V, int chunk, float temp,
                                                                int top_k, float top_p, const float* __restrict__ q_noise,
@@ -38,6 +143,7 @@ __global__ void __launch_bounds__(NT) xb_sample_cluster_kernel(const float* __re
   __shared__ float red[32];
   __shared__ float sv[NT / 32];
   __shared__ int si[NT / 32];
+  __shared__ SampleCand cand;
   cg::cluster_group cluster = cg::this_cluster();
   const int rank = (int)cluster.block_rank();
   const int rowi = blockIdx.x / CL;
@@ -49,6 +155,7 @@ __global__ void __launch_bounds__(NT) xb_sample_cluster_kernel(const float* __re
 
   // ---- load the slice once (float4 when the row allows it), scale, local max
   float mx = -INFINITY;
+  bool odd = false;                               // a NaN among this thread's numbers
   if ((V & 3) == 0 && (chunk & 3) == 0 && (reinterpret_cast<uintptr_t>(row) & 15) == 0) {
     const float4* r4 = reinterpret_cast<const float4*>(row + i0);
     float4* v4 = reinterpret_cast<float4*>(vals);
@@ -56,6 +163,7 @@ __global__ void __launch_bounds__(NT) xb_sample_cluster_kernel(const float* __re
     auto put = [&](int i, float4 a) {
       a.x *= inv_t; a.y *= inv_t; a.z *= inv_t; a.w *= inv_t;
       v4[i] = a;
+      odd = odd || !(a.x + a.y + a.z + a.w == a.x + a.y + a.z + a.w);
       mx = fmaxf(fmaxf(mx, fmaxf(a.x, a.y)), fmaxf(a.z, a.w));
     };
     int i = threadIdx.x;
@@ -68,8 +176,80 @@ __global__ void __launch_bounds__(NT) xb_sample_cluster_kernel(const float* __re
     for (int i = threadIdx.x; i < n; i += NT) {
       const float v = row[i0 + i] * inv_t;
       vals[i] = v;
+      odd = odd || v != v;
       mx = fmaxf(mx, v);
     }
+  }
+  const bool use_k = top_k > 0 && top_k < V;
+  if (use_k && top_k <= XB_TOPK_FAST) {
+    // ---- candidates: everything from the k-th largest bucket maximum on
+    const int lane = threadIdx.x & 31, per = top_k <= 64 ? 32 : 8;   // lanes of a bucket: 32 or 128 buckets a block
+    const int nb = NT / per;
+    float bm = mx;
+    for (int o = 1; o < per; o <<= 1) bm = fmaxf(bm, __shfl_xor_sync(0xffffffffu, bm, o));
+    if (lane % per == 0) cand.bucket[threadIdx.x / per] = bm;
+    const int any_odd = __syncthreads_or(odd);
+    if (threadIdx.x == 0) cand.n = any_odd ? XB_TOPK_CAND + 1 : 0;
+    cluster.sync();
+    float* all = mfh;                             // [CL * nb] bucket maxima of the row (mfh | mh: 512 numbers)
+    static_assert(CL * 128 <= 512, "bucket maxima of a row");
+    for (int i = threadIdx.x; i < CL * nb; i += NT) {
+      const float b = cluster.map_shared_rank(&cand, i / nb)->bucket[i % nb];
+      if (i < 256) mfh[i] = b; else mh[i - 256] = __float_as_uint(b);
+    }
+    __syncthreads();
+    if (threadIdx.x < CL * nb) {
+      auto at = [&](int i) { return i < 256 ? all[i] : __uint_as_float(mh[i - 256]); };
+      const float b = at(threadIdx.x);
+      int gt = 0, ge = 0;
+      for (int i = 0; i < CL * nb; ++i) {
+        const float o = at(i);
+        gt += o > b;
+        ge += o >= b;
+      }
+      if (gt < top_k && ge >= top_k) s_needf = b;   // all that write write the same
+    }
+    __syncthreads();
+    const float low = s_needf;
+    if (!any_odd) {
+      for (int i = threadIdx.x; i < n; i += NT) {
+        const float v = vals[i];
+        if (v >= low) {
+          const int at = atomicAdd(&cand.n, 1);
+          if (at < XB_TOPK_CAND) { cand.v[at] = v; cand.i[at] = i0 + i; }
+        }
+      }
+    }
+    cluster.sync();
+    int total = 0;
+    bool fits = true;
+    for (int r = 0; r < CL; ++r) {
+      const int c = cluster.map_shared_rank(&cand, r)->n;
+      fits = fits && c <= XB_TOPK_CAND;
+      total += c;
+    }
+    if (fits && total <= 2 * NT && 4 * total <= chunk) {   // the same answer in every block of the cluster
+      if (rank == 0) {
+        float* cv = vals;                         // the slice is not needed any more
+        int* ci = reinterpret_cast<int*>(vals + total);
+        float* es = vals + 2 * total;
+        float* cum = vals + 3 * total;
+        int at = 0;
+        for (int r = 0; r < CL; ++r) {
+          const SampleCand* pc = cluster.map_shared_rank(&cand, r);
+          const int c = pc->n;
+          for (int i = threadIdx.x; i < c; i += NT) { cv[at + i] = pc->v[i]; ci[at + i] = pc->i[i]; }
+          at += c;
+        }
+        __syncthreads();
+        const int bi = sample_candidates<NT>(cv, ci, total, top_k, top_p, q_noise != nullptr ? q_noise + (long long)rowi * V : nullptr, seed, rowi, es, cum,
+                                             mfh, si);
+        if (threadIdx.x == 0) out[rowi] = bi == 0x7fffffff ? 0 : bi;
+      }
+      cluster.sync();                             // the peers' candidates outlive the first block's reads
+      return;
+    }
+    __syncthreads();
   }
   mx = warp_max(mx);
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = mx;
@@ -85,7 +265,6 @@ __global__ void __launch_bounds__(NT) xb_sample_cluster_kernel(const float* __re
   float mxv = -INFINITY;                          // global max = max of the kept set
   bool have_max = false;
   uint32_t pivot_key = 0;
-  const bool use_k = top_k > 0 && top_k < V;
   if (use_k) {
     uint32_t prefix = 0;
     int need = top_k;
@@ -113,14 +292,25 @@ __global__ void __launch_bounds__(NT) xb_sample_cluster_kernel(const float* __re
       }
       __syncthreads();
       if (!have_max) { mxv = s_needf; have_max = true; }
-      if (threadIdx.x == 0) {
-        int nn = need, b = 255;
-        for (; b > 0; --b) {
-          if ((int)mh[b] >= nn) break;
-          nn -= (int)mh[b];
+      if (threadIdx.x < 32) {
+        // lane l holds bins 255 - 8 l downwards: the first bin whose running count from the top reaches `need`
+        int c[8], mine = 0;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) { c[j] = (int)mh[255 - 8 * (int)threadIdx.x - j]; mine += c[j]; }
+        int before = mine;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int y = __shfl_up_sync(0xffffffffu, before, o);
+          if ((int)threadIdx.x >= o) before += y;
         }
-        s_prefix = prefix | ((uint32_t)b << shift);
-        s_need = nn;
+        const unsigned hit = __ballot_sync(0xffffffffu, before >= need);
+        const int who = hit != 0 ? __ffs(hit) - 1 : 31;
+        if ((int)threadIdx.x == who) {
+          int nn = need - (before - mine), j = 0;
+          for (; j < 7 && c[j] < nn; ++j) nn -= c[j];
+          s_prefix = prefix | ((uint32_t)(255 - 8 * who - j) << shift);
+          s_need = nn;
+        }
       }
       __syncthreads();
       prefix = s_prefix;
@@ -253,4 +443,47 @@ __global__ void __launch_bounds__(NT) xb_sample_cluster_kernel(const float* __re
     out[rowi] = bi == 0x7fffffff ? 0 : bi;
   }
   cluster.sync();                                 // peers' shared memory must outlive rank 0's reads
+}
+
+// First-index arg-max of a row by a cluster of CL blocks: one block reads a 128256-entry row at about 50 GB/s.
+template <int NT, int CL>
+__global__ void __launch_bounds__(NT) xb_argmax_cluster_kernel(const float* __restrict__ logits, int V, int chunk, int* __restrict__ out) {
+  __shared__ float sv[NT / 32];
+  __shared__ int si[NT / 32];
+  cg::cluster_group cluster = cg::this_cluster();
+  const int rank = (int)cluster.block_rank(), rowi = blockIdx.x / CL;
+  const float* row = logits + (long long)rowi * V;
+  const int i0 = rank * chunk, i1 = i0 + chunk < V ? i0 + chunk : V;
+  float best = -INFINITY;
+  int bi = 0x7fffffff;
+  auto take = [&](float v, int i) { if (v > best || (v == best && i < bi)) { best = v; bi = i; } };
+  if ((V & 3) == 0 && (reinterpret_cast<uintptr_t>(row) & 15) == 0) {   // chunk is a multiple of 4
+    const float4* r4 = reinterpret_cast<const float4*>(row);
+#pragma unroll 4
+    for (int i = (i0 >> 2) + threadIdx.x; i < (i1 >> 2); i += NT) {
+      const float4 a = r4[i];
+      take(a.x, 4 * i); take(a.y, 4 * i + 1); take(a.z, 4 * i + 2); take(a.w, 4 * i + 3);
+    }
+  } else {
+    for (int i = i0 + threadIdx.x; i < i1; i += NT) take(row[i], i);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const float ov = __shfl_xor_sync(0xffffffffu, best, o);
+    const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
+    take(ov, oi);
+  }
+  if ((threadIdx.x & 31) == 0) { sv[threadIdx.x >> 5] = best; si[threadIdx.x >> 5] = bi; }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < NT / 32; ++w) take(sv[w], si[w]);
+    sv[0] = best;
+    si[0] = bi;
+  }
+  cluster.sync();
+  if (rank == 0 && threadIdx.x == 0) {
+    for (int r = 1; r < CL; ++r) take(cluster.map_shared_rank(sv, r)[0], cluster.map_shared_rank(si, r)[0]);
+    out[rowi] = bi == 0x7fffffff ? 0 : bi;
+  }
+  cluster.sync();
 }

@@ -4,6 +4,7 @@
 // CUDA-graph replay of decode steps, sampling and the loader are the engine's own.
 #pragma once
 #include "xb_hybrid_kernels.cuh"
+#include "xb_delta_chunk.cuh"
 #include <set>
 #include <tuple>
 
@@ -109,6 +110,8 @@ struct HyModel {
   int recur_lpc = 0;         // XB_HY_LPC=4|8|16 pins the lanes per state column (A/B); 0: by the step's shape
   float *seg_ws = nullptr, *seg_decay = nullptr;   // recurrences cut into segments: a state and the decays per segment
   size_t maxSeg = 0, maxSegK = 0;                  // state numbers / key channels of the largest such layer
+  float* chunk_ws = nullptr;                       // delta rules by chunks: the prepared blocks (xb_delta_chunk.cuh)
+  size_t maxChunk = 0, chunk_entries = 0;          // floats of a chunk over all heads of the largest such layer, chunks it holds
   int use_seg = 1;           // XB_HY_SEG=0: recurrences always as one chain per sequence (A/B); XB_HY_SEG=n >= 64: segments of n tokens
   int seg_len = 0;           // pinned segment length, 0: by the step's shape
   int use_tc_attn = 1;       // XB_HY_TC_ATTN=0: attention through the per-token kernel everywhere (A/B)
@@ -171,6 +174,12 @@ static void hy_name_cols(HyModel* hy, const std::string& name, bf16* base, long 
 static void hy_segment_room(HyModel* hy, long long numbers, long long keys) {
   if ((size_t)numbers > hy->maxSeg) hy->maxSeg = numbers;
   if ((size_t)keys > hy->maxSegK) hy->maxSegK = keys;
+}
+
+static void hy_chunk_room(HyModel* hy, int mode, int heads, int dk) {
+  const int dkp = dk <= 64 ? 64 : dk <= 128 ? 128 : 256;
+  const size_t n = (size_t)heads * hy_chunk_block(mode, dkp);
+  if (n > hy->maxChunk) hy->maxChunk = n;
 }
 
 // A norm of the stream: one vector (or one number), for the tanh norm also an offset per channel and the input's factor.
@@ -324,6 +333,7 @@ static int hy_create_mixer(xb_engine* e, int i, bool own, size_t& st, uint64_t& 
     if ((size_t)l.n_o > hy->maxO) hy->maxO = l.n_o;
   } else if (c.mixer == XB_MIX_GDELTA) {
     const long long HN = H * n, rk = c.m_rank;
+    hy_chunk_room(hy, HY_REC_GDELTA, (int)H, (int)n);
     XB_CHECK(n <= HY_MAX_KDIM && rk > 0, "layer %d: bad delta-rule sizes (key dim <= %d)", i, HY_MAX_KDIM);
     l.off_r = 0; l.off_k = (int)HN; l.off_v = (int)(2 * HN); l.off_g = (int)(3 * HN); l.off_a = (int)(4 * HN); l.off_w1 = (int)(5 * HN);
     l.n_in = l.off_w1 + (int)rk;
@@ -657,6 +667,7 @@ static int hy_create(xb_engine* e, const xb_hybrid_desc& d, const xb_hybrid_laye
       const long long H = c.d_heads, G = c.d_kv_heads, dk = c.d_dim, dv = c.d_vdim, tp = c.d_taps;
       XB_CHECK(H > 0 && G > 0 && H % G == 0 && dk > 0 && dk <= HY_MAX_KDIM && dv > 0, "layer %d: bad delta-rule sizes (key dim <= %d)", i, HY_MAX_KDIM);
       XB_CHECK(tp >= 1 && tp <= HY_MAX_TAPS, "layer %d: short filter of %lld taps (1..%d)", i, tp, HY_MAX_TAPS);
+      hy_chunk_room(hy, HY_REC_DELTA, (int)H, (int)dk);
       l.off_q = 0; l.off_k = (int)(G * dk); l.off_v = (int)(2 * G * dk);
       l.c_conv = (int)(2 * G * dk + H * dv);
       l.off_g = l.c_conv; l.off_b = l.off_g + (int)(H * dv); l.off_a = l.off_b + (int)H;
@@ -899,6 +910,11 @@ static int hy_create(xb_engine* e, const xb_hybrid_desc& d, const xb_hybrid_laye
     const size_t entries = Tm / HY_SEG_MIN + Tm / (2 * HY_SEG_MIN) + 2;
     XB_TRY(hy_alloc_t(hy, &hy->seg_ws, entries * hy->maxSeg));
     XB_TRY(hy_alloc_t(hy, &hy->seg_decay, entries * hy->maxSegK));
+  }
+  if (hy->maxChunk > 0 && Tm >= hy_chunk_min(HY_REC_DELTA)) {
+    // steps of up to 8192 tokens; larger ones run token by token
+    hy->chunk_entries = (Tm < 8192 ? Tm : 8192) / HY_CT + d.max_seqs;
+    XB_TRY(hy_alloc_t(hy, &hy->chunk_ws, hy->chunk_entries * hy->maxChunk));
   }
   if (hy->maxQG > 0) {
     XB_TRY(hy_alloc_t(hy, &hy->qg, Tm * hy->maxQG));
@@ -1263,6 +1279,19 @@ static int hy_segments(xb_engine* e, const RecurIn& in, float* state, long long 
   return xb_fail(1, "recurrent key dim %d exceeds %d", dk, HY_MAX_KDIM);
 }
 
+// Prompts through the chunks of xb_delta_chunk.cuh (delta rules).
+template <int NCH, int MODE>
+static int hy_chunks_n(xb_engine* e, const RecurIn& in, float* state, long long ss, float* o, long long ldo, const BatchMeta& m, int n_seqs,
+                       int H, int dk, int dv, int T, cudaStream_t st) {
+  constexpr int DKP = 64 * NCH;
+  constexpr size_t ps = (size_t)hy_chunk_vectors(MODE) * HY_CT * (DKP + 4) * sizeof(float);
+  constexpr size_t cs = (size_t)2 * (hy_chunk_block(MODE, DKP) + HY_CT * 16) * sizeof(float);
+  if (ps > 48 * 1024) XB_SMEM_ATTR_ONCE((hy_chunk_prep_kernel<MODE>), 4 * HY_CT * 260 * sizeof(float));
+  if (cs > 48 * 1024) XB_SMEM_ATTR_ONCE((hy_chunk_kernel<NCH, MODE>), cs);
+  XB_TRY(hy_launch(e, hy_chunk_prep_kernel<MODE>, dim3(T / HY_CT + n_seqs, H), dim3(256), ps, st, in, e->hy->chunk_ws, m, n_seqs, H, dk, DKP));
+  return hy_launch(e, hy_chunk_kernel<NCH, MODE>, dim3(n_seqs, H, (dv + 15) / 16), dim3(128), cs, st, in, (const float*)e->hy->chunk_ws, state, ss, o, ldo,
+                   m, H, dk, dv);
+}
 template <int MODE>
 static int hy_recur(xb_engine* e, const RecurIn& in, float* state, long long ss, float* o, long long ldo, const BatchMeta& m, int n_seqs,
                     int H, int dk, int dv, int T, cudaStream_t st) {
@@ -1270,6 +1299,15 @@ static int hy_recur(xb_engine* e, const RecurIn& in, float* state, long long ss,
     const int least = e->hy->seg_len > 0 ? 2 * e->hy->seg_len : 4 * HY_SEG_MIN;   // average length from which it pays
     if (e->hy->use_seg && T / n_seqs >= least && (long long)n_seqs * (T / HY_SEG_MIN + 1) <= 65535)   // grid z
       return hy_segments<MODE>(e, in, state, ss, o, ldo, m, n_seqs, H, dk, dv, T, st);
+  }
+  if constexpr (MODE == HY_REC_DELTA || MODE == HY_REC_GDELTA) {
+    // (a pinned lane layout asks for the token-by-token kernel)
+    if (e->hy->use_seg && e->hy->recur_lpc == 0 && e->hy->chunk_ws != nullptr && T / n_seqs >= hy_chunk_min(MODE) &&
+        (size_t)(T / HY_CT + n_seqs) <= e->hy->chunk_entries) {
+      if (dk <= 64) return hy_chunks_n<1, MODE>(e, in, state, ss, o, ldo, m, n_seqs, H, dk, dv, T, st);
+      if (dk <= 128) return hy_chunks_n<2, MODE>(e, in, state, ss, o, ldo, m, n_seqs, H, dk, dv, T, st);
+      if (dk <= 256) return hy_chunks_n<4, MODE>(e, in, state, ss, o, ldo, m, n_seqs, H, dk, dv, T, st);
+    }
   }
   int lpc = e->hy->recur_lpc;
   if (lpc == 0) {

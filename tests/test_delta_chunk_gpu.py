@@ -1,0 +1,58 @@
+"""The delta rules by chunks of sixteen tokens against the same rules token by token (float32 engine): lengths around a chunk's and the
+rule's edges, key and value sizes around the kernel's tiles, shared key heads, unequal sequences, prompts that go on from a
+cached state, and decays near zero and one."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+_MLP = {"kind": "dense", "ff": 64}
+
+
+def _model(kind, dk, dv, heads, kv):
+  from xotorch_support_jetson_b200 import synth
+  if kind == "delta":
+    hf = {"architecture": "Refatar", "width": 64, "vocab": 97, "norm": {"eps": 1e-5},
+          "layers": [{"type": "delta", "mixer": {"heads": heads, "kv_heads": kv, "dim": dk, "vdim": dv, "conv": 2}, "mlp": None}]}
+    state = synth.random_refatar_state(hf, seed=dk + dv)
+    state["l0.mix.A_log"] = torch.linspace(-6.0, 4.5, heads)   # decays from about one down to exp(-90 softplus): zero within a few tokens
+  else:
+    hf = {"architecture": "Bibevik", "width": 64, "vocab": 97, "embedding": {"scale": 8.0}, "norm": {"eps": 1e-6},
+          "layers": [{"type": "general_delta", "mixer": {"heads": heads, "dim": dk, "rank": 8}, "mlp": None}]}
+    state = synth.random_bibevik_state(hf, seed=dk)
+    state["l0.mix.w0"] = torch.linspace(-9.0, 9.0, heads * dk)   # decays over their whole range
+  return hf, state
+
+
+def _run(hf, state, lens, monkeypatch, by_steps):
+  from xotorch_support_jetson_b200.model_config import hybrid_model_config, resolve_tensor_sizes
+  from xotorch_support_jetson_b200.shard import Shard
+  from xotorch_support_jetson_b200.stage import StageRuntime
+  monkeypatch.setenv("XB_HY_LPC", "16" if by_steps else "0")
+  cfg = hybrid_model_config(hf)
+  resolve_tensor_sizes(cfg, {k: tuple(v.shape) for k, v in state.items()})
+  st = StageRuntime(Shard("delta-test", 0, 0, 1), cfg, max_batch_tokens=sum(lens), max_seqs=len(lens), max_tokens_per_seq=2 * max(lens) + 8, dtype="float32")
+  st.load_state(state)
+  g = torch.Generator().manual_seed(sum(lens))
+  outs = []
+  for start in (0, 1):   # twice the same lengths: the second half goes on from the cached state
+    ids = torch.randint(0, 97, (sum(lens),), generator=g).to("cuda", torch.int32)
+    tap = torch.empty((sum(lens), 64), device="cuda")
+    st.forward(list(range(len(lens))), lens, [start * n for n in lens], tokens=ids, taps=[tap])
+    outs.append(tap.double().cpu())
+  torch.cuda.synchronize()
+  st.close()
+  return torch.cat(outs)
+
+
+@pytest.mark.parametrize("lens", [[96], [97], [111], [112], [113], [32, 300], [100, 96, 130]])
+@pytest.mark.parametrize("kind,dk,dv,heads,kv", [("delta", 32, 48, 4, 2), ("delta", 64, 16, 3, 1), ("delta", 65, 17, 2, 2), ("delta", 128, 33, 4, 4),
+                                                 ("delta", 200, 40, 2, 1), ("general", 32, 32, 3, 3), ("general", 64, 64, 2, 2), ("general", 72, 72, 2, 2),
+                                                 ("general", 130, 130, 1, 1)])
+def test_chunks_equal_steps(built_lib, monkeypatch, kind, dk, dv, heads, kv, lens):
+  hf, state = _model(kind, dk, dv, heads, kv)
+  a, b = (_run(hf, state, lens, monkeypatch, steps) for steps in (False, True))
+  assert torch.isfinite(a).all()
+  # both sum dk + 16 fp32 products in another order; read-out norm and output projection carry that on: a few 1e-6 of a row
+  err = (a - b).norm(dim=1) / b.norm(dim=1)
+  assert err.max() < 2e-5, err.max()

@@ -17,13 +17,14 @@
 // FMA), the 2 x 16 dot products of a chunk are reduced together by halving exchanges, after which lane i owns token i, and only the
 // triangular solve goes token by token.  Bound by instruction issue (about a thousand a chunk and warp, one warp a scheduler) and by that
 // solve.
-// 2048 tokens, 16 heads of 128 x 128 (gated): 741 -> @1@ us; 1800 tokens, 32 heads of 64 x 64 (general): 777 -> @2@ us, preparation
-// included.
+// 2048 tokens, 16 heads of 128 x 128 (gated): 741 -> 212 us and 38 us of preparation; 450 and 1350 tokens, 32 heads of 64 x 64
+// (general): 777 -> 213 and 98 us.  Errors against 64 bits as token by token (3.4e-7 and 2.9e-7 after 2047 tokens).
 #pragma once
 
 #define HY_CT 16          // tokens of a chunk = lanes that share a column
-// Average tokens of a sequence from which the chunks are used.  A layer, one sequence: gated 32 tokens 259 -> 249 us, 64 (two sequences) 419 -> 392;
-// general 32 236 -> 246, 64 359 -> 367 (the preparation costs more than it saves), 100 (six) 495 -> 472, 400 462 -> 393.
+#define HY_CHUNK_VP 18    // pitch of the chunk's 16 x 16 values in shared memory
+// Average tokens of a sequence from which the chunks are used.  A layer in bf16, token by token -> chunks: gated, 32 tokens 257 -> 245 us,
+// two of 64 417 -> 388; general, 32 tokens 241 -> 236, 33 237 -> 239, two of 64 363 -> 359, six of 100 493 -> 430.
 __host__ __device__ constexpr int hy_chunk_min(int mode) { return mode == HY_REC_GDELTA ? 96 : 32; }
 __host__ __device__ constexpr int hy_chunk_vectors(int mode) { return mode == HY_REC_GDELTA ? 4 : 2; }
 // floats of one (chunk, head): the row vectors [vectors][16][dkp], for the general rule P_16 [dkp], the matrices [16][16], sixteen numbers per token
@@ -32,7 +33,7 @@ __host__ __device__ constexpr int hy_chunk_scal(int mode, int dkp) { return hy_c
 __host__ __device__ constexpr int hy_chunk_block(int mode, int dkp) { return hy_chunk_scal(mode, dkp) + 6 * HY_CT; }
 
 // entry of chunk c of sequence s: start_row / 16 + s + c (no two sequences share one)
-// grid (T / 16 + n_seqs, H), 256 threads; dynamic shared memory: the row vectors at pitch dkp + 4, decays
+// grid (T / 16 + n_seqs, H), 256 threads; dynamic shared memory: the row vectors (general rule: and the decays) at pitch dkp + 4
 template <int MODE>
 __global__ void __launch_bounds__(256) hy_chunk_prep_kernel(RecurIn in, float* __restrict__ ws, BatchMeta m, int n_seqs, int H, int dk, int dkp) {
   extern __shared__ __align__(16) float cps[];
@@ -68,7 +69,7 @@ __global__ void __launch_bounds__(256) hy_chunk_prep_kernel(RecurIn in, float* _
     }
     if (tid < HY_CT) gs[tid] = tid < nt ? in.decay[(row0 + tid) * H + h] : 1.f;
     __syncthreads();
-    const int i = tid >> 4, j = tid & 15;
+    const int i = tid & 15, j = tid >> 4;   // matrices lie column by column: lane i of the walk reads its row without bank conflicts
     float kk = 0.f, qk = 0.f;
     if (j < i) {
       const float *ki = cps + i * pitch, *qi = cps + (HY_CT + i) * pitch, *kj = cps + j * pitch;
@@ -101,26 +102,40 @@ __global__ void __launch_bounds__(256) hy_chunk_prep_kernel(RecurIn in, float* _
       scal[5 * HY_CT + tid] = all;
     }
   } else {
+    float* wv = cps + 4 * HY_CT * pitch;
+    const int n4 = HY_CT * dkp;
+#pragma unroll 4
+    for (int x = tid; x < n4; x += 256) {   // u, r*w, k, a*u, w as they are
+      const int t = x / dkp, r = x - t * dkp;
+      const bool have = t < nt && r < dk;
+      const float* src = in.c + (row0 + t) * in.ldc + (long long)g * dk + r;
+      cps[t * pitch + r] = have ? src[in.koff] : 0.f;
+      cps[(HY_CT + t) * pitch + r] = have ? src[in.qoff] : 0.f;
+      cps[(2 * HY_CT + t) * pitch + r] = have ? src[in.xoff[2]] : 0.f;
+      cps[(3 * HY_CT + t) * pitch + r] = have ? src[in.xoff[1]] : 0.f;
+      wv[t * pitch + r] = have ? src[in.xoff[0]] : 1.f;
+    }
+    __syncthreads();
     for (int r = tid; r < dkp; r += 256) {
       float P = 1.f;
-      for (int t = 0; t < HY_CT; ++t) {
-        const bool have = t < nt && r < dk;
-        const float* src = in.c + (row0 + t) * in.ldc + (long long)g * dk + r;
-        const float u = have ? src[in.koff] * P : 0.f, q = have ? src[in.qoff] * P : 0.f;   // before this token's decay
-        if (have) P *= src[in.xoff[0]];
-        const float ip = 1.0f / P;
-        const float e = have ? src[in.xoff[1]] * ip : 0.f, k = have ? src[in.xoff[2]] * ip : 0.f;
-        const float v[4] = {u, q, k, e};
 #pragma unroll
-        for (int x = 0; x < 4; ++x) {
-          cps[(x * HY_CT + t) * pitch + r] = v[x];
-          blk[(x * HY_CT + t) * dkp + r] = v[x];
-        }
+      for (int t = 0; t < HY_CT; ++t) {
+        float* x = cps + t * pitch + r;
+        x[0] *= P;                          // before this token's decay
+        x[HY_CT * pitch] *= P;
+        P *= wv[t * pitch + r];
+        const float ip = 1.0f / P;
+        x[2 * HY_CT * pitch] *= ip;
+        x[3 * HY_CT * pitch] *= ip;
       }
       blk[4 * HY_CT * dkp + r] = P;
     }
     __syncthreads();
-    const int i = tid >> 4, j = tid & 15;
+    for (int x = tid; x < 4 * n4; x += 256) {
+      const int t = x / dkp, r = x - t * dkp;
+      blk[x] = cps[t * pitch + r];
+    }
+    const int i = tid & 15, j = tid >> 4;   // matrices lie column by column: lane i of the walk reads its row without bank conflicts
     float o[4] = {0.f, 0.f, 0.f, 0.f};   // u.k, u.e, q.k, q.e
     if (j < i) {
       const float *ui = cps + i * pitch, *qi = cps + (HY_CT + i) * pitch, *kj = cps + (2 * HY_CT + j) * pitch, *ej = cps + (3 * HY_CT + j) * pitch;
@@ -160,13 +175,13 @@ __device__ __forceinline__ void hy_chunk_reduce(float (&v)[HY_CT][2], int sub) {
   }
 }
 
-// grid (n_seqs, H, ceil(dv / 16)), 128 threads (16 value columns); dynamic shared memory 2 * (block + 16 x 16 values) floats
+// grid (n_seqs, H, ceil(dv / 16)), 128 threads (16 value columns); dynamic shared memory 2 * (block + 16 x 18 values) floats
 template <int NCH, int MODE>
 __global__ void __launch_bounds__(128) hy_chunk_kernel(RecurIn in, const float* __restrict__ ws, float* __restrict__ state, long long state_stride,
                                                        float* __restrict__ o, long long ldo, BatchMeta m, int H, int dk, int dv) {
   pdl_wait();   // no early trigger, as in hy_recur_kernel
   extern __shared__ __align__(16) float cks[];
-  constexpr int DKP = 64 * NCH, BLK = hy_chunk_block(MODE, DKP), NB = BLK + HY_CT * 16, RP = HY_CT * DKP;
+  constexpr int DKP = 64 * NCH, BLK = hy_chunk_block(MODE, DKP), NB = BLK + HY_CT * HY_CHUNK_VP, RP = HY_CT * DKP;
   const int s = blockIdx.x, h = blockIdx.y, tid = threadIdx.x;
   const int warp = tid >> 5, lane = tid & 31, sub = lane & 15;
   const int j0 = blockIdx.z * 16, jl = warp * 4 + (lane >> 4) * 2, col = j0 + jl;   // this lane's columns col, col + 1
@@ -179,8 +194,8 @@ __global__ void __launch_bounds__(128) hy_chunk_kernel(RecurIn in, const float* 
     for (int i = tid; i < BLK / 4; i += 128) hy_cp16(buf + 4 * i, src + 4 * i);
     for (int i = tid; i < HY_CT * 16; i += 128) {
       const int t = c * HY_CT + (i >> 4), x = i & 15;
-      if (t < sp.len && x < ncv) hy_cp4(buf + BLK + i, cv + (sp.start + t) * in.ldc + x);
-      else buf[BLK + i] = 0.f;
+      if (t < sp.len && x < ncv) hy_cp4(buf + BLK + (i >> 4) * HY_CHUNK_VP + x, cv + (sp.start + t) * in.ldc + x);
+      else buf[BLK + (i >> 4) * HY_CHUNK_VP + x] = 0.f;
     }
     hy_cp_commit();
   };
@@ -240,7 +255,7 @@ __global__ void __launch_bounds__(128) hy_chunk_kernel(RecurIn in, const float* 
     float pa[2], pb[2], ov[2];
     dots(buf, pa);
     dots(buf + RP, pb);
-    const float2 v2 = *reinterpret_cast<const float2*>(V + sub * 16);
+    const float2 v2 = *reinterpret_cast<const float2*>(V + sub * HY_CHUNK_VP);
     const float v[2] = {v2.x, v2.y};
     float coef[HY_CT][2];          // what every token writes into the two columns (the same in all sixteen lanes)
     if (MODE == HY_REC_DELTA) {
@@ -249,7 +264,7 @@ __global__ void __launch_bounds__(128) hy_chunk_kernel(RecurIn in, const float* 
       float u[2];
 #pragma unroll
       for (int j = 0; j < HY_CT; ++j) {
-        const float kk = mats[sub * HY_CT + j], qq = mats[HY_CT * HY_CT + sub * HY_CT + j], behind = scal[4 * HY_CT + j];
+        const float kk = mats[j * HY_CT + sub], qq = mats[HY_CT * HY_CT + j * HY_CT + sub], behind = scal[4 * HY_CT + j];
 #pragma unroll
         for (int x = 0; x < 2; ++x) {
           u[x] = be * (v[x] - gd * pa[x]);   // final in lane j
@@ -284,14 +299,14 @@ __global__ void __launch_bounds__(128) hy_chunk_kernel(RecurIn in, const float* 
       constexpr int M = HY_CT * HY_CT;
 #pragma unroll
       for (int j = 0; j < HY_CT; ++j) {
-        const float2 vj = *reinterpret_cast<const float2*>(V + j * 16);
-        const float uk = mats[sub * HY_CT + j], qk = mats[2 * M + sub * HY_CT + j];
+        const float2 vj = *reinterpret_cast<const float2*>(V + j * HY_CHUNK_VP);
+        const float uk = mats[j * HY_CT + sub], qk = mats[2 * M + j * HY_CT + sub];
         pa[0] = j < sub ? fmaf(uk, vj.x, pa[0]) : pa[0]; pa[1] = j < sub ? fmaf(uk, vj.y, pa[1]) : pa[1];
         pb[0] = j < sub ? fmaf(qk, vj.x, pb[0]) : pb[0]; pb[1] = j < sub ? fmaf(qk, vj.y, pb[1]) : pb[1];
       }
 #pragma unroll
       for (int j = 0; j < HY_CT; ++j) {
-        const float ue = mats[M + sub * HY_CT + j], qe = mats[3 * M + sub * HY_CT + j];
+        const float ue = mats[M + j * HY_CT + sub], qe = mats[3 * M + j * HY_CT + sub];
 #pragma unroll
         for (int x = 0; x < 2; ++x) {
           const float aj = __shfl_sync(0xffffffffu, pa[x], j, 16);   // final in lane j
@@ -305,7 +320,7 @@ __global__ void __launch_bounds__(128) hy_chunk_kernel(RecurIn in, const float* 
       for (int x = 0; x < 2; ++x) ov[x] = fmaf(rk, v[x], fmaf(-ra, pa[x], pb[x]));
 #pragma unroll
       for (int j = 0; j < HY_CT; ++j) {
-        const float2 vj = *reinterpret_cast<const float2*>(V + j * 16);
+        const float2 vj = *reinterpret_cast<const float2*>(V + j * HY_CHUNK_VP);
         const hy_f2 kv[2] = {hy_f2_pack(vj.x, vj.x), hy_f2_pack(vj.y, vj.y)};
         const hy_f2 ea[2] = {hy_f2_pack(-coef[j][0], -coef[j][0]), hy_f2_pack(-coef[j][1], -coef[j][1])};
 #pragma unroll

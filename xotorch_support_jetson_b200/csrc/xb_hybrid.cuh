@@ -1284,9 +1284,10 @@ template <int NCH, int MODE>
 static int hy_chunks_n(xb_engine* e, const RecurIn& in, float* state, long long ss, float* o, long long ldo, const BatchMeta& m, int n_seqs,
                        int H, int dk, int dv, int T, cudaStream_t st) {
   constexpr int DKP = 64 * NCH;
-  constexpr size_t ps = (size_t)hy_chunk_vectors(MODE) * HY_CT * (DKP + 4) * sizeof(float);
-  constexpr size_t cs = (size_t)2 * (hy_chunk_block(MODE, DKP) + HY_CT * 16) * sizeof(float);
-  if (ps > 48 * 1024) XB_SMEM_ATTR_ONCE((hy_chunk_prep_kernel<MODE>), 4 * HY_CT * 260 * sizeof(float));
+  constexpr int rows = MODE == HY_REC_GDELTA ? 5 : 2;
+  constexpr size_t ps = (size_t)rows * HY_CT * (DKP + 4) * sizeof(float);
+  constexpr size_t cs = (size_t)2 * (hy_chunk_block(MODE, DKP) + HY_CT * HY_CHUNK_VP) * sizeof(float);
+  if (ps > 48 * 1024) XB_SMEM_ATTR_ONCE((hy_chunk_prep_kernel<MODE>), rows * HY_CT * 260 * sizeof(float));
   if (cs > 48 * 1024) XB_SMEM_ATTR_ONCE((hy_chunk_kernel<NCH, MODE>), cs);
   XB_TRY(hy_launch(e, hy_chunk_prep_kernel<MODE>, dim3(T / HY_CT + n_seqs, H), dim3(256), ps, st, in, e->hy->chunk_ws, m, n_seqs, H, dk, DKP));
   return hy_launch(e, hy_chunk_kernel<NCH, MODE>, dim3(n_seqs, H, (dv + 15) / 16), dim3(128), cs, st, in, (const float*)e->hy->chunk_ws, state, ss, o, ldo,

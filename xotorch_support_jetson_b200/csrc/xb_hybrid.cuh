@@ -5,6 +5,7 @@
 #pragma once
 #include "xb_hybrid_kernels.cuh"
 #include "xb_delta_chunk.cuh"
+#include "xb_hybrid_quad.cuh"
 #include <set>
 #include <tuple>
 
@@ -1329,6 +1330,15 @@ static int hy_filter(xb_engine* e, int T, int n_seqs, bool no_span, const LinOut
                      const BatchMeta& m, int identity, int act_silu, OT* out, long long ld_out, cudaStream_t st) {
   const long long SS = (long long)e->hy->state_floats;
   bool tail_done = false;
+  if (T > 64 && taps >= 2 && taps <= 4 && C % 4 == 0 && ld_out % 4 == 0 && SS % 4 == 0 && hy_quad(in, col0) && hy_quad_ptr(tail) && hy_quad_ptr(out)) {
+    // prompts: four channels and eight rows per thread
+    const dim3 g((T + 7) / 8, (C / 4 + 255) / 256);
+    auto run = [&](auto kern) { return hy_launch(e, kern, g, dim3(256), 0, st, in, col0, C, w, (const float*)tail, SS, m, identity, act_silu, out, ld_out, T); };
+    if (taps == 2) XB_TRY(run(hy_taps_quad_kernel<OT, 2>));
+    else if (taps == 3) XB_TRY(run(hy_taps_quad_kernel<OT, 3>));
+    else XB_TRY(run(hy_taps_quad_kernel<OT, 4>));
+    return hy_launch(e, hy_tail_update_kernel, dim3(n_seqs, (C + 255) / 256), dim3(256), 0, st, in, col0, C, taps, tail, SS, m);
+  }
   const bool few = T <= 64;   // a block per row instead of 16 rows per thread
   const dim3 tg(few ? T : (T + 15) / 16, (C + 255) / 256);
   const int wt = no_span ? 1 : 0;
@@ -1473,6 +1483,10 @@ static int hy_row_op_launch(xb_engine* e, int T, const RowOpArgs& a, cudaStream_
     if (few) return hy_launch(e, hy_row_op_ext_kernel<AT, 1024>, dim3(T), dim3(1024), (size_t)hy->d.dim * sizeof(float), st, a);
     return hy_launch(e, hy_row_op_ext_kernel<AT, 256>, dim3(T), dim3(256), (size_t)hy->d.dim * sizeof(float), st, a);
   }
+  const LinOut* ms[3] = {&a.m1, &a.m2, &a.m3};
+  bool quad = !few && hy->d.dim % 4 == 0 && (a.bw == nullptr || hy_quad_ptr(a.bw));
+  for (const LinOut* o : ms) quad = quad && ((o->f == nullptr && o->h == nullptr) || hy_quad(*o, 0));
+  if (quad) return hy_launch(e, hy_row_op_quad_kernel<AT>, dim3(T), dim3(256), (size_t)hy->d.dim * sizeof(float), st, a);
   if (few) return hy_launch(e, hy_row_op_kernel<AT, 1024>, dim3(T), dim3(1024), (size_t)hy->d.dim * sizeof(float), st, a);
   return hy_launch(e, hy_row_op_kernel<AT, 256>, dim3(T), dim3(256), (size_t)hy->d.dim * sizeof(float), st, a);
 }
@@ -1729,6 +1743,10 @@ static int hy_ff_parallel(xb_engine* e, const HyLayer& l, int T, const void* xin
 }
 
 template <typename AT>
+static int hy_head_norm(xb_engine* e, int T, long long ldo, const float* w, const LinOut& P, int off_gate, AT* out, long long ld_out, int H, int dv,
+                        int w_hstride, int gate_sigmoid, cudaStream_t st);
+
+template <typename AT>
 static int hy_run_parallel_t(xb_engine* e, int T, int n_seqs, void* const* taps, cudaStream_t st, int with_head) {
   HyModel* hy = e->hy;
   const xb_hybrid_desc& d = hy->d;
@@ -1769,18 +1787,25 @@ static int hy_run_parallel_t(xb_engine* e, int T, int n_seqs, void* const* taps,
       LinOut Wd;
       XB_TRY(hy_launch(e, hy_act_cols_kernel<AT>, dim3(T, (rk + 255) / 256), dim3(256), 0, st, P, l.off_w1, rk, 1, a2, (long long)rk));
       XB_TRY(hy_linear<AT>(e, a2, rk, l.w_d2, l.t_d2, nullptr, T, HN, rk, hy->m2, hy->cap_m, st, &Wd));
-      XB_TRY(hy_launch(e, hy_gdelta_prep_kernel, dim3(T, (H + 7) / 8), dim3(256), 0, st, P, l.off_r, l.off_k, l.off_v, l.off_a, Wd, (const float*)l.w0,
+      if (T > 64 && n % 4 == 0 && n <= 128 && (n & (n - 1)) == 0 && hy_quad(P, l.off_r) && hy_quad(P, l.off_k) && hy_quad(P, l.off_v) && hy_quad(P, l.off_a) &&
+          hy_quad(Wd, 0) && hy_quad_ptr(l.w0))
+        XB_TRY(hy_launch(e, hy_gdelta_prep_quad_kernel, dim3((unsigned)(((long long)T * HN / 4 + 255) / 256)), dim3(256), 0, st, P, l.off_r, l.off_k, l.off_v,
+                         l.off_a, Wd, (const float*)l.w0, hy->c, 6LL * HN, hy->beta, hy->decay, H, n, T));
+      else
+        XB_TRY(hy_launch(e, hy_gdelta_prep_kernel, dim3(T, (H + 7) / 8), dim3(256), 0, st, P, l.off_r, l.off_k, l.off_v, l.off_a, Wd, (const float*)l.w0,
                        hy->c, (long long)6 * HN, hy->beta, hy->decay, H, n));
       RecurIn in;
       in.c = hy->c; in.ldc = 6LL * HN; in.qoff = 0; in.koff = HN; in.xoff[0] = 2LL * HN; in.xoff[1] = 3LL * HN; in.xoff[2] = 4LL * HN;
       in.voff = 5LL * HN; in.q_heads = H; in.beta = hy->beta; in.decay = hy->decay; in.qk = nullptr; in.hdecay = nullptr;
       XB_TRY(hy_recur<HY_REC_GDELTA>(e, in, hy->state + l.st_rec, SS, hy->o, (long long)l.n_o, m, n_seqs, H, n, n, T, st));
-      XB_TRY(hy_launch(e, hy_head_norm_kernel<AT>, dim3(T, (H + 7) / 8), dim3(256), 0, st, (const float*)hy->o, (long long)l.n_o,
-                       (const float*)l.head_norm, P, l.off_g, d.norm_eps, 1.0f, a1, (long long)l.n_o, H, n, n, 1));
+      XB_TRY(hy_head_norm<AT>(e, T, (long long)l.n_o, (const float*)l.head_norm, P, l.off_g, a1, (long long)l.n_o, H, n, n, 1, st));
     } else {
       const int dv = c.m_vdim;
       const int nc = 2 * H * n + H * dv;
-      XB_TRY(hy_launch(e, hy_act_cols_kernel<float>, dim3(T, (nc + 255) / 256), dim3(256), 0, st, P, l.off_q, nc, 0, hy->c, (long long)nc));
+      if (T > 64 && nc % 4 == 0 && hy_quad(P, l.off_q))
+        XB_TRY(hy_launch(e, hy_act_cols_quad_kernel<float>, dim3(T, (nc / 4 + 255) / 256), dim3(256), 0, st, P, l.off_q, nc, 0, hy->c, (long long)nc));
+      else
+        XB_TRY(hy_launch(e, hy_act_cols_kernel<float>, dim3(T, (nc + 255) / 256), dim3(256), 0, st, P, l.off_q, nc, 0, hy->c, (long long)nc));
       RecurIn in;
       in.c = hy->c; in.ldc = nc; in.qoff = 0; in.koff = (long long)H * n; in.voff = 2LL * H * n; in.q_heads = H;
       in.xoff[0] = in.xoff[1] = in.xoff[2] = 0;
@@ -2046,10 +2071,10 @@ template <typename AT>
 static int hy_head_norm(xb_engine* e, int T, long long ldo, const float* w, const LinOut& P, int off_gate, AT* out, long long ld_out, int H, int dv,
                         int w_hstride, int gate_sigmoid, cudaStream_t st) {
   const int per = dv / 8;
-  if (T > 64 && off_gate >= 0 && P.h != nullptr && P.bias == nullptr && P.ld % 8 == 0 && off_gate % 8 == 0 && dv % 8 == 0 && per <= 32 && (per & (per - 1)) == 0 &&
+  if (T > 64 && off_gate >= 0 && P.h != nullptr && hy_quad_ptr(P.bias) && P.ld % 8 == 0 && off_gate % 8 == 0 && dv % 8 == 0 && per <= 32 && (per & (per - 1)) == 0 &&
       ldo % 8 == 0 && ld_out % 8 == 0)
     return hy_launch(e, hy_head_norm_vec_kernel<AT>, dim3((unsigned)(((long long)T * H * per + 255) / 256)), dim3(256), 0, st, (const float*)e->hy->o, ldo, w,
-                     P.h + off_gate, P.ld, e->hy->d.norm_eps, out, ld_out, H, dv, w_hstride, gate_sigmoid, T);
+                     P.h + off_gate, P.ld, P.bias != nullptr ? P.bias + off_gate : nullptr, e->hy->d.norm_eps, out, ld_out, H, dv, w_hstride, gate_sigmoid, T);
   return hy_launch(e, hy_head_norm_kernel<AT>, dim3(T, (H + 7) / 8), dim3(256), 0, st, (const float*)e->hy->o, ldo, w, P, off_gate, e->hy->d.norm_eps, 1.0f,
                    out, ld_out, H, dv, w_hstride, gate_sigmoid);
 }
@@ -2287,8 +2312,7 @@ static int hy_run_body_t(xb_engine* e, int T, int n_seqs, int n_tiles, void* con
         in.xoff[0] = in.xoff[1] = in.xoff[2] = 0;
         XB_TRY(hy_recur<HY_REC_DELTA>(e, in, hy->state + l.st_rec, SS, hy->o, (long long)l.n_o, m, n_seqs, H, dk, dv, T, st));
       }
-      XB_TRY(hy_launch(e, hy_head_norm_kernel<AT>, dim3(T, (H + 7) / 8), dim3(256), 0, st, (const float*)hy->o, (long long)l.n_o,
-                       (const float*)l.head_norm, P, l.off_g, d.norm_eps, 1.0f, a1, (long long)l.n_o, H, dv, 0, 0));
+      XB_TRY(hy_head_norm<AT>(e, T, (long long)l.n_o, (const float*)l.head_norm, P, l.off_g, a1, (long long)l.n_o, H, dv, 0, 0, st));
       XB_TRY(hy_linear<AT>(e, a1, l.n_o, l.w_o, l.t_o, nullptr, T, D, l.n_o, hy->m1, hy->cap_m, st, &y1));
     } else if (c.mixer == XB_MIX_SOFTMAX) {
       XB_TRY(hy_softmax_mixer<AT>(e, l, T, n_seqs, n_tiles, P, m, st));
@@ -2328,8 +2352,12 @@ static int hy_run_body_t(xb_engine* e, int T, int n_seqs, int n_tiles, void* con
                          (long long)l.n_o, AttnOpt{nullptr, 0.f, G, 0}));
       }
       const long long ldc = 2LL * Hr * rk + (long long)Hr * rv;
-      XB_TRY(hy_launch(e, hy_hgrn_prep_kernel, dim3(T, (2 * Hr * rk + Hr * rv + 255) / 256), dim3(256), 0, st, P, l.off_rq, l.off_rf, l.off_rv, (const float*)l.lower, hy->c,
-                       ldc, Hr * rk, Hr * rv));
+      if (T > 64 && (Hr * rk) % 4 == 0 && (Hr * rv) % 4 == 0 && hy_quad(P, l.off_rq) && hy_quad(P, l.off_rf) && hy_quad(P, l.off_rv))
+        XB_TRY(hy_launch(e, hy_hgrn_prep_quad_kernel, dim3(T, ((2 * Hr * rk + Hr * rv) / 4 + 255) / 256), dim3(256), 0, st, P, l.off_rq, l.off_rf, l.off_rv,
+                         (const float*)l.lower, hy->c, ldc, Hr * rk, Hr * rv));
+      else
+        XB_TRY(hy_launch(e, hy_hgrn_prep_kernel, dim3(T, (2 * Hr * rk + Hr * rv + 255) / 256), dim3(256), 0, st, P, l.off_rq, l.off_rf, l.off_rv, (const float*)l.lower, hy->c,
+                         ldc, Hr * rk, Hr * rv));
       {
         RecurIn in;
         in.c = hy->c; in.ldc = ldc; in.qoff = 0; in.koff = (long long)Hr * rk; in.voff = 2LL * Hr * rk; in.q_heads = Hr;

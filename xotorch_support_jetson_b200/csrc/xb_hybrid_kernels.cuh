@@ -1533,10 +1533,10 @@ __global__ void __launch_bounds__(256) hy_head_norm_kernel(const float* __restri
 }
 
 // The same for prompts whose gate is part of one bf16 matrix: eight neighbouring channels per thread, dv / 8 (a power of two up to 32)
-// neighbouring lanes per head.  off_gate, the pitches and dv are multiples of 8; no bias.  grid ceil(T * H * dv / 8 / 256), 256 threads.
+// neighbouring lanes per head.  off_gate, the pitches and dv are multiples of 8; gb: the gate's bias or nullptr.  grid ceil(T * H * dv / 8 / 256), 256 threads.
 template <typename AT>
 __global__ void __launch_bounds__(256) hy_head_norm_vec_kernel(const float* __restrict__ o, long long ldo, const float* __restrict__ w, const bf16* __restrict__ g,
-                                                               long long ldg, float eps, AT* __restrict__ out, long long ld_out, int H, int dv,
+                                                               long long ldg, const float* __restrict__ gb, float eps, AT* __restrict__ out, long long ld_out, int H, int dv,
                                                                int w_hstride, int gate_sigmoid, int T) {
   pdl_launch_dependents();
   pdl_wait();
@@ -1549,7 +1549,7 @@ __global__ void __launch_bounds__(256) hy_head_norm_vec_kernel(const float* __re
   const int h = (int)(th - t * H);
   float v[8], wv[8], gv[8];
   hy_ld8f(o + t * ldo + (long long)h * dv + j, v);
-  hy_load8(g + t * ldg + (long long)h * dv + j, nullptr, gv);
+  hy_load8(g + t * ldg + (long long)h * dv + j, gb != nullptr ? gb + (long long)h * dv + j : nullptr, gv);
   hy_ld8f(w + (long long)h * w_hstride + j, wv);
   float ss = 0.f;
 #pragma unroll

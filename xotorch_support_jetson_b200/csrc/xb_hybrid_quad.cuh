@@ -1,0 +1,288 @@
+// Row-wise kernels of hybrid prompts, four neighbouring channels per thread.
+//
+// The one-channel forms (hy_taps_tile_kernel, hy_hgrn_prep_kernel, hy_act_cols_kernel, hy_row_op_kernel, hy_gdelta_prep_kernel) issue 2- and
+// 4-byte accesses and were bound by instructions and by loads in flight, at 0.15 to 0.35 of the copy rate.  These take
+// 8- and 16-byte accesses where the operand is one bf16 or fp32 matrix (prompts; split-K planes of few rows keep the others), rows,
+// columns and pitches are multiples of four and pointers are aligned (hy_quad).  Per channel the arithmetic is the same;
+// sums over a row are taken in another order.
+// us a launch, before -> now, 2048 rows: filter of 2048 channels fp32 -> bf16 27.9 -> 15.8, q|k|v filter of 6144 channels 59 -> 38, HGRN2
+// preparation 53.5 -> 17.4, residual + norm of the stream 24.3 -> 17.4; 1800 rows: parallel block's residual + norm 27.1 -> 14.6, SiLU of
+// 6144 columns 46.8 -> 15.6, general delta rule's preparation 55.6 -> 28.3.
+#pragma once
+
+__device__ __forceinline__ void hy_quad_bf(const bf16* p, float* v) {
+  const uint2 u = *reinterpret_cast<const uint2*>(p);
+  const float2 a = bf2_to_f2(u.x), b = bf2_to_f2(u.y);
+  v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
+}
+__device__ __forceinline__ void hy_quad_f(const float* p, float* v) {
+  const float4 a = *reinterpret_cast<const float4*>(p);
+  v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+}
+// one matrix (no planes), see hy_quad
+__device__ __forceinline__ void lin_quad(const LinOut& o, long long row, int col, float* v) {
+  if (o.h != nullptr) hy_quad_bf(o.h + row * o.ld + col, v);
+  else hy_quad_f(o.f + row * o.ld + col, v);
+  if (o.bias != nullptr) {
+    float b[4];
+    hy_quad_f(o.bias + col, b);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) v[j] += b[j];
+  }
+}
+__device__ __forceinline__ void hy_quad_st(float* p, const float* v) { *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]); }
+__device__ __forceinline__ void hy_quad_st(bf16* p, const float* v) {
+  *reinterpret_cast<uint2*>(p) = make_uint2(f2_to_bf2(v[0], v[1]), f2_to_bf2(v[2], v[3]));
+}
+// can `o` be read four columns at a time from column `col` (a multiple of four) on?
+static bool hy_quad(const LinOut& o, int col) {
+  if (o.ld % 4 != 0 || col % 4 != 0 || (o.bias != nullptr && (reinterpret_cast<uintptr_t>(o.bias) & 15) != 0)) return false;
+  if (o.h != nullptr) return (reinterpret_cast<uintptr_t>(o.h) & 7) == 0;
+  return o.f != nullptr && o.si.splits == 0 && (reinterpret_cast<uintptr_t>(o.f) & 15) == 0;
+}
+static bool hy_quad_ptr(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+
+// hy_taps_tile_kernel with TT = 8 rows and four channels per thread; C, ld_out and tail_stride multiples of four
+template <typename OT, int TAPS>
+__global__ void __launch_bounds__(256) hy_taps_quad_kernel(LinOut in, int col0, int C, const float* __restrict__ w, const float* __restrict__ tail,
+                                                           long long tail_stride, BatchMeta m, int identity, int act_silu, OT* __restrict__ out,
+                                                           long long ld_out, int T) {
+  constexpr int TT = 8;
+  pdl_launch_dependents();
+  pdl_wait();
+  const int c = (blockIdx.y * blockDim.x + threadIdx.x) * 4;
+  if (c >= C) return;
+  const int r0 = blockIdx.x * TT;
+  const int last_row = (r0 + TT < T ? r0 + TT : T) - 1;
+  const bool uniform = m.tok_seq[r0] == m.tok_seq[last_row];
+  const int s_first = m.tok_seq[r0];
+  float wv[TAPS][4];
+#pragma unroll
+  for (int e = 0; e < 4; ++e)
+#pragma unroll
+    for (int j = 0; j < TAPS; ++j) wv[j][e] = w[(long long)(c + e) * TAPS + j];
+  float win[TAPS][4];   // win[d - 1]: the input d steps back (TAPS - 1 used)
+#pragma unroll
+  for (int d = 0; d < TAPS; ++d)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) win[d][e] = 0.f;
+  float cur[TT][4];
+#pragma unroll
+  for (int i = 0; i < TT; ++i) lin_quad(in, r0 + i <= last_row ? r0 + i : last_row, col0 + c, cur[i]);
+#pragma unroll
+  for (int i = 0; i < TT; ++i) {
+    const int row = r0 + i;
+    if (row > last_row) break;
+    const int s = uniform ? s_first : m.tok_seq[row];
+    const bool begins = !uniform && i > 0 && m.tok_seq[row - 1] != s;
+    if (i == 0 || begins) {
+      const float* tl = tail + (long long)m.seq_slot[s] * tail_stride;
+      const int start = begins ? row : (s > 0 ? m.seq_last[s - 1] + 1 : 0);
+      const int pos = m.tok_pos[row], pos0 = m.tok_pos[start];
+#pragma unroll
+      for (int d = 1; d < TAPS; ++d) {
+        const int p = pos - d;
+        float v[4] = {0.f, 0.f, 0.f, 0.f};
+        if (p >= 0) {
+          if (row - d >= start) lin_quad(in, row - d, col0 + c, v);
+          else hy_quad_f(tl + (long long)(p - (pos0 - (TAPS - 1))) * C + c, v);
+        }
+#pragma unroll
+        for (int e = 0; e < 4; ++e) win[d - 1][e] = v[e];
+      }
+    }
+    float acc[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      acc[e] = identity ? cur[i][e] : 0.f;
+#pragma unroll
+      for (int j = 0; j < TAPS - 1; ++j) acc[e] += wv[j][e] * win[TAPS - 2 - j][e];   // oldest first
+      acc[e] += wv[TAPS - 1][e] * cur[i][e];
+      if (act_silu) acc[e] = hy_silu(acc[e]);
+#pragma unroll
+      for (int d = TAPS - 1; d >= 2; --d) win[d - 1][e] = win[d - 2][e];
+      win[0][e] = cur[i][e];
+    }
+    hy_quad_st(out + (long long)row * ld_out + c, acc);
+  }
+}
+
+// hy_hgrn_prep_kernel; HK and HV multiples of four
+__global__ void __launch_bounds__(256) hy_hgrn_prep_quad_kernel(LinOut P, int off_q, int off_f, int off_v, const float* __restrict__ lower,
+                                                                float* __restrict__ c, long long ldc, int HK, int HV) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const long long t = blockIdx.x;
+  const int i = (blockIdx.y * 256 + threadIdx.x) * 4;
+  if (i >= 2 * HK + HV) return;
+  float v[4];
+  if (i < HK) {
+    lin_quad(P, t, off_q + i, v);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) v[e] = hy_silu(v[e]);
+  } else if (i < 2 * HK) {
+    lin_quad(P, t, off_f + i - HK, v);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float lo = lower[i - HK + e];
+      v[e] = lo + (1.0f - lo) * hy_sigmoid(v[e]);
+    }
+  } else {
+    lin_quad(P, t, off_v + i - 2 * HK, v);
+  }
+  hy_quad_st(c + t * ldc + i, v);
+}
+
+// hy_act_cols_kernel; n a multiple of four
+template <typename OT>
+__global__ void __launch_bounds__(256) hy_act_cols_quad_kernel(LinOut P, int off, int n, int act, OT* __restrict__ out, long long ld_out) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const long long t = blockIdx.x;
+  const int i = (blockIdx.y * 256 + threadIdx.x) * 4;
+  if (i >= n) return;
+  float v[4];
+  lin_quad(P, t, off + i, v);
+#pragma unroll
+  for (int e = 0; e < 4; ++e) v[e] = act == 0 ? hy_silu(v[e]) : tanhf(v[e]);
+  hy_quad_st(out + t * ld_out + i, v);
+}
+
+// hy_row_op_kernel (every form of it); D a multiple of four
+template <typename AT>
+__global__ void __launch_bounds__(256) hy_row_op_quad_kernel(RowOpArgs a) {
+  constexpr int NT = 256;
+  pdl_launch_dependents();
+  pdl_wait();
+  extern __shared__ __align__(16) float row[];
+  __shared__ float red[32];
+  const long long t = blockIdx.x;
+  const int D = a.D;
+  float* x = a.x + t * D;
+  const bool branch = a.m1.f != nullptr || a.m1.h != nullptr;
+  const bool two = a.m2.f != nullptr || a.m2.h != nullptr;
+  const bool three = a.plain_add && (a.m3.f != nullptr || a.m3.h != nullptr);
+  float s2 = 0.f;
+  float inv = 0.f;
+  if (branch && !a.plain_add) {   // the branch's own norm
+    float ss = 0.f;
+    for (int i = threadIdx.x * 4; i < D; i += NT * 4) {
+      float v[4], b[4];
+      lin_quad(a.m1, t, i, v);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) v[e] *= a.s1;
+      if (two) {
+        lin_quad(a.m2, t, i, b);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) v[e] += a.s2 * b[e];
+      }
+#pragma unroll
+      for (int e = 0; e < 4; ++e) ss += v[e] * v[e];
+      hy_quad_st(row + i, v);
+    }
+    ss = block_sum<NT>(ss, red);
+    inv = 1.0f / sqrtf(ss / (float)D + a.eps);
+  }
+  for (int i = threadIdx.x * 4; i < D; i += NT * 4) {
+    float v[4], b[4];
+    hy_quad_f(x + i, v);
+    if (branch && a.plain_add) {
+      float y[4];
+      lin_quad(a.m1, t, i, y);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) y[e] *= a.s1;
+      if (two) {
+        lin_quad(a.m2, t, i, b);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) y[e] += a.s2 * b[e];
+      }
+      if (three) {
+        lin_quad(a.m3, t, i, b);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) y[e] += b[e];
+      }
+#pragma unroll
+      for (int e = 0; e < 4; ++e) v[e] += y[e];
+    } else if (branch) {
+      float w[4];
+      hy_quad_f(row + i, b);   // this thread wrote them
+      hy_quad_f(a.bw + i, w);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) v[e] += b[e] * inv * (w[e] + a.bw_one);
+    }
+    if (branch) hy_quad_st(x + i, v);
+    hy_quad_st(row + i, v);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) s2 += v[e] * v[e];
+  }
+  if (a.nw != nullptr) {
+    s2 = block_sum<NT>(s2, red);
+    const float inv2 = 1.0f / sqrtf(s2 / (float)D + a.eps);
+    for (int i = threadIdx.x * 4; i < D; i += NT * 4) {
+      float v[4];
+      hy_quad_f(row + i, v);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) v[e] = v[e] * inv2 * hy_norm_weight(a.nw, a.nw_mode, i + e);
+      hy_quad_st(a.hn + t * D + i, v);
+      if (a.ha != nullptr) hy_quad_st(reinterpret_cast<AT*>(a.ha) + t * D + i, v);
+    }
+  }
+  if (a.xa != nullptr) {
+    AT* xa = reinterpret_cast<AT*>(a.xa) + t * D;
+    for (int i = threadIdx.x * 4; i < D; i += NT * 4) {
+      float v[4];
+      hy_quad_f(row + i, v);
+      hy_quad_st(xa + i, v);
+    }
+  }
+}
+
+// hy_gdelta_prep_kernel; n / 4 lanes per head (a power of two up to 32), grid ceil(T * H * n / 4 / 256)
+__global__ void __launch_bounds__(256) hy_gdelta_prep_quad_kernel(LinOut P, int off_r, int off_k, int off_v, int off_a, LinOut Wd,
+                                                                  const float* __restrict__ w0, float* __restrict__ c, long long ldc,
+                                                                  float* __restrict__ ra, float* __restrict__ rk, int H, int n, int T) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int per = n >> 2;
+  const long long idx = (long long)blockIdx.x * 256 + threadIdx.x, all = (long long)T * H * per;
+  const bool live = idx < all;
+  const long long th = (live ? idx : all - 1) / per;
+  const int i = (int)((live ? idx : all - 1) - th * per) * 4;
+  const long long t = th / H, HN = (long long)H * n;
+  const int h = (int)(th - t * H), b = h * n + i;
+  float r[4], k[4], v[4], z[4], aa[4], w[4];
+  lin_quad(P, t, off_r + b, r);
+  lin_quad(P, t, off_k + b, k);
+  lin_quad(P, t, off_v + b, v);
+  lin_quad(P, t, off_a + b, aa);
+  lin_quad(Wd, t, b, w);
+  hy_quad_f(w0 + b, z);
+  float sk = 0.f;
+#pragma unroll
+  for (int e = 0; e < 4; ++e) sk = fmaf(k[e], k[e], sk);
+  for (int off = per >> 1; off > 0; off >>= 1) sk += __shfl_xor_sync(0xffffffffu, sk, off);
+  const float ik = 1.0f / sqrtf(sk + 1e-6f);
+  float s_ra = 0.f, s_rk = 0.f, rw[4], u[4], au[4];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    w[e] = expf(-0.6065306597126334f * hy_sigmoid(w[e] + z[e]));
+    u[e] = k[e] * ik;
+    au[e] = hy_sigmoid(aa[e]) * u[e];
+    rw[e] = r[e] * w[e];
+    s_ra = fmaf(r[e], au[e], s_ra);
+    s_rk = fmaf(r[e], k[e], s_rk);
+  }
+  for (int off = per >> 1; off > 0; off >>= 1) {
+    s_ra += __shfl_xor_sync(0xffffffffu, s_ra, off);
+    s_rk += __shfl_xor_sync(0xffffffffu, s_rk, off);
+  }
+  if (!live) return;
+  float* row = c + t * ldc + b;
+  hy_quad_st(row, rw);
+  hy_quad_st(row + HN, u);
+  hy_quad_st(row + 2 * HN, w);
+  hy_quad_st(row + 3 * HN, au);
+  hy_quad_st(row + 4 * HN, k);
+  hy_quad_st(row + 5 * HN, v);
+  if (i == 0) { ra[t * H + h] = s_ra; rk[t * H + h] = s_rk; }
+}

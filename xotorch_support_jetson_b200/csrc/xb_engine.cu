@@ -117,6 +117,7 @@ struct xb_engine {
   unsigned long long* ts_buf = nullptr;
   int ts_cap = 0, ts_next = 0, ts_blocks = 160;
   int meta_T = 0;         // token rows the device metadata currently describes
+  int step_ctx = 0;       // prompts: longest context of the step, its own rows included; steps of single tokens (captured once for every length): no bound
   std::map<long long, GemmPlan> plans;
   xb_counters c{};
   std::map<long long, int> loaded;   // (layer + 1) * 64 + kind -> seen by xb_load_weight / xb_load_safetensors
@@ -1188,6 +1189,7 @@ static int forward_impl(xb_engine* e, const xb_batch* b, void* out, void* const*
     XB_CUDA(cudaMemcpyAsync(e->d_meta, hm, e->meta_ints * 4, cudaMemcpyHostToDevice, st));
   }
   e->meta_T = T;
+  e->step_ctx = decode_only ? 1 << 30 : max_ctx;
   XB_CUDA(cudaEventRecord(e->meta_ev[ring], st));
 
   // ---- inputs to fixed addresses

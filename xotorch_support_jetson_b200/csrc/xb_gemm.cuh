@@ -16,8 +16,7 @@
 //   MODE_SKINNY  (decode, T <= 128): A = W tile (128 output features), B = x (all T tokens).
 //       HBM-bound weight streaming; K is split across CTAs so every SM pulls weights;
 //       output = fp32 partial sums  out[split][t][n]  reduced by the consumer kernel.
-//   MODE_WIDE    (prefill): A = x tile (128 tokens), B = W tile (BN features);
-//       tensor-bound; output = bf16  out[t][n] (+ bias, rounded once like nn.Linear).
+//   MODE_WIDE    (more than 128 rows): the kernels of xb_wide.cuh, bf16 out[t][n] (+ bias, rounded once like nn.Linear).
 //
 // The engine stores weights TILE-MAJOR in HBM ([N/128][K/64][128][64] bf16): every TMA box is
 // one contiguous 16 KB read instead of 128 rows x 128 B at a K*2-byte pitch.

@@ -193,7 +193,7 @@ xb_gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
 
   // Roles are entered by elect.sync and weights and activations have a producer thread each: under `lane == 0` one thread
   // needed 0.35 us to issue a k-block, as long as HBM takes to deliver its 16 KB to every SM, so no gap was ever made up.
-  // llama-3.2-1b, one sequence: 929 -> 795 us a step; four 8B layers: one sequence 450 -> 390, 32 sequences 835 -> 786.
+  // llama-3.2-1b, one sequence: 845 -> 770 us a step; four 8B layers: one sequence 397 -> 372, 32 sequences 764 -> 746.
   if (warp == 0) {
     // ===================== TMA producer of the weights =====================
     // They never depend on the preceding kernel: their boxes go out at once, as far as the ring reaches.

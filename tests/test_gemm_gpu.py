@@ -47,11 +47,11 @@ def test_wide_linear_matches_fp32(built_lib, T, N, K):
   assert (y != ref_b).float().mean().item() < 0.02
 
 
-@pytest.mark.parametrize("variant", range(1, 9))
+@pytest.mark.parametrize("variant", range(1, 5))
 @pytest.mark.parametrize("T,N,K", [(129, 512, 1024), (257, 1000, 328), (130, 200, 2048), (700, 640, 1088)])
 def test_wide_linear_variants_match_fp64(built_lib, variant, T, N, K):
-  """Every tile shape of the prompt Linear (pairs of CTAs, K in two or four parts, tiles of 128 to 256 columns) at one row past
-  a tile, at features that end inside a tile and inside a 16-column chunk, and at odd numbers of k-blocks."""
+  """Every tile shape of the prompt Linear (pairs of CTAs, tiles of 128 to 256 columns) at one row past a tile, at features that end
+  inside a tile and inside a 16-column chunk, and at odd numbers of k-blocks."""
   from xotorch_support_jetson_b200.stage import debug_linear
   g = torch.Generator(device="cuda").manual_seed(T + N + K)
   x = (torch.randn(T, K, device="cuda", generator=g) * 0.5).to(torch.bfloat16)
@@ -62,4 +62,4 @@ def test_wide_linear_variants_match_fp64(built_lib, variant, T, N, K):
   # one bf16 rounding of a sum that is off by at most K fp32 roundings of its largest partial sum
   bound = ref.abs() * 2 ** -8 + K * 2 ** -24 * (x.double().abs() @ w.double().abs().t())
   assert ((y.double() - ref).abs() <= bound).all()
-  assert torch.equal(y, debug_linear(x, w, use_tensor_cores=True, force_splits=variant))
+  assert torch.equal(y, debug_linear(x, w, use_tensor_cores=True, force_splits=2))   # all sum in one order

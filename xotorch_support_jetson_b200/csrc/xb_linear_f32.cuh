@@ -12,7 +12,7 @@
 // refatar-1b layers, 73 GFLOP: 7.06 ms with plain FMA on 64 x 64 tiles, 1.55 ms now (all kernels); one row 774 -> 506 us, so
 // few rows take it too.
 // S > 1: S CTAs of a cluster share a tile, each a part of K, and add their totals in rank order through distributed shared
-// memory, as in xb_wide.cuh.
+// memory.
 #pragma once
 #include "xb_wide.cuh"
 

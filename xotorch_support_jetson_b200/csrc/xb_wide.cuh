@@ -6,12 +6,14 @@
 // drain TMEM, persistent over tiles with two accumulators.  What varies is how the tiles cover the chip:
 //   CG = 2  a pair of CTAs works on one 256 x BN tile (cta_group::2): each stages its own 128 token rows and HALF of the
 //           weight rows, 32 KB instead of 48 KB a k-block at BN = 256.
-//   S > 1   S CTAs of a cluster share one tile, each a part of K; the fp32 partial tiles meet through distributed shared
-//           memory, every CTA reduces its share of the columns in rank order (same bits every time) and stores it.
+//   BN      128, 192 or 256 features a tile, by what fills the SMs evenly.
+// Every variant sums K in the same order, k-block by k-block into one accumulator, so a row's numbers depend neither on the tile
+// it falls into nor on what else the step carries: a prompt in portions has the bits of the whole.  (K in two or four parts over a
+// cluster was faster below 512 rows and gave that up.)
 #pragma once
 #include "xb_gemm.cuh"
 
-template <int BN, int CG, int S>
+template <int BN, int CG>
 struct WideCfg {
   static constexpr int BROWS = BN / CG;                       // weight rows this CTA stages
   static constexpr int BOX = BROWS % 128 == 0 ? 128 : 64;     // rows of one TMA box (divides 128: a box stays in its weight tile)
@@ -20,14 +22,14 @@ struct WideCfg {
   static constexpr int KS = BN <= 128 ? 2 : 1;                // k-blocks of one stage: narrow tiles halve the barrier round trips a k-block
   static constexpr int STAGES_RAW = (216 * 1024) / (KS * (A_BYTES + B_BYTES));
   static constexpr int STAGES = STAGES_RAW > 8 ? 8 : STAGES_RAW;
-  static constexpr int ACC_STAGES = S > 1 ? 1 : 2;
+  static constexpr int ACC_STAGES = 2;
   static constexpr int TM_RAW = ACC_STAGES * BN;
   static constexpr int TM_COLS = TM_RAW <= 128 ? 128 : TM_RAW <= 256 ? 256 : 512;
   static constexpr int ACC_COLS = TM_COLS / ACC_STAGES;
   static constexpr int PAIRS = BN / 32;                       // column pairs (two chunks of 16) of a tile
   static constexpr int RING_BYTES = STAGES * KS * (A_BYTES + B_BYTES);
   static constexpr int SMEM_BYTES = RING_BYTES + 1024 + 256;
-  static_assert(BROWS % BOX == 0 && PAIRS % S == 0 && (S - 1) * (BN / S) * 128 * 4 <= RING_BYTES, "tile");
+  static_assert(BROWS % BOX == 0, "tile");
 };
 
 __device__ __forceinline__ uint32_t cluster_rank() {
@@ -191,10 +193,10 @@ __device__ __forceinline__ void wide_emit(const GemmArgs& g, int t, int pos, int
 // Roles are entered by elect.sync, not by lane == 0, and the two operands have a producer thread each: one thread doing
 // everything under `lane == 0` spent 0.35 us a k-block whatever the tile (a 128 x 64 tile took as long as 128 x 256), most of
 // it issuing.  4096^3, CUDA events: 256x256 pair 103 -> 94 us, 128x256 107 -> 103, 128x128 166 -> 116, 128x64 306 -> 202.
-template <int BN, int CG, int S>
+template <int BN, int CG>
 __global__ void __launch_bounds__(224, 1)
 xb_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, GemmArgs g) {
-  using Cfg = WideCfg<BN, CG, S>;
+  using Cfg = WideCfg<BN, CG>;
   constexpr int STAGES = Cfg::STAGES, KS = Cfg::KS;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -208,12 +210,10 @@ xb_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const uint32_t rank = CG * S > 1 ? cluster_rank() : 0;
+  const uint32_t rank = CG > 1 ? cluster_rank() : 0;
   const int a_units = (g.a_tiles + CG - 1) / CG;
   const int n_units = a_units * g.b_tiles;
-  const int u0 = blockIdx.x / (CG * S), u_step = S > 1 ? n_units : gridDim.x / CG;
-  const int kb0 = S > 1 ? (int)(((long long)rank * g.k_blocks) / S) : 0;
-  const int kb1 = S > 1 ? (int)(((long long)(rank + 1) * g.k_blocks) / S) : g.k_blocks;
+  const int u0 = blockIdx.x / CG, u_step = gridDim.x / CG;
 
   if (warp == 0 && lane == 0) {
     tma_prefetch_desc(&tmA);
@@ -236,7 +236,7 @@ xb_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   }
   tc_fence_before();
   __syncthreads();
-  if (CG * S > 1) cluster_sync_aligned();   // barriers of the peers are ready too
+  if (CG > 1) cluster_sync_aligned();   // barriers of the peer are ready too
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   pdl_launch_dependents();
@@ -258,8 +258,8 @@ xb_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       if (warp == 6) pdl_wait();   // weights never depend on the preceding kernel: their boxes go out at once
       for (int u = u0; u < n_units; u += u_step) {
         const int ta = (u % a_units) * CG + (CG == 2 ? (int)rank : 0), tb = u / a_units;
-        for (int kb = kb0; kb < kb1; kb += KS) {
-          const int nk = KS == 1 || kb + 1 == kb1 ? 1 : KS;
+        for (int kb = 0; kb < g.k_blocks; kb += KS) {
+          const int nk = KS == 1 || kb + 1 == g.k_blocks ? 1 : KS;
           mbar_wait(&empty_bar[stage], phase ^ 1);
           if (warp == 6) {
             expect(nk * Cfg::A_BYTES);
@@ -296,17 +296,17 @@ xb_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         mbar_wait(&tempty_bar[acc], acc_phase ^ 1);   // epilogue has drained this accumulator
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + (uint32_t)(acc * Cfg::ACC_COLS);
-        for (int kb = kb0; kb < kb1; kb += KS) {
+        for (int kb = 0; kb < g.k_blocks; kb += KS) {
           mbar_wait(&full_bar[stage], phase);
           tc_fence_after();
 #pragma unroll
           for (int q = 0; q < KS; ++q) {
-            if (q > 0 && kb + q >= kb1) break;
+            if (q > 0 && kb + q >= g.k_blocks) break;
             const uint64_t da = desc_a0 + (uint64_t)((stage * KS + q) * (Cfg::A_BYTES >> 4));
             const uint64_t db = desc_b0 + (uint64_t)((stage * KS + q) * (Cfg::B_BYTES >> 4));
 #pragma unroll
             for (int k = 0; k < 4; ++k)               // 4 x (K = 16) per 64-wide k-block
-              wide_mma<CG>(d_tmem, da + k * 2, db + k * 2, idesc, (kb > kb0 || q > 0 || k > 0) ? 1u : 0u);
+              wide_mma<CG>(d_tmem, da + k * 2, db + k * 2, idesc, (kb > 0 || q > 0 || k > 0) ? 1u : 0u);
           }
           wide_commit<CG>(&empty_bar[stage]);
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
@@ -321,99 +321,35 @@ xb_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     const int row_in_tile = quad * 32 + lane;
     const uint32_t lane_base = tmem_base + ((uint32_t)(quad * 32) << 16);
     pdl_wait();                                       // `out` may still be read by the upstream grid
-    if (S == 1) {
-      int acc = 0;
-      uint32_t acc_phase = 0;
-      for (int u = u0; u < n_units; u += u_step) {
-        const int ta = (u % a_units) * CG + (CG == 2 ? (int)rank : 0), tb = u / a_units;
-        const int t = ta * 128 + row_in_tile;
-        const int pos = g.epi == XB_EPI_QKV && t < g.a_rows ? g.tok_pos[t] : 0;
-        mbar_wait(&tfull_bar[acc], acc_phase);
-        tc_fence_after();
-        const uint32_t t_addr = lane_base + (uint32_t)(acc * Cfg::ACC_COLS);
-#pragma unroll 1
-        for (int p = 0; p < Cfg::PAIRS; ++p) {
-          int c0, c1;
-          wide_pair_cols(g, p, c0, c1);
-          uint32_t v0[16], v1[16];
-          tmem_ld16(t_addr + c0, v0);
-          tmem_ld16(t_addr + c1, v1);
-          tmem_ld_wait();
-          wide_emit(g, t, pos, tb * BN + c0, tb * BN + c1, reinterpret_cast<float*>(v0), reinterpret_cast<float*>(v1));
-        }
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) {
-          if (CG == 1) mbar_arrive(&tempty_bar[acc]);
-          else mbar_arrive_cluster(cluster_map(smem_u32(&tempty_bar[acc]), 0));
-        }
-        if (++acc == Cfg::ACC_STAGES) { acc = 0; acc_phase ^= 1; }
-      }
-    } else {
-      mbar_wait(&tfull_bar[0], 0);                    // all MMAs of this CTA have retired: its ring is free for the exchange
+    int acc = 0;
+    uint32_t acc_phase = 0;
+    for (int u = u0; u < n_units; u += u_step) {
+      const int ta = (u % a_units) * CG + (CG == 2 ? (int)rank : 0), tb = u / a_units;
+      const int t = ta * 128 + row_in_tile;
+      const int pos = g.epi == XB_EPI_QKV && t < g.a_rows ? g.tok_pos[t] : 0;
+      mbar_wait(&tfull_bar[acc], acc_phase);
       tc_fence_after();
+      const uint32_t t_addr = lane_base + (uint32_t)(acc * Cfg::ACC_COLS);
+#pragma unroll 1
+      for (int p = 0; p < Cfg::PAIRS; ++p) {
+        int c0, c1;
+        wide_pair_cols(g, p, c0, c1);
+        uint32_t v0[16], v1[16];
+        tmem_ld16(t_addr + c0, v0);
+        tmem_ld16(t_addr + c1, v1);
+        tmem_ld_wait();
+        wide_emit(g, t, pos, tb * BN + c0, tb * BN + c1, reinterpret_cast<float*>(v0), reinterpret_cast<float*>(v1));
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) {
+        if (CG == 1) mbar_arrive(&tempty_bar[acc]);
+        else mbar_arrive_cluster(cluster_map(smem_u32(&tempty_bar[acc]), 0));
+      }
+      if (++acc == Cfg::ACC_STAGES) { acc = 0; acc_phase ^= 1; }
     }
   }
   __syncwarp();
-  if (S > 1) {
-    constexpr int OWN = Cfg::PAIRS / S;               // pairs this CTA finishes
-    cluster_sync_aligned();                           // every CTA's ring is free
-    float* xch = reinterpret_cast<float*>(smem);      // [S - 1 senders][OWN pairs][32 columns][128 rows]
-    const int quad = warp & 3, row_in_tile = quad * 32 + lane;
-    const uint32_t lane_base = tmem_base + ((uint32_t)(quad * 32) << 16);
-    if (warp >= 2 && warp < 6) {
-#pragma unroll 1
-      for (int d = 0; d < S; ++d) {
-        if (d == (int)rank) continue;
-        const uint32_t dst = cluster_map(smem_u32(xch), d) + (uint32_t)(((int)rank < d ? rank : rank - 1) * OWN * 32 * 128 + row_in_tile) * 4;
-#pragma unroll 1
-        for (int p = 0; p < OWN; ++p) {
-          int c0, c1;
-          wide_pair_cols(g, d * OWN + p, c0, c1);
-          uint32_t v0[16], v1[16];
-          tmem_ld16(lane_base + c0, v0);
-          tmem_ld16(lane_base + c1, v1);
-          tmem_ld_wait();
-#pragma unroll
-          for (int j = 0; j < 16; ++j) {
-            asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(dst + (uint32_t)((p * 32 + j) * 128) * 4), "r"(v0[j]) : "memory");
-            asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(dst + (uint32_t)((p * 32 + 16 + j) * 128) * 4), "r"(v1[j]) : "memory");
-          }
-        }
-      }
-    }
-    __syncwarp();
-    cluster_sync_aligned();                           // the partial columns of the peers have arrived
-    if (warp >= 2 && warp < 6) {
-      const int ta = u0 % a_units, tb = u0 / a_units;
-      const int t = ta * 128 + row_in_tile;
-      const int pos = g.epi == XB_EPI_QKV && t < g.a_rows ? g.tok_pos[t] : 0;
-#pragma unroll 1
-      for (int p = 0; p < OWN; ++p) {
-        int c0, c1;
-        wide_pair_cols(g, (int)rank * OWN + p, c0, c1);
-        uint32_t v0[16], v1[16];
-        tmem_ld16(lane_base + c0, v0);
-        tmem_ld16(lane_base + c1, v1);
-        tmem_ld_wait();
-        float x0[16], x1[16];
-#pragma unroll
-        for (int j = 0; j < 16; ++j) x0[j] = x1[j] = 0.f;
-#pragma unroll
-        for (int s = 0; s < S; ++s) {                 // rank order: the same sums every time
-          if (s == (int)rank) {
-#pragma unroll
-            for (int j = 0; j < 16; ++j) { x0[j] += __uint_as_float(v0[j]); x1[j] += __uint_as_float(v1[j]); }
-          } else {
-            const float* src = xch + (size_t)((s < (int)rank ? s : s - 1) * OWN + p) * 32 * 128 + row_in_tile;
-#pragma unroll
-            for (int j = 0; j < 16; ++j) { x0[j] += src[j * 128]; x1[j] += src[(16 + j) * 128]; }
-          }
-        }
-        wide_emit(g, t, pos, tb * BN + c0, tb * BN + c1, x0, x1);
-      }
-    }
-  }
   tc_fence_before();
   __syncthreads();
   if (CG == 2) cluster_sync_aligned();                // no CTA of a pair leaves while the other still uses its memory
@@ -425,19 +361,19 @@ xb_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 
 // ----------------------------------------------------------------------------- host side
 struct WideVariant {
-  int bn, cg, split;
+  int bn, cg;
   int (*run)(const CUtensorMap&, const CUtensorMap&, const GemmArgs&, int grid, cudaStream_t, int pdl);
 };
 
-template <int BN, int CG, int S>
+template <int BN, int CG>
 static int xb_wide_launch_t(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmArgs& g, int grid, cudaStream_t st, int pdl) {
-  using Cfg = WideCfg<BN, CG, S>;
+  using Cfg = WideCfg<BN, CG>;
   {
     static bool done[XB_MAX_DEVICES] = {false};
     int dev = 0;
     XB_CUDA(cudaGetDevice(&dev));
     if (dev < 0 || dev >= XB_MAX_DEVICES || !done[dev]) {
-      XB_CUDA(cudaFuncSetAttribute(xb_wide_kernel<BN, CG, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES));
+      XB_CUDA(cudaFuncSetAttribute(xb_wide_kernel<BN, CG>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES));
       if (dev >= 0 && dev < XB_MAX_DEVICES) done[dev] = true;
     }
   }
@@ -453,34 +389,30 @@ static int xb_wide_launch_t(const CUtensorMap& tmA, const CUtensorMap& tmB, cons
     attr[na].val.programmaticStreamSerializationAllowed = 1;
     ++na;
   }
-  if (CG * S > 1) {
+  if (CG > 1) {
     attr[na].id = cudaLaunchAttributeClusterDimension;
-    attr[na].val.clusterDim.x = CG * S;
+    attr[na].val.clusterDim.x = CG;
     attr[na].val.clusterDim.y = 1;
     attr[na].val.clusterDim.z = 1;
     ++na;
   }
   cfg.attrs = attr;
   cfg.numAttrs = na;
-  XB_CUDA(cudaLaunchKernelEx(&cfg, xb_wide_kernel<BN, CG, S>, tmA, tmB, g));
+  XB_CUDA(cudaLaunchKernelEx(&cfg, xb_wide_kernel<BN, CG>, tmA, tmB, g));
   return 0;
 }
 
-#define XB_WIDE_VARIANT(BN, CG, S) {BN, CG, S, xb_wide_launch_t<BN, CG, S>}
+#define XB_WIDE_VARIANT(BN, CG) {BN, CG, xb_wide_launch_t<BN, CG>}
 static const WideVariant g_wide_variants[] = {
-  XB_WIDE_VARIANT(256, 2, 1), XB_WIDE_VARIANT(256, 1, 1), XB_WIDE_VARIANT(192, 1, 1), XB_WIDE_VARIANT(128, 1, 1),
-  XB_WIDE_VARIANT(256, 1, 2), XB_WIDE_VARIANT(192, 1, 2), XB_WIDE_VARIANT(128, 1, 2), XB_WIDE_VARIANT(128, 1, 4),
+  XB_WIDE_VARIANT(256, 2), XB_WIDE_VARIANT(256, 1), XB_WIDE_VARIANT(192, 1), XB_WIDE_VARIANT(128, 1),
 };
 #undef XB_WIDE_VARIANT
 enum { XB_WIDE_VARIANTS = sizeof(g_wide_variants) / sizeof(g_wide_variants[0]) };
 
-// The variant with the least estimated time: waves x (k-blocks of a CTA x time of one) + epilogue, exchange and launch.
-// The times (us) are fitted to a sweep of T = 192 .. 4096 over the Linears of the registered models (K 2048 .. 18944, N 2048 ..
-// 37888): the rule's choice is on average within 1 % of the best variant.  What the variants are for, us cold, old 128 x 256
-// tiling -> choice: T 192, 2048 x 8192: 54.8 -> 18.9 (K in four); T 373, 3072 x 8192: 57 -> 28 (K in two); T 733, 4096 x 14336:
-// 96 -> 87 (192 columns); T 4096, 28672 x 4096: 664 -> 644 (pairs).
-// K goes in parts up to 512 rows only: above, that is best for a few shapes (by 18 % at most, 1024 x 2048 x 8192), and without it
-// a long prompt and its portions sum alike.
+// The variant with the least estimated time: waves x (k-blocks x time of one) + epilogue.  The times (us) are fitted to a sweep of T =
+// 192 .. 4096 over the Linears of the registered models (K 2048 .. 18944, N 2048 .. 37888).
+// What the variants are for, us cold, old 128 x 256 tiling -> choice: T 733, 4096 x 14336: 96 -> 87 (192 columns); T 4096, 28672 x
+// 4096: 664 -> 644 (pairs).
 // col_unit: columns that have to stay together in a tile (a head where the rotation pairs its halves).
 static int xb_pick_wide(int T, int N, int K, int col_unit, int num_sms) {
   int best = 1;
@@ -488,13 +420,12 @@ static int xb_pick_wide(int T, int N, int K, int col_unit, int num_sms) {
   const int a_tiles = (T + 127) / 128, k_blocks = (K + 63) / 64;
   for (int i = 0; i < XB_WIDE_VARIANTS; ++i) {
     const WideVariant& v = g_wide_variants[i];
-    if (v.bn % col_unit != 0 || k_blocks < 4 * v.split || (v.split > 1 && T > 512)) continue;
+    if (v.bn % col_unit != 0) continue;
     const long long units = (long long)((a_tiles + v.cg - 1) / v.cg) * ((N + v.bn - 1) / v.bn);
-    const int slots = v.split == 4 ? (num_sms - 4) / 4 : num_sms / (v.cg * v.split);   // clusters of four leave some SMs idle
+    const int slots = num_sms / v.cg;
     const long long waves = (units + slots - 1) / slots;
     const double kb = v.cg == 2 ? 0.36 : v.bn == 256 ? 0.40 : v.bn == 192 ? 0.31 : 0.26;
-    const double epi = v.bn * 0.02;
-    const double t = (double)waves * k_blocks / v.split * kb + (v.split > 1 ? 0.6 * epi + 1.7 + 5.0 * (double)(waves - 1) : epi);
+    const double t = (double)waves * k_blocks * kb + v.bn * 0.02;
     if (t < best_t) { best_t = t; best = i; }
   }
   return best;
@@ -506,7 +437,6 @@ static int xb_wide_plan(GemmPlan* p, const bf16* x, long long ldx, const bf16* w
   XB_CHECK(vi < XB_WIDE_VARIANTS, "wide Linear variant %d of %d", vi + 1, (int)XB_WIDE_VARIANTS);
   const WideVariant& v = g_wide_variants[vi];
   GemmArgs& g = p->args;
-  XB_CHECK(g.k_blocks >= v.split, "K=%d is too short for %d parts", K, v.split);
   p->wide = vi;
   p->bn = v.bn;
   g.a_tiles = (T + 127) / 128;
@@ -514,8 +444,7 @@ static int xb_wide_plan(GemmPlan* p, const bf16* x, long long ldx, const bf16* w
   g.a_rows = T;
   g.b_rows = N;
   const int units = (g.a_tiles + v.cg - 1) / v.cg * g.b_tiles;
-  if (v.split > 1) p->grid = units * v.split;
-  else p->grid = (units < num_sms / v.cg ? units : num_sms / v.cg) * v.cg;
+  p->grid = (units < num_sms / v.cg ? units : num_sms / v.cg) * v.cg;
   const int box = (v.bn / v.cg) % 128 == 0 ? 128 : 64;
   const long long w_tiles = (N + 127) / 128;
   XB_TRY(xb_make_tmap(&p->tmA, x, T, K, ldx, 128));

@@ -1136,13 +1136,18 @@ static int hy_launch(xb_engine* e, void (*kern)(KArgs...), dim3 grid, dim3 block
   return 0;
 }
 
-// Keys a query of this step can see at most.
-static int hy_most_keys(const xb_engine* e, int window) { return e->step_ctx < window ? e->step_ctx : window; }
-// Warps of a (token, head) block of hy_attn_window_kernel: one per `per` visible keys, at most 16.  Warps beyond the keys only cost: 300 tokens
-// of a float32 layer with a window of 1028, 32 heads, 16 warps 557 us, five 288 us.
-static int hy_window_warps(int keys, int per) {
-  const int n = keys / per + (keys % per != 0);
-  return n < 1 ? 1 : (n > 16 ? 16 : n);
+// Warps of a (token, head) block of hy_attn_window_kernel.  most: the layer's number; single tokens take it.  Prompts take one per 64
+// keys that a query of the step can see, because warps beyond the keys only cost (300 tokens of a float32 layer with a window of 1028, 32
+// heads: 16 warps 557 us, five 288 us); each query then works with as many of them as its own keys ask for (hy_warps_for), so that its
+// sums do not depend on the other rows of the step.
+struct WindowWarps {
+  int launch, own;   // warps of a block; AttnOpt::own_warps
+};
+static WindowWarps hy_window_warps(const xb_engine* e, int span, int most) {
+  const int n = most < 1 ? 1 : most > 16 ? 16 : most;
+  if (e->step_len == 1) return {n, 0};
+  const int asked = hy_warps_for(e->step_ctx < span ? e->step_ctx : span);
+  return {asked < n ? asked : n, 1};
 }
 
 static LinOut hy_plain(const float* f, long long ld) {
@@ -1612,16 +1617,18 @@ static int hy_latent_mixer(xb_engine* e, const HyLayer& l, int T, const LinOut& 
       XB_TRY(hy_launch(e, hy_latent_merge_kernel, dim3(T * H), dim3(128), 0, st, (const float*)hy->lat_part, ns, T * H, H, R, hy->o, (long long)H * R));
   }
   if (!done) {
-    const int aw = hy_window_warps(hy_most_keys(e, hy_latent_window(c)), 64);   // the block's warps share out the visible keys
+    const WindowWarps ww = hy_window_warps(e, hy_latent_window(c), 16);   // the block's warps share out the visible keys
+    const int aw = ww.launch;
+    const AttnOpt lopt{nullptr, 0.f, 1, 0, nullptr, nullptr, 0, ww.own};
     const size_t asm_bytes = (size_t)(((W + 3) & ~3) + aw * (2 + R)) * sizeof(float);
     const LinOut QA = hy_plain(hy->qa, (long long)H * W);
     const int far = hy_latent_window(c);
     if (R <= 256)
       XB_TRY(hy_launch(e, hy_attn_window_kernel<KT, float, 8>, dim3(T, H), dim3(32 * aw), asm_bytes, st, QA, 0, -1, (const KT*)l.k_pool,
-                       (const KT*)l.k_pool, m, H, 1, W, R, W, W, far, 0, c.m_scale, 1.0f, hy->o, (long long)H * R, AttnOpt{nullptr, 0.f, 1, 0}));
+                       (const KT*)l.k_pool, m, H, 1, W, R, W, W, far, 0, c.m_scale, 1.0f, hy->o, (long long)H * R, lopt));
     else
       XB_TRY(hy_launch(e, hy_attn_window_kernel<KT, float, 16>, dim3(T, H), dim3(32 * aw), asm_bytes, st, QA, 0, -1, (const KT*)l.k_pool,
-                       (const KT*)l.k_pool, m, H, 1, W, R, W, W, far, 0, c.m_scale, 1.0f, hy->o, (long long)H * R, AttnOpt{nullptr, 0.f, 1, 0}));
+                       (const KT*)l.k_pool, m, H, 1, W, R, W, W, far, 0, c.m_scale, 1.0f, hy->o, (long long)H * R, lopt));
   }
   if (tiles)
     return hy_launch(e, hy_head_mm_mma_kernel, dim3((T + HY_HG_M - 1) / HY_HG_M, H, (dv + HY_HG_N - 1) / HY_HG_N), dim3(128), 0, st, (const float*)hy->o,
@@ -1986,7 +1993,9 @@ static int hy_softmax_mixer(xb_engine* e, const HyLayer& l, int T, int n_seqs, i
     return 0;
   }
   const int far = c.s_window > 0 ? c.s_window : 1 << 30;   // no window: the block's warps share out all earlier keys
-  const int aw = hy_window_warps(hy_most_keys(e, c.s_chunk > 0 && c.s_chunk < far ? c.s_chunk : far), 32);
+  // one warp per 32 visible keys at most: up to 512 keys a warp takes one tile, so that leaving out warps beyond the step's keys changes no sum
+  const int most = c.s_chunk > 0 && c.s_chunk < far ? c.s_chunk : far, seen = e->step_ctx < most ? e->step_ctx : most;
+  const int aw = seen >= 512 ? 16 : (seen + 31) / 32;
   const size_t asm_bytes = (size_t)(((dk + 3) & ~3) + aw * (2 + (vch ? vch : dvo))) * sizeof(float);
   const LinOut Q = hy_plain(hy->qa, (long long)H * dk);
   const KT* kp = (const KT*)l.k_pool;
@@ -2351,11 +2360,12 @@ static int hy_run_body_t(xb_engine* e, int T, int n_seqs, int n_tiles, void* con
         if (dk == 128) XB_TRY(hy_attn_tc<128>(e, l, m, in, reinterpret_cast<bf16*>(hy->a1), st));
         else XB_TRY(hy_attn_tc<64>(e, l, m, in, reinterpret_cast<bf16*>(hy->a1), st));
       } else {
-        const int aw = hy_window_warps(hy_most_keys(e, c.a_window + c.a_keep_first), 64);
+        const WindowWarps ww = hy_window_warps(e, c.a_window + c.a_keep_first, (c.a_window + c.a_keep_first + 63) / 64);   // at most one per 64 visible keys
+        const int aw = ww.launch;
         const size_t asm_bytes = (size_t)(((dk + 3) & ~3) + aw * (2 + dv)) * sizeof(float);
         XB_TRY(hy_launch(e, hy_attn_window_kernel<KT, AT, 8>, dim3(T, H), dim3(32 * aw), asm_bytes, st, P, l.off_q, l.off_g,
                          (const KT*)l.k_pool, (const KT*)l.v_pool, m, H, G, dk, dv, dk, dv, c.a_window, c.a_keep_first, c.a_scale, 1.0f, a1,
-                         (long long)l.n_o, AttnOpt{nullptr, 0.f, G, 0}));
+                         (long long)l.n_o, AttnOpt{nullptr, 0.f, G, 0, nullptr, nullptr, 0, ww.own}));
       }
       const long long ldc = 2LL * Hr * rk + (long long)Hr * rv;
       if (T > 64 && (Hr * rk) % 4 == 0 && (Hr * rv) % 4 == 0 && hy_quad(P, l.off_rq) && hy_quad(P, l.off_rf) && hy_quad(P, l.off_rv))

@@ -1658,6 +1658,7 @@ __global__ void hy_qg_pack_kernel(LinOut P, int off_q, int nq, int off_g, int ng
 // block's lanes can carry; every block recomputes the scores).
 // r1 / r2 (per head, both or neither): r1[h] * ln(1 + r2[h] * (query position - key position)) is taken off the scaled score.
 // chunk > 0: a query sees only keys of its own chunk of positions, floor(i / chunk) = floor(j / chunk) (keep_first = 0 then).
+// own_warps: a query works with hy_warps_for(its visible keys) warps of its block instead of all of them.
 struct AttnOpt {
   const float* sink;
   float softcap;
@@ -1666,7 +1667,13 @@ struct AttnOpt {
   const float* r1;
   const float* r2;
   int chunk;
+  int own_warps;
 };
+// one warp per 64 keys; up to 128 keys one per tile of 32
+__host__ __device__ __forceinline__ int hy_warps_for(int keys) {
+  const int tiles = keys / 32 + (keys % 32 != 0);
+  return tiles <= 4 ? tiles : tiles <= 8 ? 4 : tiles / 2 + (tiles & 1);
+}
 template <typename KT, typename AT, int NACC>
 __global__ void __launch_bounds__(512) hy_attn_window_kernel(LinOut P, int off_q, int off_gate, const KT* __restrict__ k_pool,
                                                              const KT* __restrict__ v_pool, BatchMeta m, int H, int G, int dk, int dv,
@@ -1695,6 +1702,7 @@ __global__ void __launch_bounds__(512) hy_attn_window_kernel(LinOut P, int off_q
   if (opt.chunk > 0 && pos - pos % opt.chunk > lo) lo = pos - pos % opt.chunk;
   const int n_first = keep_first < lo ? keep_first : lo;   // kept keys that the window does not already cover
   const int n_vis = n_first + (pos - lo + 1);
+  const int asked = opt.own_warps ? hy_warps_for(n_vis) : nw, work = asked < nw ? asked : nw;   // working warps
   float mx = -INFINITY, l = 0.f;
   float acc[NACC];
 #pragma unroll
@@ -1702,7 +1710,7 @@ __global__ void __launch_bounds__(512) hy_attn_window_kernel(LinOut P, int off_q
   // even dv: a lane owns channel pairs (2 * (lane + 32 c), + 1), c < 4, and takes four keys per round so that their value
   // loads are in flight together; odd dv: a lane owns channels lane + 32 c, one key per round
   const bool pairs = ((dv | ldv) & 1) == 0;
-  for (int base = warp * 32; base < n_vis; base += nw * 32) {
+  for (int base = warp < work ? warp * 32 : n_vis; base < n_vis; base += work * 32) {
     const int idx = base + lane;
     float sc = -INFINITY;
     long long prow = 0;

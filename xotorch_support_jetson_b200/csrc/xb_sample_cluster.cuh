@@ -24,14 +24,21 @@ struct SampleXchg {
   int pad;
 };
 
-// Top-k of up to XB_TOPK_FAST: the row is dealt into buckets (what eight lanes, or a warp, have read); the k-th largest bucket
+// Top-k from candidates: the row is dealt into buckets (what eight lanes, or a warp, have read); the k-th largest bucket
 // maximum has k elements at or above it, so the elements from there on contain the kept set -- about k + k^2 / (2 buckets) of
 // 128256, 41 for k = 35.  Only these candidates are looked at again: pivot, softmax, nucleus and draw run over them in the first
-// block of the cluster.  Bound by reading the row and by four cluster barriers: 32 x 128256 logits, top-k 35, 26.6 -> 19.9 us a call (what the host needs to enqueue it),
-// top-k 35 + top-p 0.9 45 -> 35, against four radix passes over every element.  Rows with more candidates than fit (many ties), or with a NaN, and larger k
-// take the radix passes.
-#define XB_TOPK_FAST 256
-#define XB_TOPK_CAND 512    // candidates a block can hold
+// block of the cluster.  Bound by reading the row and by three cluster barriers: 32 x 128256 logits, top-k 35, 26.6 -> 19.9 us a call
+// (what the host needs to enqueue it), against four radix passes over every element.
+// The radix passes keep what they are better at; device time of 32 rows, 128256 / 32768 entries, us.  k = 35: 15 / 13 with the usual 41 candidates,
+// radix 27 / 15.  Candidates are ranked all against all: 26 / 24 for 250, 43 / 40 for 500; handed on to the radix passes 32 / 20 for 300, 33 / 21 for 500.
+// From k = 65 on 512 bucket maxima are ranked too: 40 / 37 for k = 200, radix 27 / 15.  A nucleus costs the radix passes four more, over mass: 57 / 41 for k = 257,
+// candidates 40 / 37 for k = 200, 65 / 62 for 760 of them, 95 / 92 for 1000, handed on 84 / 71.
+// Rows with more candidates than a block holds (many ties) or with a NaN are handed on as well.
+#define XB_TOPK_PLAIN 64       // largest k without and with a nucleus
+#define XB_TOPK_NUCLEUS 256
+#define XB_CAND_PLAIN 256      // most candidates of a row without and with a nucleus
+#define XB_CAND_NUCLEUS 768
+#define XB_TOPK_CAND 512       // candidates a block can hold
 struct SampleCand {
   float bucket[128];        // this block's bucket maxima
   float v[XB_TOPK_CAND];
@@ -39,7 +46,7 @@ struct SampleCand {
   int n;                    // > XB_TOPK_CAND: take the radix passes
 };
 
-// the first block's last steps over n candidates (v, i in shared memory, any order): the chosen index, in every thread
+// the first block's last steps over n <= NT candidates (v, i in shared memory, any order): the chosen index, in every thread
 template <int NT>
 __device__ int sample_candidates(const float* v, const int* idx, int n, int top_k, float top_p, const float* __restrict__ q_row, unsigned long long seed,
                                  int rowi, float* sorted_e, float* cum, float* s_f, int* s_i) {
@@ -47,29 +54,24 @@ __device__ int sample_candidates(const float* v, const int* idx, int n, int top_
   if (tid == 0) { s_f[0] = -INFINITY; s_f[1] = -INFINITY; }
   __syncthreads();
   // rank of every candidate by (value down, index up): a fixed order whatever order they arrived in
-  float my_v[2];
-  int my_i[2], my_r[2], gt[2], ge[2];
-#pragma unroll
-  for (int c = 0; c < 2; ++c) {
-    const int a = tid + c * NT;
-    my_r[c] = gt[c] = ge[c] = 0;
-    if (a < n) {
-      my_v[c] = v[a]; my_i[c] = idx[a];
-      for (int b = 0; b < n; ++b) {
-        const float o = v[b];
-        gt[c] += o > my_v[c];
-        ge[c] += o >= my_v[c];
-        my_r[c] += o > my_v[c] || (o == my_v[c] && idx[b] < my_i[c]);
-      }
-      if (my_r[c] == 0) s_f[1] = my_v[c];                       // largest value
-      if (gt[c] < top_k && ge[c] >= top_k) s_f[0] = my_v[c];    // k-th largest value (every thread that writes has the same)
+  float my_v = 0.f;
+  int my_i = 0, my_r = 0;
+  if (tid < n) {
+    int gt = 0, ge = 0;
+    my_v = v[tid]; my_i = idx[tid];
+    for (int b = 0; b < n; ++b) {
+      const float o = v[b];
+      gt += o > my_v;
+      ge += o >= my_v;
+      my_r += o > my_v || (o == my_v && idx[b] < my_i);
     }
+    if (my_r == 0) s_f[1] = my_v;                       // largest value
+    if (gt < top_k && ge >= top_k) s_f[0] = my_v;       // k-th largest value (every thread that writes has the same)
   }
   __syncthreads();
   const float pivot = s_f[0], mxv = s_f[1];
-#pragma unroll
-  for (int c = 0; c < 2; ++c)
-    if (tid + c * NT < n) sorted_e[my_r[c]] = my_v[c] >= pivot ? expf(my_v[c] - mxv) : 0.f;
+  const float my_e = tid < n && my_v >= pivot ? expf(my_v - mxv) : 0.f;
+  if (tid < n) sorted_e[my_r] = my_e;
   __syncthreads();
   if (tid < 32) {               // running sums in rank order, a fixed tree
     float base = 0.f;
@@ -84,33 +86,32 @@ __device__ int sample_candidates(const float* v, const int* idx, int n, int top_
       if (a + tid < n) cum[a + tid] = x;
       base = __shfl_sync(0xffffffffu, x, 31);
     }
-    if (tid == 0) { s_f[2] = base; s_f[3] = 0.f; }
+    if (tid == 0) { s_f[2] = base; s_i[0] = n - 1; }
   }
   __syncthreads();
   const float sum = s_f[2];
+  float p_cut = 0.f;
   if (top_p > 0.f && top_p < 1.f) {   // smallest probability of the shortest head that reaches top_p, equal ones with it
+    // the lanes of the scan add up in different trees, so where weights are tiny a sum can come out an ulp below its predecessor
+    // and top_p be crossed more than once: the first crossing counts
     for (int a = tid; a < n; a += NT)
-      if (cum[a] >= top_p * sum && (a == 0 || cum[a - 1] < top_p * sum)) s_f[3] = sorted_e[a];
+      if (cum[a] >= top_p * sum && (a == 0 || cum[a - 1] < top_p * sum)) atomicMin(&s_i[0], a);
     __syncthreads();
+    p_cut = sorted_e[s_i[0]];
   }
-  const float p_cut = s_f[3];
   float best = -INFINITY;
   int bi = 0x7fffffff;
-#pragma unroll
-  for (int c = 0; c < 2; ++c) {
-    if (tid + c * NT >= n || my_v[c] < pivot) continue;
-    const float e = expf(my_v[c] - mxv);
-    if (e < p_cut) continue;
+  if (tid < n && my_v >= pivot && my_e >= p_cut) {
     float qv;
     if (q_row != nullptr) {
-      qv = q_row[my_i[c]];
+      qv = q_row[my_i];
     } else {
-      const uint32_t r = mix32(seed * 0x9E3779B97F4A7C15ULL + ((unsigned long long)rowi << 32) + (unsigned)my_i[c]);
+      const uint32_t r = mix32(seed * 0x9E3779B97F4A7C15ULL + ((unsigned long long)rowi << 32) + (unsigned)my_i);
       const float u = ((float)(r & 0xffffff) + 0.5f) * (1.0f / 16777216.0f);
       qv = -logf(u);
     }
-    const float sc = (e / sum) / qv;
-    if (sc > best || (sc == best && my_i[c] < bi)) { best = sc; bi = my_i[c]; }
+    const float sc = (my_e / sum) / qv;
+    if (sc > best || (sc == best && my_i < bi)) { best = sc; bi = my_i; }
   }
   auto better = [](float a, int ai, float b, int bj) { return a > b || (a == b && ai < bj); };
 #pragma unroll
@@ -181,7 +182,8 @@ __global__ void __launch_bounds__(NT) xb_sample_cluster_kernel(const float* __re
     }
   }
   const bool use_k = top_k > 0 && top_k < V;
-  if (use_k && top_k <= XB_TOPK_FAST) {
+  const bool nucleus = top_p > 0.f && top_p < 1.f;
+  if (use_k && top_k <= (nucleus ? XB_TOPK_NUCLEUS : XB_TOPK_PLAIN)) {
     // ---- candidates: everything from the k-th largest bucket maximum on
     const int lane = threadIdx.x & 31, per = top_k <= 64 ? 32 : 8;   // lanes of a bucket: 32 or 128 buckets a block
     const int nb = NT / per;
@@ -228,7 +230,8 @@ __global__ void __launch_bounds__(NT) xb_sample_cluster_kernel(const float* __re
       fits = fits && c <= XB_TOPK_CAND;
       total += c;
     }
-    if (fits && total <= 2 * NT && 4 * total <= chunk) {   // the same answer in every block of the cluster
+    static_assert(XB_CAND_PLAIN <= NT && XB_CAND_NUCLEUS <= NT, "a thread per candidate");
+    if (fits && total <= (nucleus ? XB_CAND_NUCLEUS : XB_CAND_PLAIN) && 4 * total <= chunk) {   // the same answer in every block of the cluster
       if (rank == 0) {
         float* cv = vals;                         // the slice is not needed any more
         int* ci = reinterpret_cast<int*>(vals + total);

@@ -56,3 +56,70 @@ def test_chunks_equal_steps(built_lib, monkeypatch, kind, dk, dv, heads, kv, len
   # both sum dk + 16 fp32 products in another order; read-out norm and output projection carry that on: a few 1e-6 of a row
   err = (a - b).norm(dim=1) / b.norm(dim=1)
   assert err.max() < 2e-5, err.max()
+
+
+def _stage(hf, state, rows, seqs, per_seq):
+  from xotorch_support_jetson_b200.model_config import hybrid_model_config, resolve_tensor_sizes
+  from xotorch_support_jetson_b200.shard import Shard
+  from xotorch_support_jetson_b200.stage import StageRuntime
+  cfg = hybrid_model_config(hf)
+  resolve_tensor_sizes(cfg, {k: tuple(v.shape) for k, v in state.items()})
+  st = StageRuntime(Shard("delta-test", 0, 0, 1), cfg, max_batch_tokens=rows, max_seqs=seqs, max_tokens_per_seq=per_seq, dtype="float32")
+  st.load_state(state)
+  return st
+
+
+def _calls(st, calls):
+  """Stream rows of calls (slots, lengths, starts); the ids depend on slot and position alone."""
+  outs = []
+  for slots, lens, starts in calls:
+    ids = [torch.randint(0, 97, (2048,), generator=torch.Generator().manual_seed(s))[a:a + n] for s, n, a in zip(slots, lens, starts)]
+    tap = torch.empty((sum(lens), 64), device="cuda")
+    st.forward(slots, lens, starts, tokens=torch.cat(ids).to("cuda", torch.int32), taps=[tap])
+    outs.append(tap.cpu())
+  torch.cuda.synchronize()
+  return torch.cat(outs)
+
+
+def _by_steps(monkeypatch, hf, state, calls, rows, seqs, per_seq):
+  monkeypatch.setenv("XB_HY_LPC", "16")
+  st = _stage(hf, state, rows, seqs, per_seq)
+  out = _calls(st, calls)
+  st.close()
+  monkeypatch.setenv("XB_HY_LPC", "0")
+  return out
+
+
+_MIXES = [
+  [[31]], [[32]], [[33]], [[95]], [[1, 32]],                            # where the rules change over
+  [[1, 400, 3, 2, 15, 17, 300]], [[5, 4, 3, 2, 1, 100]],                # several sequences that begin inside the same sixteen rows
+  [[100, 40, 200], [1, 300, 17]], [[200, 97], [3, 1], [16, 112]],       # continuations of other lengths
+]
+
+
+@pytest.mark.parametrize("lens", _MIXES)
+@pytest.mark.parametrize("kind,dk,dv,heads,kv", [("delta", 64, 33, 3, 1), ("delta", 128, 16, 2, 2), ("general", 64, 64, 2, 2), ("general", 72, 72, 2, 2)])
+def test_mixed_lengths_equal_steps(built_lib, monkeypatch, kind, dk, dv, heads, kv, lens):
+  hf, state = _model(kind, dk, dv, heads, kv)
+  calls, at = [], [0] * len(lens[0])
+  for part in lens:
+    calls.append((list(range(len(part))), part, list(at[: len(part)])))
+    at = [a + n for a, n in zip(at, part)] + at[len(part):]
+  rows, seqs, per = max(sum(p) for p in lens), len(lens[0]), max(at) + 8
+  ref = _by_steps(monkeypatch, hf, state, calls, rows, seqs, per).double()
+  st = _stage(hf, state, rows, seqs, per)
+  got = _calls(st, calls).double()
+  st.close()
+  assert torch.isfinite(got).all()
+  err = (got - ref).norm(dim=1) / ref.norm(dim=1)
+  assert err.max() < 2e-5, err.max()   # as above
+
+
+@pytest.mark.parametrize("kind", ["delta", "general"])
+def test_short_neighbours_do_not_change_a_long_prompt(built_lib, kind):
+  hf, state = _model(kind, 64, 64, 2, 2)
+  st = _stage(hf, state, 430, 24, 512)
+  alone = _calls(st, [([0], [400], [0])])
+  beside = _calls(st, [(list(range(1, 23)) + [0], [1] * 22 + [400], [0] * 23)])[22:]
+  st.close()
+  assert torch.equal(alone, beside)

@@ -23,8 +23,14 @@
 
 #define HY_CT 16          // tokens of a chunk = lanes that share a column
 #define HY_CHUNK_VP 18    // pitch of the chunk's 16 x 16 values in shared memory
-// Average tokens of a sequence from which the chunks are used.  A layer in bf16, token by token -> chunks: gated, 32 tokens 257 -> 245 us,
+// Tokens of the step's longest sequence from which the chunks are used: the longest one sets the time of either form while the chip has room
+// for all of them.  A layer in bf16, token by token -> chunks: gated, 32 tokens 257 -> 245 us,
 // two of 64 417 -> 388; general, 32 tokens 241 -> 236, 33 237 -> 239, two of 64 363 -> 359, six of 100 493 -> 430.
+// Where sequences fill the chip token by token is as fast or faster, hence a limit on the blocks of the walk per SM that run abreast.  A bf16 step of
+// one layer (128 blocks a sequence), token by token -> chunks, us, gated / general: 2 x 200 tokens 410 -> 373 / 382 -> 333, 4 x 500 782 -> 717 / 782 -> 696, 10 x
+// 500 1470 -> 1412 / 1465 -> 1471, 14 x 500 1877 -> 1895 / 2245 -> 2023, 20 x 200 1164 -> 1188 / 1200 -> 1219; below 200 tokens 4 x 100 388 -> 380 / 347 -> 340,
+// 6 x 100 423 -> 434 / 386 -> 389, 10 x 100 510 -> 510 / 461 -> 474, 64 x 40 (gated) 913 -> 995.  One of 1000 beside 60 of one: 981 -> 769 / 1074 -> 791.
+__host__ __device__ constexpr int hy_chunk_abreast(int mode, long long longest_chunks) { return longest_chunks < 13 ? 4 : mode == HY_REC_GDELTA ? 16 : 11; }
 __host__ __device__ constexpr int hy_chunk_min(int mode) { return mode == HY_REC_GDELTA ? 96 : 32; }
 __host__ __device__ constexpr int hy_chunk_vectors(int mode) { return mode == HY_REC_GDELTA ? 4 : 2; }
 // floats of one (chunk, head): the row vectors [vectors][16][dkp], for the general rule P_16 [dkp], the matrices [16][16], sixteen numbers per token

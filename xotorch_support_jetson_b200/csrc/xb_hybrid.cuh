@@ -1318,8 +1318,9 @@ static int hy_recur(xb_engine* e, const RecurIn& in, float* state, long long ss,
   }
   if constexpr (MODE == HY_REC_DELTA || MODE == HY_REC_GDELTA) {
     // (a pinned lane layout asks for the token-by-token kernel)
-    if (e->hy->use_seg && e->hy->recur_lpc == 0 && e->hy->chunk_ws != nullptr && T / n_seqs >= hy_chunk_min(MODE) &&
-        (size_t)(T / HY_CT + n_seqs) <= e->hy->chunk_entries) {
+    const long long abreast = (long long)(T / HY_CT + n_seqs) * H * ((dv + 15) / 16), longest = (e->step_len + HY_CT - 1) / HY_CT;
+    if (e->hy->use_seg && e->hy->recur_lpc == 0 && e->hy->chunk_ws != nullptr && e->step_len >= hy_chunk_min(MODE) &&
+        abreast <= hy_chunk_abreast(MODE, longest) * longest * e->num_sms && (size_t)(T / HY_CT + n_seqs) <= e->hy->chunk_entries) {
       if (dk <= 64) return hy_chunks_n<1, MODE>(e, in, state, ss, o, ldo, m, n_seqs, H, dk, dv, T, st);
       if (dk <= 128) return hy_chunks_n<2, MODE>(e, in, state, ss, o, ldo, m, n_seqs, H, dk, dv, T, st);
       if (dk <= 256) return hy_chunks_n<4, MODE>(e, in, state, ss, o, ldo, m, n_seqs, H, dk, dv, T, st);

@@ -123,3 +123,37 @@ def test_short_neighbours_do_not_change_a_long_prompt(built_lib, kind):
   beside = _calls(st, [(list(range(1, 23)) + [0], [1] * 22 + [400], [0] * 23)])[22:]
   st.close()
   assert torch.equal(alone, beside)
+
+
+# a chunk's block of 32 general or 64 gated heads of 256 channels is 2.3 MB: the workspace holds 88 or 89 of them
+@pytest.mark.parametrize("kind,dv,lens,first", [("general", 256, [1700], [1408]), ("general", 256, [900, 30, 800], [448, 30, 464]), ("general", 256, [20] * 10 + [1400], None),
+                                                ("delta", 16, [1500], [1424]), ("delta", 16, [700, 900], [688, 704])])
+def test_steps_beyond_the_workspace(built_lib, monkeypatch, kind, dv, lens, first):
+  heads = 32 if kind == "general" else 64
+  hf, state = _model(kind, 256, dv, heads, heads)
+  n, rows, per = len(lens), sum(lens), max(lens) + 8
+  whole = [(list(range(n)), lens, [0] * n)]
+  ref = _by_steps(monkeypatch, hf, state, whole, rows, n, per).double()
+  st = _stage(hf, state, rows, n, per)
+  got = _calls(st, whole)
+  err = (got.double() - ref).norm(dim=1) / ref.norm(dim=1)
+  assert torch.isfinite(got).all() and err.max() < 2e-5, err.max()   # as above
+  if first is not None:   # the same rows in two steps that the workspace holds: the state passes in fp32, so the bits are the same
+    rest = [(s, a - b, b) for s, (a, b) in enumerate(zip(lens, first)) if a > b]
+    parts = _calls(st, [(list(range(n)), first, [0] * n), ([s for s, _, _ in rest], [k for _, k, _ in rest], [b for _, _, b in rest])])
+    heads, tails = parts[: sum(first)].split(first), dict(zip([s for s, _, _ in rest], parts[sum(first):].split([k for _, k, _ in rest])))
+    again = torch.cat([torch.cat([heads[s], tails[s]]) if s in tails else heads[s] for s in range(n)])
+    assert torch.equal(got, again)
+  st.close()
+
+
+def test_workspaces_follow_the_caches(built_lib):
+  """Reserving the caches anew frees the workspaces first and makes them again: the same bits from another place."""
+  hf, state = _model("delta", 64, 64, 2, 2)
+  st = _stage(hf, state, 300, 3, 512)
+  calls = [([0, 1], [200, 97], [0, 0]), ([0, 1], [1, 1], [200, 97])]
+  first = _calls(st, calls)
+  from xotorch_support_jetson_b200 import _cabi
+  _cabi.check(st.lib.xb_kv_reserve(st._h, 3, 512, st.page_tokens))
+  assert torch.equal(first, _calls(st, calls))
+  st.close()

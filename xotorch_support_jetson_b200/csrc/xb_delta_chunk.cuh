@@ -23,6 +23,7 @@
 
 #define HY_CT 16          // tokens of a chunk = lanes that share a column
 #define HY_CHUNK_VP 18    // pitch of the chunk's 16 x 16 values in shared memory
+#define HY_CHUNK_BYTES ((size_t)192 << 20)   // most the prepared blocks may take (bibevik-1b: 4500 tokens, refatar-1b: 10000); steps beyond that go in parts
 // Tokens of the step's longest sequence from which the chunks are used: the longest one sets the time of either form while the chip has room
 // for all of them.  A layer in bf16, token by token -> chunks: gated, 32 tokens 257 -> 245 us,
 // two of 64 417 -> 388; general, 32 tokens 241 -> 236, 33 237 -> 239, two of 64 363 -> 359, six of 100 493 -> 430.
@@ -38,23 +39,36 @@ __host__ __device__ constexpr int hy_chunk_mats(int mode, int dkp) { return hy_c
 __host__ __device__ constexpr int hy_chunk_scal(int mode, int dkp) { return hy_chunk_mats(mode, dkp) + hy_chunk_vectors(mode) * HY_CT * HY_CT; }
 __host__ __device__ constexpr int hy_chunk_block(int mode, int dkp) { return hy_chunk_scal(mode, dkp) + 6 * HY_CT; }
 
-// entry of chunk c of sequence s: start_row / 16 + s + c (no two sequences share one)
-// grid (T / 16 + n_seqs, H), 256 threads; dynamic shared memory: the row vectors (general rule: and the decays) at pitch dkp + 4
+// Where the blocks of a step lie.  per = 0, all of them at once: chunk c of sequence s at entry start_row / 16 + s + c (no two sequences share
+// one), grid T / 16 + n_seqs.  per > 0, the chunks [c0, c0 + per) of every sequence: entry s * per + c - c0, grid n_seqs * per.
+struct ChunkPart {
+  int c0, per;
+};
+// grid (entries, H), 256 threads; dynamic shared memory: the row vectors (general rule: and the decays) at pitch dkp + 4
 template <int MODE>
-__global__ void __launch_bounds__(256) hy_chunk_prep_kernel(RecurIn in, float* __restrict__ ws, BatchMeta m, int n_seqs, int H, int dk, int dkp) {
+__global__ void __launch_bounds__(256) hy_chunk_prep_kernel(RecurIn in, float* __restrict__ ws, BatchMeta m, ChunkPart part, int n_seqs, int H, int dk,
+                                                            int dkp) {
   extern __shared__ __align__(16) float cps[];
   __shared__ float gs[HY_CT];
   pdl_launch_dependents();
   pdl_wait();
   int s = 0, start = 0, len = 0, c = -1;
-  for (; s < n_seqs; ++s) {
+  if (part.per > 0) {
+    s = blockIdx.x / part.per;
+    c = part.c0 + (int)blockIdx.x - s * part.per;
     start = s > 0 ? m.seq_last[s - 1] + 1 : 0;
     len = m.seq_last[s] - start + 1;
-    c = (int)blockIdx.x - (start / HY_CT + s);
-    if (c < 0) return;
-    if (c * HY_CT < len) break;
+    if (c * HY_CT >= len) return;
+  } else {
+    for (; s < n_seqs; ++s) {
+      start = s > 0 ? m.seq_last[s - 1] + 1 : 0;
+      len = m.seq_last[s] - start + 1;
+      c = (int)blockIdx.x - (start / HY_CT + s);
+      if (c < 0) return;
+      if (c * HY_CT < len) break;
+    }
+    if (s == n_seqs) return;
   }
-  if (s == n_seqs) return;
   const int h = blockIdx.y, g = h / (H / in.q_heads), tid = threadIdx.x;
   const int nt = len - c * HY_CT < HY_CT ? len - c * HY_CT : HY_CT;
   const long long row0 = start + c * HY_CT;
@@ -184,7 +198,7 @@ __device__ __forceinline__ void hy_chunk_reduce(float (&v)[HY_CT][2], int sub) {
 // grid (n_seqs, H, ceil(dv / 16)), 128 threads (16 value columns); dynamic shared memory 2 * (block + 16 x 18 values) floats
 template <int NCH, int MODE>
 __global__ void __launch_bounds__(128) hy_chunk_kernel(RecurIn in, const float* __restrict__ ws, float* __restrict__ state, long long state_stride,
-                                                       float* __restrict__ o, long long ldo, BatchMeta m, int H, int dk, int dv) {
+                                                       float* __restrict__ o, long long ldo, BatchMeta m, ChunkPart part, int H, int dk, int dv) {
   pdl_wait();   // no early trigger, as in hy_recur_kernel
   extern __shared__ __align__(16) float cks[];
   constexpr int DKP = 64 * NCH, BLK = hy_chunk_block(MODE, DKP), NB = BLK + HY_CT * HY_CHUNK_VP, RP = HY_CT * DKP;
@@ -192,7 +206,10 @@ __global__ void __launch_bounds__(128) hy_chunk_kernel(RecurIn in, const float* 
   const int warp = tid >> 5, lane = tid & 31, sub = lane & 15;
   const int j0 = blockIdx.z * 16, jl = warp * 4 + (lane >> 4) * 2, col = j0 + jl;   // this lane's columns col, col + 1
   const SeqSpan sp = seq_span(m, s);
-  const int e0 = sp.start / HY_CT + s, chunks = (sp.len + HY_CT - 1) / HY_CT;
+  // this launch's chunks [c0, c1); chunk c at entry e0 + c
+  const int all = (sp.len + HY_CT - 1) / HY_CT, c0 = part.c0, c1 = part.per > 0 && c0 + part.per < all ? c0 + part.per : all;
+  const int e0 = part.per > 0 ? s * part.per - c0 : sp.start / HY_CT + s;
+  if (c0 >= c1) return;
   const float* cv = in.c + in.voff + (long long)h * dv + j0;
   const int ncv = dv - j0 < 16 ? dv - j0 : 16;
   auto stage = [&](int c, float* buf) {
@@ -209,7 +226,7 @@ __global__ void __launch_bounds__(128) hy_chunk_kernel(RecurIn in, const float* 
   float* st[2];
 #pragma unroll
   for (int c = 0; c < 2; ++c) {
-    const bool live = col + c < dv, have = live && sp.pos0 > 0;
+    const bool live = col + c < dv, have = live && (sp.pos0 > 0 || c0 > 0);   // the part before left its state there
     st[c] = state + (long long)sp.slot * state_stride + ((long long)h * dv + (live ? col + c : 0)) * dk;
 #pragma unroll
     for (int ch = 0; ch < NCH; ++ch) {
@@ -249,10 +266,10 @@ __global__ void __launch_bounds__(128) hy_chunk_kernel(RecurIn in, const float* 
     out[0] = v[0][0];
     out[1] = v[0][1];
   };
-  stage(0, cks);
-  for (int c = 0; c < chunks; ++c) {
+  stage(c0, cks + (c0 & 1) * NB);
+  for (int c = c0; c < c1; ++c) {
     const float* buf = cks + (c & 1) * NB;
-    if (c + 1 < chunks) { stage(c + 1, cks + ((c + 1) & 1) * NB); hy_cp_wait<1>(); }
+    if (c + 1 < c1) { stage(c + 1, cks + ((c + 1) & 1) * NB); hy_cp_wait<1>(); }
     else hy_cp_wait<0>();
     __syncthreads();
     const float* mats = buf + hy_chunk_mats(MODE, DKP);

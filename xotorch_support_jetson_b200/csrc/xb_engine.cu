@@ -43,6 +43,7 @@ struct xb_engine;
 struct HyModel;
 static void hy_destroy(HyModel* hy);
 static int hy_reserve(xb_engine* e);
+static int hy_make_spare_rooms(xb_engine* e);
 static int hy_finalize(xb_engine* e);
 static void hy_drop_plans(xb_engine* e);
 static int hy_kv_splits(xb_engine* e, int T, int max_ctx);
@@ -730,6 +731,7 @@ extern "C" int xb_kv_reserve(xb_engine* e, int n_slots, int max_tokens_per_slot,
   XB_CUDA(cudaMemset(e->d_page_table, 0, e->h_page_table.size() * 4));
   e->c.kv_pages_total = e->n_pages;
   e->c.kv_pages_free = e->free_pages.size();
+  if (e->hy != nullptr) XB_TRY(hy_make_spare_rooms(e));
   return 0;
 }
 

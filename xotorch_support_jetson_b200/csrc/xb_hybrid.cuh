@@ -152,8 +152,17 @@ static void hy_name_vec(HyModel* hy, const std::string& name, float* dst, long l
 // a latent attention layer that reads the cache rows of an earlier one has no pool of its own
 static bool hy_borrows_rows(const HyLayer& l) { return l.d.mixer == XB_MIX_LATENT && l.d.m_kv_from >= 0; }
 
+static void hy_free_spare_rooms(HyModel* hy) {
+  cudaFree(hy->chunk_ws);
+  cudaFree(hy->pieces);
+  hy->chunk_ws = nullptr;
+  hy->pieces = nullptr;
+  hy->chunk_entries = 0;
+  hy->pieces_rows = 0;
+}
 static void hy_destroy(HyModel* hy) {
   if (hy == nullptr) return;
+  hy_free_spare_rooms(hy);
   for (void* p : hy->allocs) cudaFree(p);
   for (HyLayer& l : hy->L) {
     if (!hy_borrows_rows(l)) { cudaFree(l.k_pool); cudaFree(l.v_pool); }
@@ -861,11 +870,6 @@ static int hy_create(xb_engine* e, const xb_hybrid_desc& d, const xb_hybrid_laye
   XB_TRY(hy_alloc(hy, &hy->a1, Tm * hy->maxK * as));
   XB_TRY(hy_alloc(hy, &hy->a2, Tm * hy->maxK * as));
   XB_TRY(hy_alloc(hy, &hy->head_in, R * D * as));
-  if (d.compute_fp32) {
-    const size_t most = Tm > R ? Tm : R;
-    hy->pieces_rows = most < XB_F32_ROWS ? (int)most : XB_F32_ROWS;
-    XB_TRY(hy_alloc_t(hy, &hy->pieces, 3 * (size_t)hy->pieces_rows * hy->maxK));
-  }
   if (d.block == XB_BLOCK_PARALLEL || d.block == XB_BLOCK_PRENORM) XB_TRY(hy_alloc(hy, &hy->ah, Tm * D * as));
   {
     // the first layer that blends values leaves them for the others, whose value rows must have the same width
@@ -911,11 +915,6 @@ static int hy_create(xb_engine* e, const xb_hybrid_desc& d, const xb_hybrid_laye
     const size_t entries = Tm / HY_SEG_MIN + Tm / (2 * HY_SEG_MIN) + 2;
     XB_TRY(hy_alloc_t(hy, &hy->seg_ws, entries * hy->maxSeg));
     XB_TRY(hy_alloc_t(hy, &hy->seg_decay, entries * hy->maxSegK));
-  }
-  if (hy->maxChunk > 0 && Tm >= hy_chunk_min(HY_REC_DELTA)) {
-    // steps of up to 8192 tokens; larger ones run token by token
-    hy->chunk_entries = (Tm < 8192 ? Tm : 8192) / HY_CT + d.max_seqs;
-    XB_TRY(hy_alloc_t(hy, &hy->chunk_ws, hy->chunk_entries * hy->maxChunk));
   }
   if (hy->maxQG > 0) {
     XB_TRY(hy_alloc_t(hy, &hy->qg, Tm * hy->maxQG));
@@ -1048,8 +1047,43 @@ static int hy_missing(xb_engine* e, char* buf, size_t buflen, int* n_missing) {
 }
 
 // ----------------------------------------------------------------------------- slots: KV pools + state
+// Workspaces that make steps faster but that none needs, made once weights and caches have their place: each takes at most a quarter of what is
+// left, the tile-major copies of the weights taken off, so that a model that fills the device still runs (delta rules token by token, float32
+// Linears through the plain kernels).
+template <typename T>
+static int hy_spare_room(T** p, size_t unit, size_t least, size_t to_come, size_t* units) {
+  size_t left = 0, total = 0;
+  XB_CUDA(cudaMemGetInfo(&left, &total));
+  const size_t fit = left > to_come ? (left - to_come) / 4 / (unit * sizeof(T)) : 0;
+  if (*units > fit) *units = fit;
+  if (*units < least) { *units = 0; return 0; }
+  XB_TRY(dmalloc((void**)p, *units * unit * sizeof(T)));
+  XB_CUDA(cudaMemset(*p, 0, *units * unit * sizeof(T)));
+  return 0;
+}
+static int hy_make_spare_rooms(xb_engine* e) {
+  HyModel* hy = e->hy;
+  const xb_hybrid_desc& d = hy->d;
+  const size_t Tm = d.max_batch_tokens, R = hy_max_rows(e), to_come = d.compute_fp32 || !hy->use_tc || hy->finalized ? 0 : e->c.weight_bytes;
+  if (hy->maxChunk > 0 && Tm >= hy_chunk_min(HY_REC_DELTA)) {
+    const size_t most = HY_CHUNK_BYTES / (hy->maxChunk * sizeof(float)), whole = Tm / HY_CT + d.max_seqs;
+    hy->chunk_entries = whole < most ? whole : most;
+    XB_TRY(hy_spare_room(&hy->chunk_ws, hy->maxChunk, 1, to_come, &hy->chunk_entries));
+  }
+  if (d.compute_fp32) {
+    const size_t most = Tm > R ? Tm : R;
+    size_t rows = most < XB_F32_ROWS ? most : XB_F32_ROWS;
+    XB_TRY(hy_spare_room(&hy->pieces, 3 * hy->maxK, rows < 128 ? rows : 128, to_come, &rows));
+    hy->pieces_rows = (int)rows;
+  }
+  XB_CUDA(cudaDeviceSynchronize());   // the zeroing ran on the default stream, which the caller's does not wait for
+  return 0;
+}
+
 static int hy_reserve(xb_engine* e) {
   HyModel* hy = e->hy;
+  hy_free_spare_rooms(hy);
+  hy->f32_plans.clear();   // they hold the room's address
   const size_t es = hy->d.compute_fp32 ? 4 : 2;
   for (HyLayer& l : hy->L) {
     if (hy_borrows_rows(l)) {   // an earlier layer's pool (made before this one)
@@ -1304,9 +1338,21 @@ static int hy_chunks_n(xb_engine* e, const RecurIn& in, float* state, long long 
   constexpr size_t cs = (size_t)2 * (hy_chunk_block(MODE, DKP) + HY_CT * HY_CHUNK_VP) * sizeof(float);
   if (ps > 48 * 1024) XB_SMEM_ATTR_ONCE((hy_chunk_prep_kernel<MODE>), rows * HY_CT * 260 * sizeof(float));
   if (cs > 48 * 1024) XB_SMEM_ATTR_ONCE((hy_chunk_kernel<NCH, MODE>), cs);
-  XB_TRY(hy_launch(e, hy_chunk_prep_kernel<MODE>, dim3(T / HY_CT + n_seqs, H), dim3(256), ps, st, in, e->hy->chunk_ws, m, n_seqs, H, dk, DKP));
-  return hy_launch(e, hy_chunk_kernel<NCH, MODE>, dim3(n_seqs, H, (dv + 15) / 16), dim3(128), cs, st, in, (const float*)e->hy->chunk_ws, state, ss, o, ldo,
-                   m, H, dk, dv);
+  // parts of as many chunks of every sequence as the workspace holds; the state passes from part to part through its place in the cache, so
+  // the sums are those of one launch
+  ChunkPart part{0, 0};
+  int entries = T / HY_CT + n_seqs;
+  if ((size_t)entries > e->hy->chunk_entries) {
+    part.per = (int)(e->hy->chunk_entries / n_seqs);
+    entries = n_seqs * part.per;
+  }
+  do {
+    XB_TRY(hy_launch(e, hy_chunk_prep_kernel<MODE>, dim3(entries, H), dim3(256), ps, st, in, e->hy->chunk_ws, m, part, n_seqs, H, dk, DKP));
+    XB_TRY(hy_launch(e, hy_chunk_kernel<NCH, MODE>, dim3(n_seqs, H, (dv + 15) / 16), dim3(128), cs, st, in, (const float*)e->hy->chunk_ws, state, ss, o, ldo,
+                     m, part, H, dk, dv));
+    part.c0 += part.per;
+  } while (part.per > 0 && part.c0 * HY_CT < e->step_len);
+  return 0;
 }
 template <int MODE>
 static int hy_recur(xb_engine* e, const RecurIn& in, float* state, long long ss, float* o, long long ldo, const BatchMeta& m, int n_seqs,
@@ -1317,10 +1363,11 @@ static int hy_recur(xb_engine* e, const RecurIn& in, float* state, long long ss,
       return hy_segments<MODE>(e, in, state, ss, o, ldo, m, n_seqs, H, dk, dv, T, st);
   }
   if constexpr (MODE == HY_REC_DELTA || MODE == HY_REC_GDELTA) {
-    // (a pinned lane layout asks for the token-by-token kernel)
+    // (a pinned lane layout asks for the token-by-token kernel; so do many sequences of huge heads, of which the workspace holds less than four chunks)
     const long long abreast = (long long)(T / HY_CT + n_seqs) * H * ((dv + 15) / 16), longest = (e->step_len + HY_CT - 1) / HY_CT;
     if (e->hy->use_seg && e->hy->recur_lpc == 0 && e->hy->chunk_ws != nullptr && e->step_len >= hy_chunk_min(MODE) &&
-        abreast <= hy_chunk_abreast(MODE, longest) * longest * e->num_sms && (size_t)(T / HY_CT + n_seqs) <= e->hy->chunk_entries) {
+        abreast <= hy_chunk_abreast(MODE, longest) * longest * e->num_sms &&
+        (size_t)(T / HY_CT + n_seqs <= 4 * n_seqs ? T / HY_CT + n_seqs : 4 * n_seqs) <= e->hy->chunk_entries) {
       if (dk <= 64) return hy_chunks_n<1, MODE>(e, in, state, ss, o, ldo, m, n_seqs, H, dk, dv, T, st);
       if (dk <= 128) return hy_chunks_n<2, MODE>(e, in, state, ss, o, ldo, m, n_seqs, H, dk, dv, T, st);
       if (dk <= 256) return hy_chunks_n<4, MODE>(e, in, state, ss, o, ldo, m, n_seqs, H, dk, dv, T, st);

@@ -43,3 +43,20 @@ def test_pieces_on_tensor_cores_equal_plain_fma(built_lib, monkeypatch, mid, n):
   if n <= 300:
     ref = _ORACLE[mid](hf, state, ids)[rows].double()
     assert (tc - ref).norm() <= max(1.5 * float((plain - ref).norm()), 1e-6 * float(ref.norm()))
+
+
+@pytest.mark.parametrize("n", [1, 300])
+def test_infinite_weights_answer_as_plain_fma(built_lib, monkeypatch, n):
+  """One infinite weight per logit: the product is an infinity of the activation's sign, whatever its low bits."""
+  from xotorch_support_jetson_b200 import synth
+  from xotorch_support_jetson_b200.models import model_cards
+  hf = model_cards["bibevik-tiny"]["hf_config"]
+  state = synth.random_bibevik_state(hf, seed=3)
+  V, D = state["head"].shape
+  state["head"][torch.arange(V), torch.arange(V) % D] = float("inf")
+  ids = torch.randint(0, hf["vocab"], (n,), generator=torch.Generator().manual_seed(n)).to(torch.int32)
+  rows, tc = _logits("bibevik-tiny", hf, state, ids.tolist(), monkeypatch, True)
+  _, plain = _logits("bibevik-tiny", hf, state, ids.tolist(), monkeypatch, False)
+  assert torch.isinf(plain).any()
+  assert torch.equal(torch.isnan(tc), torch.isnan(plain))
+  assert torch.equal(tc.sign()[torch.isinf(plain)], plain.sign()[torch.isinf(plain)]) and torch.equal(torch.isinf(tc), torch.isinf(plain))

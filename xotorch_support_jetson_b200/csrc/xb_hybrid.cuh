@@ -121,6 +121,8 @@ struct HyModel {
   std::map<std::tuple<const void*, const void*, const void*, int>, GemmPlan> plans;
   bf16* pieces = nullptr;    // float32 mode: the rows of a Linear's input as three planes of bf16 pieces [3][pieces_rows][K]
   int pieces_rows = 0;
+  std::set<std::string> nonfinite;   // float32 mode: loaded matrices that hold an infinity or a NaN
+  int* d_flag = nullptr;
   std::map<std::tuple<const void*, const void*, const void*, int, int, int>, F32Plan> f32_plans;
 };
 
@@ -958,6 +960,22 @@ static int hy_store(xb_engine* e, const std::string& name, const void* src, int 
   XB_CUDA(cudaGetLastError());
   XB_CUDA(cudaDeviceSynchronize());
   if (staging) cudaFree(staging);
+  if (hy->d.compute_fp32 && !t.f32) {   // see hy_f32_linear_takes
+    int bad = 0;
+    if (hy->d_flag == nullptr) XB_TRY(hy_alloc_t(hy, &hy->d_flag, 1));
+    XB_CUDA(cudaMemset(hy->d_flag, 0, sizeof(int)));
+    hy_nonfinite_kernel<<<(unsigned)t.rows, 256>>>((const bf16*)t.dst, t.cols, t.ld, hy->d_flag);
+    XB_CUDA(cudaGetLastError());
+    XB_CUDA(cudaMemcpy(&bad, hy->d_flag, sizeof(int), cudaMemcpyDeviceToHost));
+    const bool was = !hy->nonfinite.empty();
+    if (bad != 0) hy->nonfinite.insert(name);
+    else hy->nonfinite.erase(name);
+    if (was != !hy->nonfinite.empty()) {   // captured steps hold the other kernels
+      for (auto& kv : e->graphs)
+        if (kv.second.exec != nullptr) cudaGraphExecDestroy(kv.second.exec);
+      e->graphs.clear();
+    }
+  }
   hy->loaded.insert(name);
   hy->finalized = false;
   return 0;
@@ -1219,9 +1237,10 @@ static bool hy_tc_linear(xb_engine* e, const void* x, long long ldx, const bf16*
   return true;
 }
 
-// The float32 mode on the tensor cores (xb_linear_f32.cuh); input widths off its grid take the plain kernels.
+// The float32 mode on the tensor cores (xb_linear_f32.cuh); input widths off its grid take the plain kernels.  So does a model with a weight that
+// is not finite: against a row's zero pieces an infinity would come out as NaN where the plain product is infinite.
 static bool hy_f32_linear_takes(const xb_engine* e, const bf16* w, int K) {
-  return e->hy->use_tc && e->hy->pieces != nullptr && (size_t)K <= e->hy->maxK && xb_f32_takes(w, K);
+  return e->hy->use_tc && e->hy->pieces != nullptr && e->hy->nonfinite.empty() && (size_t)K <= e->hy->maxK && xb_f32_takes(w, K);
 }
 static int hy_f32_linear(xb_engine* e, const float* x, long long ldx, const bf16* w, const float* bias, int T, int N, int K, float* out, cudaStream_t st,
                          LinOut* y) {

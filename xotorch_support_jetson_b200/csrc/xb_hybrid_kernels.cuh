@@ -3287,6 +3287,12 @@ __global__ void hy_load_convert_kernel(const void* __restrict__ src, int dt, lon
   const long long r = idx / cols, c = idx - r * cols;
   act_store<OT>(dst + r * ld_dst + c, hy_src_at(src, idx, dt));
 }
+// *flag <- 1 if the matrix holds an infinity or a NaN; a block per row
+__global__ void hy_nonfinite_kernel(const bf16* __restrict__ w, long long cols, long long ld, int* __restrict__ flag) {
+  bool bad = false;
+  for (long long c = threadIdx.x; c < cols; c += blockDim.x) bad = bad || !isfinite(bf2f(w[blockIdx.x * ld + c]));
+  if (bad) *flag = 1;
+}
 
 #include "xb_hyper.cuh"
 #include "xb_qkv_prep.cuh"

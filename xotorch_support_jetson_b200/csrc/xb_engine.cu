@@ -753,7 +753,7 @@ extern "C" int xb_kv_slot_len(xb_engine* e, int slot, int* len) {
 // ----------------------------------------------------------------------------- forward
 // every Linear of the engine goes through here (timeline instrumentation hooks in when enabled)
 static int run_gemm(xb_engine* e, const GemmPlan& gp, cudaStream_t st) {
-  if (e->ts_buf != nullptr && e->ts_next < e->ts_cap && gp.grid <= e->ts_blocks) {
+  if (e->ts_buf != nullptr && gp.stages > 0 && e->ts_next < e->ts_cap && gp.grid <= e->ts_blocks) {   // decode Linears
     GemmPlan p = gp;
     p.args.ts = e->ts_buf + (size_t)e->ts_next * e->ts_blocks * XB_TS_SLOTS;
     ++e->ts_next;

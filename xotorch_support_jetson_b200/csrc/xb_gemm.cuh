@@ -55,9 +55,10 @@ struct GemmArgs {
   float* out2;             // SKINNY: second copy of the result (same layout as `out`), e.g. pinned host memory
   unsigned long long* ts;  // timeline instrumentation (XB_GEMM_TS=1): [gridDim.x][XB_TS_SLOTS] globaltimer stamps, else nullptr
 };
-// stamps: 0 block entry, 1 producer: first stages issued (before the dependency wait), 2 producer: dependency resolved,
+// stamps (decode Linears; prompt Linears record none): 0 block entry, 1 weight producer: first boxes issued (as many as the ring
+// holds, or all of the block's), 2 activation producer: dependency resolved,
 // 3 first MMA issued, 4 last MMA committed, 5 (not a time) %smid of the block, 6 epilogue: last unit stored, 7 block exit,
-// 8 epilogue: accumulator of the last unit complete, 9 producer: last load issued, 10 MMA thread: last stage landed
+// 8 epilogue: accumulator of the last unit complete, 9 weight producer: last box issued, 10 MMA thread: last stage landed
 #define XB_TS(g, slot)                                                                   \
   do {                                                                                   \
     if ((g).ts != nullptr) (g).ts[(size_t)blockIdx.x * XB_TS_SLOTS + (slot)] = xb_gtimer(); \
@@ -211,6 +212,7 @@ xb_gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
       }
+      if (issued < STAGES) XB_TS(g, 1);
       XB_TS(g, 9);
     }
   } else if (warp == 6) {

@@ -6,14 +6,19 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
-def _stage(kind, max_rows):
+def _stage(kind, max_rows, sizes=None):
   from oracle import torch_oracle as O
   from xotorch_support_jetson_b200 import models
   from xotorch_support_jetson_b200.shard import Shard
   from xotorch_support_jetson_b200.stage import StageRuntime
   from xotorch_support_jetson_b200.synth import random_hf_state
   # long enough sums (1024 and 2816) and few enough tiles that splitting K over blocks would look worthwhile at 129 to 512 rows
-  if kind == "interleaved":
+  if sizes is not None:   # (heads, kv heads, head dim, feed-forward)
+    H, KV, hd, ff = sizes
+    mid, hf = ("llama-3.2-tiny", dict(models.model_cards["llama-3.2-tiny"]["hf_config"], hidden_size=640, num_attention_heads=H, num_key_value_heads=KV,
+                                      head_dim=hd, intermediate_size=ff, num_hidden_layers=2)) if kind == "interleaved" else \
+              ("qwen-2.5-odd", models._qwen(640, H, KV, ff, 2, vocab=1536, max_pos=4096))
+  elif kind == "interleaved":
     mid, hf = "llama-3.2-tiny", dict(models.model_cards["llama-3.2-tiny"]["hf_config"], hidden_size=1024, num_attention_heads=16, num_key_value_heads=4,
                                      head_dim=64, intermediate_size=2816, num_hidden_layers=2)
   else:
@@ -61,3 +66,23 @@ def test_neighbours_do_not_change_a_prompt(built_lib, kind, lens):
       st.release_slot(3)
   torch.cuda.synchronize()
   st.close()
+
+
+@pytest.mark.parametrize("kind", ["interleaved", "half-split"])
+@pytest.mark.parametrize("sizes", [(10, 2, 64, 992), (5, 1, 128, 1120)])   # 896 q/k/v, 640 o and down, 1984 or 2240 gate/up features: ends inside every tile
+@pytest.mark.parametrize("n", [129, 257, 300])
+def test_every_tile_has_the_same_bits(built_lib, monkeypatch, kind, sizes, n):
+  """CTA pairs and tiles of 256, 192 and 128 features on tile-major weights, with the rotation, cache-append and SiLU epilogues: the whole
+  forward and a token step that reads the cached keys and values."""
+  outs = []
+  for variant in range(1, 5):
+    monkeypatch.setenv("XB_WIDE_VARIANT", str(variant))
+    st, cfg = _stage(kind, n, sizes)
+    ids = torch.randint(1, cfg["vocab_size"], (n + 1,), generator=torch.Generator().manual_seed(n)).to("cuda", torch.int32)
+    rows = _rows(st, cfg, [0], [n], [0], ids[:n].contiguous())
+    step = _rows(st, cfg, [0], [1], [n], ids[n:].contiguous())
+    outs.append(torch.cat([rows, step]).cpu())
+    st.close()
+  assert torch.isfinite(outs[0].float()).all()
+  for o in outs[1:]:
+    assert torch.equal(outs[0], o)

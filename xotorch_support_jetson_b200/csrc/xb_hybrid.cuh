@@ -115,6 +115,7 @@ struct HyModel {
   size_t maxChunk = 0, chunk_entries = 0;          // floats of a chunk over all heads of the largest such layer, chunks it holds
   int use_seg = 1;           // XB_HY_SEG=0: recurrences always as one chain per sequence (A/B); XB_HY_SEG=n >= 64: segments of n tokens
   int seg_len = 0;           // pinned segment length, 0: by the step's shape
+  int use_quad = 1;          // XB_HY_QUAD=0: row kernels of prompts one channel per thread (A/B)
   int use_tc_attn = 1;       // XB_HY_TC_ATTN=0: attention through the per-token kernel everywhere (A/B)
   int use_tc = 1;            // XB_HY_TC=0: every Linear through the plain kernels (A/B)
   size_t cap_P = 0, cap_m = 0, cap_head = 0;   // bytes of the Linear output buffers
@@ -908,6 +909,8 @@ static int hy_create(xb_engine* e, const xb_hybrid_desc& d, const xb_hybrid_laye
     if (ps != nullptr && ps[0] == '0') hy->p_split = 0;
     const char* sl = getenv("XB_HY_SEG");
     if (sl != nullptr) { hy->use_seg = atoi(sl) > 0 ? 1 : 0; hy->seg_len = atoi(sl) >= HY_SEG_MIN ? atoi(sl) : 0; }
+    const char* qd = getenv("XB_HY_QUAD");
+    if (qd != nullptr && qd[0] == '0') hy->use_quad = 0;
     const char* lp = getenv("XB_HY_LPC");
     if (lp != nullptr && (atoi(lp) == 4 || atoi(lp) == 8 || atoi(lp) == 16)) hy->recur_lpc = atoi(lp);
   }
@@ -1411,7 +1414,7 @@ static int hy_filter(xb_engine* e, int T, int n_seqs, bool no_span, const LinOut
                      const BatchMeta& m, int identity, int act_silu, OT* out, long long ld_out, cudaStream_t st) {
   const long long SS = (long long)e->hy->state_floats;
   bool tail_done = false;
-  if (T > 64 && taps >= 2 && taps <= 4 && C % 4 == 0 && ld_out % 4 == 0 && SS % 4 == 0 && hy_quad(in, col0) && hy_quad_ptr(tail) && hy_quad_ptr(out)) {
+  if (e->hy->use_quad && T > 64 && taps >= 2 && taps <= 4 && C % 4 == 0 && ld_out % 4 == 0 && SS % 4 == 0 && hy_quad(in, col0) && hy_quad_ptr(tail) && hy_quad_ptr(out)) {
     // prompts: four channels and eight rows per thread
     const dim3 g((T + 7) / 8, (C / 4 + 255) / 256);
     auto run = [&](auto kern) { return hy_launch(e, kern, g, dim3(256), 0, st, in, col0, C, w, (const float*)tail, SS, m, identity, act_silu, out, ld_out, T); };
@@ -1565,7 +1568,7 @@ static int hy_row_op_launch(xb_engine* e, int T, const RowOpArgs& a, cudaStream_
     return hy_launch(e, hy_row_op_ext_kernel<AT, 256>, dim3(T), dim3(256), (size_t)hy->d.dim * sizeof(float), st, a);
   }
   const LinOut* ms[3] = {&a.m1, &a.m2, &a.m3};
-  bool quad = !few && hy->d.dim % 4 == 0 && (a.bw == nullptr || hy_quad_ptr(a.bw));
+  bool quad = hy->use_quad && !few && hy->d.dim % 4 == 0 && (a.bw == nullptr || hy_quad_ptr(a.bw));
   for (const LinOut* o : ms) quad = quad && ((o->f == nullptr && o->h == nullptr) || hy_quad(*o, 0));
   if (quad) return hy_launch(e, hy_row_op_quad_kernel<AT>, dim3(T), dim3(256), (size_t)hy->d.dim * sizeof(float), st, a);
   if (few) return hy_launch(e, hy_row_op_kernel<AT, 1024>, dim3(T), dim3(1024), (size_t)hy->d.dim * sizeof(float), st, a);
@@ -1870,7 +1873,7 @@ static int hy_run_parallel_t(xb_engine* e, int T, int n_seqs, void* const* taps,
       LinOut Wd;
       XB_TRY(hy_launch(e, hy_act_cols_kernel<AT>, dim3(T, (rk + 255) / 256), dim3(256), 0, st, P, l.off_w1, rk, 1, a2, (long long)rk));
       XB_TRY(hy_linear<AT>(e, a2, rk, l.w_d2, l.t_d2, nullptr, T, HN, rk, hy->m2, hy->cap_m, st, &Wd));
-      if (T > 64 && n % 4 == 0 && n <= 128 && (n & (n - 1)) == 0 && hy_quad(P, l.off_r) && hy_quad(P, l.off_k) && hy_quad(P, l.off_v) && hy_quad(P, l.off_a) &&
+      if (hy->use_quad && T > 64 && n % 4 == 0 && n <= 128 && (n & (n - 1)) == 0 && hy_quad(P, l.off_r) && hy_quad(P, l.off_k) && hy_quad(P, l.off_v) && hy_quad(P, l.off_a) &&
           hy_quad(Wd, 0) && hy_quad_ptr(l.w0))
         XB_TRY(hy_launch(e, hy_gdelta_prep_quad_kernel, dim3((unsigned)(((long long)T * HN / 4 + 255) / 256)), dim3(256), 0, st, P, l.off_r, l.off_k, l.off_v,
                          l.off_a, Wd, (const float*)l.w0, hy->c, 6LL * HN, hy->beta, hy->decay, H, n, T));
@@ -1885,7 +1888,7 @@ static int hy_run_parallel_t(xb_engine* e, int T, int n_seqs, void* const* taps,
     } else {
       const int dv = c.m_vdim;
       const int nc = 2 * H * n + H * dv;
-      if (T > 64 && nc % 4 == 0 && hy_quad(P, l.off_q))
+      if (hy->use_quad && T > 64 && nc % 4 == 0 && hy_quad(P, l.off_q))
         XB_TRY(hy_launch(e, hy_act_cols_quad_kernel<float>, dim3(T, (nc / 4 + 255) / 256), dim3(256), 0, st, P, l.off_q, nc, 0, hy->c, (long long)nc));
       else
         XB_TRY(hy_launch(e, hy_act_cols_kernel<float>, dim3(T, (nc + 255) / 256), dim3(256), 0, st, P, l.off_q, nc, 0, hy->c, (long long)nc));
@@ -2155,7 +2158,7 @@ template <typename AT>
 static int hy_head_norm(xb_engine* e, int T, long long ldo, const float* w, const LinOut& P, int off_gate, AT* out, long long ld_out, int H, int dv,
                         int w_hstride, int gate_sigmoid, cudaStream_t st) {
   const int per = dv / 8;
-  if (T > 64 && off_gate >= 0 && P.h != nullptr && hy_quad_ptr(P.bias) && P.ld % 8 == 0 && off_gate % 8 == 0 && dv % 8 == 0 && per <= 32 && (per & (per - 1)) == 0 &&
+  if (e->hy->use_quad && T > 64 && off_gate >= 0 && P.h != nullptr && hy_quad_ptr(P.bias) && P.ld % 8 == 0 && off_gate % 8 == 0 && dv % 8 == 0 && per <= 32 && (per & (per - 1)) == 0 &&
       ldo % 8 == 0 && ld_out % 8 == 0)
     return hy_launch(e, hy_head_norm_vec_kernel<AT>, dim3((unsigned)(((long long)T * H * per + 255) / 256)), dim3(256), 0, st, (const float*)e->hy->o, ldo, w,
                      P.h + off_gate, P.ld, P.bias != nullptr ? P.bias + off_gate : nullptr, e->hy->d.norm_eps, out, ld_out, H, dv, w_hstride, gate_sigmoid, T);
@@ -2435,7 +2438,7 @@ static int hy_run_body_t(xb_engine* e, int T, int n_seqs, int n_tiles, void* con
                          (long long)l.n_o, AttnOpt{nullptr, 0.f, G, 0, nullptr, nullptr, 0, ww.own}));
       }
       const long long ldc = 2LL * Hr * rk + (long long)Hr * rv;
-      if (T > 64 && (Hr * rk) % 4 == 0 && (Hr * rv) % 4 == 0 && hy_quad(P, l.off_rq) && hy_quad(P, l.off_rf) && hy_quad(P, l.off_rv))
+      if (hy->use_quad && T > 64 && (Hr * rk) % 4 == 0 && (Hr * rv) % 4 == 0 && hy_quad(P, l.off_rq) && hy_quad(P, l.off_rf) && hy_quad(P, l.off_rv))
         XB_TRY(hy_launch(e, hy_hgrn_prep_quad_kernel, dim3(T, ((2 * Hr * rk + Hr * rv) / 4 + 255) / 256), dim3(256), 0, st, P, l.off_rq, l.off_rf, l.off_rv,
                          (const float*)l.lower, hy->c, ldc, Hr * rk, Hr * rv));
       else

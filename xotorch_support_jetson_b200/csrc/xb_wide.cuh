@@ -433,7 +433,10 @@ static int xb_pick_wide(int T, int N, int K, int col_unit, int num_sms) {
 
 static int xb_wide_plan(GemmPlan* p, const bf16* x, long long ldx, const bf16* w, int w_tiled, int T, int N, int K, int col_unit, int num_sms,
                         int force_variant) {
-  const int vi = force_variant > 0 ? force_variant - 1 : xb_pick_wide(T, N, K, col_unit, num_sms);
+  int vi = force_variant > 0 ? force_variant - 1 : xb_pick_wide(T, N, K, col_unit, num_sms);
+  const char* ev = getenv("XB_WIDE_VARIANT");   // pins the variant (from 1) where it does not cut a column unit (tests, A/B)
+  const int pin = ev != nullptr ? atoi(ev) : 0;
+  if (force_variant == 0 && pin >= 1 && pin <= XB_WIDE_VARIANTS && g_wide_variants[pin - 1].bn % col_unit == 0) vi = pin - 1;
   XB_CHECK(vi < XB_WIDE_VARIANTS, "wide Linear variant %d of %d", vi + 1, (int)XB_WIDE_VARIANTS);
   const WideVariant& v = g_wide_variants[vi];
   GemmArgs& g = p->args;

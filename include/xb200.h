@@ -3,7 +3,7 @@
  * The reference (satoutahhaithem/xotorch_support_jetson) is 100% Python and has no FFI;
  * its plugin boundary is the Python class `InferenceEngine`
  * (xotorch/inference/inference_engine.py:11-51).  This header is the native layer that a
- * drop-in `InferenceEngine` subclass binds with ctypes (see INTEGRATION.md); each entry
+ * drop-in `InferenceEngine` subclass binds with ctypes; each entry
  * point cites the reference code whose work it replaces.  Paths are relative to the
  * reference repository root.
  *

@@ -17,8 +17,8 @@
 // FMA), the 2 x 16 dot products of a chunk are reduced together by halving exchanges, after which lane i owns token i, and only the
 // triangular solve goes token by token.  Bound by instruction issue (about a thousand a chunk and warp, one warp a scheduler) and by that
 // solve.
-// 2048 tokens, 16 heads of 128 x 128 (gated): 741 -> 212 us and 38 us of preparation; 450 and 1350 tokens, 32 heads of 64 x 64
-// (general): 777 -> 213 and 98 us.  Errors against 64 bits as token by token (3.4e-7 and 2.9e-7 after 2047 tokens).
+// 2048 tokens, 16 heads of 128 x 128 (gated): 741 -> 212 us and 41 us of preparation; 450 and 1350 tokens, 32 heads of 64 x 64
+// (general): 777 -> 218 and 84 us.  Errors against 64 bits as token by token (3.4e-7 and 2.9e-7 after 2047 tokens).
 #pragma once
 
 #define HY_CT 16          // tokens of a chunk = lanes that share a column

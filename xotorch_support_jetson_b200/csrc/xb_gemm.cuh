@@ -74,7 +74,7 @@ __device__ __forceinline__ void gemm_w_coord(const GemmArgs& g, int wt, int kb, 
 struct GemmUnit {
   int ta, tb, kb0, kb1, slot;
 };
-// Walks the work units of one block; all three warp roles walk the same sequence.
+// Walks the work units of one block; all warp roles walk the same sequence.
 struct UnitWalker {
   int u, it, end;
   __device__ __forceinline__ void init(const GemmArgs& g) {
@@ -194,7 +194,8 @@ xb_gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
 
   // Roles are entered by elect.sync and weights and activations have a producer thread each: under `lane == 0` one thread
   // needed 0.35 us to issue a k-block, as long as HBM takes to deliver its 16 KB to every SM, so no gap was ever made up.
-  // llama-3.2-1b, one sequence: 845 -> 770 us a step; four 8B layers: one sequence 397 -> 372, 32 sequences 764 -> 746.
+  // A step, with the build in one optimiser run (build.py), which these loops also gain from: llama-3.2-1b, one sequence 847 -> 768 us;
+  // four 8B layers, one sequence 398 -> 372, 32 sequences, bound by HBM before, 769 -> 756.
   if (warp == 0) {
     // ===================== TMA producer of the weights =====================
     // They never depend on the preceding kernel: their boxes go out at once, as far as the ring reaches.
@@ -508,7 +509,7 @@ static int xb_wide_run(const GemmPlan& p, cudaStream_t st, int pdl);
 //   16 columns (bs=1):  5: 3.294  6: 3.249  7: 3.227  8: 3.280  9: 3.299  10: 3.335
 //   32 columns (bs=32): 5: 4.85   6: 4.67   7: 4.68   8: 4.70   9: 4.72   10: 4.76
 //   64 columns (bs=64): 4: 6.85   5: 6.60   6: 6.59   7: 6.59   8: 6.57
-// XB_GEMM_STAGES=r1 selects the round-1 depths (5 / 5 / 4 / 6) for an A/B; a number selects that depth for the widths
+// XB_GEMM_STAGES=r1 selects the former depths (5 / 5 / 4 / 6) for an A/B; a number selects that depth for the widths
 // that have it instantiated (xb_gemm_run) and leaves the others at their default.
 static int xb_skinny_stages(int bn) {
   const int w = bn <= 16 ? 0 : bn <= 32 ? 1 : bn <= 64 ? 2 : 3;

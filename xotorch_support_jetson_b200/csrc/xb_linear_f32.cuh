@@ -9,8 +9,9 @@
 //   D[128 rows x 128 features] (TMEM) = sum over pieces  A_p[128 x 64] (smem) * B[128 x 64]^T (W, smem)
 //
 // Bound by the tensor cores (12 MMAs a k-block, 0.4 us) and by the 64 KB an SM takes in for them (0.55 us).  300 rows of two
-// refatar-1b layers, 73 GFLOP: 7.06 ms with plain FMA on 64 x 64 tiles, 1.55 ms now (all kernels); one row 774 -> 506 us, so
-// few rows take it too.
+// refatar-1b layers, 73 GFLOP: 7.06 ms with plain FMA on 64 x 64 tiles, 1.55 ms with this kernel (all kernels of the
+// step; 1.19 ms today); one row 774 -> 506 us, so few rows take it too.  The layers' Linears of 300 rows, 37 to 50 MB of weights: 46 to 62 us, tensor pipe
+// 0.5 to 0.7 busy.
 // S > 1: S CTAs of a cluster share a tile, each a part of K, and add their totals in rank order through distributed shared
 // memory.
 #pragma once

@@ -4,7 +4,7 @@
 encode / sample / decode / infer_tensor / load_checkpoint, concrete infer_prompt), and
 ``get_inference_engine`` mirrors the factory at ``inference_engine.py:54-70`` with one
 new key, ``"b200"``.  A reference checkout registers the engine by adding that key to
-its own ``inference_engine_classes`` / ``get_inference_engine`` (INTEGRATION.md).
+its own ``inference_engine_classes`` / ``get_inference_engine``.
 """
 from abc import ABC, abstractmethod
 from typing import Optional

@@ -1,0 +1,182 @@
+// Softmax attention of float32 prompts by tiles of queries.  Included by xb_hybrid_kernels.cuh.
+//
+// hy_attn_window_kernel gives every (token, query head) a block that reads all of its keys and values: 300 tokens x 32 heads of 64 pull 0.7 GB
+// through L2 and are bound by that (290 us).  Here a block takes 32 query rows of one key head -- 32 / R consecutive tokens of a sequence x
+// its R query heads -- against 32 keys at a time from shared memory, so that a key row is read once for 32 queries.  All sums are fp32 FMA:
+// what bounds it is their issue and the shared-memory reads that feed them.  Half a warp owns two query rows from scores to output.
+// That layer 290 -> 55 us, two float32 layers on a prompt of 300 rows 1196 -> 959.
+//
+// Key tiles start at multiples of 32 positions whatever the queries, and a tile that a query does not see changes none of its sums: a query's
+// result depends on its own position and context alone.  Sequences below `min_len` rows stay with the other kernel: it has a block for every
+// (token, head), where 63 rows make 16 to 64 tiles, too few to share out a long context.  The choice is a sequence's own, too.
+#pragma once
+
+#define HY_AT_ROWS 32
+#define HY_AT_KEYS 32
+#define HY_AT_MIN_LEN 64
+
+__device__ __forceinline__ void hy_at_copy16(float* dst, const float* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+
+struct AttnTile {
+  int H, G, dk, dv;          // query heads, key heads, key and value channels (rows of the pools: dk / dv floats)
+  int v_in_k;                // 1: a value is the head of its key row (v_pool unused)
+  int window, keep_first;
+  float scale, out_scale;
+  int tiles;                 // blocks of a sequence: grid (sequences x tiles, G)
+  int min_len;
+};
+// queries + two stages of keys (and values) + weights; 64 floats behind the last row, which wide value reads may touch
+static size_t hy_at_smem(const AttnTile& a, int nv) {
+  return ((size_t)HY_AT_ROWS * (a.dk + 4) + 2 * HY_AT_KEYS * ((size_t)a.dk + 4 + (a.v_in_k ? 0 : 64 * nv)) + HY_AT_ROWS * (HY_AT_KEYS + 4) + 64) * sizeof(float);
+}
+
+// NV: 64-channel groups of a value row (dv <= 64 NV).  sigmoid(gate column) and out_scale as in hy_attn_window_kernel.
+template <int NV, typename AT>
+__global__ void __launch_bounds__(256) hy_attn_tile_kernel(LinOut P, int off_q, int off_gate, const float* __restrict__ k_pool, const float* __restrict__ v_pool,
+                                                           BatchMeta m, AttnTile a, AT* __restrict__ out, long long ld_out) {
+  pdl_launch_dependents();
+  pdl_wait();
+  extern __shared__ __align__(16) float at_smem[];
+  const int R = a.H / a.G, TQ = HY_AT_ROWS / R, dk = a.dk, dv = a.dv, KP = dk + 4, VP = a.v_in_k ? KP : 64 * NV;
+  const int s = blockIdx.x / a.tiles, i0 = (blockIdx.x - s * a.tiles) * TQ, g = blockIdx.y;
+  const int first = s > 0 ? m.seq_last[s - 1] + 1 : 0, len = m.seq_last[s] + 1 - first;
+  if (len < a.min_len || i0 >= len) return;
+  const int n_tok = min(TQ, len - i0), pos0 = m.tok_pos[first] + i0, pos_last = pos0 + n_tok - 1;
+  const int* pages = m.page_table + (long long)m.seq_slot[s] * m.max_pages;
+  float* sQ = at_smem;
+  float* sK = sQ + HY_AT_ROWS * KP;
+  float* sV = sK + 2 * HY_AT_KEYS * KP;
+  float* sP = sV + (a.v_in_k ? 0 : 2 * HY_AT_KEYS * VP);
+  const int tid = threadIdx.x, hw = tid >> 4, l16 = tid & 15;
+  for (int i = tid; i < HY_AT_ROWS * dk; i += 256) {
+    const int r = i / dk, d = i - r * dk, t = r / R;
+    sQ[r * KP + d] = t < n_tok && r < TQ * R ? lin_at(P, first + i0 + t, off_q + (g * R + r - t * R) * dk + d) * a.scale : 0.f;
+  }
+  // the two rows of this half-warp: position (-1: no such row), newest first key of the window
+  int pos[2], row[2];
+#pragma unroll
+  for (int u = 0; u < 2; ++u) {
+    const int r = hw * 2 + u, t = r / R;
+    row[u] = t < n_tok && r < TQ * R ? t : -1;
+    pos[u] = row[u] >= 0 ? pos0 + t : -1;
+  }
+  auto fetch = [&](int kt, int stage) {   // eight threads a key; keys behind the last query are not read
+    const int j = tid >> 3, key = kt * HY_AT_KEYS + j;
+    float* kd = sK + (stage * HY_AT_KEYS + j) * KP;
+    float* vd = sV + (stage * HY_AT_KEYS + j) * VP;
+    if (key <= pos_last) {
+      const long long kr = ((long long)pages[key / m.page_tokens] * a.G + g) * m.page_tokens + key % m.page_tokens;
+      for (int c = (tid & 7) * 4; c < dk; c += 32) hy_at_copy16(kd + c, k_pool + kr * dk + c);
+      if (!a.v_in_k)
+        for (int c = (tid & 7) * 4; c < dv; c += 32) hy_at_copy16(vd + c, v_pool + kr * dv + c);
+    } else {   // zero rows: their weights are 0
+      for (int c = (tid & 7) * 4; c < dk; c += 32) *reinterpret_cast<float4*>(kd + c) = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (!a.v_in_k)
+        for (int c = (tid & 7) * 4; c < dv; c += 32) *reinterpret_cast<float4*>(vd + c) = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  const int last = pos_last / HY_AT_KEYS, lo = max(0, pos0 - a.window + 1);   // lo: oldest key of the tile's windows
+  auto next = [&](int kt) {   // the next tile that some query sees: kept first keys, then the windows
+    ++kt;
+    return kt * HY_AT_KEYS >= a.keep_first && kt < lo / HY_AT_KEYS ? lo / HY_AT_KEYS : kt;
+  };
+  float mx[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};
+  float4 acc[2][NV];
+#pragma unroll
+  for (int u = 0; u < 2; ++u)
+#pragma unroll
+    for (int v = 0; v < NV; ++v) acc[u][v] = make_float4(0.f, 0.f, 0.f, 0.f);
+  const float* q0 = sQ + hw * 2 * KP;
+  int kt = next(-1), stage = 0;
+  fetch(kt, 0);
+  while (kt <= last) {
+    const int kn = next(kt);
+    if (kn <= last) fetch(kn, stage ^ 1);
+    else asm volatile("cp.async.commit_group;" ::: "memory");
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    __syncthreads();
+    // ---- scores of two rows against keys l16 and l16 + 16
+    const float* k0 = sK + (stage * HY_AT_KEYS + l16) * KP;
+    float sc[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
+#pragma unroll 4
+    for (int c = 0; c < dk; c += 4) {
+      const float4 qa = *reinterpret_cast<const float4*>(q0 + c), qb = *reinterpret_cast<const float4*>(q0 + KP + c);
+      const float4 ka = *reinterpret_cast<const float4*>(k0 + c), kb = *reinterpret_cast<const float4*>(k0 + 16 * KP + c);
+      sc[0][0] = fmaf(qa.x, ka.x, sc[0][0]); sc[0][0] = fmaf(qa.y, ka.y, sc[0][0]); sc[0][0] = fmaf(qa.z, ka.z, sc[0][0]); sc[0][0] = fmaf(qa.w, ka.w, sc[0][0]);
+      sc[0][1] = fmaf(qa.x, kb.x, sc[0][1]); sc[0][1] = fmaf(qa.y, kb.y, sc[0][1]); sc[0][1] = fmaf(qa.z, kb.z, sc[0][1]); sc[0][1] = fmaf(qa.w, kb.w, sc[0][1]);
+      sc[1][0] = fmaf(qb.x, ka.x, sc[1][0]); sc[1][0] = fmaf(qb.y, ka.y, sc[1][0]); sc[1][0] = fmaf(qb.z, ka.z, sc[1][0]); sc[1][0] = fmaf(qb.w, ka.w, sc[1][0]);
+      sc[1][1] = fmaf(qb.x, kb.x, sc[1][1]); sc[1][1] = fmaf(qb.y, kb.y, sc[1][1]); sc[1][1] = fmaf(qb.z, kb.z, sc[1][1]); sc[1][1] = fmaf(qb.w, kb.w, sc[1][1]);
+    }
+    const int key = kt * HY_AT_KEYS + l16;
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int j = key + 16 * h;
+        if (j > pos[u] || (pos[u] - j >= a.window && j >= a.keep_first)) sc[u][h] = -INFINITY;
+      }
+      float t = fmaxf(sc[u][0], sc[u][1]);
+#pragma unroll
+      for (int o = 8; o > 0; o >>= 1) t = fmaxf(t, __shfl_xor_sync(0xffffffffu, t, o));
+      const float nm = fmaxf(mx[u], t), ref = nm == -INFINITY ? 0.f : nm;   // (no key seen yet: every weight below is 0)
+      const float corr = expf(mx[u] - ref), p0 = expf(sc[u][0] - ref), p1 = expf(sc[u][1] - ref);
+      mx[u] = nm;
+      l[u] = l[u] * corr + (p0 + p1);
+      float* sp = sP + (hw * 2 + u) * (HY_AT_KEYS + 4) + l16;
+      sp[0] = p0;
+      sp[16] = p1;
+#pragma unroll
+      for (int v = 0; v < NV; ++v) {
+        acc[u][v].x *= corr; acc[u][v].y *= corr; acc[u][v].z *= corr; acc[u][v].w *= corr;
+      }
+    }
+    __syncwarp();   // a row's weights are its half-warp's own
+    // ---- weighted values: channels 4 l16 .. of each group of 64
+    const float* vs = (a.v_in_k ? sK : sV) + stage * HY_AT_KEYS * VP + l16 * 4;
+    const float* pr = sP + hw * 2 * (HY_AT_KEYS + 4);
+#pragma unroll 2
+    for (int j = 0; j < HY_AT_KEYS; j += 4) {
+      const float4 pa = *reinterpret_cast<const float4*>(pr + j), pb = *reinterpret_cast<const float4*>(pr + HY_AT_KEYS + 4 + j);
+      const float pja[4] = {pa.x, pa.y, pa.z, pa.w}, pjb[4] = {pb.x, pb.y, pb.z, pb.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int v = 0; v < NV; ++v) {
+          const float4 x = *reinterpret_cast<const float4*>(vs + (j + i) * VP + v * 64);
+          acc[0][v].x = fmaf(pja[i], x.x, acc[0][v].x); acc[0][v].y = fmaf(pja[i], x.y, acc[0][v].y);
+          acc[0][v].z = fmaf(pja[i], x.z, acc[0][v].z); acc[0][v].w = fmaf(pja[i], x.w, acc[0][v].w);
+          acc[1][v].x = fmaf(pjb[i], x.x, acc[1][v].x); acc[1][v].y = fmaf(pjb[i], x.y, acc[1][v].y);
+          acc[1][v].z = fmaf(pjb[i], x.z, acc[1][v].z); acc[1][v].w = fmaf(pjb[i], x.w, acc[1][v].w);
+        }
+    }
+    __syncthreads();   // the stage may be filled again
+    kt = kn;
+    stage ^= 1;
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+#pragma unroll
+  for (int u = 0; u < 2; ++u) {
+    float L = l[u];
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) L += __shfl_xor_sync(0xffffffffu, L, o);
+    if (row[u] < 0) continue;
+    const long long t = first + i0 + row[u];
+    const int h = g * R + hw * 2 + u - row[u] * R;
+    const float inv = a.out_scale / L;
+#pragma unroll
+    for (int v = 0; v < NV; ++v) {
+      const float x[4] = {acc[u][v].x, acc[u][v].y, acc[u][v].z, acc[u][v].w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int d = v * 64 + l16 * 4 + i;
+        if (d >= dv) break;
+        float y = x[i] * inv;
+        if (off_gate >= 0) y *= hy_sigmoid(lin_at(P, t, off_gate + h * dv + d));
+        act_store<AT>(out + t * ld_out + (long long)h * dv + d, y);
+      }
+    }
+  }
+}

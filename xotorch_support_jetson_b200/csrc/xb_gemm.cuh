@@ -595,6 +595,7 @@ static int xb_gemm_plan(GemmPlan* p, const bf16* x, long long ldx, const bf16* w
   p->stages = xb_skinny_stages(p->bn);
   p->split.k_blocks = g.k_blocks;
   p->split.q = g.sk_q;
+  p->split.inv = xb_split_inv(g.sk_q, g.sk_items);
   p->split.splits = g.splits;
   return 0;
 }

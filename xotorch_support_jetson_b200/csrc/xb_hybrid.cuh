@@ -1746,15 +1746,19 @@ static int hy_latent_mixer(xb_engine* e, const HyLayer& l, int T, const LinOut& 
 
 // The logits of a step: the wanted rows of the model's last norm (hn), or every sequence's last one, through the head.
 template <typename AT>
-static int hy_run_head(xb_engine* e, int n_seqs, const BatchMeta& m, cudaStream_t st) {
+static int hy_run_head(xb_engine* e, int n_seqs, const BatchMeta& m, cudaStream_t st, const void* rows = nullptr) {
   HyModel* hy = e->hy;
   const xb_hybrid_desc& d = hy->d;
   const int n = e->sel_rows != nullptr ? e->sel_n : n_seqs, D = d.dim;
   if (n <= 0) return 0;
   const int* idx = e->sel_rows != nullptr ? hy->d_rows : m.seq_last;
   LinOut y;
-  XB_TRY(hy_launch(e, hy_gather_rows_kernel<AT>, dim3(n), dim3(256), 0, st, (const float*)hy->hn, idx, reinterpret_cast<AT*>(hy->head_in), D));
-  XB_TRY(hy_linear<AT>(e, hy->head_in, D, hy->head, hy->t_head, nullptr, n, d.vocab, D, hy->head_raw, hy->cap_head, st, &y));
+  const void* in = hy->head_in;
+  if (rows != nullptr && e->sel_rows == nullptr)   // one row a sequence, in order: what a gather would copy
+    in = rows;
+  else
+    XB_TRY(hy_launch(e, hy_gather_rows_kernel<AT>, dim3(n), dim3(256), 0, st, (const float*)hy->hn, idx, reinterpret_cast<AT*>(hy->head_in), D));
+  XB_TRY(hy_linear<AT>(e, in, D, hy->head, hy->t_head, nullptr, n, d.vocab, D, hy->head_raw, hy->cap_head, st, &y));
   const long long tot = (long long)n * d.vocab;
   return hy_launch(e, hy_logits_kernel, dim3((unsigned)((tot + 255) / 256)), dim3(256), 0, st, y, d.logit_softcap, e->logits, n, d.vocab);
 }
@@ -1893,7 +1897,7 @@ static int hy_run_parallel_t(xb_engine* e, int T, int n_seqs, void* const* taps,
     a.xa = nullptr; a.ha = hy->ah; a.eps = d.norm_eps; a.D = D; a.plain_add = 1; a.nw_mode = nwm; a.groups = 1; a.res_mult = 1.f; a.ext = 0;
     return hy_row_op_launch<AT>(e, T, a, st);
   };
-  XB_TRY(hy_launch(e, hy_embed_kernel, dim3(T), dim3(128), 0, st, (const int*)e->in_tokens, (const bf16*)hy->embed, hy->x, D, d.vocab,
+  XB_TRY(hy_launch(e, hy_embed_kernel, dim3(T), dim3(T <= 64 ? 512 : 128), 0, st, (const int*)e->in_tokens, (const bf16*)hy->embed, hy->x, D, d.vocab,
                    d.embed_scale));
   XB_TRY(row_op(hy_none(), hy_none(), hy->L[0].norm1));
   for (int li = 0; li < d.n_layers; ++li) {
@@ -1934,8 +1938,12 @@ static int hy_run_parallel_t(xb_engine* e, int T, int n_seqs, void* const* taps,
       in.xoff[0] = in.xoff[1] = in.xoff[2] = 0;
       in.beta = in.decay = in.qk = nullptr; in.hdecay = l.hdecay;
       XB_TRY(hy_recur<HY_REC_LIGHTNING>(e, in, hy->state + l.st_rec, SS, hy->o, (long long)l.n_o, m, n_seqs, H, n, dv, T, st));
-      XB_TRY(hy_launch(e, hy_all_heads_norm_kernel<AT>, dim3(T), dim3(256), 0, st, (const float*)hy->o, (long long)l.n_o,
-                       (const float*)l.head_norm, P, l.off_g, d.norm_eps, a1, (long long)l.n_o, H * dv));
+      if (T <= 64)
+        XB_TRY(hy_launch(e, hy_all_heads_norm_kernel<AT, 1024>, dim3(T), dim3(1024), 0, st, (const float*)hy->o, (long long)l.n_o,
+                         (const float*)l.head_norm, P, l.off_g, d.norm_eps, a1, (long long)l.n_o, H * dv));
+      else
+        XB_TRY(hy_launch(e, hy_all_heads_norm_kernel<AT, 256>, dim3(T), dim3(256), 0, st, (const float*)hy->o, (long long)l.n_o,
+                         (const float*)l.head_norm, P, l.off_g, d.norm_eps, a1, (long long)l.n_o, H * dv));
     }
     XB_TRY(hy_linear<AT>(e, a1, l.n_o, l.w_o, l.t_o, nullptr, T, D, l.n_o, hy->m1, hy->cap_m, st, &y1));
     if (c.ff > 0) XB_TRY(hy_ff_parallel<AT>(e, l, T, hy->ah, st, &y2));
@@ -1943,7 +1951,7 @@ static int hy_run_parallel_t(xb_engine* e, int T, int n_seqs, void* const* taps,
     if (taps != nullptr && taps[li] != nullptr)
       XB_CUDA(cudaMemcpyAsync(taps[li], hy->x, (size_t)T * D * sizeof(float), cudaMemcpyDeviceToDevice, st));
   }
-  return with_head ? hy_run_head<AT>(e, n_seqs, m, st) : 0;
+  return with_head ? hy_run_head<AT>(e, n_seqs, m, st, T == n_seqs ? hy->ah : nullptr) : 0;
 }
 
 // Rotary-position softmax attention of one layer: P = [q | k | v | head gates] of the step's rows -> a1 = what the output
@@ -2199,7 +2207,10 @@ static int hy_head_norm(xb_engine* e, int T, long long ldo, const float* w, cons
       ldo % 8 == 0 && ld_out % 8 == 0)
     return hy_launch(e, hy_head_norm_vec_kernel<AT>, dim3((unsigned)(((long long)T * H * per + 255) / 256)), dim3(256), 0, st, (const float*)e->hy->o, ldo, w,
                      P.h + off_gate, P.ld, P.bias != nullptr ? P.bias + off_gate : nullptr, e->hy->d.norm_eps, out, ld_out, H, dv, w_hstride, gate_sigmoid, T);
-  return hy_launch(e, hy_head_norm_kernel<AT>, dim3(T, (H + 7) / 8), dim3(256), 0, st, (const float*)e->hy->o, ldo, w, P, off_gate, e->hy->d.norm_eps, 1.0f,
+  if (T <= 64)
+    return hy_launch(e, hy_head_norm_kernel<AT, 4>, dim3(T, (H + 7) / 8), dim3(256), 0, st, (const float*)e->hy->o, ldo, w, P, off_gate, e->hy->d.norm_eps, 1.0f,
+                     out, ld_out, H, dv, w_hstride, gate_sigmoid);
+  return hy_launch(e, hy_head_norm_kernel<AT, 1>, dim3(T, (H + 7) / 8), dim3(256), 0, st, (const float*)e->hy->o, ldo, w, P, off_gate, e->hy->d.norm_eps, 1.0f,
                    out, ld_out, H, dv, w_hstride, gate_sigmoid);
 }
 
@@ -2317,7 +2328,7 @@ static int hy_run_prenorm_t(xb_engine* e, int T, int n_seqs, int n_tiles, void* 
     XB_TRY(hy_launch(e, hy_embed_tanh_kernel<AT>, dim3(T), dim3(256), 0, st, (const int*)e->in_tokens, (const bf16*)hy->embed, hy->x, D, d.vocab,
                      d.embed_scale, TanhNorm{l0.norm1, l0.norm1_b, l0.norm1_a}, ah));
   } else {
-    XB_TRY(hy_launch(e, hy_embed_kernel, dim3(T), dim3(128), 0, st, (const int*)e->in_tokens, (const bf16*)hy->embed, hy->x, D, d.vocab, d.embed_scale));
+    XB_TRY(hy_launch(e, hy_embed_kernel, dim3(T), dim3(T <= 64 ? 512 : 128), 0, st, (const int*)e->in_tokens, (const bf16*)hy->embed, hy->x, D, d.vocab, d.embed_scale));
     XB_TRY(add_norm(hy_none(), hy->L[0].norm1, nullptr, nullptr, false));
   }
   for (int li = 0; li < d.n_layers; ++li) {
@@ -2411,7 +2422,7 @@ static int hy_run_body_t(xb_engine* e, int T, int n_seqs, int n_tiles, void* con
   const bool side_fused = T <= 64 && (size_t)(2 * D + d.side_dim + 8) * sizeof(float) <= 48 * 1024;
   AT* a1 = reinterpret_cast<AT*>(hy->a1);
   AT* a2 = reinterpret_cast<AT*>(hy->a2);
-  XB_TRY(hy_launch(e, hy_embed_kernel, dim3(T), dim3(128), 0, st, (const int*)e->in_tokens, (const bf16*)hy->embed, hy->x, D, d.vocab,
+  XB_TRY(hy_launch(e, hy_embed_kernel, dim3(T), dim3(T <= 64 ? 512 : 128), 0, st, (const int*)e->in_tokens, (const bf16*)hy->embed, hy->x, D, d.vocab,
                    d.embed_scale));
   XB_TRY(hy_row_op<AT>(e, T, hy_none(), 0.f, hy_none(), 0.f, nullptr, 0.f, hy->L[0].norm1, nullptr, st));
   for (int li = 0; li < d.n_layers; ++li) {
@@ -2493,7 +2504,7 @@ static int hy_run_body_t(xb_engine* e, int T, int n_seqs, int n_tiles, void* con
         in.xoff[0] = in.xoff[1] = in.xoff[2] = 0;
         XB_TRY(hy_recur<HY_REC_HGRN>(e, in, hy->state + l.st_rec, SS, hy->o, (long long)l.n_o2, m, n_seqs, Hr, rk, rv, T, st));
       }
-      XB_TRY(hy_launch(e, hy_head_norm_kernel<AT>, dim3(T, (Hr + 7) / 8), dim3(256), 0, st, (const float*)hy->o, (long long)l.n_o2,
+      XB_TRY(hy_launch(e, hy_head_norm_kernel<AT, 1>, dim3(T, (Hr + 7) / 8), dim3(256), 0, st, (const float*)hy->o, (long long)l.n_o2,
                        (const float*)l.head_norm, P, -1, d.norm_eps, 1.0f, a2, (long long)l.n_o2, Hr, rv, 0, 0));
       XB_TRY(hy_linear<AT>(e, a1, l.n_o, l.w_o, l.t_o, nullptr, T, D, l.n_o, hy->m1, hy->cap_m, st, &y1));
       XB_TRY(hy_linear<AT>(e, a2, l.n_o2, l.w_o2, l.t_o2, nullptr, T, D, l.n_o2, hy->m2, hy->cap_m, st, &y2));

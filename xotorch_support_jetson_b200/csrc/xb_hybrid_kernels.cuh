@@ -205,14 +205,28 @@ __global__ void __launch_bounds__(NT) hy_row_op_kernel(RowOpArgs a) {
   if (branch && a.plain_add) {
     const bool three = a.m3.f != nullptr || a.m3.h != nullptr;
     float s2 = 0.f;
-    for (int i = threadIdx.x; i < D; i += NT) {
-      float b = a.s1 * lin_at(a.m1, t, i);
-      if (two) b += a.s2 * lin_at(a.m2, t, i);
-      if (three) b += lin_at(a.m3, t, i);
-      const float v = x[i] + b;
-      x[i] = v;
-      row[i] = v;
-      s2 += v * v;
+    for (int i = threadIdx.x; i < D; i += 2 * NT) {   // both columns' loads go out before the first sum
+      const int col[2] = {i, i + NT < D ? i + NT : -1};
+      const float xv[2] = {x[i], col[1] >= 0 ? x[col[1]] : 0.f};
+      float b[2], u[2];
+      lin_at_cols<2, 12>(a.m1, t, col, u);
+      b[0] = a.s1 * u[0]; b[1] = a.s1 * u[1];
+      if (two) {
+        lin_at_cols<2, 12>(a.m2, t, col, u);
+        b[0] += a.s2 * u[0]; b[1] += a.s2 * u[1];
+      }
+      if (three) {
+        lin_at_cols<2, 12>(a.m3, t, col, u);
+        b[0] += u[0]; b[1] += u[1];
+      }
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        if (col[c] < 0) break;
+        const float v = xv[c] + b[c];
+        x[col[c]] = v;
+        row[col[c]] = v;
+        s2 += v * v;
+      }
     }
     if (a.nw == nullptr && a.xa == nullptr) return;
     s2 = block_sum<NT>(s2, red);
@@ -226,11 +240,21 @@ __global__ void __launch_bounds__(NT) hy_row_op_kernel(RowOpArgs a) {
     }
   } else if (branch) {
     float ss = 0.f;
-    for (int i = threadIdx.x; i < D; i += NT) {
-      float v = a.s1 * lin_at(a.m1, t, i);
-      if (two) v += a.s2 * lin_at(a.m2, t, i);
-      row[i] = v;
-      ss += v * v;
+    for (int i = threadIdx.x; i < D; i += 2 * NT) {
+      const int col[2] = {i, i + NT < D ? i + NT : -1};
+      float v[2], u[2];
+      lin_at_cols<2, 12>(a.m1, t, col, v);
+      v[0] *= a.s1; v[1] *= a.s1;
+      if (two) {
+        lin_at_cols<2, 12>(a.m2, t, col, u);
+        v[0] += a.s2 * u[0]; v[1] += a.s2 * u[1];
+      }
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        if (col[c] < 0) break;
+        row[col[c]] = v[c];
+        ss += v[c] * v[c];
+      }
     }
     ss = block_sum<NT>(ss, red);
     const float inv = 1.0f / sqrtf(ss / (float)D + a.eps);
@@ -1506,8 +1530,9 @@ __global__ void hy_hgrn_prep_kernel(LinOut P, int off_q, int off_f, int off_v, c
 // ----------------------------------------------------------------------------- per-head RMS norm (+ SiLU gate) of a read-out
 // out[t, h*dv + j] = scale * o / rms_over_dv(o) * w[h * w_hstride + j] * (gate ? act(P[t, off_gate + h*dv + j]) : 1)
 // w_hstride: 0 = one weight vector for all heads, dv = a vector per head; gate_sigmoid: 0 = SiLU gate, 1 = sigmoid gate.
-// H = 1 with dv = all heads' size norms the concatenated read-out as one vector.
-template <typename AT>
+// H = 1 with dv = all heads' size norms the concatenated read-out as one vector.  G: gate columns of a lane read at once, ahead of the sum (4 up to 64
+// rows, where the planes' latency counts; 1 in prompts).
+template <typename AT, int G>
 __global__ void __launch_bounds__(256) hy_head_norm_kernel(const float* __restrict__ o, long long ldo, const float* __restrict__ w,
                                                            LinOut P, int off_gate, float eps, float scale, AT* __restrict__ out,
                                                            long long ld_out, int H, int dv, int w_hstride, int gate_sigmoid) {
@@ -1519,15 +1544,27 @@ __global__ void __launch_bounds__(256) hy_head_norm_kernel(const float* __restri
     const float* p = o + t * ldo + (long long)h * dv;
     float ss = 0.f;
     for (int j = lane; j < dv; j += 32) ss += p[j] * p[j];
+    float gz[G] = {0.f};
+    auto gates = [&](int j0) {
+      if (off_gate < 0) return;
+      int col[G];
+#pragma unroll
+      for (int c = 0; c < G; ++c) col[c] = j0 + 32 * c < dv ? off_gate + h * dv + j0 + 32 * c : -1;
+      lin_at_cols<G, 4>(P, t, col, gz);
+    };
+    if (G > 1) gates(lane);   // they arrive while the sum is made
     ss = warp_sum(ss);
     const float inv = scale / sqrtf(ss / (float)dv + eps);
-    for (int j = lane; j < dv; j += 32) {
-      float v = p[j] * inv * w[(long long)h * w_hstride + j];
-      if (off_gate >= 0) {
-        const float gz = lin_at(P, t, off_gate + h * dv + j);
-        v *= gate_sigmoid ? hy_sigmoid(gz) : hy_silu(gz);
+    for (int j0 = lane; j0 < dv; j0 += 32 * G) {
+      if (G == 1 || j0 >= 32 * G) gates(j0);
+#pragma unroll
+      for (int c = 0; c < G; ++c) {
+        const int j = j0 + 32 * c;
+        if (j >= dv) break;
+        float v = p[j] * inv * w[(long long)h * w_hstride + j];
+        if (off_gate >= 0) v *= gate_sigmoid ? hy_sigmoid(gz[c]) : hy_silu(gz[c]);
+        act_store<AT>(out + t * ld_out + (long long)h * dv + j, v);
       }
-      act_store<AT>(out + t * ld_out + (long long)h * dv + j, v);
     }
   }
 }
@@ -2314,31 +2351,49 @@ __global__ void __launch_bounds__(NT) hy_latent_down_kernel(LinOut P, int off_dk
   __shared__ float red[32];
   const int row = blockIdx.x;
   const bool rows = off_dkv >= 0;
+  __shared__ int at[2];   // position, page of the row
   float sq = 0.f, sk = 0.f;
+  if (rows && threadIdx.x == NT - 64) {   // three dependent lookups, by a thread that has no latent column where threads abound
+    const int pos = m.tok_pos[row];
+    at[0] = pos;
+    at[1] = m.page_table[(long long)m.seq_slot[m.tok_seq[row]] * m.max_pages + pos / m.page_tokens];
+  }
   for (int i = threadIdx.x; i < qr; i += NT) { const float v = lin_at(P, row, off_dq + i); dsm[i] = v; sq = fmaf(v, v, sq); }
   if (rows)
-    for (int i = threadIdx.x; i < R; i += NT) { const float v = lin_at(P, row, off_dkv + i); dsm[qr + i] = v; sk = fmaf(v, v, sk); }
+    for (int i = threadIdx.x; i < R; i += NT) {
+      const int col[1] = {off_dkv + i};
+      float v[1];
+      lin_at_cols<1, 8>(P, row, col, v);
+      dsm[qr + i] = v[0];
+      sk = fmaf(v[0], v[0], sk);
+    }
+  const int half = r.dims >> 1;   // `half` pairs, then the entries that pass unchanged
+  const int i0 = NT - 1 - threadIdx.x;
+  float uv[2] = {0.f, 0.f};
+  if (rows && i0 < dr - half) {   // this thread's first pair
+    const int d0 = i0 >= half ? half + i0 : r.half ? i0 : 2 * i0, d1 = i0 >= half ? -1 : r.half ? i0 + half : 2 * i0 + 1;
+    const int col[2] = {off_dkv + R + d0, d1 >= 0 ? off_dkv + R + d1 : -1};
+    lin_at_cols<2, 8>(P, row, col, uv);
+  }
   if (qr > 0) {
     const float inv = 1.0f / sqrtf(block_sum<NT>(sq, red) / (float)qr + eps);
     for (int i = threadIdx.x; i < qr; i += NT) act_store<AT>(cq + (long long)row * qr + i, dsm[i] * inv * qnw[i]);   // its own entries
   }
   if (!rows) return;
-  const int s = m.tok_seq[row], pos = m.tok_pos[row];
-  const int page = m.page_table[(long long)m.seq_slot[s] * m.max_pages + pos / m.page_tokens];
-  KT* kr = k_pool + ((long long)page * m.page_tokens + pos % m.page_tokens) * (R + dr);
   const float inv = 1.0f / sqrtf(block_sum<NT>(sk, red) / (float)R + eps);
+  const int pos = at[0];
+  KT* kr = k_pool + ((long long)at[1] * m.page_tokens + pos % m.page_tokens) * (R + dr);
   for (int i = threadIdx.x; i < R; i += NT) act_store<KT>(kr + i, dsm[qr + i] * inv * nw[i]);
-  const int half = r.dims >> 1;   // `half` pairs, then the entries that pass unchanged
-  for (int i = NT - 1 - threadIdx.x; i < dr - half; i += NT) {
+  for (int i = i0; i < dr - half; i += NT) {
     if (i < half) {
       const int d0 = r.half ? i : 2 * i, d1 = r.half ? i + half : 2 * i + 1;
-      const float u = lin_at(P, row, off_dkv + R + d0), v = lin_at(P, row, off_dkv + R + d1);
+      const float u = i == i0 ? uv[0] : lin_at(P, row, off_dkv + R + d0), v = i == i0 ? uv[1] : lin_at(P, row, off_dkv + R + d1);
       float cs, sn;
       hy_rot_cs(r, pos, i, &cs, &sn);
       act_store<KT>(kr + R + d0, u * cs - v * sn);
       act_store<KT>(kr + R + d1, v * cs + u * sn);
     } else {
-      act_store<KT>(kr + R + half + i, lin_at(P, row, off_dkv + R + half + i));
+      act_store<KT>(kr + R + half + i, i == i0 ? uv[0] : lin_at(P, row, off_dkv + R + half + i));
     }
   }
 }
@@ -2352,11 +2407,17 @@ template <int ROWS>
 __global__ void __launch_bounds__(256) hy_latent_absorb_kernel(LinOut Q, int qoff, int dr, const bf16* __restrict__ W, float* __restrict__ qa,
                                                                int H, int T, int K, int N, RotArgs r, const int* __restrict__ tok_pos) {
   pdl_launch_dependents();
-  pdl_wait();
   extern __shared__ __align__(16) float xsm[];
   const int t0 = blockIdx.x * ROWS, h = blockIdx.y;
   const int nt = T - t0 < ROWS ? T - t0 : ROWS;
   const int qh = qoff + h * (K + dr), ld = N + dr;
+  // one row: the block waits for its weights, which depend on no kernel before -- PRE of a thread's first column are under way early
+  constexpr int PRE = ROWS == 1 ? 32 : 0;
+  const bf16* Wh = W + (long long)h * K * N;
+  bf16 pre[PRE > 0 ? PRE : 1];
+#pragma unroll
+  for (int k = 0; k < PRE; ++k) pre[k] = k < K && threadIdx.x < N ? Wh[(long long)k * N + threadIdx.x] : bf16();
+  pdl_wait();
   for (int i = threadIdx.x; i < ROWS * K; i += 256) {
     const int rr = i / K, k = i - rr * K;
     xsm[i] = rr < nt ? lin_at(Q, t0 + rr, qh + k) : 0.f;
@@ -2377,13 +2438,19 @@ __global__ void __launch_bounds__(256) hy_latent_absorb_kernel(LinOut Q, int qof
     }
   }
   __syncthreads();
-  const bf16* Wh = W + (long long)h * K * N;
   for (int n = threadIdx.x; n < N; n += 256) {
     float acc[ROWS];
 #pragma unroll
     for (int rr = 0; rr < ROWS; ++rr) acc[rr] = 0.f;
-#pragma unroll 8
-    for (int k = 0; k < K; ++k) {
+    int k0 = 0;
+    if (PRE > 0 && n == threadIdx.x) {
+#pragma unroll
+      for (int k = 0; k < PRE; ++k)
+        if (k < K) acc[0] = fmaf(xsm[k], bf2f(pre[k]), acc[0]);
+      k0 = PRE;
+    }
+#pragma unroll(ROWS == 1 ? 32 : 8)
+    for (int k = k0; k < K; ++k) {
       const float w = bf2f(Wh[(long long)k * N + n]);
 #pragma unroll
       for (int rr = 0; rr < ROWS; ++rr) acc[rr] = fmaf(xsm[rr * K + k], w, acc[rr]);
@@ -2444,19 +2511,37 @@ __global__ void __launch_bounds__(128) hy_head_mm_kernel(const float* __restrict
 // up-projection and the head's gate in one block.
 //   x = sum_s O_s 2^(m_s - M) / sum_s l_s 2^(m_s - M);  y[t, h * N + n] = sigmoid(G) * sum_k x[k] W[(h * N + n) * R + k]
 // part [n_splits][T * H][2 + R] = (m, l, O) per share.  grid (T, H), 256 threads; R + n_splits floats of shared memory.
+// Shares behind the last one that holds a key (a short sequence has fewer tiles than the step has shares) are not read: they would add zeros.
+// The first eight weight rows of a warp are under way before the kernel before this one is done.  Latency-bound (128 blocks, 1 MB): 38 shares read
+// in rounds of eight and weights in rounds of four took 24 us cold at 8 tokens of 24 to 36 keys.
 template <typename AT>
 __global__ void __launch_bounds__(256) hy_latent_readout_kernel(const float* __restrict__ part, int n_splits, int NR, int H, int R, const bf16* __restrict__ W,
                                                                 AT* __restrict__ y, long long ldy, int N, LinOut G, int off_gate) {
   pdl_launch_dependents();
-  pdl_wait();
   extern __shared__ __align__(16) float xsm[];
+  __shared__ int used;
   float* fac = xsm + R;
   const int t = blockIdx.x, h = blockIdx.y, row = t * H + h;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const bf16* Wh = W + (long long)h * N * R;
+  const bool vec = (R & 7) == 0 && (reinterpret_cast<uintptr_t>(W) & 15) == 0;
+  constexpr int PRE = 8;
+  uint4 pre[PRE];
+#pragma unroll
+  for (int i = 0; i < PRE; ++i)
+    pre[i] = vec && lane * 8 < R && warp + 8 * i < N ? *reinterpret_cast<const uint4*>(Wh + (long long)(warp + 8 * i) * R + lane * 8) : make_uint4(0u, 0u, 0u, 0u);
+  pdl_wait();
+  const float g = off_gate >= 0 ? hy_sigmoid(lin_at(G, t, off_gate + h)) : 1.0f;
   if (warp == 0) {
     float M = HY_LAT_NEG;
-    for (int s = lane; s < n_splits; s += 32) M = fmaxf(M, part[((long long)s * NR + row) * (R + 2)]);
+    int last = 0;
+    for (int s = lane; s < n_splits; s += 32) {
+      const float v = part[((long long)s * NR + row) * (R + 2)];
+      if (v > HY_LAT_NEG) last = s + 1;
+      M = fmaxf(M, v);
+    }
     M = warp_max(M);
+    last = __reduce_max_sync(0xffffffffu, last);
     float L = 0.f;
     for (int s = lane; s < n_splits; s += 32) {
       const float* p = part + ((long long)s * NR + row) * (R + 2);
@@ -2466,29 +2551,45 @@ __global__ void __launch_bounds__(256) hy_latent_readout_kernel(const float* __r
     }
     L = warp_sum(L);
     for (int s = lane; s < n_splits; s += 32) fac[s] /= L;
+    if (lane == 0) used = last > 0 ? last : 1;   // a row without a finite score keeps its NaN
   }
   __syncthreads();
+  const int shares = used;
   for (int c = threadIdx.x; c < R; c += 256) {
     float acc = 0.f;
     const float* p = part + (long long)row * (R + 2) + 2 + c;
 #pragma unroll 8
-    for (int s = 0; s < n_splits; ++s) acc = fmaf(p[(long long)s * NR * (R + 2)], fac[s], acc);
+    for (int s = 0; s < shares; ++s) acc = fmaf(p[(long long)s * NR * (R + 2)], fac[s], acc);
     xsm[c] = acc;
   }
   __syncthreads();
-  const float g = off_gate >= 0 ? hy_sigmoid(lin_at(G, t, off_gate + h)) : 1.0f;
-  const bf16* Wh = W + (long long)h * N * R;
-  const bool vec = (R & 7) == 0 && (reinterpret_cast<uintptr_t>(W) & 15) == 0;
-#pragma unroll 4
-  for (int n = warp; n < N; n += 8) {
-    float acc = 0.f;
-    if (vec) {
-      for (int k = lane * 8; k < R; k += 256) acc = hy_dot8(xsm + k, *reinterpret_cast<const uint4*>(Wh + (long long)n * R + k), acc);
-    } else {
-      for (int k = lane; k < R; k += 32) acc = fmaf(bf2f(Wh[(long long)n * R + k]), xsm[k], acc);
-    }
+  auto emit = [&](int n, float acc) {
     acc = warp_sum(acc);
     if (lane == 0) act_store<AT>(y + (long long)t * ldy + (long long)h * N + n, acc * g);
+  };
+  if (vec) {
+#pragma unroll
+    for (int i = 0; i < PRE; ++i) {
+      const int n = warp + 8 * i;
+      if (n >= N) break;
+      float acc = 0.f;
+      if (lane * 8 < R) acc = hy_dot8(xsm + lane * 8, pre[i], acc);
+      for (int k = lane * 8 + 256; k < R; k += 256) acc = hy_dot8(xsm + k, *reinterpret_cast<const uint4*>(Wh + (long long)n * R + k), acc);
+      emit(n, acc);
+    }
+#pragma unroll 8
+    for (int n = warp + 8 * PRE; n < N; n += 8) {
+      float acc = 0.f;
+      for (int k = lane * 8; k < R; k += 256) acc = hy_dot8(xsm + k, *reinterpret_cast<const uint4*>(Wh + (long long)n * R + k), acc);
+      emit(n, acc);
+    }
+  } else {
+#pragma unroll 4
+    for (int n = warp; n < N; n += 8) {
+      float acc = 0.f;
+      for (int k = lane; k < R; k += 32) acc = fmaf(bf2f(Wh[(long long)n * R + k]), xsm[k], acc);
+      emit(n, acc);
+    }
   }
 }
 
@@ -2558,20 +2659,30 @@ __global__ void __launch_bounds__(128) hy_head_mm_mma_kernel(const float* __rest
 }
 
 // The read-out of all heads normed as ONE vector (RMS over the n entries of a token), weighted and gated by sigmoid:
-// out[t, i] = o[t, i] / rms(o[t, :]) * w[i] * sigmoid(P[t, off_gate + i]).  grid (T), 256 threads.
-template <typename AT>
-__global__ void __launch_bounds__(256) hy_all_heads_norm_kernel(const float* __restrict__ o, long long ldo, const float* __restrict__ w, LinOut P,
-                                                                int off_gate, float eps, AT* __restrict__ out, long long ld_out, int n) {
+// out[t, i] = o[t, i] / rms(o[t, :]) * w[i] * sigmoid(P[t, off_gate + i]).  grid (T), NT threads: 256 for prompts, 1024 in steps of few rows.
+template <typename AT, int NT>
+__global__ void __launch_bounds__(NT) hy_all_heads_norm_kernel(const float* __restrict__ o, long long ldo, const float* __restrict__ w, LinOut P,
+                                                               int off_gate, float eps, AT* __restrict__ out, long long ld_out, int n) {
   pdl_launch_dependents();
   pdl_wait();
   __shared__ float red[32];
   const long long t = blockIdx.x;
   const float* p = o + t * ldo;
   float ss = 0.f;
-  for (int i = threadIdx.x; i < n; i += 256) ss = fmaf(p[i], p[i], ss);
-  ss = block_sum<256>(ss, red);
-  const float inv = 1.0f / sqrtf(ss / (float)n + eps);
-  for (int i = threadIdx.x; i < n; i += 256) act_store<AT>(out + t * ld_out + i, p[i] * inv * w[i] * hy_sigmoid(lin_at(P, t, off_gate + i)));
+#pragma unroll 8
+  for (int i = threadIdx.x; i < n; i += NT) ss = fmaf(p[i], p[i], ss);
+  float inv = 0.f;
+  for (int base = 0; base < n; base += 2 * NT) {
+    const int i = base + threadIdx.x, col[2] = {i < n ? off_gate + i : -1, i + NT < n ? off_gate + i + NT : -1};
+    float gz[2];
+    lin_at_cols<2, 8>(P, t, col, gz);
+    if (base == 0) inv = 1.0f / sqrtf(block_sum<NT>(ss, red) / (float)n + eps);
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      const int j = i + c * NT;
+      if (j < n) act_store<AT>(out + t * ld_out + j, p[j] * inv * w[j] * hy_sigmoid(gz[c]));
+    }
+  }
 }
 
 // ----------------------------------------------------------------------------- element-wise activations of projection columns
@@ -2604,27 +2715,49 @@ __global__ void __launch_bounds__(256) hy_gdelta_prep_kernel(LinOut P, int off_r
   float* row = c + t * ldc;
   for (int h = blockIdx.y * nw + warp; h < H; h += nw * gridDim.y) {
     const int b = h * n;
-    float sk = 0.f;
-    for (int i = lane; i < n; i += 32) {
+    // two channels a lane and turn; those of the first turn (all of them up to 64 channels) are read once, ahead of the sum
+    float sk = 0.f, ik = 0.f, s_ra = 0.f, s_rk = 0.f;
+    for (int i = lane + 64; i < n; i += 32) {
       const float k = lin_at(P, t, off_k + b + i);
       sk = fmaf(k, k, sk);
     }
-    sk = warp_sum(sk);
-    const float ik = 1.0f / sqrtf(sk + 1e-6f);
-    float s_ra = 0.f, s_rk = 0.f;
-    for (int i = lane; i < n; i += 32) {
-      const float r = lin_at(P, t, off_r + b + i), k = lin_at(P, t, off_k + b + i);
-      const float w = expf(-0.6065306597126334f * hy_sigmoid(lin_at(Wd, t, b + i) + w0[b + i]));
-      const float a = hy_sigmoid(lin_at(P, t, off_a + b + i));
-      const float u = k * ik, au = a * u;
-      row[b + i] = r * w;
-      row[HN + b + i] = u;
-      row[2 * HN + b + i] = w;
-      row[3 * HN + b + i] = au;
-      row[4 * HN + b + i] = k;
-      row[5 * HN + b + i] = lin_at(P, t, off_v + b + i);
-      s_ra = fmaf(r, au, s_ra);
-      s_rk = fmaf(r, k, s_rk);
+    for (int base = 0; base < n; base += 64) {
+      int col[8], cw[2];
+      float v[8], z[2];
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        const int i = base + lane + 32 * c;
+        const bool in = i < n;
+        col[c] = in ? off_r + b + i : -1;
+        col[2 + c] = in ? off_k + b + i : -1;
+        col[4 + c] = in ? off_a + b + i : -1;
+        col[6 + c] = in ? off_v + b + i : -1;
+        cw[c] = in ? b + i : -1;
+      }
+      lin_at_cols<8, 4>(P, t, col, v);
+      lin_at_cols<2, 4>(Wd, t, cw, z);
+      if (base == 0) {
+        float first = v[2] * v[2];
+        first = fmaf(v[3], v[3], first);
+        ik = 1.0f / sqrtf(warp_sum(first + sk) + 1e-6f);
+      }
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        const int i = base + lane + 32 * c;
+        if (i >= n) break;
+        const float r = v[c], k = v[2 + c];
+        const float w = expf(-0.6065306597126334f * hy_sigmoid(z[c] + w0[b + i]));
+        const float a = hy_sigmoid(v[4 + c]);
+        const float u = k * ik, au = a * u;
+        row[b + i] = r * w;
+        row[HN + b + i] = u;
+        row[2 * HN + b + i] = w;
+        row[3 * HN + b + i] = au;
+        row[4 * HN + b + i] = k;
+        row[5 * HN + b + i] = v[6 + c];
+        s_ra = fmaf(r, au, s_ra);
+        s_rk = fmaf(r, k, s_rk);
+      }
     }
     s_ra = warp_sum(s_ra);
     s_rk = warp_sum(s_rk);

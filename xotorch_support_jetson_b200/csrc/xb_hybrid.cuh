@@ -1620,7 +1620,7 @@ static int hy_sublayer_input(xb_engine* e, int T, int n_seqs, bool no_span, cons
 static int hy_latent_window(const xb_hybrid_layer& c) { return c.m_window > 0 ? c.m_window : 1 << 30; }
 // Latent attention through hy_latent_attn_mma_kernel.  0: launched; 1: not applicable (shared memory); < 0: -error.  n_splits > 1 leaves
 // the key shares in hy->lat_part.
-template <int WARPS, int DVC, int LOADW, bool EXT>
+template <int WARPS, int DVC, int LOADW, bool EXT, bool FULL>
 static int hy_latent_mma_launch_x(xb_engine* e, const HyLayer& l, const BatchMeta& m, int T, int n_splits, cudaStream_t st) {
   HyModel* hy = e->hy;
   const xb_hybrid_layer& c = l.d;
@@ -1633,20 +1633,22 @@ static int hy_latent_mma_launch_x(xb_engine* e, const HyLayer& l, const BatchMet
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= XB_MAX_DEVICES) return 1;
     if (granted[dev] < smem) {
-      if (cudaFuncSetAttribute(hy_latent_attn_mma_kernel<WARPS, DVC, LOADW, EXT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) != cudaSuccess) return 1;
+      if (cudaFuncSetAttribute(hy_latent_attn_mma_kernel<WARPS, DVC, LOADW, EXT, FULL>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) != cudaSuccess) return 1;
       granted[dev] = 200 * 1024;
     }
   }
   const dim3 grid((NR + 16 * WARPS - 1) / (16 * WARPS), n_splits, (R + DVC - 1) / DVC);
-  if (hy_launch(e, hy_latent_attn_mma_kernel<WARPS, DVC, LOADW, EXT>, grid, dim3(32 * LOADW), smem, st, (const float*)hy->qa, (const bf16*)l.k_pool, m, T, H, W,
+  if (hy_launch(e, hy_latent_attn_mma_kernel<WARPS, DVC, LOADW, EXT, FULL>, grid, dim3(32 * LOADW), smem, st, (const float*)hy->qa, (const bf16*)l.k_pool, m, T, H, W,
                 R, c.m_scale * 1.4426950408889634f, n_splits, hy->lat_part, hy->o, (long long)H * R, hy_latent_window(c)) != 0)
     return -1;
   return 0;
 }
 template <int WARPS, int DVC, int LOADW>
 static int hy_latent_mma_launch(xb_engine* e, const HyLayer& l, const BatchMeta& m, int T, int n_splits, cudaStream_t st) {
-  if (l.d.m_window > 0) return hy_latent_mma_launch_x<WARPS, DVC, LOADW, true>(e, l, m, T, n_splits, st);
-  return hy_latent_mma_launch_x<WARPS, DVC, LOADW, false>(e, l, m, T, n_splits, st);
+  const bool full = l.d.m_kv_rank % DVC == 0;
+  if (l.d.m_window > 0)
+    return full ? hy_latent_mma_launch_x<WARPS, DVC, LOADW, true, true>(e, l, m, T, n_splits, st) : hy_latent_mma_launch_x<WARPS, DVC, LOADW, true, false>(e, l, m, T, n_splits, st);
+  return full ? hy_latent_mma_launch_x<WARPS, DVC, LOADW, false, true>(e, l, m, T, n_splits, st) : hy_latent_mma_launch_x<WARPS, DVC, LOADW, false, false>(e, l, m, T, n_splits, st);
 }
 static int hy_latent_mma(xb_engine* e, const HyLayer& l, const BatchMeta& m, int T, int* n_splits, cudaStream_t st) {
   *n_splits = 1;

@@ -131,17 +131,6 @@ __device__ __forceinline__ void epi_store16(bf16* dst, const float* x) {
   reinterpret_cast<uint4*>(dst)[0] = p0;
   reinterpret_cast<uint4*>(dst)[1] = p1;
 }
-// where 16 elements [e, e+16) of fused-QKV head `head` of token row t go: q buffer or the paged cache
-__device__ __forceinline__ bf16* epi_qkv_dst(const GemmArgs& g, int t, int pos, int head, int e) {
-  const int H = g.n_heads, KV = g.n_kv_heads, hd = g.head_dim;
-  if (head < H) return g.q_out + ((long long)t * H + head) * hd + e;
-  const int slot = g.seq_slot[g.tok_seq[t]];
-  const int page = g.page_table[(long long)slot * g.max_pages + pos / g.page_tokens];
-  const int off = pos % g.page_tokens;
-  const int kvh = (head - H) % KV;
-  bf16* pool = head < H + KV ? g.k_pool : g.v_pool;
-  return pool + (((long long)page * KV + kvh) * g.page_tokens + off) * hd + e;
-}
 
 template <int BN, int STAGES>
 __global__ void __launch_bounds__(224, 1)

@@ -132,8 +132,36 @@ __device__ __forceinline__ void wide_store_plain(const GemmArgs& g, int t, int n
       if (n0 + j < g.b_rows) dst[j] = f2bf(x[j]);
   }
 }
+// What the fused-QKV epilogue needs of a token row beside its sums.  A block of a prompt of a few hundred rows has one tile, so what its epilogue
+// waits for adds to the Linear: the row's place in the cache (three dependent lookups) is found while the products run, the rotation factors of a
+// column pair (32 neighbouring floats) arrive while the pair before is written.  Looked up where they were used, the fused projection of
+// 373 rows x 3072 -> 5120 took 27 us cold, the plain one of 3072 columns 19; seven 3B layers of such a prompt 995 -> 973 us in all.
+struct WideQkvRow {
+  long long kv;       // element offset of (page, head 0, place in the page) in a pool
+  float cs[32];       // (cos, sin) of the pair at hand
+};
+__device__ __forceinline__ long long wide_kv_row(const GemmArgs& g, int t, int pos) {
+  const int slot = g.seq_slot[g.tok_seq[t]], block = pos / g.page_tokens;
+  const int page = g.page_table[(long long)slot * g.max_pages + block];
+  return ((long long)page * g.n_kv_heads * g.page_tokens + (pos - block * g.page_tokens)) * g.head_dim;
+}
+// the factors of the pair whose first column is n0; columns that turn in no head load nothing
+__device__ __forceinline__ void wide_rope_load(const GemmArgs& g, int pos, int n0, float* cs) {
+  const int hd = g.head_dim, head = hd == 128 ? n0 >> 7 : n0 >> 6, e0 = n0 - head * hd;   // head_dim is 64 or 128, a pair lies in one head
+  if (head >= g.n_heads + g.n_kv_heads) return;
+  const float4* src = reinterpret_cast<const float4*>(g.rope + (long long)pos * hd + (g.rope_kind != 0 ? 2 * e0 : e0));
+#pragma unroll
+  for (int i = 0; i < 8; ++i) *reinterpret_cast<float4*>(cs + 4 * i) = src[i];
+}
+// where 16 elements [e, e + 16) of fused-QKV head `head` of token row t go: q buffer or the paged cache
+__device__ __forceinline__ bf16* wide_qkv_dst(const GemmArgs& g, int t, long long kv, int head, int e) {
+  const int H = g.n_heads, KV = g.n_kv_heads, hd = g.head_dim;
+  if (head < H) return g.q_out + ((long long)t * H + head) * hd + e;
+  const bool k = head < H + KV;
+  return (k ? g.k_pool : g.v_pool) + kv + (long long)(head - (k ? H : H + KV)) * g.page_tokens * hd + e;
+}
 // x0 / x1: fp32 sums of the columns n0.. and n1.. of token row t
-__device__ __forceinline__ void wide_emit(const GemmArgs& g, int t, int pos, int n0, int n1, float* x0, float* x1) {
+__device__ __forceinline__ void wide_emit(const GemmArgs& g, int t, const WideQkvRow& r, int n0, int n1, float* x0, float* x1) {
   if (t >= g.a_rows) return;
   if (g.epi == XB_EPI_SILU) {
     // gate/up rows are interleaved in blocks of 16 features: act = bf16(bf16(silu(gate)) * up)
@@ -147,41 +175,37 @@ __device__ __forceinline__ void wide_emit(const GemmArgs& g, int t, int pos, int
   } else if (g.epi == XB_EPI_QKV) {
     if (n0 >= g.b_rows) return;
     const int hd = g.head_dim, half = hd >> 1, turned = g.n_heads + g.n_kv_heads;
-    const float* rope_row = g.rope + (long long)pos * half * 2;
     wide_bias_round(g, n0, x0);
     if (n1 < g.b_rows) wide_bias_round(g, n1, x1);
-    const int h0 = n0 / hd, e0 = n0 - h0 * hd;
+    const int h0 = hd == 128 ? n0 >> 7 : n0 >> 6, e0 = n0 - h0 * hd;
     if (g.rope_kind != 0) {
       if (h0 < turned) {
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
-          const float2 cs = *reinterpret_cast<const float2*>(rope_row + (e0 + j) * 2);
-          const float cc = rbf(cs.x), ss = rbf(cs.y);
+          const float cc = rbf(r.cs[2 * j]), ss = rbf(r.cs[2 * j + 1]);
           const float a = x0[j], b = x1[j];
           x0[j] = __fadd_rn(rbf(__fmul_rn(a, cc)), rbf(__fmul_rn(-b, ss)));
           x1[j] = __fadd_rn(rbf(__fmul_rn(b, cc)), rbf(__fmul_rn(a, ss)));
         }
       }
-      bf16* dst = epi_qkv_dst(g, t, pos, h0, e0);
+      bf16* dst = wide_qkv_dst(g, t, r.kv, h0, e0);
       epi_store16(dst, x0);
       epi_store16(dst + half, x1);
     } else {
 #pragma unroll
       for (int c = 0; c < 2; ++c) {
         float* x = c == 0 ? x0 : x1;
-        const int n = c == 0 ? n0 : n1;
-        if (n >= g.b_rows) break;
-        const int head = n / hd, e = n - head * hd;
-        if (head < turned) {
+        const float* cs = r.cs + 16 * c;
+        if ((c == 0 ? n0 : n1) >= g.b_rows) break;
+        if (h0 < turned) {
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
-            const float2 cs = *reinterpret_cast<const float2*>(rope_row + (e / 2 + j) * 2);
             const float a = x[2 * j], b = x[2 * j + 1];
-            x[2 * j] = __fsub_rn(__fmul_rn(a, cs.x), __fmul_rn(b, cs.y));
-            x[2 * j + 1] = __fadd_rn(__fmul_rn(b, cs.x), __fmul_rn(a, cs.y));
+            x[2 * j] = __fsub_rn(__fmul_rn(a, cs[2 * j]), __fmul_rn(b, cs[2 * j + 1]));
+            x[2 * j + 1] = __fadd_rn(__fmul_rn(b, cs[2 * j]), __fmul_rn(a, cs[2 * j + 1]));
           }
         }
-        epi_store16(epi_qkv_dst(g, t, pos, head, e), x);
+        epi_store16(wide_qkv_dst(g, t, r.kv, h0, e0 + 16 * c), x);
       }
     }
   } else {
@@ -326,7 +350,16 @@ xb_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     for (int u = u0; u < n_units; u += u_step) {
       const int ta = (u % a_units) * CG + (CG == 2 ? (int)rank : 0), tb = u / a_units;
       const int t = ta * 128 + row_in_tile;
-      const int pos = g.epi == XB_EPI_QKV && t < g.a_rows ? g.tok_pos[t] : 0;
+      const bool qkv = g.epi == XB_EPI_QKV && t < g.a_rows;
+      const int pos = qkv ? g.tok_pos[t] : 0;
+      WideQkvRow row;
+      row.kv = qkv && tb * BN + BN > g.n_heads * g.head_dim ? wide_kv_row(g, t, pos) : 0;
+      float next[32];
+      if (qkv) {
+        int c0, c1;
+        wide_pair_cols(g, 0, c0, c1);
+        wide_rope_load(g, pos, tb * BN + c0, next);
+      }
       mbar_wait(&tfull_bar[acc], acc_phase);
       tc_fence_after();
       const uint32_t t_addr = lane_base + (uint32_t)(acc * Cfg::ACC_COLS);
@@ -337,8 +370,17 @@ xb_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         uint32_t v0[16], v1[16];
         tmem_ld16(t_addr + c0, v0);
         tmem_ld16(t_addr + c1, v1);
+        if (qkv) {
+#pragma unroll
+          for (int j = 0; j < 32; ++j) row.cs[j] = next[j];
+          if (p + 1 < Cfg::PAIRS) {
+            int d0, d1;
+            wide_pair_cols(g, p + 1, d0, d1);
+            wide_rope_load(g, pos, tb * BN + d0, next);
+          }
+        }
         tmem_ld_wait();
-        wide_emit(g, t, pos, tb * BN + c0, tb * BN + c1, reinterpret_cast<float*>(v0), reinterpret_cast<float*>(v1));
+        wide_emit(g, t, row, tb * BN + c0, tb * BN + c1, reinterpret_cast<float*>(v0), reinterpret_cast<float*>(v1));
       }
       tc_fence_before();
       __syncwarp();

@@ -89,30 +89,75 @@ __global__ void __launch_bounds__(NT) xb_resid_norm_kernel(const float* __restri
                                                            const bf16* __restrict__ nw, bf16* __restrict__ hn, int D,
                                                            float eps, int two_round) {
   pdl_launch_dependents();
-  pdl_wait();
   __shared__ float red[32];
   extern __shared__ float row[];  // D floats: the new residual row
   const int t = blockIdx.x;
+  if (SRC != 0) {
+    // prompts: a row's loads go out together, the norm's weights (which wait for no kernel) before the wait; the sums keep their order.  One load
+    // after the other a block of a few hundred rows took six round trips to memory
+    constexpr int U = 8;
+    uint32_t wv[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int i = (u * NT + threadIdx.x) * 2;
+      wv[u] = nw != nullptr && i < D ? *reinterpret_cast<const uint32_t*>(nw + i) : 0u;
+    }
+    pdl_wait();
+    float ss = 0.f;
+    for (int i0 = 0; i0 < D; i0 += U * NT * 2) {
+      uint32_t hw[U], yw[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int i = i0 + (u * NT + threadIdx.x) * 2;
+        const long long o = (long long)t * D + i;
+        hw[u] = i < D ? *reinterpret_cast<const uint32_t*>(h + o) : 0u;
+        yw[u] = SRC == 1 && i < D ? *reinterpret_cast<const uint32_t*>(y + o) : 0u;
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int i = i0 + (u * NT + threadIdx.x) * 2;
+        if (i >= D) break;
+        float2 hv = bf2_to_f2(hw[u]);
+        if (SRC == 1) {
+          const float2 yv = bf2_to_f2(yw[u]);
+          hv.x = rbf(hv.x + yv.x);
+          hv.y = rbf(hv.y + yv.y);
+          *reinterpret_cast<uint32_t*>(h + (long long)t * D + i) = f2_to_bf2(hv.x, hv.y);
+        }
+        row[i] = hv.x;
+        row[i + 1] = hv.y;
+        ss += hv.x * hv.x + hv.y * hv.y;
+      }
+    }
+    if (nw == nullptr) return;
+    ss = block_sum<NT>(ss, red);
+    const float inv = 1.0f / sqrtf(ss / (float)D + eps);
+    for (int i0 = 0; i0 < D; i0 += U * NT * 2) {
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int i = i0 + (u * NT + threadIdx.x) * 2;
+        if (i >= D) break;
+        const float2 w = bf2_to_f2(i0 == 0 ? wv[u] : *reinterpret_cast<const uint32_t*>(nw + i));
+        *reinterpret_cast<uint32_t*>(hn + (long long)t * D + i) = f2_to_bf2(rms_apply(row[i], inv, w.x, two_round), rms_apply(row[i + 1], inv, w.y, two_round));
+      }
+    }
+    return;
+  }
+  pdl_wait();
   float ss = 0.f;
   for (int i = threadIdx.x * 2; i < D; i += NT * 2) {
     const long long o = (long long)t * D + i;
     float2 hv = bf2_to_f2(*reinterpret_cast<const uint32_t*>(h + o));
-    if (SRC == 0) {
-      float a = 0.f, b = 0.f;
-      const int splits = xb_n_segments(si, i);
-      for (int s = 0; s < splits; ++s) {
-        const float2 p = *reinterpret_cast<const float2*>(part + s * split_stride + o);
-        a += p.x;
-        b += p.y;
-      }
-      hv.x = rbf(hv.x + rbf(a));
-      hv.y = rbf(hv.y + rbf(b));
-    } else if (SRC == 1) {
-      const float2 yv = bf2_to_f2(*reinterpret_cast<const uint32_t*>(y + o));
-      hv.x = rbf(hv.x + yv.x);
-      hv.y = rbf(hv.y + yv.y);
+    float a = 0.f, b = 0.f;
+    const int splits = xb_n_segments(si, i);
+    for (int s = 0; s < splits; ++s) {
+      const float2 p = *reinterpret_cast<const float2*>(part + s * split_stride + o);
+      a += p.x;
+      b += p.y;
     }
-    if (SRC != 2) *reinterpret_cast<uint32_t*>(h + o) = f2_to_bf2(hv.x, hv.y);
+    hv.x = rbf(hv.x + rbf(a));
+    hv.y = rbf(hv.y + rbf(b));
+    *reinterpret_cast<uint32_t*>(h + o) = f2_to_bf2(hv.x, hv.y);
     row[i] = hv.x;
     row[i + 1] = hv.y;
     ss += hv.x * hv.x + hv.y * hv.y;

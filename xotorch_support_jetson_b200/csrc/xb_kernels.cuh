@@ -94,7 +94,7 @@ __global__ void __launch_bounds__(NT) xb_resid_norm_kernel(const float* __restri
   const int t = blockIdx.x;
   if (SRC != 0) {
     // prompts: a row's loads go out together, the norm's weights (which wait for no kernel) before the wait; the sums keep their order.  One load
-    // after the other a block of a few hundred rows took six round trips to memory
+    // after the other a block of a few hundred rows took six round trips to memory (373 rows of 3072, fourteen norms: 973 -> 966 us in all)
     constexpr int U = 8;
     uint32_t wv[U];
 #pragma unroll

@@ -6,8 +6,8 @@
 // what bounds it is their issue and the shared-memory reads that feed them.  Half a warp owns two query rows from scores to output.
 // That layer 290 -> 55 us, two float32 layers on a prompt of 300 rows 1196 -> 959.
 //
-// Key tiles start at multiples of 32 positions whatever the queries, and a tile that a query does not see changes none of its sums: a query's
-// result depends on its own position and context alone.  Sequences below `min_len` rows stay with the other kernel: it has a block for every
+// Key tiles start at multiples of 32 positions whatever the queries, and keys that a query does not see change none of its sums, whatever they hold: a
+// query's result depends on its own position and context alone.  Sequences below `min_len` rows stay with the other kernel: it has a block for every
 // (token, head), where 63 rows make 16 to 64 tiles, too few to share out a long context.  The choice is a sequence's own, too.
 #pragma once
 
@@ -90,6 +90,8 @@ __global__ void __launch_bounds__(256) hy_attn_tile_kernel(LinOut P, int off_q, 
 #pragma unroll
     for (int v = 0; v < NV; ++v) acc[u][v] = make_float4(0.f, 0.f, 0.f, 0.f);
   const float* q0 = sQ + hw * 2 * KP;
+  const int newest = (int)__reduce_max_sync(0xffffffffu, (unsigned)(max(pos[0], pos[1]) + 1));   // keys [0, newest) are all that this warp's rows see
+  auto sees = [&](int u, int j) { return j <= pos[u] && (pos[u] - j < a.window || j < a.keep_first); };
   int kt = next(-1), stage = 0;
   fetch(kt, 0);
   while (kt <= last) {
@@ -116,7 +118,7 @@ __global__ void __launch_bounds__(256) hy_attn_tile_kernel(LinOut P, int off_q, 
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         const int j = key + 16 * h;
-        if (j > pos[u] || (pos[u] - j >= a.window && j >= a.keep_first)) sc[u][h] = -INFINITY;
+        if (!sees(u, j)) sc[u][h] = -INFINITY;
       }
       float t = fmaxf(sc[u][0], sc[u][1]);
 #pragma unroll
@@ -134,24 +136,38 @@ __global__ void __launch_bounds__(256) hy_attn_tile_kernel(LinOut P, int off_q, 
       }
     }
     __syncwarp();   // a row's weights are its half-warp's own
-    // ---- weighted values: channels 4 l16 .. of each group of 64
+    // ---- weighted values: channels 4 l16 .. of each group of 64.  In a tile that some row does not see whole, the values of its masked keys enter as 0:
+    // their weights are 0, but 0 x inf and 0 x NaN are not
     const float* vs = (a.v_in_k ? sK : sV) + stage * HY_AT_KEYS * VP + l16 * 4;
     const float* pr = sP + hw * 2 * (HY_AT_KEYS + 4);
+    auto add_values = [&](auto mask) {
+      constexpr bool MASK = decltype(mask)::value;
+      const int n = MASK ? min(HY_AT_KEYS, newest - kt * HY_AT_KEYS) : HY_AT_KEYS;
 #pragma unroll 2
-    for (int j = 0; j < HY_AT_KEYS; j += 4) {
-      const float4 pa = *reinterpret_cast<const float4*>(pr + j), pb = *reinterpret_cast<const float4*>(pr + HY_AT_KEYS + 4 + j);
-      const float pja[4] = {pa.x, pa.y, pa.z, pa.w}, pjb[4] = {pb.x, pb.y, pb.z, pb.w};
+      for (int j = 0; j < n; j += 4) {
+        const float4 pa = *reinterpret_cast<const float4*>(pr + j), pb = *reinterpret_cast<const float4*>(pr + HY_AT_KEYS + 4 + j);
+        const float pja[4] = {pa.x, pa.y, pa.z, pa.w}, pjb[4] = {pb.x, pb.y, pb.z, pb.w};
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+        for (int i = 0; i < 4; ++i) {
+          const bool sa = !MASK || sees(0, kt * HY_AT_KEYS + j + i), sb = !MASK || sees(1, kt * HY_AT_KEYS + j + i);
 #pragma unroll
-        for (int v = 0; v < NV; ++v) {
-          const float4 x = *reinterpret_cast<const float4*>(vs + (j + i) * VP + v * 64);
-          acc[0][v].x = fmaf(pja[i], x.x, acc[0][v].x); acc[0][v].y = fmaf(pja[i], x.y, acc[0][v].y);
-          acc[0][v].z = fmaf(pja[i], x.z, acc[0][v].z); acc[0][v].w = fmaf(pja[i], x.w, acc[0][v].w);
-          acc[1][v].x = fmaf(pjb[i], x.x, acc[1][v].x); acc[1][v].y = fmaf(pjb[i], x.y, acc[1][v].y);
-          acc[1][v].z = fmaf(pjb[i], x.z, acc[1][v].z); acc[1][v].w = fmaf(pjb[i], x.w, acc[1][v].w);
+          for (int v = 0; v < NV; ++v) {
+            const float4 x = *reinterpret_cast<const float4*>(vs + (j + i) * VP + v * 64);
+            const float4 xa = sa ? x : make_float4(0.f, 0.f, 0.f, 0.f), xb = sb ? x : make_float4(0.f, 0.f, 0.f, 0.f);
+            acc[0][v].x = fmaf(pja[i], xa.x, acc[0][v].x); acc[0][v].y = fmaf(pja[i], xa.y, acc[0][v].y);
+            acc[0][v].z = fmaf(pja[i], xa.z, acc[0][v].z); acc[0][v].w = fmaf(pja[i], xa.w, acc[0][v].w);
+            acc[1][v].x = fmaf(pjb[i], xb.x, acc[1][v].x); acc[1][v].y = fmaf(pjb[i], xb.y, acc[1][v].y);
+            acc[1][v].z = fmaf(pjb[i], xb.z, acc[1][v].z); acc[1][v].w = fmaf(pjb[i], xb.w, acc[1][v].w);
+          }
         }
-    }
+      }
+    };
+    const int k_lo = kt * HY_AT_KEYS, k_hi = k_lo + HY_AT_KEYS - 1;
+    bool whole = true;   // every key of the tile is seen by this thread's rows
+#pragma unroll
+    for (int u = 0; u < 2; ++u) whole = whole && (row[u] < 0 || (k_hi <= pos[u] && (pos[u] - k_lo < a.window || k_hi < a.keep_first)));
+    if (__all_sync(0xffffffffu, whole)) add_values(std::false_type());
+    else add_values(std::true_type());
     __syncthreads();   // the stage may be filled again
     kt = kn;
     stage ^= 1;

@@ -1,5 +1,5 @@
-"""A token whose row is not finite spoils the queries that see it and no others: earlier tokens of its prompt and later ones that its window has left
-behind answer as if it were an ordinary one.  Attention of float32 prompts by tiles of queries (hy_attn_tile_kernel) against one block per
+"""A token whose row is not finite spoils the queries that see it and no others: earlier tokens of its prompt, later ones that its window has left
+behind, and other sequences answer as if it were an ordinary one.  Attention of hybrid models by tiles of queries (hy_attn_tile_kernel) and by
 (token, head) (hy_attn_window_kernel)."""
 import pytest
 import torch
@@ -73,3 +73,21 @@ def test_only_the_queries_that_see_it(built_lib, monkeypatch, model, bad):
   assert (a - b)[fine].abs().max() <= 2e-5 * b[fine].abs().max()
   # rows before it: the same bits as without it
   assert torch.equal(a[:bad], rows["1", "plain"][:bad])
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("model", ["window", "latent"])
+def test_another_sequence_in_the_first_row_of_the_pool(built_lib, monkeypatch, model, dtype):
+  """37 keys end inside a round of four: what fills the round up must not be the pool's first row, another sequence's."""
+  monkeypatch.setenv("XB_HY_TC_ATTN", "0")
+  monkeypatch.setenv("XB_HY_LAT_MMA", "0")
+  hf, state = {"window": lambda: _window(3, 70), "latent": _latent}[model]()
+  got = []
+  for bad in ([], [0]):
+    st = _stage(hf, state, dtype)
+    _rows(st, 0, _ids(5, 1, bad))   # pages are handed out from the first on
+    ids = _ids(38, 2)
+    got.append(torch.cat([_rows(st, 1, ids[:37]), _rows(st, 1, ids[37:], 37)]))
+    st.close()
+  assert torch.isfinite(got[0]).all()
+  assert torch.equal(got[0], got[1])

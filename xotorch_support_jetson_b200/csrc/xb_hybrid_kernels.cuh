@@ -1713,6 +1713,8 @@ __host__ __device__ __forceinline__ int hy_warps_for(int keys) {
   const int tiles = keys / 32 + (keys % 32 != 0);
   return tiles <= 4 ? tiles : tiles <= 8 ? 4 : tiles / 2 + (tiles & 1);
 }
+// value row of the keys that fill up a round of four: a row of the pool may be any sequence's, and 0 x inf is NaN
+__device__ __align__(16) float hy_zero_row[512];
 template <typename KT, typename AT, int NACC>
 __global__ void __launch_bounds__(512) hy_attn_window_kernel(LinOut P, int off_q, int off_gate, const KT* __restrict__ k_pool,
                                                              const KT* __restrict__ v_pool, BatchMeta m, int H, int G, int dk, int dv,
@@ -1754,13 +1756,13 @@ __global__ void __launch_bounds__(512) hy_attn_window_kernel(LinOut P, int off_q
   for (int base = warp < work ? warp * 32 : n_vis; base < n_vis; base += work * 32) {
     const int idx = base + lane;
     float sc = -INFINITY;
-    long long prow = 0;
+    const KT* vrow = reinterpret_cast<const KT*>(hy_zero_row);   // this lane's value row
     if (idx < n_vis) {
       const int kp = idx < n_first ? idx : lo + (idx - n_first);
       const long long pg = pages[kp / m.page_tokens];
       const int ip = kp % m.page_tokens;
       const long long krow = (pg * G + g) * m.page_tokens + ip;
-      prow = opt.v_heads == G ? krow : pg * m.page_tokens + ip;   // the value row (shared with the other lanes below)
+      vrow = v_pool + (opt.v_heads == G ? krow : pg * m.page_tokens + ip) * ldv;
       sc = (ldk & 7) == 0 ? hy_dot_row<KT>(q, k_pool + krow * ldk, dk) : hy_dot_row_any<KT>(q, k_pool + krow * ldk, dk);
       if (opt.softcap > 0.f) sc = opt.softcap * tanhf(sc / opt.softcap);
       if (opt.r1 != nullptr) sc -= opt.r1[h] * log1pf(opt.r2[h] * (float)(pos - kp));
@@ -1775,14 +1777,13 @@ __global__ void __launch_bounds__(512) hy_attn_window_kernel(LinOut P, int off_q
     mx = nm;
     const int cnt = n_vis - base < 32 ? n_vis - base : 32;
     if (pairs) {
-      for (int jj = 0; jj < cnt; jj += 4) {   // lanes past cnt hold p = 0 and row 0 of the pool (finite values)
+      for (int jj = 0; jj < cnt; jj += 4) {   // lanes past cnt hold p = 0 and a row of zeros
         float pj[4];
         float2 vv[4][NACC / 2];
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
           pj[u] = __shfl_sync(0xffffffffu, p, jj + u);
-          const long long pr = __shfl_sync(0xffffffffu, prow, jj + u);
-          const KT* vr = v_pool + pr * ldv;
+          const KT* vr = reinterpret_cast<const KT*>(__shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(vrow), jj + u));
 #pragma unroll
           for (int c = 0; c < NACC / 2; ++c) {
             const int d = 2 * (lane + 32 * c);
@@ -1801,8 +1802,7 @@ __global__ void __launch_bounds__(512) hy_attn_window_kernel(LinOut P, int off_q
     } else {
       for (int jj = 0; jj < cnt; ++jj) {
         const float pj = __shfl_sync(0xffffffffu, p, jj);
-        const long long pr = __shfl_sync(0xffffffffu, prow, jj);
-        const KT* vr = v_pool + pr * ldv;
+        const KT* vr = reinterpret_cast<const KT*>(__shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(vrow), jj));
 #pragma unroll
         for (int c = 0; c < NACC; ++c) {
           const int d = lane + 32 * c;

@@ -57,14 +57,14 @@ def _rows(st, slot, ids, pos=0):
 def test_only_the_queries_that_see_it(built_lib, monkeypatch, model, bad):
   hf, state = {"window": lambda: _window(3, 70), "window_one_head": lambda: _window(0, 40, 2, 2), "latent": _latent}[model]()
   rows = {}
-  for tile in ("1", "0"):
+  for tile in ("64", "0"):
     monkeypatch.setenv("XB_HY_ATTN_TILE", tile)
     st = _stage(hf, state)
     rows[tile] = _rows(st, 0, _ids(150, 7, [bad]))
     rows[tile, "plain"] = _rows(st, 1, _ids(150, 7))
     st.close()
-  a, b = rows["1"], rows["0"]
-  assert not torch.equal(rows["1", "plain"], rows["0", "plain"])   # two kernels
+  a, b = rows["64"], rows["0"]
+  assert not torch.equal(rows["64", "plain"], rows["0", "plain"])   # two kernels
   fine = torch.isfinite(b).all(1)
   assert fine[:bad].all() and not fine[bad]
   if model == "latent":
@@ -72,7 +72,7 @@ def test_only_the_queries_that_see_it(built_lib, monkeypatch, model, bad):
   assert torch.equal(torch.isfinite(a).all(1), fine)
   assert (a - b)[fine].abs().max() <= 2e-5 * b[fine].abs().max()
   # rows before it: the same bits as without it
-  assert torch.equal(a[:bad], rows["1", "plain"][:bad])
+  assert torch.equal(a[:bad], rows["64", "plain"][:bad])
 
 
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])

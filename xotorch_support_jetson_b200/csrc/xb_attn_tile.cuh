@@ -1,4 +1,4 @@
-// Softmax attention of float32 prompts by tiles of queries.  Included by xb_hybrid_kernels.cuh.
+// Softmax attention of float32 prompts by tiles of queries.  Included by xb_hybrid_kernels.cuh, ahead of the other kernel.
 //
 // hy_attn_window_kernel gives every (token, query head) a block that reads all of its keys and values: 300 tokens x 32 heads of 64 pull 0.7 GB
 // through L2 and are bound by that (290 us).  Here a block takes 32 query rows of one key head -- 32 / R consecutive tokens of a sequence x
@@ -7,13 +7,26 @@
 // That layer 290 -> 55 us, two float32 layers on a prompt of 300 rows 1196 -> 959.
 //
 // Key tiles start at multiples of 32 positions whatever the queries, and keys that a query does not see change none of its sums, whatever they hold: a
-// query's result depends on its own position and context alone.  Sequences below `min_len` rows stay with the other kernel: it has a block for every
-// (token, head), where 63 rows make 16 to 64 tiles, too few to share out a long context.  The choice is a sequence's own, too.
+// query's result depends on its own position and context alone.  Which sequences go by tiles: hy_at_takes.
 #pragma once
 
 #define HY_AT_ROWS 32
 #define HY_AT_KEYS 32
 #define HY_AT_MIN_LEN 64
+
+// Whether the rows of a sequence (len new ones behind ctx) go by tiles.  A tile walks all keys of its rows by itself, so a sequence takes about as long as
+// its last tile however few it has; the other kernel has a block for every (token, head) and takes as long as there is work.  Both grow with the context,
+// so the line lies at a number of tiles, each counted by the share of the last one's keys that an average one sees: a half without a context, all of them
+// behind a long one.  Tiles against (token, head), us of the kernel: latents of 320 / 256 channels, 16 heads, 64 rows without a context (32 tiles that count
+// 16) 38 against 23, 96 rows (24) 45 against 48, 64 rows behind 256 (29) 97 against 154, behind 4096 985 against 1573; 4 heads behind 4096, 128 rows (16)
+// 999 against 905, 192 rows (24) 1013 against 1357; 32 heads over 8, 64 rows (32) 16 against 24.  Below 64 rows it was not measured, those stay.
+// The choice hangs on the sequence and the layer alone.  from > 1: from so many rows on, whatever the tiles.
+__host__ __device__ __forceinline__ bool hy_at_takes(int len, int ctx, int H, int G, int window, int from) {
+  if (from > 1) return len >= from;
+  const int tq = HY_AT_ROWS / (H / G), seen = ctx < window ? ctx : window;
+  const long long tiles = (long long)((len + tq - 1) / tq) * G;
+  return len >= HY_AT_MIN_LEN && tiles * (2LL * seen + len) > 32LL * (seen + len);
+}
 
 __device__ __forceinline__ void hy_at_copy16(float* dst, const float* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
@@ -25,7 +38,7 @@ struct AttnTile {
   int window, keep_first;
   float scale, out_scale;
   int tiles;                 // blocks of a sequence: grid (sequences x tiles, G)
-  int min_len;
+  int from;                  // see hy_at_takes
 };
 // queries + two stages of keys (and values) + weights; 64 floats behind the last row, which wide value reads may touch
 static size_t hy_at_smem(const AttnTile& a, int nv) {
@@ -42,8 +55,10 @@ __global__ void __launch_bounds__(256) hy_attn_tile_kernel(LinOut P, int off_q, 
   const int R = a.H / a.G, TQ = HY_AT_ROWS / R, dk = a.dk, dv = a.dv, KP = dk + 4, VP = a.v_in_k ? KP : 64 * NV;
   const int s = blockIdx.x / a.tiles, i0 = (blockIdx.x - s * a.tiles) * TQ, g = blockIdx.y;
   const int first = s > 0 ? m.seq_last[s - 1] + 1 : 0, len = m.seq_last[s] + 1 - first;
-  if (len < a.min_len || i0 >= len) return;
-  const int n_tok = min(TQ, len - i0), pos0 = m.tok_pos[first] + i0, pos_last = pos0 + n_tok - 1;
+  if (i0 >= len) return;
+  const int ctx = m.tok_pos[first];
+  if (!hy_at_takes(len, ctx, a.H, a.G, a.window, a.from)) return;
+  const int n_tok = min(TQ, len - i0), pos0 = ctx + i0, pos_last = pos0 + n_tok - 1;
   const int* pages = m.page_table + (long long)m.seq_slot[s] * m.max_pages;
   float* sQ = at_smem;
   float* sK = sQ + HY_AT_ROWS * KP;

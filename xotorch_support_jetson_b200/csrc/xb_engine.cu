@@ -119,7 +119,8 @@ struct xb_engine {
   int ts_cap = 0, ts_next = 0, ts_blocks = 160;
   int meta_T = 0;         // token rows the device metadata currently describes
   int step_len = 0;       // rows of the step's longest sequence
-  int step_min = 0, step_seqs = 0;   // ... of its shortest, and how many there are
+  struct StepSeq { int len, ctx; };
+  std::vector<StepSeq> step_seqs;   // new rows of each, and what its cache held before
   int step_ctx = 0;       // prompts: longest context of the step, its own rows included; steps of single tokens (captured once for every length): no bound
   std::map<long long, GemmPlan> plans;
   xb_counters c{};
@@ -1091,7 +1092,7 @@ static int forward_impl(xb_engine* e, const xb_batch* b, void* out, void* const*
            first ? "first shard needs token ids" : "non-first shard needs a hidden state");
   XB_CHECK(!last || b->n_seqs <= 128, "LM head path supports up to 128 sequences per call");
   // ---- host-side batch bookkeeping
-  int T = 0, max_ctx = 0, max_len = 0, min_len = 1 << 30;
+  int T = 0, max_ctx = 0, max_len = 0;
   bool decode_only = true;
   for (int i = 0; i < b->n_seqs; ++i) {
     const int slot = b->slot_ids[i], ql = b->q_lens[i], pos = b->positions[i];
@@ -1105,7 +1106,6 @@ static int forward_impl(xb_engine* e, const xb_batch* b, void* out, void* const*
     T += ql;
     if (ql != 1) decode_only = false;
     if (ql > max_len) max_len = ql;
-    if (ql < min_len) min_len = ql;
     if (pos + ql > max_ctx) max_ctx = pos + ql;
   }
   XB_CHECK(T <= d.max_batch_tokens, "batch carries %d token rows, engine was created for %d", T, d.max_batch_tokens);
@@ -1197,8 +1197,8 @@ static int forward_impl(xb_engine* e, const xb_batch* b, void* out, void* const*
   e->meta_T = T;
   e->step_ctx = decode_only ? 1 << 30 : max_ctx;
   e->step_len = max_len;
-  e->step_min = min_len;
-  e->step_seqs = b->n_seqs;
+  e->step_seqs.clear();
+  for (int i = 0; i < b->n_seqs; ++i) e->step_seqs.push_back({b->q_lens[i], b->positions[i]});
   XB_CUDA(cudaEventRecord(e->meta_ev[ring], st));
 
   // ---- inputs to fixed addresses

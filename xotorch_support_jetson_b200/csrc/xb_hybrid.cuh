@@ -115,7 +115,7 @@ struct HyModel {
   size_t maxChunk = 0, chunk_entries = 0;          // floats of a chunk over all heads of the largest such layer, chunks it holds
   int use_seg = 1;           // XB_HY_SEG=0: recurrences always as one chain per sequence (A/B); XB_HY_SEG=n >= 64: segments of n tokens
   int seg_len = 0;           // pinned segment length, 0: by the step's shape
-  int use_attn_tile = 1;     // XB_HY_ATTN_TILE=0: attention of float32 prompts one (token, head) per block (A/B)
+  int use_attn_tile = 1;     // XB_HY_ATTN_TILE=0: attention of float32 prompts one (token, head) per block (A/B); n > 1: by tiles from n rows of a sequence on
   int use_quad = 1;          // XB_HY_QUAD=0: row kernels of prompts one channel per thread (A/B)
   int use_tc_attn = 1;       // XB_HY_TC_ATTN=0: attention through the per-token kernel everywhere (A/B)
   int use_tc = 1;            // XB_HY_TC=0: every Linear through the plain kernels (A/B)
@@ -913,7 +913,7 @@ static int hy_create(xb_engine* e, const xb_hybrid_desc& d, const xb_hybrid_laye
     const char* qd = getenv("XB_HY_QUAD");
     if (qd != nullptr && qd[0] == '0') hy->use_quad = 0;
     const char* at = getenv("XB_HY_ATTN_TILE");
-    if (at != nullptr && at[0] == '0') hy->use_attn_tile = 0;
+    if (at != nullptr && (atoi(at) > 0 || at[0] == '0')) hy->use_attn_tile = atoi(at);
     const char* lp = getenv("XB_HY_LPC");
     if (lp != nullptr && (atoi(lp) == 4 || atoi(lp) == 8 || atoi(lp) == 16)) hy->recur_lpc = atoi(lp);
   }
@@ -1208,27 +1208,35 @@ static WindowWarps hy_window_warps(const xb_engine* e, int span, int most) {
   return {asked < n ? asked : n, 1};
 }
 
-// The sequences of a float32 prompt step that have HY_AT_MIN_LEN rows or more through hy_attn_tile_kernel; *left: rows remain for
-// hy_attn_window_kernel (with `below` in its options).  v_pool == nullptr: a value is the head of its key row.  Takes head sizes of whole float4s up to 384 / 256 channels
+// The sequences of a float32 prompt step that hy_at_takes takes through hy_attn_tile_kernel; *left: rows remain for hy_attn_window_kernel, *tiled: how
+// it tells them apart (AttnOpt::tiled).  v_pool == nullptr: a value is the head of its key row.  Takes head sizes of whole float4s up to 384 / 256 channels
 // and up to 32 query heads a key head.
 template <typename KT, typename AT>
 static int hy_attn_tiles(xb_engine* e, const LinOut& P, int off_q, int off_gate, const KT* k_pool, const KT* v_pool, const BatchMeta& m, int H, int G, int dk, int dv,
-                         int window, int keep_first, float scale, float out_scale, AT* out, long long ld_out, cudaStream_t st, bool* left, int* below) {
+                         int window, int keep_first, float scale, float out_scale, AT* out, long long ld_out, cudaStream_t st, bool* left, int* tiled) {
   *left = true;
-  *below = 0;
+  *tiled = 0;
   if constexpr (std::is_same<KT, float>::value) {
-    if (!e->hy->use_attn_tile || e->step_len < HY_AT_MIN_LEN || dk % 4 != 0 || dv % 4 != 0 || dk > 384 || dv > 256 || H / G > HY_AT_ROWS) return 0;
-    AttnTile a{H, G, dk, dv, v_pool == nullptr, window, keep_first, scale, out_scale, 0, HY_AT_MIN_LEN};
+    const int from = e->hy->use_attn_tile;
+    if (from == 0 || e->step_len < (from > 1 ? from : HY_AT_MIN_LEN) || dk % 4 != 0 || dv % 4 != 0 || dk > 384 || dv > 256 || H / G > HY_AT_ROWS) return 0;
+    int longest = 0;
+    bool rest = false;
+    for (const auto& q : e->step_seqs) {
+      if (hy_at_takes(q.len, q.ctx, H, G, window, from)) longest = q.len > longest ? q.len : longest;
+      else rest = true;
+    }
+    if (longest == 0) return 0;
+    AttnTile a{H, G, dk, dv, v_pool == nullptr, window, keep_first, scale, out_scale, 0, from};
     const int TQ = HY_AT_ROWS / (H / G);
-    a.tiles = (e->step_len + TQ - 1) / TQ;
-    const dim3 grid(e->step_seqs * a.tiles, G);
+    a.tiles = (longest + TQ - 1) / TQ;
+    const dim3 grid((unsigned)(e->step_seqs.size() * a.tiles), G);
 #define HY_AT_CASE(NV)                                                                                                                      \
   if (dv <= 64 * NV) {                                                                                                                      \
     const size_t smem = hy_at_smem(a, NV);                                                                                                  \
     XB_SMEM_ATTR_ONCE((hy_attn_tile_kernel<NV, AT>), 227 * 1024);                                                                           \
     XB_TRY(hy_launch(e, hy_attn_tile_kernel<NV, AT>, grid, dim3(256), smem, st, P, off_q, off_gate, k_pool, v_pool, m, a, out, ld_out));     \
-    *left = e->step_min < HY_AT_MIN_LEN;                                                                                                    \
-    *below = HY_AT_MIN_LEN;                                                                                                                 \
+    *left = rest;                                                                                                                           \
+    *tiled = from;                                                                                                                          \
     return 0;                                                                                                                               \
   }
     HY_AT_CASE(1)
@@ -1728,9 +1736,9 @@ static int hy_latent_mixer(xb_engine* e, const HyLayer& l, int T, const LinOut& 
     const LinOut QA = hy_plain(hy->qa, (long long)H * W);
     const int far = hy_latent_window(c);
     bool left;
-    int below;
-    XB_TRY((hy_attn_tiles<KT, float>(e, QA, 0, -1, (const KT*)l.k_pool, (const KT*)nullptr, m, H, 1, W, R, far, 0, c.m_scale, 1.0f, hy->o, (long long)H * R, st, &left, &below)));
-    const AttnOpt lopt{nullptr, 0.f, 1, 0, nullptr, nullptr, 0, ww.own, below};
+    int tiled;
+    XB_TRY((hy_attn_tiles<KT, float>(e, QA, 0, -1, (const KT*)l.k_pool, (const KT*)nullptr, m, H, 1, W, R, far, 0, c.m_scale, 1.0f, hy->o, (long long)H * R, st, &left, &tiled)));
+    const AttnOpt lopt{nullptr, 0.f, 1, 0, nullptr, nullptr, 0, ww.own, tiled};
     if (!left) {
     } else if (R <= 256)
       XB_TRY(hy_launch(e, hy_attn_window_kernel<KT, float, 8>, dim3(T, H), dim3(32 * aw), asm_bytes, st, QA, 0, -1, (const KT*)l.k_pool,
@@ -2484,13 +2492,13 @@ static int hy_run_body_t(xb_engine* e, int T, int n_seqs, int n_tiles, void* con
         const int aw = ww.launch;
         const size_t asm_bytes = (size_t)(((dk + 3) & ~3) + aw * (2 + dv)) * sizeof(float);
         bool left;
-        int below;
+        int tiled;
         XB_TRY((hy_attn_tiles<KT, AT>(e, P, l.off_q, l.off_g, (const KT*)l.k_pool, (const KT*)l.v_pool, m, H, G, dk, dv, c.a_window, c.a_keep_first, c.a_scale, 1.0f,
-                                      a1, (long long)l.n_o, st, &left, &below)));
+                                      a1, (long long)l.n_o, st, &left, &tiled)));
         if (left)
           XB_TRY(hy_launch(e, hy_attn_window_kernel<KT, AT, 8>, dim3(T, H), dim3(32 * aw), asm_bytes, st, P, l.off_q, l.off_g,
                            (const KT*)l.k_pool, (const KT*)l.v_pool, m, H, G, dk, dv, dk, dv, c.a_window, c.a_keep_first, c.a_scale, 1.0f, a1,
-                           (long long)l.n_o, AttnOpt{nullptr, 0.f, G, 0, nullptr, nullptr, 0, ww.own, below}));
+                           (long long)l.n_o, AttnOpt{nullptr, 0.f, G, 0, nullptr, nullptr, 0, ww.own, tiled}));
       }
       const long long ldc = 2LL * Hr * rk + (long long)Hr * rv;
       if (hy->use_quad && T > 64 && (Hr * rk) % 4 == 0 && (Hr * rv) % 4 == 0 && hy_quad(P, l.off_rq) && hy_quad(P, l.off_rf) && hy_quad(P, l.off_rv))

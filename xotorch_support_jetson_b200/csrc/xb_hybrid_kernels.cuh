@@ -1679,6 +1679,8 @@ __global__ void hy_qg_pack_kernel(LinOut P, int off_q, int nq, int off_g, int ng
   out[t * (nq + ng) + i] = f2bf(lin_at(P, t, i < nq ? off_q + i : off_g + (i - nq)));
 }
 
+#include "xb_attn_tile.cuh"
+
 // One block per (token, query head); its warps split the visible keys 32 at a time.  Query i sees key j when j <= i and
 // (i - j < window or j < keep_first): the kept first keys, then the window.  In a 32-key tile a lane scores one key (fp32
 // dot with the query in shared memory), the warp does the online softmax, then lanes own value channels for the weighted
@@ -1696,7 +1698,7 @@ __global__ void hy_qg_pack_kernel(LinOut P, int off_q, int nq, int off_g, int ng
 // r1 / r2 (per head, both or neither): r1[h] * ln(1 + r2[h] * (query position - key position)) is taken off the scaled score.
 // chunk > 0: a query sees only keys of its own chunk of positions, floor(i / chunk) = floor(j / chunk) (keep_first = 0 then).
 // own_warps: a query works with hy_warps_for(its visible keys) warps of its block instead of all of them.
-// below > 0: queries of sequences with fewer rows in this step only (the others went through hy_attn_tile_kernel).
+// tiled > 0: only the queries of sequences that hy_at_takes (with from = tiled) leaves; the others went through hy_attn_tile_kernel.
 struct AttnOpt {
   const float* sink;
   float softcap;
@@ -1706,7 +1708,7 @@ struct AttnOpt {
   const float* r2;
   int chunk;
   int own_warps;
-  int below;
+  int tiled;
 };
 // one warp per 64 keys; up to 128 keys one per tile of 32
 __host__ __device__ __forceinline__ int hy_warps_for(int keys) {
@@ -1725,8 +1727,11 @@ __global__ void __launch_bounds__(512) hy_attn_window_kernel(LinOut P, int off_q
   extern __shared__ __align__(16) float qsm[];
   const int row = blockIdx.x, h = blockIdx.y;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-  const int s = m.tok_seq[row];
-  if (opt.below > 0 && m.seq_last[s] - (s > 0 ? m.seq_last[s - 1] : -1) >= opt.below) return;
+  if (opt.tiled > 0) {
+    const int s = m.tok_seq[row];
+    const int first = s > 0 ? m.seq_last[s - 1] + 1 : 0;
+    if (hy_at_takes(m.seq_last[s] + 1 - first, m.tok_pos[first], H, G, window, opt.tiled)) return;
+  }
   const int dv_full = dv;
   int voff = 0;
   if (opt.v_chunk > 0) {
@@ -1739,7 +1744,7 @@ __global__ void __launch_bounds__(512) hy_attn_window_kernel(LinOut P, int off_q
   for (int i = threadIdx.x; i < dk; i += blockDim.x) q[i] = lin_at(P, row, off_q + h * dk + i) * scale;
   __syncthreads();
   const int g = h / (H / G);
-  const int pos = m.tok_pos[row];
+  const int s = m.tok_seq[row], pos = m.tok_pos[row];
   const int* pages = m.page_table + (long long)m.seq_slot[s] * m.max_pages;
   int lo = pos - window + 1 > 0 ? pos - window + 1 : 0;
   if (opt.chunk > 0 && pos - pos % opt.chunk > lo) lo = pos - pos % opt.chunk;
@@ -3431,7 +3436,6 @@ __global__ void hy_nonfinite_kernel(const bf16* __restrict__ w, long long cols, 
   if (bad) *flag = 1;
 }
 
-#include "xb_attn_tile.cuh"
 #include "xb_hyper.cuh"
 #include "xb_qkv_prep.cuh"
 #include "xb_mlstm.cuh"

@@ -429,10 +429,20 @@ class StageRuntime:
 
   def sample(self, logits: torch.Tensor, temp: float = 0.0, top_k: int = 0, top_p: float = 0.0,
              q: Optional[torch.Tensor] = None, seed: int = 0, out: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """int32 [n] ids of fp32 logits [n, vocab] (xb_sample), with q = Exp(1) noise [n, vocab] or noise counted from seed.  The library reads n * vocab numbers
+    behind each address: a buffer that holds fewer, or anything but what it takes, raises ValueError.  Wider rows are not told apart -- the first n * vocab
+    numbers are sampled as n rows -- so a caller whose rows are padded packs them first."""
     assert logits.dtype == torch.float32 and logits.is_cuda and logits.is_contiguous()
     n = logits.shape[0]
+    need = n * self.vocab
+    if logits.numel() < need:
+      raise ValueError(f"logits {tuple(logits.shape)} are not {n} rows of {self.vocab} numbers")
+    if q is not None and (q.numel() < need or q.dtype != torch.float32 or q.device != logits.device or not q.is_contiguous()):
+      raise ValueError(f"noise {q.dtype} {tuple(q.shape)} on {q.device}: wants contiguous float32 [{n}, {self.vocab}] on {logits.device}")
     if out is None:
       out = torch.empty((n,), dtype=torch.int32, device=self.device)
+    elif out.numel() < n or out.dtype != torch.int32 or out.device != logits.device or not out.is_contiguous():
+      raise ValueError(f"out {out.dtype} {tuple(out.shape)} on {out.device}: wants contiguous int32 [{n}] on {logits.device}")
     stream = torch.cuda.current_stream(self.device).cuda_stream
     _cabi.check(self.lib.xb_sample(self._h, C.c_void_p(logits.data_ptr()), n, float(temp), int(top_k), float(top_p),
                                    C.c_void_p(q.data_ptr()) if q is not None else None, int(seed),

@@ -1948,12 +1948,13 @@ static int hy_run_parallel_t(xb_engine* e, int T, int n_seqs, void* const* taps,
       in.xoff[0] = in.xoff[1] = in.xoff[2] = 0;
       in.beta = in.decay = in.qk = nullptr; in.hdecay = l.hdecay;
       XB_TRY(hy_recur<HY_REC_LIGHTNING>(e, in, hy->state + l.st_rec, SS, hy->o, (long long)l.n_o, m, n_seqs, H, n, dv, T, st));
-      if (T <= 64)
-        XB_TRY(hy_launch(e, hy_all_heads_norm_kernel<AT, 1024>, dim3(T), dim3(1024), 0, st, (const float*)hy->o, (long long)l.n_o,
-                         (const float*)l.head_norm, P, l.off_g, d.norm_eps, a1, (long long)l.n_o, H * dv));
-      else
-        XB_TRY(hy_launch(e, hy_all_heads_norm_kernel<AT, 256>, dim3(T), dim3(256), 0, st, (const float*)hy->o, (long long)l.n_o,
-                         (const float*)l.head_norm, P, l.off_g, d.norm_eps, a1, (long long)l.n_o, H * dv));
+      auto norm = [&](auto kern, int threads) {
+        return hy_launch(e, kern, dim3(T), dim3(threads), 0, st, (const float*)hy->o, (long long)l.n_o, (const float*)l.head_norm, P, l.off_g, d.norm_eps, a1,
+                         (long long)l.n_o, H * dv);
+      };
+      if (T <= 64) XB_TRY(norm(hy_all_heads_norm_kernel<AT, 1024, true>, 1024));
+      else if (P.h == nullptr && P.si.splits > 0) XB_TRY(norm(hy_all_heads_norm_kernel<AT, 256, true>, 256));
+      else XB_TRY(norm(hy_all_heads_norm_kernel<AT, 256, false>, 256));
     }
     XB_TRY(hy_linear<AT>(e, a1, l.n_o, l.w_o, l.t_o, nullptr, T, D, l.n_o, hy->m1, hy->cap_m, st, &y1));
     if (c.ff > 0) XB_TRY(hy_ff_parallel<AT>(e, l, T, hy->ah, st, &y2));

@@ -2653,8 +2653,10 @@ __global__ void __launch_bounds__(128) hy_head_mm_mma_kernel(const float* __rest
 }
 
 // The read-out of all heads normed as ONE vector (RMS over the n entries of a token), weighted and gated by sigmoid:
-// out[t, i] = o[t, i] / rms(o[t, :]) * w[i] * sigmoid(P[t, off_gate + i]).  grid (T), NT threads: 256 for prompts, 1024 in steps of few rows.
-template <typename AT, int NT>
+// out[t, i] = o[t, i] / rms(o[t, :]) * w[i] * sigmoid(P[t, off_gate + i]).  grid (T), NT threads: 1024 up to 64 rows, else 256.
+// PLANES: the planes of two gate columns in flight, ahead of the sum, as the projection of few rows leaves them.  A prompt's one matrix is read column by
+// column: its blocks hide the latency, and the other form's 80 registers instead of 40 cost 18.2 against 14.6 us at 1024 rows x 2048.
+template <typename AT, int NT, bool PLANES>
 __global__ void __launch_bounds__(NT) hy_all_heads_norm_kernel(const float* __restrict__ o, long long ldo, const float* __restrict__ w, LinOut P,
                                                                int off_gate, float eps, AT* __restrict__ out, long long ld_out, int n) {
   pdl_launch_dependents();
@@ -2663,18 +2665,24 @@ __global__ void __launch_bounds__(NT) hy_all_heads_norm_kernel(const float* __re
   const long long t = blockIdx.x;
   const float* p = o + t * ldo;
   float ss = 0.f;
+  if constexpr (!PLANES) {
+    for (int i = threadIdx.x; i < n; i += NT) ss = fmaf(p[i], p[i], ss);
+    const float inv = 1.0f / sqrtf(block_sum<NT>(ss, red) / (float)n + eps);
+    for (int i = threadIdx.x; i < n; i += NT) act_store<AT>(out + t * ld_out + i, p[i] * inv * w[i] * hy_sigmoid(lin_at(P, t, off_gate + i)));
+  } else {
 #pragma unroll 8
-  for (int i = threadIdx.x; i < n; i += NT) ss = fmaf(p[i], p[i], ss);
-  float inv = 0.f;
-  for (int base = 0; base < n; base += 2 * NT) {
-    const int i = base + threadIdx.x, col[2] = {i < n ? off_gate + i : -1, i + NT < n ? off_gate + i + NT : -1};
-    float gz[2];
-    lin_at_cols<2, 8>(P, t, col, gz);
-    if (base == 0) inv = 1.0f / sqrtf(block_sum<NT>(ss, red) / (float)n + eps);
+    for (int i = threadIdx.x; i < n; i += NT) ss = fmaf(p[i], p[i], ss);
+    float inv = 0.f;
+    for (int base = 0; base < n; base += 2 * NT) {
+      const int i = base + threadIdx.x, col[2] = {i < n ? off_gate + i : -1, i + NT < n ? off_gate + i + NT : -1};
+      float gz[2];
+      lin_at_cols<2, 8>(P, t, col, gz);
+      if (base == 0) inv = 1.0f / sqrtf(block_sum<NT>(ss, red) / (float)n + eps);
 #pragma unroll
-    for (int c = 0; c < 2; ++c) {
-      const int j = i + c * NT;
-      if (j < n) act_store<AT>(out + t * ld_out + j, p[j] * inv * w[j] * hy_sigmoid(gz[c]));
+      for (int c = 0; c < 2; ++c) {
+        const int j = i + c * NT;
+        if (j < n) act_store<AT>(out + t * ld_out + j, p[j] * inv * w[j] * hy_sigmoid(gz[c]));
+      }
     }
   }
 }

@@ -1,10 +1,10 @@
 // Softmax attention of float32 prompts by tiles of queries.  Included by xb_hybrid_kernels.cuh, ahead of the other kernel.
 //
 // hy_attn_window_kernel gives every (token, query head) a block that reads all of its keys and values: 300 tokens x 32 heads of 64 pull 0.7 GB
-// through L2 and are bound by that (290 us).  Here a block takes 32 query rows of one key head -- 32 / R consecutive tokens of a sequence x
+// through L2 and are bound by that (268 us).  Here a block takes 32 query rows of one key head -- 32 / R consecutive tokens of a sequence x
 // its R query heads -- against 32 keys at a time from shared memory, so that a key row is read once for 32 queries.  All sums are fp32 FMA:
 // what bounds it is their issue and the shared-memory reads that feed them.  Half a warp owns two query rows from scores to output.
-// That layer 290 -> 55 us, two float32 layers on a prompt of 300 rows 1196 -> 959.
+// That layer 268 -> 49 us with the caches flushed, two float32 layers on a prompt of 300 rows 1196 -> 959 in all.
 //
 // Key tiles start at multiples of 32 positions whatever the queries, and keys that a query does not see change none of its sums, whatever they hold: a
 // query's result depends on its own position and context alone.  Which sequences go by tiles: hy_at_takes.
@@ -105,8 +105,9 @@ __global__ void __launch_bounds__(256) hy_attn_tile_kernel(LinOut P, int off_q, 
 #pragma unroll
     for (int v = 0; v < NV; ++v) acc[u][v] = make_float4(0.f, 0.f, 0.f, 0.f);
   const float* q0 = sQ + hw * 2 * KP;
-  const int newest = (int)__reduce_max_sync(0xffffffffu, (unsigned)(max(pos[0], pos[1]) + 1));   // keys [0, newest) are all that this warp's rows see
-  auto sees = [&](int u, int j) { return j <= pos[u] && (pos[u] - j < a.window || j < a.keep_first); };
+  // oldest and newest position of the warp's rows: tiles that all of them see whole need no mask
+  const int first_pos = __reduce_min_sync(0xffffffffu, min(row[0] < 0 ? 0x7fffffff : pos[0], row[1] < 0 ? 0x7fffffff : pos[1]));
+  const int last_pos = __reduce_max_sync(0xffffffffu, max(pos[0], pos[1]));
   int kt = next(-1), stage = 0;
   fetch(kt, 0);
   while (kt <= last) {
@@ -127,14 +128,22 @@ __global__ void __launch_bounds__(256) hy_attn_tile_kernel(LinOut P, int off_q, 
       sc[1][0] = fmaf(qb.x, ka.x, sc[1][0]); sc[1][0] = fmaf(qb.y, ka.y, sc[1][0]); sc[1][0] = fmaf(qb.z, ka.z, sc[1][0]); sc[1][0] = fmaf(qb.w, ka.w, sc[1][0]);
       sc[1][1] = fmaf(qb.x, kb.x, sc[1][1]); sc[1][1] = fmaf(qb.y, kb.y, sc[1][1]); sc[1][1] = fmaf(qb.z, kb.z, sc[1][1]); sc[1][1] = fmaf(qb.w, kb.w, sc[1][1]);
     }
-    const int key = kt * HY_AT_KEYS + l16;
+    const int k_lo = kt * HY_AT_KEYS, k_hi = k_lo + HY_AT_KEYS - 1;
+    const bool whole = k_hi <= first_pos && (last_pos - k_lo < a.window || k_hi < a.keep_first);
+    uint32_t seen[2] = {0u, 0u};   // else: the keys of the tile that a row sees
+    if (!whole) {
+#pragma unroll
+      for (int u = 0; u < 2; ++u)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int j = k_lo + l16 + 16 * h;
+          const bool sees = j <= pos[u] && (pos[u] - j < a.window || j < a.keep_first);
+          if (!sees) sc[u][h] = -INFINITY;
+          seen[u] |= ((__ballot_sync(0xffffffffu, sees) >> (threadIdx.x & 16)) & 0xffffu) << (16 * h);
+        }
+    }
 #pragma unroll
     for (int u = 0; u < 2; ++u) {
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int j = key + 16 * h;
-        if (!sees(u, j)) sc[u][h] = -INFINITY;
-      }
       float t = fmaxf(sc[u][0], sc[u][1]);
 #pragma unroll
       for (int o = 8; o > 0; o >>= 1) t = fmaxf(t, __shfl_xor_sync(0xffffffffu, t, o));
@@ -157,14 +166,14 @@ __global__ void __launch_bounds__(256) hy_attn_tile_kernel(LinOut P, int off_q, 
     const float* pr = sP + hw * 2 * (HY_AT_KEYS + 4);
     auto add_values = [&](auto mask) {
       constexpr bool MASK = decltype(mask)::value;
-      const int n = MASK ? min(HY_AT_KEYS, newest - kt * HY_AT_KEYS) : HY_AT_KEYS;
-#pragma unroll 2
+      const int n = MASK ? min(HY_AT_KEYS, last_pos + 1 - k_lo) : HY_AT_KEYS;
+#pragma unroll(MASK ? 1 : 2)
       for (int j = 0; j < n; j += 4) {
         const float4 pa = *reinterpret_cast<const float4*>(pr + j), pb = *reinterpret_cast<const float4*>(pr + HY_AT_KEYS + 4 + j);
         const float pja[4] = {pa.x, pa.y, pa.z, pa.w}, pjb[4] = {pb.x, pb.y, pb.z, pb.w};
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          const bool sa = !MASK || sees(0, kt * HY_AT_KEYS + j + i), sb = !MASK || sees(1, kt * HY_AT_KEYS + j + i);
+          const bool sa = !MASK || (seen[0] >> (j + i) & 1), sb = !MASK || (seen[1] >> (j + i) & 1);
 #pragma unroll
           for (int v = 0; v < NV; ++v) {
             const float4 x = *reinterpret_cast<const float4*>(vs + (j + i) * VP + v * 64);
@@ -177,11 +186,7 @@ __global__ void __launch_bounds__(256) hy_attn_tile_kernel(LinOut P, int off_q, 
         }
       }
     };
-    const int k_lo = kt * HY_AT_KEYS, k_hi = k_lo + HY_AT_KEYS - 1;
-    bool whole = true;   // every key of the tile is seen by this thread's rows
-#pragma unroll
-    for (int u = 0; u < 2; ++u) whole = whole && (row[u] < 0 || (k_hi <= pos[u] && (pos[u] - k_lo < a.window || k_hi < a.keep_first)));
-    if (__all_sync(0xffffffffu, whole)) add_values(std::false_type());
+    if (whole) add_values(std::false_type());
     else add_values(std::true_type());
     __syncthreads();   // the stage may be filled again
     kt = kn;

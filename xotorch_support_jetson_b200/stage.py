@@ -444,9 +444,9 @@ class StageRuntime:
     elif out.numel() < n or out.dtype != torch.int32 or out.device != logits.device or not out.is_contiguous():
       raise ValueError(f"out {out.dtype} {tuple(out.shape)} on {out.device}: wants contiguous int32 [{n}] on {logits.device}")
     stream = torch.cuda.current_stream(self.device).cuda_stream
-    _cabi.check(self.lib.xb_sample(self._h, C.c_void_p(logits.data_ptr()), n, float(temp), int(top_k), float(top_p),
-                                   C.c_void_p(q.data_ptr()) if q is not None else None, int(seed),
-                                   C.c_void_p(out.data_ptr()), C.c_void_p(stream)))
+    # (addresses as integers: ctypes converts them for less than a c_void_p made here costs, which pays for the checks above)
+    _cabi.check(self.lib.xb_sample(self._h, logits.data_ptr(), n, float(temp), int(top_k), float(top_p),
+                                   q.data_ptr() if q is not None else None, int(seed), out.data_ptr(), stream))
     return out
 
   def bench_linears(self, T: int, iters: int) -> int:

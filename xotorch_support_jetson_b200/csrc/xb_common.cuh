@@ -256,7 +256,7 @@ __device__ __forceinline__ float lin_at(const LinOut& o, long long row, int col)
 // v[c] = o[row][col[c]] for C columns at once (col[c] < 0: not read, 0), F planes of every column in flight: a kernel of few rows waits for
 // the latency of these loads, one round trip instead of one for every four planes of every column.  The planes of a column add up as
 // (p0 + p1) + (p2 + p3) + ..., the last one to three one by one, whatever C and F: lin_at's order.  A token step of three bibevik-1b layers (8 rows, 36 kernels, 13
-// of them waiting for such reads): 414 -> 366 us with the changes below it in the latent layer's kernels.
+// of them waiting for such reads; 35 since): 414 -> 366 us with what changed in the latent layer's kernels beside it.
 template <int C, int F>
 __device__ __forceinline__ void lin_at_cols(const LinOut& o, long long row, const int (&col)[C], float (&v)[C]) {
   static_assert(F % 4 == 0, "whole groups of four planes");

@@ -903,7 +903,7 @@ static int launch_resid_norm(xb_engine* e, const GemmPlan* gp, int T, const bf16
   return 0;
 }
 
-// kv splits of a decode batch.  Measured on B200 (profiles/attn_sweep.py, Llama-3.1-8B geometry,
+// kv splits of a decode batch.  Measured on B200 (Llama-3.1-8B geometry,
 // ctx 2048): the kernel is fastest when the whole grid is ONE wave of about two blocks per SM --
 // 32 seqs x 8 kv heads unsplit (45 us, 5.96 TB/s) beats any split; 8 seqs want 4 splits, 1 seq 16.
 // More splits only add partial traffic and combine work.

@@ -278,7 +278,7 @@ xb_gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
       }
       if (last_unit) {
         // The block's LAST unit is pure tail: nothing overlaps its epilogue (earlier units drain while the next
-        // unit's MMAs run).  Measured on B200 with per-block timestamps (profiles/gemm_timeline.py): the per-token
+        // unit's MMAs run).  Measured on B200 with per-block timestamps: the per-token
         // strided fp32 stores of the general path take 2.4 us per unit at 32 token rows -- more than the whole gap
         // the weight prefetch of the next Linear can cover (32 separate 512-byte bulk copies, one per lane, were no
         // faster: ~64 ns of issue time each).  All loads of the block have landed and all its MMAs have retired by

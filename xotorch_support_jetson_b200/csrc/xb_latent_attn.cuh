@@ -15,8 +15,8 @@
 // softmax weights entering O += P V as hi + lo bf16 pairs instead of one rounding.
 // Prompts are bound by instruction issue and the latency between them (registers and shared memory leave two warps a scheduler), hence no division or
 // page lookup per 16-byte chunk, no branch between the products, masks only in tiles that need one, a rescale only where a maximum rose, the
-// longest walks first.  Two prompts of 900 rows, 16 heads, cache rows of 320: 321 -> 163 us (by the step that holds it, 1730 -> 1572), numbers
-// unchanged.
+// longest walks first.  Two prompts of 900 rows, 16 heads, cache rows of 320: 321 -> 149 us with the caches flushed, the step that holds it
+// 1730 -> 1572, numbers unchanged.
 #pragma once
 #include "xb_attn_mma.cuh"
 

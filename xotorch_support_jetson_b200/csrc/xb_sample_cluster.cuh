@@ -27,8 +27,8 @@ struct SampleXchg {
 // Top-k from candidates: the row is dealt into buckets (what eight lanes, or a warp, have read); the k-th largest bucket
 // maximum has k elements at or above it, so the elements from there on contain the kept set -- about k + k^2 / (2 buckets) of
 // 128256, 41 for k = 35.  Only these candidates are looked at again: pivot, softmax, nucleus and draw run over them in the first
-// block of the cluster.  Bound by reading the row and by three cluster barriers: 32 x 128256 logits, top-k 35, 26.6 -> 19.9 us a call
-// (what the host needs to enqueue it), against four radix passes over every element.
+// block of the cluster.  Bound by reading the row and by three cluster barriers: 32 x 128256 logits, top-k 35, 20.7 us a call
+// on inputs in turn (19.9 the kernel alone, caches flushed), against four radix passes over every element.
 // The radix passes keep what they are better at; device time of 32 rows, 128256 / 32768 entries, us.  k = 35: 15 / 13 with the usual 41 candidates,
 // radix 27 / 15.  Candidates are ranked all against all: 26 / 24 for 250, 43 / 40 for 500; handed on to the radix passes 32 / 20 for 300, 33 / 21 for 500.
 // From k = 65 on 512 bucket maxima are ranked too: 40 / 37 for k = 200, radix 27 / 15.  A nucleus costs the radix passes four more, over mass: 57 / 41 for k = 257,

@@ -4,8 +4,12 @@
 //
 // Same pipeline as the decode Linear (xb_gemm.cuh): one thread feeds each operand by TMA, one issues tcgen05.mma, four warps
 // drain TMEM, persistent over tiles with two accumulators.  What varies is how the tiles cover the chip:
-//   CG = 2  a pair of CTAs works on one 256 x BN tile (cta_group::2): each stages its own 128 token rows and HALF of the
-//           weight rows, 32 KB instead of 48 KB a k-block at BN = 256.
+//   CG = 2  a pair of CTAs works on one tile of 2 RM rows (cta_group::2): each stages its own token rows and HALF of the
+//           weight rows, with 128 rows 32 KB instead of 48 KB a k-block at BN = 256.
+//   RM = 64 pairs on a tile of 128 rows, 64 a CTA.  A k-block takes as long as its operands need into the SM (64 bytes a clock), so what counts is how
+//           many SMs share them: 3072 features of 373 rows are 72 tiles of 128 x 128 on 72 SMs at 32 KB a k-block, or the same 72 tiles on 72 pairs
+//           at 16 KB a CTA.  Back to back, us: 373 rows x 8192 -> 3072 34.7 -> 22.1, x 3072 -> 3072 16.3 -> 12.0, 192 rows x 18944 -> 3584 76.8 -> 42.9;
+//           2048 rows x 8192 -> 3072 93.9 (192 columns) -> 84.4 (256 columns on pairs of 64 rows).
 //   BN      128, 192 or 256 features a tile, by what fills the SMs evenly.
 // Every variant sums K in the same order, k-block by k-block into one accumulator, so a row's numbers depend neither on the tile
 // it falls into nor on what else the step carries: a prompt in portions has the bits of the whole.  (K in two or four parts over a
@@ -13,20 +17,23 @@
 #pragma once
 #include "xb_gemm.cuh"
 
-template <int BN, int CG>
+template <int BN, int CG, int RM>
 struct WideCfg {
+  static_assert(RM == 128 || (RM == 64 && CG == 2), "token rows of a CTA");
   static constexpr int BROWS = BN / CG;                       // weight rows this CTA stages
   static constexpr int BOX = BROWS % 128 == 0 ? 128 : 64;     // rows of one TMA box (divides 128: a box stays in its weight tile)
-  static constexpr int A_BYTES = 128 * 64 * 2;
+  static constexpr int A_BYTES = RM * 64 * 2;
   static constexpr int B_BYTES = BROWS * 64 * 2;
-  static constexpr int KS = BN <= 128 ? 2 : 1;                // k-blocks of one stage: narrow tiles halve the barrier round trips a k-block
+  static constexpr int KS = RM == 64 || BN <= 128 ? 2 : 1;    // k-blocks of a stage: small tiles halve the barrier round trips (192 rows x 8192 -> 3072 28.8 -> 21.1 us; four a stage 21.6)
   static constexpr int STAGES_RAW = (216 * 1024) / (KS * (A_BYTES + B_BYTES));
   static constexpr int STAGES = STAGES_RAW > 8 ? 8 : STAGES_RAW;
   static constexpr int ACC_STAGES = 2;
-  static constexpr int TM_RAW = ACC_STAGES * BN;
+  // A pair with 64 token rows a CTA keeps its rows' lower half of the columns in lanes 0-63 of tensor memory, the upper in lanes 64-127.
+  static constexpr int COLS = RM == 64 ? BN / 2 : BN;         // columns a lane holds
+  static constexpr int TM_RAW = ACC_STAGES * COLS;
   static constexpr int TM_COLS = TM_RAW <= 128 ? 128 : TM_RAW <= 256 ? 256 : 512;
   static constexpr int ACC_COLS = TM_COLS / ACC_STAGES;
-  static constexpr int PAIRS = BN / 32;                       // column pairs (two chunks of 16) of a tile
+  static constexpr int PAIRS = COLS / 32;                       // column pairs (two chunks of 16) a thread drains
   static constexpr int RING_BYTES = STAGES * KS * (A_BYTES + B_BYTES);
   static constexpr int SMEM_BYTES = RING_BYTES + 1024 + 256;
   static_assert(BROWS % BOX == 0, "tile");
@@ -217,10 +224,10 @@ __device__ __forceinline__ void wide_emit(const GemmArgs& g, int t, const WideQk
 // Roles are entered by elect.sync, not by lane == 0, and the two operands have a producer thread each: one thread doing
 // everything under `lane == 0` spent 0.35 us a k-block whatever the tile (a 128 x 64 tile took as long as 128 x 256), most of
 // it issuing.  4096^3, CUDA events: 256x256 pair 103 -> 94 us, 128x256 107 -> 103, 128x128 166 -> 116, 128x64 306 -> 202.
-template <int BN, int CG>
+template <int BN, int CG, int RM>
 __global__ void __launch_bounds__(224, 1)
 xb_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, GemmArgs g) {
-  using Cfg = WideCfg<BN, CG>;
+  using Cfg = WideCfg<BN, CG, RM>;
   constexpr int STAGES = Cfg::STAGES, KS = Cfg::KS;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -235,7 +242,8 @@ xb_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const uint32_t rank = CG > 1 ? cluster_rank() : 0;
-  const int a_units = (g.a_tiles + CG - 1) / CG;
+  constexpr int ROWS = RM * CG;                         // token rows of a tile
+  const int a_units = (g.a_rows + ROWS - 1) / ROWS;
   const int n_units = a_units * g.b_tiles;
   const int u0 = blockIdx.x / CG, u_step = gridDim.x / CG;
 
@@ -281,7 +289,7 @@ xb_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       };
       if (warp == 6) pdl_wait();   // weights never depend on the preceding kernel: their boxes go out at once
       for (int u = u0; u < n_units; u += u_step) {
-        const int ta = (u % a_units) * CG + (CG == 2 ? (int)rank : 0), tb = u / a_units;
+        const int t0 = (u % a_units) * ROWS + (CG == 2 ? (int)rank * RM : 0), tb = u / a_units;
         for (int kb = 0; kb < g.k_blocks; kb += KS) {
           const int nk = KS == 1 || kb + 1 == g.k_blocks ? 1 : KS;
           mbar_wait(&empty_bar[stage], phase ^ 1);
@@ -289,7 +297,7 @@ xb_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             expect(nk * Cfg::A_BYTES);
 #pragma unroll
             for (int q = 0; q < KS; ++q)
-              if (q < nk) load(sA + (stage * KS + q) * Cfg::A_BYTES, &tmA, (kb + q) * 64, ta * 128);
+              if (q < nk) load(sA + (stage * KS + q) * Cfg::A_BYTES, &tmA, (kb + q) * 64, t0);
           } else {
             expect(nk * Cfg::B_BYTES);
 #pragma unroll
@@ -312,7 +320,7 @@ xb_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   } else if (warp == 1) {
     // ===================== MMA issuer (one elected thread, of a pair: of its first CTA) =====================
     if ((CG == 1 || rank == 0) && elect_one()) {
-      constexpr uint32_t idesc = (umma_idesc_bf16(BN) & ~(0x1fu << 24)) | ((uint32_t)(128 * CG >> 4) << 24);
+      constexpr uint32_t idesc = (umma_idesc_bf16(BN) & ~(0x1fu << 24)) | ((uint32_t)(ROWS >> 4) << 24);
       int stage = 0, acc = 0;
       uint32_t phase = 0, acc_phase = 0;
       const uint64_t desc_a0 = umma_desc_sw128(smem_u32(sA)), desc_b0 = umma_desc_sw128(smem_u32(sB));
@@ -342,23 +350,24 @@ xb_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   } else {
     // ===================== epilogue warps 2..5 =====================
     const int quad = warp & 3;
-    const int row_in_tile = quad * 32 + lane;
+    const int row_in_tile = RM == 64 ? (quad & 1) * 32 + lane : quad * 32 + lane;
+    const int col0 = RM == 64 ? (quad >> 1) * Cfg::COLS : 0;
     const uint32_t lane_base = tmem_base + ((uint32_t)(quad * 32) << 16);
     pdl_wait();                                       // `out` may still be read by the upstream grid
     int acc = 0;
     uint32_t acc_phase = 0;
     for (int u = u0; u < n_units; u += u_step) {
-      const int ta = (u % a_units) * CG + (CG == 2 ? (int)rank : 0), tb = u / a_units;
-      const int t = ta * 128 + row_in_tile;
+      const int tb = u / a_units, n0 = tb * BN + col0;
+      const int t = (u % a_units) * ROWS + (CG == 2 ? (int)rank * RM : 0) + row_in_tile;
       const bool qkv = g.epi == XB_EPI_QKV && t < g.a_rows;
       const int pos = qkv ? g.tok_pos[t] : 0;
       WideQkvRow row;
-      row.kv = qkv && tb * BN + BN > g.n_heads * g.head_dim ? wide_kv_row(g, t, pos) : 0;
+      row.kv = qkv && n0 + Cfg::COLS > g.n_heads * g.head_dim ? wide_kv_row(g, t, pos) : 0;
       float next[32];
       if (qkv) {
         int c0, c1;
         wide_pair_cols(g, 0, c0, c1);
-        wide_rope_load(g, pos, tb * BN + c0, next);
+        wide_rope_load(g, pos, n0 + c0, next);
       }
       mbar_wait(&tfull_bar[acc], acc_phase);
       tc_fence_after();
@@ -376,11 +385,11 @@ xb_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           if (p + 1 < Cfg::PAIRS) {
             int d0, d1;
             wide_pair_cols(g, p + 1, d0, d1);
-            wide_rope_load(g, pos, tb * BN + d0, next);
+            wide_rope_load(g, pos, n0 + d0, next);
           }
         }
         tmem_ld_wait();
-        wide_emit(g, t, row, tb * BN + c0, tb * BN + c1, reinterpret_cast<float*>(v0), reinterpret_cast<float*>(v1));
+        wide_emit(g, t, row, n0 + c0, n0 + c1, reinterpret_cast<float*>(v0), reinterpret_cast<float*>(v1));
       }
       tc_fence_before();
       __syncwarp();
@@ -403,19 +412,20 @@ xb_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 
 // ----------------------------------------------------------------------------- host side
 struct WideVariant {
-  int bn, cg;
+  int bn, cg, rm, cols;          // cols: columns a thread of the epilogue holds
+  double us_k_block, us_ends;    // estimated time (xb_pick_wide)
   int (*run)(const CUtensorMap&, const CUtensorMap&, const GemmArgs&, int grid, cudaStream_t, int pdl);
 };
 
-template <int BN, int CG>
+template <int BN, int CG, int RM>
 static int xb_wide_launch_t(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmArgs& g, int grid, cudaStream_t st, int pdl) {
-  using Cfg = WideCfg<BN, CG>;
+  using Cfg = WideCfg<BN, CG, RM>;
   {
     static bool done[XB_MAX_DEVICES] = {false};
     int dev = 0;
     XB_CUDA(cudaGetDevice(&dev));
     if (dev < 0 || dev >= XB_MAX_DEVICES || !done[dev]) {
-      XB_CUDA(cudaFuncSetAttribute(xb_wide_kernel<BN, CG>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES));
+      XB_CUDA(cudaFuncSetAttribute(xb_wide_kernel<BN, CG, RM>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES));
       if (dev >= 0 && dev < XB_MAX_DEVICES) done[dev] = true;
     }
   }
@@ -440,34 +450,34 @@ static int xb_wide_launch_t(const CUtensorMap& tmA, const CUtensorMap& tmB, cons
   }
   cfg.attrs = attr;
   cfg.numAttrs = na;
-  XB_CUDA(cudaLaunchKernelEx(&cfg, xb_wide_kernel<BN, CG>, tmA, tmB, g));
+  XB_CUDA(cudaLaunchKernelEx(&cfg, xb_wide_kernel<BN, CG, RM>, tmA, tmB, g));
   return 0;
 }
 
-#define XB_WIDE_VARIANT(BN, CG) {BN, CG, xb_wide_launch_t<BN, CG>}
+#define XB_WIDE_VARIANT(BN, CG, RM, KB, ENDS) {BN, CG, RM, WideCfg<BN, CG, RM>::COLS, KB, ENDS, xb_wide_launch_t<BN, CG, RM>}
 static const WideVariant g_wide_variants[] = {
-  XB_WIDE_VARIANT(256, 2), XB_WIDE_VARIANT(256, 1), XB_WIDE_VARIANT(192, 1), XB_WIDE_VARIANT(128, 1),
+  XB_WIDE_VARIANT(256, 2, 128, 0.35, 5.3), XB_WIDE_VARIANT(256, 1, 128, 0.385, 6.0), XB_WIDE_VARIANT(192, 1, 128, 0.33, 3.4),
+  XB_WIDE_VARIANT(128, 1, 128, 0.256, 1.1), XB_WIDE_VARIANT(256, 2, 64, 0.23, 1.6), XB_WIDE_VARIANT(128, 2, 64, 0.166, 1.8),
 };
 #undef XB_WIDE_VARIANT
 enum { XB_WIDE_VARIANTS = sizeof(g_wide_variants) / sizeof(g_wide_variants[0]) };
 
-// The variant with the least estimated time: waves x (k-blocks x time of one) + epilogue.  The times (us) are fitted to a sweep of T =
-// 192 .. 4096 over the Linears of the registered models (K 2048 .. 18944, N 2048 .. 37888).
-// What the variants are for, us cold, old 128 x 256 tiling -> choice: T 733, 4096 x 14336: 96 -> 87 (192 columns); T 4096, 28672 x
-// 4096: 664 -> 644 (pairs).
-// col_unit: columns that have to stay together in a tile (a head where the rotation pairs its halves).
+// The variant with the least estimated time: waves x (k-blocks x time of one) + the ends.  The times (us) are fitted to a sweep of T = 150 .. 2048 over 14
+// Linears of the registered models (K 2048 .. 18944, N 2048 .. 37888; back to back, weights from HBM): over the 126 shapes the choice is 0.3 % slower than
+// the best variant on average, 13 % at most.  Without the pairs of 64 rows it was 18 % and 79 %.
+// col_unit: columns that one thread has to hold together (a head where the rotation pairs its halves).
 static int xb_pick_wide(int T, int N, int K, int col_unit, int num_sms) {
   int best = 1;
   double best_t = 1e30;
-  const int a_tiles = (T + 127) / 128, k_blocks = (K + 63) / 64;
+  const int k_blocks = (K + 63) / 64;
   for (int i = 0; i < XB_WIDE_VARIANTS; ++i) {
     const WideVariant& v = g_wide_variants[i];
-    if (v.bn % col_unit != 0) continue;
-    const long long units = (long long)((a_tiles + v.cg - 1) / v.cg) * ((N + v.bn - 1) / v.bn);
+    if (v.cols % col_unit != 0) continue;
+    const int rows = v.rm * v.cg;
+    const long long units = (long long)((T + rows - 1) / rows) * ((N + v.bn - 1) / v.bn);
     const int slots = num_sms / v.cg;
     const long long waves = (units + slots - 1) / slots;
-    const double kb = v.cg == 2 ? 0.36 : v.bn == 256 ? 0.40 : v.bn == 192 ? 0.31 : 0.26;
-    const double t = (double)waves * k_blocks * kb + v.bn * 0.02;
+    const double t = (double)waves * k_blocks * v.us_k_block + v.us_ends;
     if (t < best_t) { best_t = t; best = i; }
   }
   return best;
@@ -478,7 +488,7 @@ static int xb_wide_plan(GemmPlan* p, const bf16* x, long long ldx, const bf16* w
   int vi = force_variant > 0 ? force_variant - 1 : xb_pick_wide(T, N, K, col_unit, num_sms);
   const char* ev = getenv("XB_WIDE_VARIANT");   // pins the variant (from 1) where it does not cut a column unit (tests, A/B)
   const int pin = ev != nullptr ? atoi(ev) : 0;
-  if (force_variant == 0 && pin >= 1 && pin <= XB_WIDE_VARIANTS && g_wide_variants[pin - 1].bn % col_unit == 0) vi = pin - 1;
+  if (force_variant == 0 && pin >= 1 && pin <= XB_WIDE_VARIANTS && g_wide_variants[pin - 1].cols % col_unit == 0) vi = pin - 1;
   XB_CHECK(vi < XB_WIDE_VARIANTS, "wide Linear variant %d of %d", vi + 1, (int)XB_WIDE_VARIANTS);
   const WideVariant& v = g_wide_variants[vi];
   GemmArgs& g = p->args;
@@ -488,11 +498,11 @@ static int xb_wide_plan(GemmPlan* p, const bf16* x, long long ldx, const bf16* w
   g.b_tiles = (N + v.bn - 1) / v.bn;
   g.a_rows = T;
   g.b_rows = N;
-  const int units = (g.a_tiles + v.cg - 1) / v.cg * g.b_tiles;
+  const int rows = v.rm * v.cg, units = (T + rows - 1) / rows * g.b_tiles;
   p->grid = (units < num_sms / v.cg ? units : num_sms / v.cg) * v.cg;
   const int box = (v.bn / v.cg) % 128 == 0 ? 128 : 64;
   const long long w_tiles = (N + 127) / 128;
-  XB_TRY(xb_make_tmap(&p->tmA, x, T, K, ldx, 128));
+  XB_TRY(xb_make_tmap(&p->tmA, x, T, K, ldx, v.rm));
   if (w_tiled) XB_TRY(xb_make_tmap(&p->tmB, w, w_tiles * g.k_blocks * 128, 64, 64, box));
   else XB_TRY(xb_make_tmap(&p->tmB, w, N, K, K, box));
   p->tmC = p->tmA;

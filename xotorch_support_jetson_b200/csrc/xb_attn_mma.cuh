@@ -313,11 +313,11 @@ __global__ void __launch_bounds__(160) xb_attn_decode_mma_kernel(
       }
     }
   } else {
-    pdl_wait();   // compute warps: q (or the projection's partial planes), and the newest K/V row
-
     constexpr int KS = HD / 16, DT = HD / 8;
     if (FUSED) {
-      // ---- finish q of this head group (every split needs it) and, where the newest tile lives, the k / v row
+      // ---- finish q of this head group (every split needs it) and, where the newest tile lives, the k / v row.  What waits for no kernel (the row's
+      // place in the cache, rotation factors, biases, plane counts of a thread's first item) is fetched ahead of the wait: 0.5 us less at one
+      // token of llama-3.2-1b.
       const int heads = H + 2 * KV, half = HD >> 1;
       const long long base = (long long)t * heads * HD;
       const float* rope_row = f.rope + (long long)pos * half * 2;
@@ -326,15 +326,20 @@ __global__ void __launch_bounds__(160) xb_attn_decode_mma_kernel(
       const int n_items = (G + (owns_last ? 2 : 0)) * iph;
       const int page = pt[pos / m.page_tokens], off = pos % m.page_tokens;
       const long long grow = (((long long)page * KV + kvh) * m.page_tokens + off) * HD;
+      auto head_of = [&](int hsel) { return hsel < G ? kvh * G + hsel : hsel == G ? H + kvh : H + KV + kvh; };
+      auto pre = [&](int it) {
+        const int head = head_of(it / iph);
+        return qkv_pre(f.si, head, (it % iph) * 4, HD, head < H + KV, f.bias, rope_row, f.rope_kind);
+      };
+      QkvPre r = pre(threadIdx.x < n_items ? threadIdx.x : 0);
+      pdl_wait();   // the projection's partial planes
       for (int it = threadIdx.x; it < n_items; it += 128) {
-        const int hsel = it / iph, c = (it % iph) * 4;
-        int head;
-        bf16 *sdst, *gdst = nullptr;
-        if (hsel < G) { head = kvh * G + hsel; sdst = sQ + hsel * HD; }
-        else if (hsel == G) { head = H + kvh; sdst = sKrow; gdst = f.k_pool + grow; }
-        else { head = H + KV + kvh; sdst = sVrow; gdst = f.v_pool + grow; }
+        if (it != threadIdx.x) r = pre(it);
+        const int hsel = it / iph, c = (it % iph) * 4, head = head_of(hsel);
+        bf16* sdst = hsel < G ? sQ + hsel * HD : hsel == G ? sKrow : sVrow;
+        bf16* gdst = hsel < G ? nullptr : (hsel == G ? f.k_pool : f.v_pool) + grow;
         float x[4], y[4];
-        qkv_item(f.part, f.si, f.split_stride, base, head, c, HD, head < H + KV, f.bias, rope_row, f.rope_kind, x, y);
+        qkv_item(r, f.part, f.split_stride, base, head, c, HD, head < H + KV, f.bias != nullptr, f.rope_kind, x, y);
         qkv_store4(sdst + c, x);
         if (gdst != nullptr) qkv_store4(gdst + c, x);        // KVCache.update: later steps read it from the pool
         if (f.rope_kind != 0) {
@@ -343,6 +348,8 @@ __global__ void __launch_bounds__(160) xb_attn_decode_mma_kernel(
         }
       }
       named_bar_sync(1, 128);
+    } else {
+      pdl_wait();   // q and the newest K/V row
     }
 
     // ===================== 4 compute warps: each takes 16 keys of every tile =====================

@@ -888,11 +888,16 @@ static int launch_resid_norm(xb_engine* e, const GemmPlan* gp, int T, const bf16
   if (gp->args.mode == XB_GEMM_SKINNY) {
     // decode-sized batches: one 1024-thread block per row
     if (d.dim % 4 == 0 && d.dim <= 1024 * 4 * 2) {
-      if (d.dim <= 1024 * 4)
-        return launch_k(e, xb_resid_norm_row_kernel<1024, 1>, dim3(T), dim3(1024), 0, st, 1, (const float*)e->gemm_out, gp->split,
-                        (long long)T * d.dim, e->h, nw, e->hn, d.dim, d.norm_eps, d.rmsnorm_two_round);
-      return launch_k(e, xb_resid_norm_row_kernel<1024, 2>, dim3(T), dim3(1024), 0, st, 1, (const float*)e->gemm_out, gp->split,
-                      (long long)T * d.dim, e->h, nw, e->hn, d.dim, d.norm_eps, d.rmsnorm_two_round);
+      // As many threads as a row has groups of four columns: the warps left out would add zeros.
+#define XB_RN_CASE(NT, VPT, F)                                                                                                                        \
+  if (d.dim <= NT * VPT * 4)                                                                                                                          \
+    return launch_k(e, xb_resid_norm_row_kernel<NT, VPT, F>, dim3(T), dim3(NT), 0, st, 1, (const float*)e->gemm_out, gp->split, (long long)T * d.dim, \
+                    e->h, nw, e->hn, d.dim, d.norm_eps, d.rmsnorm_two_round);
+      XB_RN_CASE(512, 1, 12)
+      XB_RN_CASE(768, 1, 8)
+      XB_RN_CASE(1024, 1, 6)
+      XB_RN_CASE(1024, 2, 4)
+#undef XB_RN_CASE
     }
     XB_TRY(launch_k(e, xb_resid_norm_kernel<256, 0>, dim3(T), dim3(256), smem, st, 1, (const float*)e->gemm_out, gp->split, (long long)T * d.dim,
                                                         nullptr, e->h, nw, e->hn, d.dim, d.norm_eps, d.rmsnorm_two_round));

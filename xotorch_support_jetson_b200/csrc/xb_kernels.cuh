@@ -173,7 +173,7 @@ __global__ void __launch_bounds__(NT) xb_resid_norm_kernel(const float* __restri
 }
 
 // Decode variant: one 1024-thread block per token row, 4 consecutive columns per thread (float4
-// reads of the split-K planes, all planes' loads issued before the adds), row sum of squares by
+// reads of the split-K planes), row sum of squares by
 // shuffle + one shared-memory round.  Same arithmetic and rounding points as
 // xb_resid_norm_kernel<., 0>; planes are summed in plane order.  (An 8-block cluster per row with a
 // DSMEM exchange measured 5.7-6.0 us per launch at T <= 32: cluster scheduling and the cluster
@@ -185,16 +185,19 @@ __global__ void __launch_bounds__(NT) xb_resid_norm_kernel(const float* __restri
 __device__ __forceinline__ float row_ss4(const float* v) { return v[0] * v[0] + v[1] * v[1] + v[2] * v[2] + v[3] * v[3]; }
 
 template <int NT, int VPT>
-__device__ __forceinline__ void row_norm_store(const float (&v)[VPT][4], float ss, const bf16* __restrict__ nw, bf16* __restrict__ hn_row,
+__device__ __forceinline__ void row_norm_store(const float (&v)[VPT][4], float ss, const uint2 (&wv)[VPT], bf16* __restrict__ hn_row,
                                                int D, float eps, int two_round, float* red) {
-  ss = block_sum<NT>(ss, red);
+  // block_sum's order with one barrier: every warp adds up the warps' sums itself (`red` is used once)
+  ss = warp_sum(ss);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss;
+  __syncthreads();
+  ss = warp_sum((threadIdx.x & 31) < NT / 32 ? red[threadIdx.x & 31] : 0.f);
   const float inv = 1.0f / sqrtf(ss / (float)D + eps);
 #pragma unroll
   for (int it = 0; it < VPT; ++it) {
     const int c = (it * NT + threadIdx.x) * 4;
     if (c < D) {
-      const uint2 wu = *reinterpret_cast<const uint2*>(nw + c);
-      const float2 w0 = bf2_to_f2(wu.x), w1 = bf2_to_f2(wu.y);
+      const float2 w0 = bf2_to_f2(wv[it].x), w1 = bf2_to_f2(wv[it].y);
       uint2 r;
       r.x = f2_to_bf2(rms_apply(v[it][0], inv, w0.x, two_round), rms_apply(v[it][1], inv, w0.y, two_round));
       r.y = f2_to_bf2(rms_apply(v[it][2], inv, w1.x, two_round), rms_apply(v[it][3], inv, w1.y, two_round));
@@ -203,14 +206,26 @@ __device__ __forceinline__ void row_norm_store(const float (&v)[VPT][4], float s
   }
 }
 
+// the norm weights of a thread's columns, which wait for no kernel (nw may be nullptr)
+template <int NT, int VPT>
+__device__ __forceinline__ void row_norm_weights(const bf16* __restrict__ nw, int D, uint2 (&wv)[VPT]) {
+#pragma unroll
+  for (int it = 0; it < VPT; ++it) {
+    const int c = (it * NT + threadIdx.x) * 4;
+    wv[it] = nw != nullptr && c < D ? *reinterpret_cast<const uint2*>(nw + c) : make_uint2(0u, 0u);
+  }
+}
+
 // stage input of a decode step: hn = RMSNorm(h) (h handed in by the caller; NCCL / plugin-API path)
 template <int NT, int VPT>
 __global__ void __launch_bounds__(NT) xb_norm_row_kernel(const bf16* __restrict__ h, const bf16* __restrict__ nw, bf16* __restrict__ hn,
                                                          int D, float eps, int two_round) {
   pdl_launch_dependents();
-  pdl_wait();
   __shared__ float red[32];
   const int t = blockIdx.x;
+  uint2 wv[VPT];
+  row_norm_weights<NT, VPT>(nw, D, wv);
+  pdl_wait();
   float v[VPT][4];
   float ss = 0.f;
 #pragma unroll
@@ -224,38 +239,51 @@ __global__ void __launch_bounds__(NT) xb_norm_row_kernel(const bf16* __restrict_
       ss += row_ss4(v[it]);
     }
   }
-  row_norm_store<NT, VPT>(v, ss, nw, hn + (long long)t * D, D, eps, two_round, red);
+  row_norm_store<NT, VPT>(v, ss, wv, hn + (long long)t * D, D, eps, two_round, red);
 }
 
-template <int NT, int VPT>
-__global__ void __launch_bounds__(NT) xb_resid_norm_row_kernel(const float* __restrict__ part, SplitInfo si,
+// F planes of a column and the residual go out together behind the wait, the norm's weights (which wait for no kernel) and the plane counts ahead of it:
+// one trip to L2 for a row, where planes four at a time, then the residual, then the weights took four or five.  From the exit of the Linear before to the
+// start of the one behind, one row: 6.0 -> 4.1 us at 2048 columns, 6.7 -> 5.0 at 4096 (2.6 of it the two kernel boundaries).  (The bound of one block
+// an SM is what makes the compiler spend registers on loads in flight: without it F = 12 came out in 34 registers, two or three loads at a time.  Not more than
+// 48 K registers a block all the same: the next Linear's block has to find room beside it, or it starts when the norm is done.)
+template <int NT, int VPT, int F>
+__global__ void __launch_bounds__(NT, 1) xb_resid_norm_row_kernel(const float* __restrict__ part, SplitInfo si,
                                                                long long split_stride, bf16* __restrict__ h,
                                                                const bf16* __restrict__ nw, bf16* __restrict__ hn, int D,
                                                                float eps, int two_round) {
   pdl_launch_dependents();
-  pdl_wait();
   __shared__ float red[32];
   const int t = blockIdx.x;
+  uint2 wv[VPT];
+  row_norm_weights<NT, VPT>(nw, D, wv);
+  int planes[VPT];
+#pragma unroll
+  for (int it = 0; it < VPT; ++it) {
+    const int c = (it * NT + threadIdx.x) * 4;
+    planes[it] = c < D ? xb_n_segments(si, c) : 0;
+  }
+  pdl_wait();
   float v[VPT][4];
   float ss = 0.f;
 #pragma unroll
   for (int it = 0; it < VPT; ++it) {
     const int c = (it * NT + threadIdx.x) * 4;
     v[it][0] = v[it][1] = v[it][2] = v[it][3] = 0.f;
-    if (c < D) {
-      const long long o = (long long)t * D + c;
-      const int planes = xb_n_segments(si, c);
-      float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
-      for (int s0 = 0; s0 < planes; s0 += 4) {
-        float4 p[4];
+    const bool in = c < D;
+    const long long o = (long long)t * D + (in ? c : 0);
+    const uint2 hu = *reinterpret_cast<const uint2*>(h + o);
+    float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int s0 = 0; s0 < planes[it]; s0 += F) {
+      float4 p[F];
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
-          p[u] = (s0 + u < planes) ? *reinterpret_cast<const float4*>(part + (s0 + u) * split_stride + o)
-                                   : make_float4(0.f, 0.f, 0.f, 0.f);
+      for (int u = 0; u < F; ++u)
+        p[u] = *reinterpret_cast<const float4*>(part + (s0 + u < planes[it] ? s0 + u : 0) * split_stride + o);
 #pragma unroll
-        for (int u = 0; u < 4; ++u) { a.x += p[u].x; a.y += p[u].y; a.z += p[u].z; a.w += p[u].w; }
-      }
-      const uint2 hu = *reinterpret_cast<const uint2*>(h + o);
+      for (int u = 0; u < F; ++u)
+        if (s0 + u < planes[it]) { a.x += p[u].x; a.y += p[u].y; a.z += p[u].z; a.w += p[u].w; }
+    }
+    if (in) {
       const float2 h0 = bf2_to_f2(hu.x), h1 = bf2_to_f2(hu.y);
       v[it][0] = rbf(h0.x + rbf(a.x));
       v[it][1] = rbf(h0.y + rbf(a.y));
@@ -269,7 +297,7 @@ __global__ void __launch_bounds__(NT) xb_resid_norm_row_kernel(const float* __re
     }
   }
   if (nw == nullptr) return;
-  row_norm_store<NT, VPT>(v, ss, nw, hn + (long long)t * D, D, eps, two_round, red);
+  row_norm_store<NT, VPT>(v, ss, wv, hn + (long long)t * D, D, eps, two_round, red);
 }
 
 // ----------------------------------------------------------------------------- peer hand-off (pipeline, decode)
@@ -350,9 +378,11 @@ __global__ void __launch_bounds__(NT) xb_recv_norm_row_kernel(const bf16* __rest
                                                               bf16* __restrict__ hn, int D, float eps, int two_round,
                                                               long long timeout_cycles, int* __restrict__ err_word) {
   pdl_launch_dependents();
-  pdl_wait();
   __shared__ float red[32];
   const int t = blockIdx.x;
+  uint2 wv[VPT];
+  row_norm_weights<NT, VPT>(nw, D, wv);
+  pdl_wait();
   const int slot = ctl->slot_in;
   const uint32_t want = (uint32_t)ctl->wait_value;
   if (threadIdx.x == 0) {
@@ -385,7 +415,7 @@ __global__ void __launch_bounds__(NT) xb_recv_norm_row_kernel(const bf16* __rest
       ss += row_ss4(v[it]);
     }
   }
-  row_norm_store<NT, VPT>(v, ss, nw, hn + (long long)t * D, D, eps, two_round, red);
+  row_norm_store<NT, VPT>(v, ss, wv, hn + (long long)t * D, D, eps, two_round, red);
 }
 
 // producer tail: split-K reduce + Linear rounding + residual add (the stage's final hidden rows),
@@ -439,17 +469,25 @@ __global__ void __launch_bounds__(NT) xb_resid_send_kernel(const float* __restri
 //     rope_kind 1: half-split pairs (i,i+hd/2), every product and the sum rounded to bf16
 //                  (Qwen2RotaryPositionalEmbeddings, general_mha.py:47-51)
 //   q -> q_out[t][h*hd..]; k,v -> the paged cache (KVCache.update, llm_utils.py:320-345)
-__device__ __forceinline__ void qkv_load4(const float* __restrict__ part, const SplitInfo& si, long long split_stride,
-                                          long long base, int col, const bf16* __restrict__ bias, float* x) {
+// What a work item needs that waits for no kernel: rotation factors, biases, plane counts.
+struct QkvPre {
+  float cs[8];
+  uint2 bias[2];
+  int planes[2];
+};
+// bf16(sum of the planes of four columns + bias), planes added in their order, eight in flight
+__device__ __forceinline__ void qkv_load4(const float* __restrict__ part, int planes, long long split_stride, long long at, bool has_bias, uint2 bias, float* x) {
   float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
-  const int planes = xb_n_segments(si, col);
-  for (int s = 0; s < planes; ++s) {
-    const float4 p = *reinterpret_cast<const float4*>(part + s * split_stride + base + col);
-    a.x += p.x; a.y += p.y; a.z += p.z; a.w += p.w;
+  for (int s0 = 0; s0 < planes; s0 += 8) {
+    float4 p[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      p[u] = s0 + u < planes ? *reinterpret_cast<const float4*>(part + (s0 + u) * split_stride + at) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int u = 0; u < 8; ++u) { a.x += p[u].x; a.y += p[u].y; a.z += p[u].z; a.w += p[u].w; }
   }
-  if (bias != nullptr) {
-    const uint2 bu = *reinterpret_cast<const uint2*>(bias + col);
-    const float2 b0 = bf2_to_f2(bu.x), b1 = bf2_to_f2(bu.y);
+  if (has_bias) {
+    const float2 b0 = bf2_to_f2(bias.x), b1 = bf2_to_f2(bias.y);
     a.x += b0.x; a.y += b0.y; a.z += b1.x; a.w += b1.y;
   }
   x[0] = rbf(a.x); x[1] = rbf(a.y); x[2] = rbf(a.z); x[3] = rbf(a.w);
@@ -459,27 +497,38 @@ __device__ __forceinline__ void qkv_load4(const float* __restrict__ part, const 
 // RoPE: two pairs) or, for half-split RoPE, those 4 plus their partners [half+c, half+c+4).  x (and y) receive the
 // finished bf16-representable values.  Shared by the stand-alone kernel below and by the decode attention kernel,
 // which does this work in its prologue (xb_attn_mma.cuh) -- one arithmetic, bit-identical results.
-__device__ __forceinline__ void qkv_item(const float* __restrict__ part, const SplitInfo& si, long long split_stride,
-                                         long long base, int head, int c, int hd, bool rot, const bf16* __restrict__ bias,
-                                         const float* __restrict__ rope_row, int rope_kind, float* x, float* y) {
+__device__ __forceinline__ QkvPre qkv_pre(const SplitInfo& si, int head, int c, int hd, bool rot, const bf16* __restrict__ bias,
+                                          const float* __restrict__ rope_row, int rope_kind) {
+  QkvPre r;
+  const int cx = head * hd + c, cy = cx + (hd >> 1);
+  if (rot) {   // (cos, sin) of pairs c/2 and c/2 + 1, or of the four pairs c ..
+    *reinterpret_cast<float4*>(r.cs) = *reinterpret_cast<const float4*>(rope_row + (rope_kind == 0 ? c : 2 * c));
+    if (rope_kind != 0) *reinterpret_cast<float4*>(r.cs + 4) = *reinterpret_cast<const float4*>(rope_row + 2 * c + 4);
+  }
+  r.bias[0] = bias != nullptr ? *reinterpret_cast<const uint2*>(bias + cx) : make_uint2(0u, 0u);
+  r.bias[1] = bias != nullptr && rope_kind != 0 ? *reinterpret_cast<const uint2*>(bias + cy) : make_uint2(0u, 0u);
+  r.planes[0] = xb_n_segments(si, cx);
+  r.planes[1] = rope_kind != 0 ? xb_n_segments(si, cy) : 0;
+  return r;
+}
+__device__ __forceinline__ void qkv_item(const QkvPre& r, const float* __restrict__ part, long long split_stride, long long base, int head, int c, int hd,
+                                         bool rot, bool has_bias, int rope_kind, float* x, float* y) {
   const int half = hd >> 1;
-  qkv_load4(part, si, split_stride, base, head * hd + c, bias, x);
+  qkv_load4(part, r.planes[0], split_stride, base + head * hd + c, has_bias, r.bias[0], x);
   if (rope_kind == 0) {
     if (rot) {
-      const float4 cs = *reinterpret_cast<const float4*>(rope_row + c);   // (cos,sin) of pairs c/2, c/2+1
       const float a0 = x[0], b0 = x[1], a1 = x[2], b1 = x[3];
-      x[0] = __fsub_rn(__fmul_rn(a0, cs.x), __fmul_rn(b0, cs.y));
-      x[1] = __fadd_rn(__fmul_rn(b0, cs.x), __fmul_rn(a0, cs.y));
-      x[2] = __fsub_rn(__fmul_rn(a1, cs.z), __fmul_rn(b1, cs.w));
-      x[3] = __fadd_rn(__fmul_rn(b1, cs.z), __fmul_rn(a1, cs.w));
+      x[0] = __fsub_rn(__fmul_rn(a0, r.cs[0]), __fmul_rn(b0, r.cs[1]));
+      x[1] = __fadd_rn(__fmul_rn(b0, r.cs[0]), __fmul_rn(a0, r.cs[1]));
+      x[2] = __fsub_rn(__fmul_rn(a1, r.cs[2]), __fmul_rn(b1, r.cs[3]));
+      x[3] = __fadd_rn(__fmul_rn(b1, r.cs[2]), __fmul_rn(a1, r.cs[3]));
     }
   } else {
-    qkv_load4(part, si, split_stride, base, head * hd + half + c, bias, y);
+    qkv_load4(part, r.planes[1], split_stride, base + head * hd + half + c, has_bias, r.bias[1], y);
     if (rot) {
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        const float2 cs = *reinterpret_cast<const float2*>(rope_row + (c + j) * 2);
-        const float cc = rbf(cs.x), ss = rbf(cs.y);
+        const float cc = rbf(r.cs[2 * j]), ss = rbf(r.cs[2 * j + 1]);
         const float a = x[j], b = y[j];
         x[j] = __fadd_rn(rbf(__fmul_rn(a, cc)), rbf(__fmul_rn(-b, ss)));
         y[j] = __fadd_rn(rbf(__fmul_rn(b, cc)), rbf(__fmul_rn(a, ss)));
@@ -526,7 +575,8 @@ __global__ void __launch_bounds__(256) xb_qkv_finalize_kernel(const float* __res
       dst = pool + (((long long)page * KV + kvh) * m.page_tokens + off) * hd;
     }
     float x[4], y[4];
-    qkv_item(part, si, split_stride, base, head, c, hd, head < H + KV, bias, rope_row, rope_kind, x, y);
+    const bool rot = head < H + KV;
+    qkv_item(qkv_pre(si, head, c, hd, rot, bias, rope_row, rope_kind), part, split_stride, base, head, c, hd, rot, bias != nullptr, rope_kind, x, y);
     qkv_store4(dst + c, x);
     if (rope_kind != 0) qkv_store4(dst + half + c, y);
   }
@@ -537,7 +587,7 @@ __global__ void __launch_bounds__(256) xb_qkv_finalize_kernel(const float* __res
 // are separate bf16 ops in the reference.  Input = split-K partial planes of the fused gate/up
 // projection (decode path; the prefill GEMM does this in its epilogue, xb_gemm.cuh epi_wide_silu).
 // Fused gate/up columns are interleaved in 16-feature blocks; 4 consecutive features per thread.
-__global__ void __launch_bounds__(256) xb_silu_mul_kernel(const float* __restrict__ part, SplitInfo si, long long split_stride,
+__global__ void __launch_bounds__(256, 2) xb_silu_mul_kernel(const float* __restrict__ part, SplitInfo si, long long split_stride,
                                                           bf16* __restrict__ act, int T, int I) {
   pdl_launch_dependents();
   pdl_wait();
@@ -549,11 +599,20 @@ __global__ void __launch_bounds__(256) xb_silu_mul_kernel(const float* __restric
   const long long row = (long long)t * 2 * I;
   const int planes = xb_n_segments(si, cg);                  // cg and cu lie in one 128-column tile
   float4 g = make_float4(0.f, 0.f, 0.f, 0.f), u = g;
-  for (int s = 0; s < planes; ++s) {
-    const float4 pg = *reinterpret_cast<const float4*>(part + s * split_stride + row + cg);
-    const float4 pu = *reinterpret_cast<const float4*>(part + s * split_stride + row + cu);
-    g.x += pg.x; g.y += pg.y; g.z += pg.z; g.w += pg.w;
-    u.x += pu.x; u.y += pu.y; u.z += pu.z; u.w += pu.w;
+  for (int s0 = 0; s0 < planes; s0 += 4) {                   // four planes in flight, added in their order
+    float4 pg[4], pu[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float* p = part + (s0 + j < planes ? s0 + j : 0) * split_stride + row;
+      pg[j] = *reinterpret_cast<const float4*>(p + cg);
+      pu[j] = *reinterpret_cast<const float4*>(p + cu);
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (s0 + j < planes) {
+        g.x += pg[j].x; g.y += pg[j].y; g.z += pg[j].z; g.w += pg[j].w;
+        u.x += pu[j].x; u.y += pu[j].y; u.z += pu[j].z; u.w += pu[j].w;
+      }
   }
   const float gv[4] = {rbf(g.x), rbf(g.y), rbf(g.z), rbf(g.w)};
   const float uv[4] = {rbf(u.x), rbf(u.y), rbf(u.z), rbf(u.w)};

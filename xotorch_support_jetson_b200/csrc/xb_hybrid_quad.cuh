@@ -40,6 +40,11 @@ static bool hy_quad(const LinOut& o, int col) {
   if (o.h != nullptr) return (reinterpret_cast<uintptr_t>(o.h) & 7) == 0;
   return o.f != nullptr && o.si.splits == 0 && (reinterpret_cast<uintptr_t>(o.f) & 15) == 0;
 }
+// the same for split-K planes, each of which starts on 16 bytes
+static bool hy_planes4(const LinOut& o, int col) {
+  if (o.f == nullptr || o.si.splits == 0) return hy_quad(o, col);
+  return o.ld % 4 == 0 && o.plane % 4 == 0 && col % 4 == 0 && (reinterpret_cast<uintptr_t>(o.f) & 15) == 0 && (reinterpret_cast<uintptr_t>(o.bias) & 15) == 0;
+}
 static bool hy_quad_ptr(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
 // hy_taps_tile_kernel with TT = 8 rows and four channels per thread; C, ld_out and tail_stride multiples of four
@@ -285,4 +290,131 @@ __global__ void __launch_bounds__(256) hy_gdelta_prep_quad_kernel(LinOut P, int 
   hy_quad_st(row + 4 * HN, k);
   hy_quad_st(row + 5 * HN, v);
   if (i == 0) { ra[t * H + h] = s_ra; rk[t * H + h] = s_rk; }
+}
+
+// hy_row_op_kernel for steps of few rows: a thread holds four neighbouring channels per VPT from the loads to the stores, so a row costs one trip for
+// planes and stream, two barriers and the stores.  What waits for no kernel (weights, plane counts) is fetched ahead of the wait.  The general kernel
+// reads stream and weights behind its first sum, weights again behind the second, keeps the row in shared memory, and its 1024 threads of 64 registers
+// take a whole SM: the next Linear's block cannot come in beside them and starts its weights when the norm is done.
+// The bound of one block an SM keeps F planes of four channels in flight (see xb_resid_norm_row_kernel).  Eight chats of three bibevik-1b layers (four such
+// kernels a token) 4386 -> 4243 us.
+template <int F>
+__device__ __forceinline__ void lin_planes4(const LinOut& o, long long row, int col, int planes, float* v) {   // lin_at's order of planes
+  float b[4] = {0.f, 0.f, 0.f, 0.f};
+  if (o.bias != nullptr) hy_quad_f(o.bias + col, b);
+  if (o.h != nullptr) {
+    hy_quad_bf(o.h + row * o.ld + col, v);
+  } else {
+    const float* p = o.f + row * o.ld + col;
+    v[0] = v[1] = v[2] = v[3] = 0.f;
+    for (int s0 = 0; s0 < planes; s0 += F) {
+      float w[F][4];
+#pragma unroll
+      for (int u = 0; u < F; ++u) hy_quad_f(p + (s0 + u < planes ? s0 + u : 0) * o.plane, w[u]);
+#pragma unroll
+      for (int u = 0; u < F; u += 4) {
+        if (s0 + u + 3 < planes) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) v[j] += (w[u][j] + w[u + 1][j]) + (w[u + 2][j] + w[u + 3][j]);
+        } else {
+#pragma unroll
+          for (int q = 0; q < 3; ++q)
+            if (s0 + u + q < planes) {
+#pragma unroll
+              for (int j = 0; j < 4; ++j) v[j] += w[u + q][j];
+            }
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < 4; ++j) v[j] += b[j];
+}
+__device__ __forceinline__ int lin_planes(const LinOut& o, int col) {
+  return o.f == nullptr ? 0 : o.si.splits == 0 ? 1 : xb_n_segments(o.si, col);
+}
+template <int NT>
+__device__ __forceinline__ float row_sum_once(float v, float* red) {   // block_sum with one barrier: `red` (32 floats) is used once
+  v = warp_sum(v);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+  __syncthreads();
+  return warp_sum((threadIdx.x & 31) < NT / 32 ? red[threadIdx.x & 31] : 0.f);
+}
+
+template <typename AT, int NT, int VPT, int F>
+__global__ void __launch_bounds__(NT, 1) hy_row_op_few_kernel(RowOpArgs a) {
+  pdl_launch_dependents();
+  __shared__ float red[2][32];
+  const long long t = blockIdx.x;
+  const int D = a.D;
+  const bool branch = a.m1.f != nullptr || a.m1.h != nullptr, two = a.m2.f != nullptr || a.m2.h != nullptr, three = a.m3.f != nullptr || a.m3.h != nullptr;
+  float bw[VPT][4], nw[VPT][4], x[VPT][4], v[VPT][4];
+  int n1[VPT], n2[VPT], n3[VPT];
+#pragma unroll
+  for (int it = 0; it < VPT; ++it) {
+    const int c = (it * NT + threadIdx.x) * 4;
+    const bool in = c < D;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) bw[it][j] = nw[it][j] = x[it][j] = v[it][j] = 0.f;
+    if (in && branch && !a.plain_add) hy_quad_f(a.bw + c, bw[it]);
+    if (in && a.nw != nullptr) {
+      if (a.nw_mode == 2) nw[it][0] = nw[it][1] = nw[it][2] = nw[it][3] = a.nw[0];
+      else hy_quad_f(a.nw + c, nw[it]);
+    }
+    n1[it] = in && branch ? lin_planes(a.m1, c) : 0;
+    n2[it] = in && two ? lin_planes(a.m2, c) : 0;
+    n3[it] = in && three ? lin_planes(a.m3, c) : 0;
+  }
+  pdl_wait();
+  float ss = 0.f;
+#pragma unroll
+  for (int it = 0; it < VPT; ++it) {
+    const int c = (it * NT + threadIdx.x) * 4;
+    if (c >= D) break;
+    hy_quad_f(a.x + t * D + c, x[it]);
+    if (branch) {
+      float u[4];
+      lin_planes4<F>(a.m1, t, c, n1[it], u);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) v[it][j] = a.s1 * u[j];
+      if (two) {
+        lin_planes4<F>(a.m2, t, c, n2[it], u);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) v[it][j] += a.s2 * u[j];
+      }
+      if (a.plain_add && three) {
+        lin_planes4<F>(a.m3, t, c, n3[it], u);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) v[it][j] += u[j];
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) ss += v[it][j] * v[it][j];
+  }
+  const float inv = branch && !a.plain_add ? 1.0f / sqrtf(row_sum_once<NT>(ss, red[0]) / (float)D + a.eps) : 0.f;
+  float s2 = 0.f;
+#pragma unroll
+  for (int it = 0; it < VPT; ++it) {
+    const int c = (it * NT + threadIdx.x) * 4;
+    if (c >= D) break;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      if (branch) x[it][j] += a.plain_add ? v[it][j] : v[it][j] * inv * (bw[it][j] + a.bw_one);
+      s2 += x[it][j] * x[it][j];
+    }
+    if (branch) hy_quad_st(a.x + t * D + c, x[it]);
+    if (a.xa != nullptr) hy_quad_st(reinterpret_cast<AT*>(a.xa) + t * D + c, x[it]);
+  }
+  if (a.nw == nullptr) return;
+  const float inv2 = 1.0f / sqrtf(row_sum_once<NT>(s2, red[1]) / (float)D + a.eps);
+#pragma unroll
+  for (int it = 0; it < VPT; ++it) {
+    const int c = (it * NT + threadIdx.x) * 4;
+    if (c >= D) break;
+    float h[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) h[j] = x[it][j] * inv2 * (a.nw_mode == 0 ? 1.0f + nw[it][j] : nw[it][j]);
+    hy_quad_st(a.hn + t * D + c, h);
+    if (a.ha != nullptr) hy_quad_st(reinterpret_cast<AT*>(a.ha) + t * D + c, h);
+  }
 }

@@ -51,6 +51,11 @@ struct GemmArgs {
   bf16 *q_out, *k_pool, *v_pool;
   const int *tok_seq, *tok_pos, *seq_slot, *page_table;
   int max_pages, page_tokens, n_heads, n_kv_heads, head_dim, rope_kind;
+  // XB_EPI_GLU (hybrid feed-forwards): the weight rows are, expert after expert, [gate (glu_f) | up (glu_f)], then the shared expert's [gate (glu_sf) | up];
+  // out[t][i] = activation of the i-th gate and up row.  XB_EPI_RELU2: out = max(y, 0)^2
+  int glu_f, glu_e, glu_sf, glu_act, glu_on_input, glu_ldg, glu_sg_at;
+  float glu_limit, glu_limit_s;
+  const float *glu_bias, *glu_w;   // of the weight rows; routing weights [t][glu_ldg] (nullptr: one)
   int bulk_epi;            // SKINNY: the block's LAST unit leaves through shared memory + bulk stores (see the epilogue)
   float* out2;             // SKINNY: second copy of the result (same layout as `out`), e.g. pinned host memory
   unsigned long long* ts;  // timeline instrumentation (XB_GEMM_TS=1): [gridDim.x][XB_TS_SLOTS] globaltimer stamps, else nullptr
@@ -63,7 +68,7 @@ struct GemmArgs {
   do {                                                                                   \
     if ((g).ts != nullptr) (g).ts[(size_t)blockIdx.x * XB_TS_SLOTS + (slot)] = xb_gtimer(); \
   } while (0)
-enum { XB_EPI_PLAIN = 0, XB_EPI_QKV = 1, XB_EPI_SILU = 2 };
+enum { XB_EPI_PLAIN = 0, XB_EPI_QKV = 1, XB_EPI_SILU = 2, XB_EPI_GLU = 3, XB_EPI_RELU2 = 4 };
 
 // TMA coordinates (innermost, row) of the [128 x 64] weight box holding rows 128*wt.. of k-block kb
 __device__ __forceinline__ void gemm_w_coord(const GemmArgs& g, int wt, int kb, int& c0, int& c1) {

@@ -116,6 +116,7 @@ struct HyModel {
   int use_seg = 1;           // XB_HY_SEG=0: recurrences always as one chain per sequence (A/B); XB_HY_SEG=n >= 64: segments of n tokens
   int seg_len = 0;           // pinned segment length, 0: by the step's shape
   int use_attn_tile = 1;     // XB_HY_ATTN_TILE=0: attention of float32 prompts one (token, head) per block (A/B); n > 1: by tiles from n rows of a sequence on
+  int use_act = 1;           // activations of prompts' feed-forwards in the Linear's epilogue: XB_HY_ACT=0 never, 1 wherever it can be done (2 here), else where it pays
   int use_quad = 1;          // XB_HY_QUAD=0: row kernels of prompts one channel per thread (A/B)
   int use_tc_attn = 1;       // XB_HY_TC_ATTN=0: attention through the per-token kernel everywhere (A/B)
   int use_tc = 1;            // XB_HY_TC=0: every Linear through the plain kernels (A/B)
@@ -912,6 +913,8 @@ static int hy_create(xb_engine* e, const xb_hybrid_desc& d, const xb_hybrid_laye
     if (sl != nullptr) { hy->use_seg = atoi(sl) > 0 ? 1 : 0; hy->seg_len = atoi(sl) >= HY_SEG_MIN ? atoi(sl) : 0; }
     const char* qd = getenv("XB_HY_QUAD");
     if (qd != nullptr && qd[0] == '0') hy->use_quad = 0;
+    const char* qa = getenv("XB_HY_ACT");
+    if (qa != nullptr) hy->use_act = qa[0] == '0' ? 0 : 2;
     const char* at = getenv("XB_HY_ATTN_TILE");
     if (at != nullptr && (atoi(at) > 0 || at[0] == '0')) hy->use_attn_tile = atoi(at);
     const char* lp = getenv("XB_HY_LPC");
@@ -1278,6 +1281,30 @@ static bool hy_tc_linear(xb_engine* e, const void* x, long long ldx, const bf16*
   if (p.args.mode == XB_GEMM_SKINNY) { o.f = (const float*)out; o.h = nullptr; o.si = p.split; }
   else { o.f = nullptr; o.h = (const bf16*)out; o.si = SplitInfo{0, 0, 0}; }
   *y = o;
+  return true;
+}
+
+static bool hy_act_pays(const xb_engine* e, int T, int N, int K, int n_out) {
+  return e->hy->use_act == 2 || xb_wide_act_pays(T, N, K, n_out, e->num_sms);
+}
+// A feed-forward's up Linear of a prompt with its activation in the epilogue: out [T, n_out] (bf16).  `set` completes the plan's arguments.  False: not
+// applicable (few rows, no tile-major copy, features that do not fill 128-column halves) or not worth it.
+template <typename F>
+static bool hy_act_linear(xb_engine* e, const void* x, long long ldx, const bf16* wt, int T, int N, int K, int n_out, bf16* out, cudaStream_t st, F set, int* rc) {
+  HyModel* hy = e->hy;
+  *rc = 0;
+  if (!hy->use_act || wt == nullptr || T <= 128 || ldx % 8 != 0 || n_out % 16 != 0 || !hy_act_pays(e, T, N, K, n_out)) return false;
+  const auto key = std::make_tuple((const void*)wt, x, (const void*)out, T);
+  auto it = hy->plans.find(key);
+  if (it == hy->plans.end()) {
+    GemmPlan p;
+    const int v = xb_pick_wide(T, N, K, 32, e->num_sms, true);
+    if ((*rc = xb_gemm_plan(&p, (const bf16*)x, ldx, wt, 1, T, N, K, out, n_out, nullptr, 0, e->num_sms, v + 1)) != 0) return true;
+    set(p.args);
+    it = hy->plans.emplace(key, p).first;
+  }
+  if ((*rc = run_gemm(e, it->second, st)) != 0) return true;
+  LAUNCH_COUNT(e);
   return true;
 }
 
@@ -1851,6 +1878,27 @@ static int hy_ff_parallel(xb_engine* e, const HyLayer& l, int T, const void* xin
                      (const float*)hy->gw, ldg, c.n_experts, c.top, c.ff, sf, D, hy->m2, T));   // m2: router logits there are spent
     *y = hy_plain(hy->m2, D);
     return 0;
+  }
+  const bool moe = c.ff_kind == XB_FF_MOE, glu = c.ff_kind == XB_FF_GLU_CLAMP || c.ff_kind == XB_FF_GLU;
+  const int E = moe ? c.n_experts : 1;
+  if (std::is_same<AT, bf16>::value && up_out == nullptr && (glu || (moe && hy_ff_gated(c))) && c.ff % 128 == 0 && sf % 128 == 0 &&
+      l.n_dn == E * c.ff + sf && l.n_up == 2 * l.n_dn && T > 128 && hy->use_act && l.t_up != nullptr && (!moe || l.b_up == nullptr) &&
+      hy_act_pays(e, T, l.n_up, D, l.n_dn)) {
+    if (moe) XB_TRY(hy_router<AT>(e, l, T, xin, sg, st));
+    int rc = 0;
+    const bool done = hy_act_linear(e, xin, D, l.t_up, T, l.n_up, D, l.n_dn, reinterpret_cast<bf16*>(hy->a2), st, [&](GemmArgs& g) {
+      g.epi = XB_EPI_GLU;
+      g.glu_f = c.ff; g.glu_e = E; g.glu_sf = sf;
+      g.glu_act = c.ff_kind == XB_FF_GLU_CLAMP ? XB_ACT_GLU_CLAMP : c.ff_act;
+      g.glu_on_input = moe ? c.route_input : 0;
+      g.glu_limit = c.ff_limit; g.glu_limit_s = c.shared_limit;
+      g.glu_bias = l.b_up;
+      g.glu_w = moe ? (const float*)hy->gw : nullptr;
+      g.glu_ldg = ldg; g.glu_sg_at = sg_at;
+    }, &rc);
+    if (rc != 0) return rc;
+    XB_CHECK(done, "feed-forward Linear of %d rows: activation refused", T);
+    return hy_linear<AT>(e, a2, l.n_dn, l.w_down, l.t_down, l.b_down, T, D, l.n_dn, hy->m2, hy->cap_m, st, y);
   }
   LinOut U;
   XB_TRY(hy_linear<AT>(e, xin, D, l.w_up, l.t_up, l.b_up, T, l.n_up, D, hy->P, hy->cap_P, st, &U));
@@ -2540,6 +2588,11 @@ static int hy_run_body_t(xb_engine* e, int T, int n_seqs, int n_tiles, void* con
     } else if (has_ff) {
       LinOut u, dn;
       if (!ff_direct) XB_TRY(hy_sublayer_input<AT>(e, T, n_seqs, no_span, l.canon2, l.st_canon2, m, st));
+      int rc = 0;
+      if (std::is_same<AT, bf16>::value && hy_act_linear(e, a1, D, l.t_up, T, c.ff, D, c.ff, reinterpret_cast<bf16*>(hy->a2), st, [](GemmArgs& g) { g.epi = XB_EPI_RELU2; }, &rc)) {
+        if (rc != 0) return rc;
+        XB_TRY(hy_linear<AT>(e, a2, c.ff, l.w_down, l.t_down, nullptr, T, D, c.ff, hy->m1, hy->cap_m, st, &dn));
+      } else {
       XB_TRY(hy_linear<AT>(e, a1, D, l.w_up, l.t_up, nullptr, T, c.ff, D, hy->P, hy->cap_P, st, &u));
       const long long n = (long long)T * c.ff;
       if (std::is_same<AT, bf16>::value && u.h != nullptr && u.bias == nullptr && c.ff % 8 == 0 && u.ld % 8 == 0)
@@ -2548,6 +2601,7 @@ static int hy_run_body_t(xb_engine* e, int T, int n_seqs, int n_tiles, void* con
       else
         XB_TRY(hy_launch(e, hy_relu2_kernel<AT>, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, st, u, a1, (long long)c.ff, T, c.ff));
       XB_TRY(hy_linear<AT>(e, a1, c.ff, l.w_down, l.t_down, nullptr, T, D, c.ff, hy->m1, hy->cap_m, st, &dn));
+      }
       XB_TRY(hy_row_op<AT>(e, T, dn, 1.f, hy_none(), 0.f, l.norm2b, 1.f, has_side ? nullptr : next_norm, (has_side && !side_fused) ? (void*)a1 : nullptr, st));
     }
     if (has_side && side_fused) {

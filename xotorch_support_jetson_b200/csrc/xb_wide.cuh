@@ -223,10 +223,72 @@ __device__ __forceinline__ void wide_emit(const GemmArgs& g, int t, const WideQk
   }
 }
 
+// ---- the feed-forwards of hybrid models (ACT = 1): gate and up of the same 128 features are the two halves of a 256-column tile, so the activation leaves
+// from the epilogue in one piece and the matrix of gate and up rows is never written.  1800 rows x 2048 -> 2 x 8192, us: 111.5 with a kernel that read it,
+// 97.6 now (the products alone 91.2), experts 106.8 -> 95.6; 192 rows 26.9 -> 20.8.
+// 1 / (1 + e^-x), the quotient by __fdividef (2 ulp, no branches): four warps finish a tile while the next one is multiplied, and with the exact division
+// they took longer than that (110.7 us).
+__device__ __forceinline__ float wide_sigmoid(float x) { return __fdividef(1.0f, 1.0f + expf(-x)); }
+// first gate row (or up row) of the 128 features of tile tb
+__device__ __forceinline__ int wide_glu_row(const GemmArgs& g, int tb, bool up) {
+  const int i = tb * 128, routed = g.glu_e * g.glu_f;
+  if (i >= routed) return routed + i + (up ? g.glu_sf : 0);
+  const int e = i / g.glu_f;
+  return e * g.glu_f + i + (up ? g.glu_f : 0);
+}
+// x0 / x1: fp32 sums of 16 gate and 16 up rows from n0 / n1 on, routing weight w; features f0 ..  The choice of the activation stands outside the unrolled
+// loops: inside, three activations sixteen times over ran out of the instruction cache (211 us).
+__device__ __forceinline__ void wide_emit_glu(const GemmArgs& g, int t, int f0, int n0, int n1, float w, bool shared, float* x0, float* x1) {
+  if (t >= g.a_rows) return;
+  const float limit = shared ? g.glu_limit_s : g.glu_limit;
+#pragma unroll
+  for (int j = 0; j < 16; ++j) { x0[j] = rbf(x0[j]); x1[j] = rbf(x1[j]); }   // what the Linear hands on is bf16, here as in steps of other kernels
+  if (g.glu_bias != nullptr) {
+#pragma unroll
+    for (int j = 0; j < 16; ++j) { x0[j] += g.glu_bias[n0 + j]; x1[j] += g.glu_bias[n1 + j]; }
+  }
+  if (g.glu_on_input && !shared) {   // (w h) W^T = w (h W^T)
+#pragma unroll
+    for (int j = 0; j < 16; ++j) { x0[j] *= w; x1[j] *= w; }
+  }
+  if (w == 0.f && !shared) {         // an expert that the token does not use
+#pragma unroll
+    for (int j = 0; j < 16; ++j) x0[j] = 0.f;
+  } else if (g.glu_act == XB_ACT_SWIGLU) {
+#pragma unroll
+    for (int j = 0; j < 16; ++j) x0[j] = x0[j] * wide_sigmoid(x0[j]) * x1[j];
+  } else if (g.glu_act == XB_ACT_GEGLU) {
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {   // the tanh form: 0.5 (1 + tanh y) = 1 / (1 + e^-2y)
+      const float z = x0[j];
+      x0[j] = z * wide_sigmoid(1.5957691216057308f * (z + 0.044715f * z * z * z)) * x1[j];
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      const float a = fminf(x0[j], limit), u = fminf(fmaxf(x1[j], -limit), limit);
+      x0[j] = a * wide_sigmoid(1.702f * a) * (u + 1.0f);
+    }
+  }
+  if (!g.glu_on_input || shared) {
+    if (w != 1.f) {
+#pragma unroll
+      for (int j = 0; j < 16; ++j) x0[j] *= w;
+    }
+  }
+  epi_store16(reinterpret_cast<bf16*>(g.out) + (long long)t * g.ld_out + f0, x0);
+}
+__device__ __forceinline__ void wide_emit_relu2(const GemmArgs& g, int t, int n0, float* x) {
+  if (t >= g.a_rows || n0 >= g.b_rows) return;
+#pragma unroll
+  for (int j = 0; j < 16; ++j) { const float v = fmaxf(rbf(x[j]), 0.f); x[j] = v * v; }
+  epi_store16(reinterpret_cast<bf16*>(g.out) + (long long)t * g.ld_out + n0, x);
+}
+
 // Roles are entered by elect.sync, not by lane == 0, and the two operands have a producer thread each: one thread doing
 // everything under `lane == 0` spent 0.35 us a k-block whatever the tile (a 128 x 64 tile took as long as 128 x 256), most of
 // it issuing.  4096^3, CUDA events: 256x256 pair 103 -> 94 us, 128x256 107 -> 103, 128x128 166 -> 116, 128x64 306 -> 202.
-template <int BN, int CG, int RM>
+template <int BN, int CG, int RM, int ACT = 0>
 __global__ void __launch_bounds__(224, 1)
 xb_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, GemmArgs g) {
   using Cfg = WideCfg<BN, CG, RM>;
@@ -307,7 +369,8 @@ xb_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
               if (q >= nk) break;
 #pragma unroll
               for (int j = 0; j < Cfg::BROWS / Cfg::BOX; ++j) {
-                const int n = tb * BN + (CG == 2 ? (int)rank * Cfg::BROWS : 0) + j * Cfg::BOX;
+                int n = tb * BN + (CG == 2 ? (int)rank * Cfg::BROWS : 0) + j * Cfg::BOX;
+                if (ACT != 0 && g.epi == XB_EPI_GLU) n = wide_glu_row(g, tb, CG == 2 ? rank != 0 : j != 0);
                 uint8_t* dst = sB + (stage * KS + q) * Cfg::B_BYTES + j * Cfg::BOX * 128;
                 if (g.w_tiled) load(dst, &tmB, 0, ((n >> 7) * g.k_blocks + kb + q) * 128 + (n & 127));
                 else load(dst, &tmB, (kb + q) * 64, n);
@@ -366,7 +429,17 @@ xb_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       WideQkvRow row;
       row.kv = qkv && n0 + Cfg::COLS > g.n_heads * g.head_dim ? wide_kv_row(g, t, pos) : 0;
       float next[32];
-      if (qkv) {
+      int up0 = 0, gate0 = 0;
+      float weight = 1.f;
+      bool shared = false;
+      if (ACT != 0 && g.epi == XB_EPI_GLU) {
+        gate0 = wide_glu_row(g, tb, false);
+        up0 = wide_glu_row(g, tb, true);
+        shared = tb * 128 >= g.glu_e * g.glu_f;
+        const int at = shared ? g.glu_sg_at : tb * 128 / g.glu_f;
+        if (g.glu_w != nullptr && t < g.a_rows && at >= 0) weight = g.glu_w[(long long)t * g.glu_ldg + at];
+      }
+      if (ACT == 0 && qkv) {
         int c0, c1;
         wide_pair_cols(g, 0, c0, c1);
         wide_rope_load(g, pos, n0 + c0, next);
@@ -377,11 +450,12 @@ xb_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 #pragma unroll 1
       for (int p = 0; p < Cfg::PAIRS; ++p) {
         int c0, c1;
-        wide_pair_cols(g, p, c0, c1);
+        if (ACT != 0 && g.epi == XB_EPI_GLU) { c0 = p * 16; c1 = 128 + p * 16; }
+        else wide_pair_cols(g, p, c0, c1);
         uint32_t v0[16], v1[16];
         tmem_ld16(t_addr + c0, v0);
         tmem_ld16(t_addr + c1, v1);
-        if (qkv) {
+        if (ACT == 0 && qkv) {
 #pragma unroll
           for (int j = 0; j < 32; ++j) row.cs[j] = next[j];
           if (p + 1 < Cfg::PAIRS) {
@@ -391,7 +465,15 @@ xb_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           }
         }
         tmem_ld_wait();
-        wide_emit(g, t, row, n0 + c0, n0 + c1, reinterpret_cast<float*>(v0), reinterpret_cast<float*>(v1));
+        float *x0 = reinterpret_cast<float*>(v0), *x1 = reinterpret_cast<float*>(v1);
+        if (ACT == 0) {
+          wide_emit(g, t, row, n0 + c0, n0 + c1, x0, x1);
+        } else if (g.epi == XB_EPI_GLU) {
+          wide_emit_glu(g, t, tb * 128 + c0, gate0 + c0, up0 + c0, weight, shared, x0, x1);
+        } else {
+          wide_emit_relu2(g, t, n0 + c0, x0);
+          wide_emit_relu2(g, t, n0 + c1, x1);
+        }
       }
       tc_fence_before();
       __syncwarp();
@@ -416,10 +498,11 @@ xb_wide_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 struct WideVariant {
   int bn, cg, rm, cols;          // cols: columns a thread of the epilogue holds
   double us_k_block, us_ends;    // estimated time (xb_pick_wide)
+  int (*run_act)(const CUtensorMap&, const CUtensorMap&, const GemmArgs&, int grid, cudaStream_t, int pdl);   // with the feed-forward activations, or nullptr
   int (*run)(const CUtensorMap&, const CUtensorMap&, const GemmArgs&, int grid, cudaStream_t, int pdl);
 };
 
-template <int BN, int CG, int RM>
+template <int BN, int CG, int RM, int ACT>
 static int xb_wide_launch_t(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmArgs& g, int grid, cudaStream_t st, int pdl) {
   using Cfg = WideCfg<BN, CG, RM>;
   {
@@ -427,7 +510,7 @@ static int xb_wide_launch_t(const CUtensorMap& tmA, const CUtensorMap& tmB, cons
     int dev = 0;
     XB_CUDA(cudaGetDevice(&dev));
     if (dev < 0 || dev >= XB_MAX_DEVICES || !done[dev]) {
-      XB_CUDA(cudaFuncSetAttribute(xb_wide_kernel<BN, CG, RM>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES));
+      XB_CUDA(cudaFuncSetAttribute(xb_wide_kernel<BN, CG, RM, ACT>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES));
       if (dev >= 0 && dev < XB_MAX_DEVICES) done[dev] = true;
     }
   }
@@ -452,14 +535,15 @@ static int xb_wide_launch_t(const CUtensorMap& tmA, const CUtensorMap& tmB, cons
   }
   cfg.attrs = attr;
   cfg.numAttrs = na;
-  XB_CUDA(cudaLaunchKernelEx(&cfg, xb_wide_kernel<BN, CG, RM>, tmA, tmB, g));
+  XB_CUDA(cudaLaunchKernelEx(&cfg, xb_wide_kernel<BN, CG, RM, ACT>, tmA, tmB, g));
   return 0;
 }
 
-#define XB_WIDE_VARIANT(BN, CG, RM, KB, ENDS) {BN, CG, RM, WideCfg<BN, CG, RM>::COLS, KB, ENDS, xb_wide_launch_t<BN, CG, RM>}
+#define XB_WIDE_VARIANT(BN, CG, RM, KB, ENDS, RUN_ACT) {BN, CG, RM, WideCfg<BN, CG, RM>::COLS, KB, ENDS, RUN_ACT, xb_wide_launch_t<BN, CG, RM, 0>}
 static const WideVariant g_wide_variants[] = {
-  XB_WIDE_VARIANT(256, 2, 128, 0.35, 5.3), XB_WIDE_VARIANT(256, 1, 128, 0.385, 6.0), XB_WIDE_VARIANT(192, 1, 128, 0.33, 3.4),
-  XB_WIDE_VARIANT(128, 1, 128, 0.256, 1.1), XB_WIDE_VARIANT(256, 2, 64, 0.23, 1.6), XB_WIDE_VARIANT(128, 2, 64, 0.166, 1.8),
+  XB_WIDE_VARIANT(256, 2, 128, 0.35, 5.3, (xb_wide_launch_t<256, 2, 128, 1>)), XB_WIDE_VARIANT(256, 1, 128, 0.385, 6.0, (xb_wide_launch_t<256, 1, 128, 1>)),
+  XB_WIDE_VARIANT(192, 1, 128, 0.33, 3.4, nullptr), XB_WIDE_VARIANT(128, 1, 128, 0.256, 1.1, nullptr),
+  XB_WIDE_VARIANT(256, 2, 64, 0.23, 1.6, nullptr), XB_WIDE_VARIANT(128, 2, 64, 0.166, 1.8, nullptr),
 };
 #undef XB_WIDE_VARIANT
 enum { XB_WIDE_VARIANTS = sizeof(g_wide_variants) / sizeof(g_wide_variants[0]) };
@@ -468,13 +552,14 @@ enum { XB_WIDE_VARIANTS = sizeof(g_wide_variants) / sizeof(g_wide_variants[0]) }
 // Linears of the registered models (K 2048 .. 18944, N 2048 .. 37888; back to back, weights from HBM): over the 126 shapes the choice is 0.3 % slower than
 // the best variant on average, 13 % at most.  Without the pairs of 64 rows it was 18 % and 79 %.
 // col_unit: columns that one thread has to hold together (a head where the rotation pairs its halves).
-static int xb_pick_wide(int T, int N, int K, int col_unit, int num_sms) {
+// act: only variants with the feed-forward activations.  *us: the estimate.
+static int xb_pick_wide(int T, int N, int K, int col_unit, int num_sms, bool act = false, double* us = nullptr) {
   int best = 1;
   double best_t = 1e30;
   const int k_blocks = (K + 63) / 64;
   for (int i = 0; i < XB_WIDE_VARIANTS; ++i) {
     const WideVariant& v = g_wide_variants[i];
-    if (v.cols % col_unit != 0) continue;
+    if (v.cols % col_unit != 0 || (act && v.run_act == nullptr)) continue;
     const int rows = v.rm * v.cg;
     const long long units = (long long)((T + rows - 1) / rows) * ((N + v.bn - 1) / v.bn);
     const int slots = num_sms / v.cg;
@@ -482,6 +567,7 @@ static int xb_pick_wide(int T, int N, int K, int col_unit, int num_sms) {
     const double t = (double)waves * k_blocks * v.us_k_block + v.us_ends;
     if (t < best_t) { best_t = t; best = i; }
   }
+  if (us != nullptr) *us = best_t;
   return best;
 }
 
@@ -511,6 +597,16 @@ static int xb_wide_plan(GemmPlan* p, const bf16* x, long long ldx, const bf16* w
   return 0;
 }
 
+// Does the activation belong into the epilogue?  Yes where the tiles that can do it are not slower than the best ones by more than the kernel
+// would take that reads the finished matrix (2.5 us and 3.9 TB/s over what it reads and writes).
+static bool xb_wide_act_pays(int T, int N, int K, int n_out, int num_sms) {
+  double with = 0, without = 0;
+  xb_pick_wide(T, N, K, 32, num_sms, true, &with);
+  xb_pick_wide(T, N, K, 32, num_sms, false, &without);
+  return with < without + 2.5 + 2.0 * T * ((double)N + n_out) / 3.9e6;
+}
+
 static int xb_wide_run(const GemmPlan& p, cudaStream_t st, int pdl) {
-  return g_wide_variants[p.wide].run(p.tmA, p.tmB, p.args, p.grid, st, pdl);
+  const bool act = p.args.epi == XB_EPI_GLU || p.args.epi == XB_EPI_RELU2;
+  return (act ? g_wide_variants[p.wide].run_act : g_wide_variants[p.wide].run)(p.tmA, p.tmB, p.args, p.grid, st, pdl);
 }

@@ -54,46 +54,52 @@ __global__ void __launch_bounds__(256) hy_taps_quad_kernel(LinOut in, int col0, 
                                                            long long ld_out, int T) {
   constexpr int TT = 8;
   pdl_launch_dependents();
-  pdl_wait();
   const int c = (blockIdx.y * blockDim.x + threadIdx.x) * 4;
   if (c >= C) return;
+  // What waits for no kernel (the step's metadata, the filter) comes ahead of the wait; behind it the eight rows and the rows before them go out together.
   const int r0 = blockIdx.x * TT;
   const int last_row = (r0 + TT < T ? r0 + TT : T) - 1;
-  const bool uniform = m.tok_seq[r0] == m.tok_seq[last_row];
   const int s_first = m.tok_seq[r0];
+  const bool uniform = s_first == m.tok_seq[last_row];
+  const int first_start = s_first > 0 ? m.seq_last[s_first - 1] + 1 : 0, first_pos = m.tok_pos[r0], first_pos0 = m.tok_pos[first_start];
+  const float* first_tail = tail + (long long)m.seq_slot[s_first] * tail_stride;
   float wv[TAPS][4];
 #pragma unroll
   for (int e = 0; e < 4; ++e)
 #pragma unroll
     for (int j = 0; j < TAPS; ++j) wv[j][e] = w[(long long)(c + e) * TAPS + j];
+  pdl_wait();
   float win[TAPS][4];   // win[d - 1]: the input d steps back (TAPS - 1 used)
 #pragma unroll
   for (int d = 0; d < TAPS; ++d)
 #pragma unroll
     for (int e = 0; e < 4; ++e) win[d][e] = 0.f;
+  auto window = [&](int row, int start, int pos, int pos0, const float* tl) {
+#pragma unroll
+    for (int d = 1; d < TAPS; ++d) {
+      const int p = pos - d;
+      float v[4] = {0.f, 0.f, 0.f, 0.f};
+      if (p >= 0) {
+        if (row - d >= start) lin_quad(in, row - d, col0 + c, v);
+        else hy_quad_f(tl + (long long)(p - (pos0 - (TAPS - 1))) * C + c, v);
+      }
+#pragma unroll
+      for (int e = 0; e < 4; ++e) win[d - 1][e] = v[e];
+    }
+  };
   float cur[TT][4];
 #pragma unroll
   for (int i = 0; i < TT; ++i) lin_quad(in, r0 + i <= last_row ? r0 + i : last_row, col0 + c, cur[i]);
+  window(r0, first_start, first_pos, first_pos0, first_tail);
 #pragma unroll
   for (int i = 0; i < TT; ++i) {
     const int row = r0 + i;
     if (row > last_row) break;
-    const int s = uniform ? s_first : m.tok_seq[row];
-    const bool begins = !uniform && i > 0 && m.tok_seq[row - 1] != s;
-    if (i == 0 || begins) {
-      const float* tl = tail + (long long)m.seq_slot[s] * tail_stride;
-      const int start = begins ? row : (s > 0 ? m.seq_last[s - 1] + 1 : 0);
-      const int pos = m.tok_pos[row], pos0 = m.tok_pos[start];
-#pragma unroll
-      for (int d = 1; d < TAPS; ++d) {
-        const int p = pos - d;
-        float v[4] = {0.f, 0.f, 0.f, 0.f};
-        if (p >= 0) {
-          if (row - d >= start) lin_quad(in, row - d, col0 + c, v);
-          else hy_quad_f(tl + (long long)(p - (pos0 - (TAPS - 1))) * C + c, v);
-        }
-#pragma unroll
-        for (int e = 0; e < 4; ++e) win[d - 1][e] = v[e];
+    if (!uniform && i > 0) {
+      const int s = m.tok_seq[row];
+      if (m.tok_seq[row - 1] != s) {   // a sequence begins here
+        const int pos = m.tok_pos[row];
+        window(row, row, pos, pos, tail + (long long)m.seq_slot[s] * tail_stride);
       }
     }
     float acc[4];

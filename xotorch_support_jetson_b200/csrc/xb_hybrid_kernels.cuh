@@ -64,7 +64,18 @@ __global__ void hy_embed_kernel(const int* __restrict__ tokens, const bf16* __re
   const int t = blockIdx.x;
   int tok = tokens[t];
   tok = tok < 0 ? 0 : (tok >= V ? V - 1 : tok);
-  for (int i = threadIdx.x; i < D; i += blockDim.x) x[(long long)t * D + i] = bf2f(emb[(long long)tok * D + i]) * scale;
+  const bf16* src = emb + (long long)tok * D;
+  float* dst = x + (long long)t * D;
+  if ((D & 7) == 0 && (reinterpret_cast<uintptr_t>(emb) & 15) == 0) {   // eight channels a thread: 2048 rows x 2048 13.4 -> 9.1 us cold, 8 rows 5.3 -> 3.2
+    for (int i = threadIdx.x * 8; i < D; i += blockDim.x * 8) {
+      const uint4 u = *reinterpret_cast<const uint4*>(src + i);
+      const float2 a = bf2_to_f2(u.x), b = bf2_to_f2(u.y), c = bf2_to_f2(u.z), d = bf2_to_f2(u.w);
+      *reinterpret_cast<float4*>(dst + i) = make_float4(a.x * scale, a.y * scale, b.x * scale, b.y * scale);
+      *reinterpret_cast<float4*>(dst + i + 4) = make_float4(c.x * scale, c.y * scale, d.x * scale, d.y * scale);
+    }
+    return;
+  }
+  for (int i = threadIdx.x; i < D; i += blockDim.x) dst[i] = bf2f(src[i]) * scale;
 }
 
 // tanh(alpha * x) * w + b: a norm of the stream without statistics of the row (one channel at a time, fp32)
@@ -2406,8 +2417,8 @@ __global__ void __launch_bounds__(NT) hy_latent_down_kernel(LinOut P, int off_dk
 // Queries in the cache's space.  Q carries H heads of [K unrotated | dr rotated] (columns from qoff); per head
 //   qa[t, h, n]     = sum_k Q[t, h, k] * W[(h * K + k) * N + n]     n < N: the query folded into the latent space
 //   qa[t, h, N + i] = rot(rotated part)[i]                          i < dr
-// grid (ceil(T / ROWS), H), 256 threads over n; the rows' inputs sit in shared memory (ROWS * K floats).  The first weights fetched ahead of the wait (32 a
-// thread) lay in local memory across the rotation: a latent layer of bibevik-1b at 1 to 16 tokens 69.5 us, without 67.
+// grid (ceil(T / ROWS), H), 256 threads over n; the rows' inputs sit in shared memory (ROWS * K floats).  One row a block and N a multiple of eight:
+// hy_latent_absorb_row_kernel.
 #define HY_MM_ROWS 8
 template <int ROWS>
 __global__ void __launch_bounds__(256) hy_latent_absorb_kernel(LinOut Q, int qoff, int dr, const bf16* __restrict__ W, float* __restrict__ qa,
@@ -2450,6 +2461,70 @@ __global__ void __launch_bounds__(256) hy_latent_absorb_kernel(LinOut Q, int qof
       for (int rr = 0; rr < ROWS; ++rr) acc[rr] = fmaf(xsm[rr * K + k], w, acc[rr]);
     }
     for (int rr = 0; rr < nt; ++rr) qa[((long long)(t0 + rr) * H + h) * ld + n] = acc[rr];
+  }
+}
+// The same for one row a block (steps of few rows), N a multiple of eight: a warp takes every eighth k, a lane eight neighbouring n.  All weights of K <= 64 are on
+// their way before the kernel before this one is done (the launch bound leaves them the registers: 32 a thread spilled without it); one column a thread, eight
+// k's at a time, took eight trips to memory behind the wait (8 tokens, 16 heads of 64 x 256: 12.8 -> 5.1 us cold).  grid (T, H), 256 threads; K + 8 N floats of shared memory.
+__global__ void __launch_bounds__(256, 2) hy_latent_absorb_row_kernel(LinOut Q, int qoff, int dr, const bf16* __restrict__ W, float* __restrict__ qa, int H, int K, int N,
+                                                                      RotArgs r, const int* __restrict__ tok_pos) {
+  pdl_launch_dependents();
+  extern __shared__ __align__(16) float xsm[];
+  float* part = xsm + ((K + 3) & ~3);
+  const int t = blockIdx.x, h = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int qh = qoff + h * (K + dr), ld = N + dr;
+  const bf16* Wh = W + (long long)h * K * N;
+  constexpr int PRE = 8;
+  uint4 pre[PRE];
+#pragma unroll
+  for (int i = 0; i < PRE; ++i)
+    pre[i] = warp + 8 * i < K && lane * 8 < N ? *reinterpret_cast<const uint4*>(Wh + (long long)(warp + 8 * i) * N + lane * 8) : make_uint4(0u, 0u, 0u, 0u);
+  pdl_wait();
+  for (int k = threadIdx.x; k < K; k += 256) {
+    const int col[1] = {qh + k};
+    float v[1];
+    lin_at_cols<1, 8>(Q, t, col, v);
+    xsm[k] = v[0];
+  }
+  const int half = r.dims >> 1, per = dr - half;
+  float* qd = qa + ((long long)t * H + h) * ld;
+  for (int i = 255 - threadIdx.x; i < per; i += 256) {   // by the threads that have no k where K is small
+    if (i < half) {
+      const int d0 = r.half ? i : 2 * i, d1 = r.half ? i + half : 2 * i + 1;
+      const int col[2] = {qh + K + d0, qh + K + d1};
+      float ab[2], cs, sn;
+      lin_at_cols<2, 8>(Q, t, col, ab);
+      hy_rot_cs(r, tok_pos[t], i, &cs, &sn);
+      qd[N + d0] = ab[0] * cs - ab[1] * sn;
+      qd[N + d1] = ab[1] * cs + ab[0] * sn;
+    } else {
+      qd[N + half + i] = lin_at(Q, t, qh + K + half + i);
+    }
+  }
+  __syncthreads();
+  for (int n = lane * 8; n < N; n += 256) {
+    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    auto add = [&](uint4 u, float x) {
+      const float2 a = bf2_to_f2(u.x), b = bf2_to_f2(u.y), c = bf2_to_f2(u.z), d = bf2_to_f2(u.w);
+      acc[0] = fmaf(x, a.x, acc[0]); acc[1] = fmaf(x, a.y, acc[1]); acc[2] = fmaf(x, b.x, acc[2]); acc[3] = fmaf(x, b.y, acc[3]);
+      acc[4] = fmaf(x, c.x, acc[4]); acc[5] = fmaf(x, c.y, acc[5]); acc[6] = fmaf(x, d.x, acc[6]); acc[7] = fmaf(x, d.y, acc[7]);
+    };
+    int k = warp;
+    if (n == lane * 8) {
+#pragma unroll
+      for (int i = 0; i < PRE; ++i, k += 8)
+        if (k < K) add(pre[i], xsm[k]);
+    }
+    for (; k < K; k += 8) add(*reinterpret_cast<const uint4*>(Wh + (long long)k * N + n), xsm[k]);
+    *reinterpret_cast<float4*>(part + warp * N + n) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+    *reinterpret_cast<float4*>(part + warp * N + n + 4) = make_float4(acc[4], acc[5], acc[6], acc[7]);
+  }
+  __syncthreads();
+  for (int n = threadIdx.x; n < N; n += 256) {
+    float s = part[n];
+#pragma unroll
+    for (int w = 1; w < 8; ++w) s += part[w * N + n];
+    qd[n] = s;
   }
 }
 // Per-head products with a weight that is stored head by head,
@@ -2506,10 +2581,11 @@ __global__ void __launch_bounds__(128) hy_head_mm_kernel(const float* __restrict
 //   x = sum_s O_s 2^(m_s - M) / sum_s l_s 2^(m_s - M);  y[t, h * N + n] = sigmoid(G) * sum_k x[k] W[(h * N + n) * R + k]
 // part [n_splits][T * H][2 + R] = (m, l, O) per share.  grid (T, H), 256 threads; R + n_splits floats of shared memory.
 // Shares behind the last one that holds a key (a short sequence has fewer tiles than the step has shares) are not read: they would add zeros.
-// The first eight weight rows of a warp are under way before the kernel before this one is done.  Latency-bound (128 blocks, 1 MB): 38 shares read
-// in rounds of eight and weights in rounds of four took 24 us cold at 8 tokens of 24 to 36 keys.
+// The first sixteen weight rows of a warp are under way before the kernel before this one is done.  Latency-bound (128 blocks, 1 MB): 38 shares read
+// in rounds of eight and weights in rounds of four took 24 us cold at 8 tokens of 24 to 36 keys; with eight weight rows ahead and no bound on the blocks 17.5, now
+// 11.8.
 template <typename AT>
-__global__ void __launch_bounds__(256) hy_latent_readout_kernel(const float* __restrict__ part, int n_splits, int NR, int H, int R, const bf16* __restrict__ W,
+__global__ void __launch_bounds__(256, 2) hy_latent_readout_kernel(const float* __restrict__ part, int n_splits, int NR, int H, int R, const bf16* __restrict__ W,
                                                                 AT* __restrict__ y, long long ldy, int N, LinOut G, int off_gate) {
   pdl_launch_dependents();
   extern __shared__ __align__(16) float xsm[];
@@ -2519,7 +2595,7 @@ __global__ void __launch_bounds__(256) hy_latent_readout_kernel(const float* __r
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const bf16* Wh = W + (long long)h * N * R;
   const bool vec = (R & 7) == 0 && (reinterpret_cast<uintptr_t>(W) & 15) == 0;
-  constexpr int PRE = 8;
+  constexpr int PRE = 16;
   uint4 pre[PRE];
 #pragma unroll
   for (int i = 0; i < PRE; ++i)

@@ -541,16 +541,16 @@ static int xb_wide_launch_t(const CUtensorMap& tmA, const CUtensorMap& tmB, cons
 
 #define XB_WIDE_VARIANT(BN, CG, RM, KB, ENDS, RUN_ACT) {BN, CG, RM, WideCfg<BN, CG, RM>::COLS, KB, ENDS, RUN_ACT, xb_wide_launch_t<BN, CG, RM, 0>}
 static const WideVariant g_wide_variants[] = {
-  XB_WIDE_VARIANT(256, 2, 128, 0.35, 5.3, (xb_wide_launch_t<256, 2, 128, 1>)), XB_WIDE_VARIANT(256, 1, 128, 0.385, 6.0, (xb_wide_launch_t<256, 1, 128, 1>)),
-  XB_WIDE_VARIANT(192, 1, 128, 0.33, 3.4, nullptr), XB_WIDE_VARIANT(128, 1, 128, 0.256, 1.1, nullptr),
-  XB_WIDE_VARIANT(256, 2, 64, 0.23, 1.6, nullptr), XB_WIDE_VARIANT(128, 2, 64, 0.166, 1.8, nullptr),
+  XB_WIDE_VARIANT(256, 2, 128, 0.34, 5.3, (xb_wide_launch_t<256, 2, 128, 1>)), XB_WIDE_VARIANT(256, 1, 128, 0.38, 6.2, (xb_wide_launch_t<256, 1, 128, 1>)),
+  XB_WIDE_VARIANT(192, 1, 128, 0.33, 3.4, nullptr), XB_WIDE_VARIANT(128, 1, 128, 0.26, 0.8, nullptr),
+  XB_WIDE_VARIANT(256, 2, 64, 0.22, 1.6, nullptr), XB_WIDE_VARIANT(128, 2, 64, 0.165, 1.6, nullptr),
 };
 #undef XB_WIDE_VARIANT
 enum { XB_WIDE_VARIANTS = sizeof(g_wide_variants) / sizeof(g_wide_variants[0]) };
 
 // The variant with the least estimated time: waves x (k-blocks x time of one) + the ends.  The times (us) are fitted to a sweep of T = 150 .. 2048 over 14
-// Linears of the registered models (K 2048 .. 18944, N 2048 .. 37888; back to back, weights from HBM): over the 126 shapes the choice is 0.3 % slower than
-// the best variant on average, 13 % at most.  Without the pairs of 64 rows it was 18 % and 79 %.
+// Linears of the registered models (K 2048 .. 18944, N 2048 .. 37888; back to back, weights from HBM): over the 168 shapes the choice is 0.2 % slower than
+// the best variant on average, 9 % at most.  Without the pairs of 64 rows it was 18 % and 79 %.
 // col_unit: columns that one thread has to hold together (a head where the rotation pairs its halves).
 // act: only variants with the feed-forward activations.  *us: the estimate.
 static int xb_pick_wide(int T, int N, int K, int col_unit, int num_sms, bool act = false, double* us = nullptr) {

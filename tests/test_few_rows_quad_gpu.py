@@ -1,0 +1,43 @@
+"""Gated feed-forwards, experts and logits of hybrid steps of few rows, four columns a thread, against the kernels that take one, on split-K planes (bf16) and
+plain matrices (float32), with vocabularies and widths that do and do not divide by four.  Per element they compute the same; the switch also
+changes the order in which these narrow models sum the squares of a row, which float32 shows at a few 2^-24 a layer and bf16 as roundings that fall the other way."""
+import copy
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("model,change", [("bibevik-tiny", {}), ("bibevik-tiny", {"vocab": 386}), ("bibevik-tiny", {"ff": 66}), ("pufivik-tiny", {}), ("vusenex-tiny", {}),
+                                          ("rurutar-tiny", {}), ("sizolorn-tiny", {})])
+@pytest.mark.parametrize("dtype,tol", [("bfloat16", 2e-2), ("float32", 5e-6)])
+@pytest.mark.parametrize("rows", [1, 5, 64])
+def test_four_columns_equal_one(built_lib, monkeypatch, model, change, dtype, tol, rows):
+  import inspect
+
+  from xotorch_support_jetson_b200 import model_config, synth
+  from xotorch_support_jetson_b200.models import model_cards
+  from xotorch_support_jetson_b200.shard import Shard
+  from xotorch_support_jetson_b200.stage import StageRuntime
+  hf = copy.deepcopy(model_cards[model]["hf_config"])
+  if "vocab" in change:
+    hf["vocab"] = change["vocab"]
+  if "ff" in change:
+    for lay in hf["layers"]:
+      if lay["mlp"] and lay["mlp"]["kind"] == "dense":
+        lay["mlp"]["ff"] = change["ff"]
+  make = getattr(synth, f"random_{model.split('-')[0]}_state")
+  w = make(hf, seed=4, **({"device": "cuda"} if "device" in inspect.signature(make).parameters else {}))
+  cfg = model_config.hybrid_model_config(hf)
+  model_config.resolve_tensor_sizes(cfg, {k: tuple(v.shape) for k, v in w.items()})
+  ids = torch.randint(0, hf["vocab"], (2, rows), generator=torch.Generator().manual_seed(rows)).to("cuda", torch.int32)
+  outs = []
+  for quad in ("1", "0"):
+    monkeypatch.setenv("XB_HY_QUAD", quad)
+    st = StageRuntime(Shard("quad-test", 0, cfg["num_layers"] - 1, cfg["num_layers"]), cfg, max_batch_tokens=64, max_seqs=rows, max_tokens_per_seq=8, dtype=dtype)
+    st.load_state(w)
+    outs.append(torch.stack([st.forward(list(range(rows)), [1] * rows, [s] * rows, tokens=ids[s].contiguous()).clone() for s in range(2)]).cpu())
+    st.close()
+  assert torch.isfinite(outs[0]).all()
+  assert ((outs[0] - outs[1]).norm() / outs[1].norm()).item() < tol

@@ -1806,6 +1806,8 @@ static int hy_run_head(xb_engine* e, int n_seqs, const BatchMeta& m, cudaStream_
     XB_TRY(hy_launch(e, hy_gather_rows_kernel<AT>, dim3(n), dim3(256), 0, st, (const float*)hy->hn, idx, reinterpret_cast<AT*>(hy->head_in), D));
   XB_TRY(hy_linear<AT>(e, in, D, hy->head, hy->t_head, nullptr, n, d.vocab, D, hy->head_raw, hy->cap_head, st, &y));
   const long long tot = (long long)n * d.vocab;
+  if (hy->use_quad && d.vocab % 4 == 0 && hy_planes4(y, 0) && hy_quad_ptr(e->logits))
+    return hy_launch(e, hy_logits_few_kernel, dim3((unsigned)((d.vocab / 4 + 255) / 256), n), dim3(256), 0, st, y, d.logit_softcap, e->logits, d.vocab);
   return hy_launch(e, hy_logits_kernel, dim3((unsigned)((tot + 255) / 256)), dim3(256), 0, st, y, d.logit_softcap, e->logits, n, d.vocab);
 }
 
@@ -1908,12 +1910,15 @@ static int hy_ff_parallel(xb_engine* e, const HyLayer& l, int T, const void* xin
   if (up_out != nullptr) *up_out = U;   // rows behind the experts' (a residual gate) are read by the caller
   // a bf16 matrix out of the tcgen05 Linear (prompts): the activations read and write 16 bytes per thread
   const bool vec = std::is_same<AT, bf16>::value && U.h != nullptr && U.ld % 8 == 0 && l.n_dn % 8 == 0;
+  const bool few4 = hy->use_quad && T <= 128 && l.n_dn % 4 == 0 && hy_planes4(U, 0);   // planes or one matrix, four columns a thread
   if (c.ff_kind == XB_FF_GLU_CLAMP || c.ff_kind == XB_FF_GLU) {
     const long long n = (long long)T * c.ff;
     const int act = c.ff_kind == XB_FF_GLU ? c.ff_act : XB_ACT_GLU_CLAMP;
     if (vec && c.ff % 8 == 0)
       XB_TRY(hy_launch(e, hy_glu_vec_kernel, dim3((unsigned)((n / 8 + 255) / 256)), dim3(256), 0, st, U.h, U.ld, U.bias, c.ff, c.ff_limit, act,
                        reinterpret_cast<bf16*>(hy->a2), (long long)l.n_dn, T));
+    else if (few4 && c.ff % 4 == 0)
+      XB_TRY(hy_launch(e, hy_glu_few_kernel<AT>, dim3((unsigned)((c.ff / 4 + 127) / 128), T), dim3(128), 0, st, U, c.ff, c.ff_limit, act, a2, (long long)l.n_dn));
     else
       XB_TRY(hy_launch(e, hy_glu_kernel<AT>, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, st, U, c.ff, c.ff_limit, act, a2, (long long)l.n_dn, T));
   } else {
@@ -1929,6 +1934,9 @@ static int hy_ff_parallel(xb_engine* e, const HyLayer& l, int T, const void* xin
     } else if (vec && c.ff % 8 == 0 && sf % 8 == 0)
       XB_TRY(hy_launch(e, hy_moe_act_vec_kernel, dim3((unsigned)((n / 8 + 255) / 256)), dim3(256), 0, st, U.h, U.ld, (const float*)hy->gw, ldg, sg_at, c.n_experts,
                        c.ff, c.ff_limit, sf, c.shared_limit, c.ff_act, c.route_input, reinterpret_cast<bf16*>(hy->a2), (long long)l.n_dn, T));
+    else if (few4 && c.ff % 4 == 0 && sf % 4 == 0)
+      XB_TRY(hy_launch(e, hy_moe_act_few_kernel<AT>, dim3((unsigned)((l.n_dn / 4 + 127) / 128), T), dim3(128), 0, st, U, (const float*)hy->gw, ldg, sg_at, c.n_experts, c.ff,
+                       c.ff_limit, sf, c.shared_limit, c.ff_act, c.route_input, a2, (long long)l.n_dn));
     else
       XB_TRY(hy_launch(e, hy_moe_act_kernel<AT>, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, st, U, (const float*)hy->gw, ldg, sg_at, c.n_experts, c.ff,
                        c.ff_limit, sf, c.shared_limit, c.ff_act, c.route_input, a2, (long long)l.n_dn, T));

@@ -18,7 +18,8 @@
 // triangular solve goes token by token.  Bound by instruction issue (about a thousand a chunk and warp, one warp a scheduler) and by that
 // solve.
 // 2048 tokens, 16 heads of 128 x 128 (gated): 741 -> 212 us and 41 us of preparation; 450 and 1350 tokens, 32 heads of 64 x 64
-// (general): 777 -> 218 and 84 us.  Errors against 64 bits as token by token (3.4e-7 and 2.9e-7 after 2047 tokens).
+// (general): 777 -> 218 and 84 us, with launch bounds that leave the walk its registers and the preparation four blocks an SM 206 and 80
+// (gated 211 and 40).  Errors against 64 bits as token by token (3.4e-7 and 2.9e-7 after 2047 tokens).
 #pragma once
 
 #define HY_CT 16          // tokens of a chunk = lanes that share a column
@@ -46,7 +47,7 @@ struct ChunkPart {
 };
 // grid (entries, H), 256 threads; dynamic shared memory: the row vectors (general rule: and the decays) at pitch dkp + 4
 template <int MODE>
-__global__ void __launch_bounds__(256) hy_chunk_prep_kernel(RecurIn in, float* __restrict__ ws, BatchMeta m, ChunkPart part, int n_seqs, int H, int dk,
+__global__ void __launch_bounds__(256, 4) hy_chunk_prep_kernel(RecurIn in, float* __restrict__ ws, BatchMeta m, ChunkPart part, int n_seqs, int H, int dk,
                                                             int dkp) {
   extern __shared__ __align__(16) float cps[];
   __shared__ float gs[HY_CT];
@@ -197,7 +198,7 @@ __device__ __forceinline__ void hy_chunk_reduce(float (&v)[HY_CT][2], int sub) {
 
 // grid (n_seqs, H, ceil(dv / 16)), 128 threads (16 value columns); dynamic shared memory 2 * (block + 16 x 18 values) floats
 template <int NCH, int MODE>
-__global__ void __launch_bounds__(128) hy_chunk_kernel(RecurIn in, const float* __restrict__ ws, float* __restrict__ state, long long state_stride,
+__global__ void __launch_bounds__(128, 1) hy_chunk_kernel(RecurIn in, const float* __restrict__ ws, float* __restrict__ state, long long state_stride,
                                                        float* __restrict__ o, long long ldo, BatchMeta m, ChunkPart part, int H, int dk, int dv) {
   pdl_wait();   // no early trigger, as in hy_recur_kernel
   extern __shared__ __align__(16) float cks[];

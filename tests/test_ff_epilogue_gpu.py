@@ -62,3 +62,19 @@ def test_epilogue_equals_kernel(built_lib, monkeypatch, name, n):
     assert torch.equal(a, b)
   # the sigmoids differ by a few 1e-7, so one activation in some 1e4 rounds to a neighbouring bf16 (2^-8): 4e-5 of a row, a few times that behind a layer
   assert ((a - b).norm() / a.norm()).item() < 2e-4
+
+
+def test_layers_that_share_weights_keep_their_limits(built_lib, monkeypatch):
+  """Two layers over one set of weights, each with a limit of its own: a launch takes its layer's."""
+  from xotorch_support_jetson_b200 import synth
+  from xotorch_support_jetson_b200.models import model_cards
+  hf = copy.deepcopy(model_cards["bibevik-tiny"]["hf_config"])
+  lay = next(l for l in hf["layers"] if l["type"] == "latent_attention")
+  lay.pop("weights_of", None)
+  hf["layers"] = [dict(lay, mlp={"kind": "dense", "ff": 384, "limit": 0.05}), dict(lay, mlp={"kind": "dense", "ff": 384, "limit": 2.0}, weights_of=0)]
+  state = synth.random_bibevik_state(hf, seed=8)
+  got = {}
+  for on in ("0", "1"):
+    monkeypatch.setenv("XB_HY_ACT", on)
+    got[on], _ = _stream(hf, state, 300, "bfloat16")
+  assert ((got["0"] - got["1"]).norm() / got["0"].norm()).item() < 2e-4   # as above

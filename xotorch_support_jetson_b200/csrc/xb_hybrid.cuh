@@ -1287,7 +1287,7 @@ static bool hy_tc_linear(xb_engine* e, const void* x, long long ldx, const bf16*
 static bool hy_act_pays(const xb_engine* e, int T, int N, int K, int n_out) {
   return e->hy->use_act == 2 || xb_wide_act_pays(T, N, K, n_out, e->num_sms);
 }
-// A feed-forward's up Linear of a prompt with its activation in the epilogue: out [T, n_out] (bf16).  `set` completes the plan's arguments.  False: not
+// A feed-forward's up Linear of a prompt with its activation in the epilogue: out [T, n_out] (bf16).  `set` completes a launch's arguments.  False: not
 // applicable (few rows, no tile-major copy, features that do not fill 128-column halves) or not worth it.
 template <typename F>
 static bool hy_act_linear(xb_engine* e, const void* x, long long ldx, const bf16* wt, int T, int N, int K, int n_out, bf16* out, cudaStream_t st, F set, int* rc) {
@@ -1300,10 +1300,12 @@ static bool hy_act_linear(xb_engine* e, const void* x, long long ldx, const bf16
     GemmPlan p;
     const int v = xb_pick_wide(T, N, K, 32, e->num_sms, true);
     if ((*rc = xb_gemm_plan(&p, (const bf16*)x, ldx, wt, 1, T, N, K, out, n_out, nullptr, 0, e->num_sms, v + 1)) != 0) return true;
-    set(p.args);
+    p.args.epi = XB_EPI_PLAIN;
     it = hy->plans.emplace(key, p).first;
   }
-  if ((*rc = run_gemm(e, it->second, st)) != 0) return true;
+  GemmPlan p = it->second;   // layers that share weights share the plan, not the activation's limits
+  set(p.args);
+  if ((*rc = run_gemm(e, p, st)) != 0) return true;
   LAUNCH_COUNT(e);
   return true;
 }

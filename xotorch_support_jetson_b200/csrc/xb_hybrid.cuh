@@ -1629,9 +1629,9 @@ template <typename AT>
 static int hy_row_op_launch(xb_engine* e, int T, const RowOpArgs& a, cudaStream_t st) {
   HyModel* hy = e->hy;
   const bool few = T <= 64 && hy->d.dim >= 1024;   // decode-sized batches: few rows, so more threads per row keep more loads in flight
-  // prompts whose branch is one bf16 matrix out of the tensor-core Linear, in models with grouped norms and the like: eight channels per thread.  (The plain
-  // form is faster four at a time: 2048 rows x 2048 out of L2 16.5 us, eight at a time 20.6.)
-  if (!few && (a.ext || !hy->use_quad || hy->d.dim % 4 != 0) && !a.plain_add && a.m1.h != nullptr && a.m1.bias == nullptr && a.m1.ld % 8 == 0 && a.m2.f == nullptr && a.m2.h == nullptr &&
+  // Prompts whose branch is one bf16 matrix out of the tensor-core Linear: eight channels per thread, with and without `ext`.  (2048 rows x 2048 out of L2 20.6 us;
+  // the four-channel kernel takes 16.5 and adds a row's squares in another order, which moves every later bf16 rounding.)
+  if (!few && !a.plain_add && a.m1.h != nullptr && a.m1.bias == nullptr && a.m1.ld % 8 == 0 && a.m2.f == nullptr && a.m2.h == nullptr &&
       hy->d.dim % 8 == 0)
     return hy_launch(e, hy_row_op_vec_kernel<AT>, dim3(T), dim3(256), (size_t)hy->d.dim * sizeof(float), st, a);
   if (a.ext && !a.plain_add) {   // grouped norms, residual multiplier, plain weights, the norm as a Linear input

@@ -171,14 +171,15 @@ __device__ __forceinline__ bf16* wide_qkv_dst(const GemmArgs& g, int t, long lon
 __device__ __forceinline__ void wide_emit(const GemmArgs& g, int t, const WideQkvRow& r, int n0, int n1, float* x0, float* x1) {
   if (t >= g.a_rows) return;
   if (g.epi == XB_EPI_SILU) {
-    // gate/up rows are interleaved in blocks of 16 features: act = bf16(bf16(silu(gate)) * up).  The quotient by __fdividef (2 ulp, no branches): the exact
-    // one made a tile's epilogue of four warps longer than its products; 373 rows x 3072 -> 2 x 8192 43.1 -> 39.0 us, 192 rows 32.9 -> 28.0, 2048 rows x
-    // 4096 -> 2 x 14336 383 -> 373.  Of 16 M gates of standard deviation 0.5, 2 and 6 none rounds to another bf16; error against 64 bits 1.657e-3 either way.
+    // gate/up rows are interleaved in blocks of 16 features: act = bf16(bf16(silu(gate)) * up).  The exact division's branches made a tile's epilogue of
+    // four warps longer than its products (373 rows x 3072 -> 2 x 8192 43.1 us, without 39.0).  __fdividef has none and is off by two units in the last place; over a
+    // quarter of the denominator, which keeps it below 2^126 where __fdividef would give 0, every one of the 65536 gates that a bf16 can be rounds to the bf16 of
+    // the exact quotient.
     if (n0 >= g.b_rows) return;
 #pragma unroll
     for (int j = 0; j < 16; ++j) {
       const float gg = rbf(x0[j]), uu = rbf(x1[j]);
-      x0[j] = rbf(__fdividef(gg, 1.0f + expf(-gg))) * uu;
+      x0[j] = rbf(__fdividef(0.25f * gg, fmaf(expf(-gg), 0.25f, 0.25f))) * uu;
     }
     epi_store16(reinterpret_cast<bf16*>(g.out) + (long long)t * g.ld_out + (n0 >> 1), x0);
   } else if (g.epi == XB_EPI_QKV) {

@@ -39,12 +39,7 @@ template <typename AT> __device__ __forceinline__ float act_load(const AT* p);
 template <> __device__ __forceinline__ float act_load<float>(const float* p) { return *p; }
 template <> __device__ __forceinline__ float act_load<bf16>(const bf16* p) { return bf2f(*p); }
 
-__device__ __forceinline__ float hy_sigmoid(float x) { return 1.0f / (1.0f + expf(-x)); }
-__device__ __forceinline__ float hy_silu(float x) { return x / (1.0f + expf(-x)); }
 __device__ __forceinline__ float hy_softplus(float x) { return x > 20.0f ? x : log1pf(expf(x)); }
-__device__ __forceinline__ float hy_gelu_tanh(float z) {
-  return 0.5f * z * (1.0f + tanhf(0.7978845608028654f * (z + 0.044715f * z * z * z)));
-}
 
 // first row, length, first position and slot of the sequence with index s
 struct SeqSpan { int start, len, pos0, slot; };
@@ -2986,20 +2981,6 @@ __global__ void __launch_bounds__(512) hy_gla_token_kernel(LinOut P, int off_q, 
 }
 
 // ----------------------------------------------------------------------------- clamped gated feed-forward, experts
-__device__ __forceinline__ float hy_glu_clamp(float g, float u, float limit) {
-  g = fminf(g, limit);
-  u = fminf(fmaxf(u, -limit), limit);
-  return g * hy_sigmoid(1.702f * g) * (u + 1.0f);
-}
-// One channel of one expert with routing weight w.  act: XB_ACT_GLU_CLAMP, XB_ACT_SWIGLU (silu(g) u) or XB_ACT_GEGLU (gelu(g) u,
-// tanh form), the last two without limits.
-// on_input: the weight multiplies what the expert reads, and since both projections are linear, (w h) W^T = w (h W^T):
-// gate and up are scaled before the activation; otherwise the weight multiplies the activation (and so the output).
-__device__ __forceinline__ float hy_expert_act(float g, float u, float w, float limit, int act, int on_input) {
-  if (on_input) { g *= w; u *= w; }
-  const float y = act == XB_ACT_SWIGLU ? hy_silu(g) * u : (act == XB_ACT_GEGLU ? hy_gelu_tanh(g) * u : hy_glu_clamp(g, u, limit));
-  return on_input ? y : w * y;
-}
 // The shared expert's weight: entry `at` of the routing row (behind the router's outputs), or one (at < 0).
 __device__ __forceinline__ float hy_shared_weight(const float* gwrow, int at) { return at >= 0 ? gwrow[at] : 1.0f; }
 // U carries [gate (F) | up (F)] (biases on read): out[t, i] = act(gate_i, up_i) (XB_ACT_*, see above).  grid over T * F.

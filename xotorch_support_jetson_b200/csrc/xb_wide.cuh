@@ -227,9 +227,21 @@ __device__ __forceinline__ void wide_emit(const GemmArgs& g, int t, const WideQk
 // ---- the feed-forwards of hybrid models (ACT = 1): gate and up of the same 128 features are the two halves of a 256-column tile, so the activation leaves
 // from the epilogue in one piece and the matrix of gate and up rows is never written.  1800 rows x 2048 -> 2 x 8192, us: 111.5 with a kernel that read it,
 // 97.6 now (the products alone 91.2), experts 106.8 -> 95.6; 192 rows 26.9 -> 20.8.
-// 1 / (1 + e^-x), the quotient by __fdividef (2 ulp, no branches): four warps finish a tile while the next one is multiplied, and with the exact division
-// they took longer than that (110.7 us).
-__device__ __forceinline__ float wide_sigmoid(float x) { return __fdividef(1.0f, 1.0f + expf(-x)); }
+// Four warps finish a tile while the next one is multiplied; with the division's branches, one an element, they took longer than that (110.7 us).  Results have the
+// bits of hy_glu_vec_kernel and hy_moe_act_vec_kernel, so a row's do not hang on which of the two its step takes; the divisions are made without branches: 1 / d by one Newton step on the approximate reciprocal, which for every d from 1 to 2^126 is the correctly rounded one
+// (all 126 * 2^23 of them compared), and from it a / d = q + (a - d q) / d with q = a / d rounded (Markstein 1990), correctly rounded as well.  Sixteen
+// elements of which one is beyond `WIDE_NEAR` (d could leave that range, or a / d the normal numbers) take the divisions themselves.
+#define WIDE_NEAR 32.f
+__device__ __forceinline__ float wide_recip(float d) {
+  const float r = __fdividef(1.0f, d);
+  return fmaf(r, fmaf(-d, r, 1.0f), r);
+}
+__device__ __forceinline__ bool wide_near(const float* x) {
+  float far = 0.f;
+#pragma unroll
+  for (int j = 0; j < 16; ++j) far = fmaxf(far, fabsf(x[j]));
+  return far < WIDE_NEAR;
+}
 // first gate row (or up row) of the 128 features of tile tb
 __device__ __forceinline__ int wide_glu_row(const GemmArgs& g, int tb, bool up) {
   const int i = tb * 128, routed = g.glu_e * g.glu_f;
@@ -242,40 +254,48 @@ __device__ __forceinline__ int wide_glu_row(const GemmArgs& g, int tb, bool up) 
 __device__ __forceinline__ void wide_emit_glu(const GemmArgs& g, int t, int f0, int n0, int n1, float w, bool shared, float* x0, float* x1) {
   if (t >= g.a_rows) return;
   const float limit = shared ? g.glu_limit_s : g.glu_limit;
+  const bool on_input = g.glu_on_input && !shared;
 #pragma unroll
   for (int j = 0; j < 16; ++j) { x0[j] = rbf(x0[j]); x1[j] = rbf(x1[j]); }   // what the Linear hands on is bf16, here as in steps of other kernels
   if (g.glu_bias != nullptr) {
 #pragma unroll
     for (int j = 0; j < 16; ++j) { x0[j] += g.glu_bias[n0 + j]; x1[j] += g.glu_bias[n1 + j]; }
   }
-  if (g.glu_on_input && !shared) {   // (w h) W^T = w (h W^T)
+  if (on_input) {   // (w h) W^T = w (h W^T)
 #pragma unroll
     for (int j = 0; j < 16; ++j) { x0[j] *= w; x1[j] *= w; }
   }
   if (w == 0.f && !shared) {         // an expert that the token does not use
 #pragma unroll
     for (int j = 0; j < 16; ++j) x0[j] = 0.f;
-  } else if (g.glu_act == XB_ACT_SWIGLU) {
-#pragma unroll
-    for (int j = 0; j < 16; ++j) x0[j] = x0[j] * wide_sigmoid(x0[j]) * x1[j];
   } else if (g.glu_act == XB_ACT_GEGLU) {
 #pragma unroll
-    for (int j = 0; j < 16; ++j) {   // the tanh form: 0.5 (1 + tanh y) = 1 / (1 + e^-2y)
-      const float z = x0[j];
-      x0[j] = z * wide_sigmoid(1.5957691216057308f * (z + 0.044715f * z * z * z)) * x1[j];
+    for (int j = 0; j < 16; ++j) x0[j] = hy_gelu_tanh(x0[j]) * x1[j];
+  } else if (g.glu_act == XB_ACT_SWIGLU) {
+    if (wide_near(x0)) {
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        const float d = 1.0f + expf(-x0[j]), r = wide_recip(d), q = x0[j] * r;
+        x0[j] = fmaf(fmaf(-d, q, x0[j]), r, q) * x1[j];
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < 16; ++j) x0[j] = hy_silu(x0[j]) * x1[j];
     }
   } else {
 #pragma unroll
-    for (int j = 0; j < 16; ++j) {
-      const float a = fminf(x0[j], limit), u = fminf(fmaxf(x1[j], -limit), limit);
-      x0[j] = a * wide_sigmoid(1.702f * a) * (u + 1.0f);
+    for (int j = 0; j < 16; ++j) x0[j] = fminf(x0[j], limit);
+    if (wide_near(x0)) {
+#pragma unroll
+      for (int j = 0; j < 16; ++j) x0[j] = x0[j] * wide_recip(1.0f + expf(-(1.702f * x0[j]))) * (fminf(fmaxf(x1[j], -limit), limit) + 1.0f);
+    } else {
+#pragma unroll
+      for (int j = 0; j < 16; ++j) x0[j] = hy_glu_clamp(x0[j], x1[j], limit);
     }
   }
-  if (!g.glu_on_input || shared) {
-    if (w != 1.f) {
+  if (!on_input && w != 1.f) {
 #pragma unroll
-      for (int j = 0; j < 16; ++j) x0[j] *= w;
-    }
+    for (int j = 0; j < 16; ++j) x0[j] *= w;
   }
   epi_store16(reinterpret_cast<bf16*>(g.out) + (long long)t * g.ld_out + f0, x0);
 }

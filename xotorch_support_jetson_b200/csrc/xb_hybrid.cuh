@@ -1645,8 +1645,8 @@ static int hy_row_op_launch(xb_engine* e, int T, const RowOpArgs& a, cudaStream_
   if (few) {
     bool ok = hy->use_quad && hy->d.dim % 4 == 0 && (a.bw == nullptr || hy_quad_ptr(a.bw)) && (a.nw == nullptr || a.nw_mode == 2 || hy_quad_ptr(a.nw));
     for (const LinOut* o : ms) ok = ok && ((o->f == nullptr && o->h == nullptr) || hy_planes4(*o, 0));
-    if (ok && hy->d.dim <= 2048) return hy_launch(e, hy_row_op_few_kernel<AT, 512, 1, 8>, dim3(T), dim3(512), 0, st, a);
-    if (ok && hy->d.dim <= 4096) return hy_launch(e, hy_row_op_few_kernel<AT, 512, 2, 4>, dim3(T), dim3(512), 0, st, a);
+    if (ok && hy->d.dim <= 2048) return hy_launch(e, hy_row_op_few_kernel<AT, 1, 8>, dim3(T), dim3(512), 0, st, a);
+    if (ok && hy->d.dim <= 4096) return hy_launch(e, hy_row_op_few_kernel<AT, 2, 4>, dim3(T), dim3(512), 0, st, a);
     return hy_launch(e, hy_row_op_kernel<AT, 1024>, dim3(T), dim3(1024), (size_t)hy->d.dim * sizeof(float), st, a);
   }
   return hy_launch(e, hy_row_op_kernel<AT, 256>, dim3(T), dim3(256), (size_t)hy->d.dim * sizeof(float), st, a);

@@ -299,11 +299,11 @@ __global__ void __launch_bounds__(256) hy_gdelta_prep_quad_kernel(LinOut P, int 
 }
 
 // hy_row_op_kernel for steps of few rows: a thread holds four neighbouring channels per VPT from the loads to the stores, so a row costs one trip for
-// planes and stream, two barriers and the stores.  What waits for no kernel (weights, plane counts) is fetched ahead of the wait.  The general kernel
+// planes and stream, four barriers and the stores; sums and squares add up in the general kernel's order, bit for bit.  What waits for no kernel (weights, plane counts) is fetched ahead of the wait.  The general kernel
 // reads stream and weights behind its first sum, weights again behind the second, keeps the row in shared memory, and its 1024 threads of 64 registers
 // take a whole SM: the next Linear's block cannot come in beside them and starts its weights when the norm is done.
 // The bound of one block an SM keeps F planes of four channels in flight (see xb_resid_norm_row_kernel).  Eight chats of three bibevik-1b layers (four such
-// kernels a token) 4386 -> 4243 us.
+// kernels a token) 4386 -> 4243 us; with an order of its own for the squares and two barriers it took the same.
 template <int F>
 __device__ __forceinline__ void lin_planes4(const LinOut& o, long long row, int col, int planes, float* v) {   // lin_at's order of planes
   float b[4] = {0.f, 0.f, 0.f, 0.f};
@@ -339,44 +339,71 @@ __device__ __forceinline__ void lin_planes4(const LinOut& o, long long row, int 
 __device__ __forceinline__ int lin_planes(const LinOut& o, int col) {
   return o.f == nullptr ? 0 : o.si.splits == 0 ? 1 : xb_n_segments(o.si, col);
 }
-template <int NT>
-__device__ __forceinline__ float row_sum_once(float v, float* red) {   // block_sum with one barrier: `red` (32 floats) is used once
-  v = warp_sum(v);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+// The sum of squares of a row of up to 2 VPT * 1024 channels in the order of hy_row_op_kernel<., 1024>: its thread i adds the channels i, i + 1024, ..; then warps,
+// then their sums.  Here thread q of each half of 512 threads holds VPT pieces of the channels 4 q .. 4 q + 3 (mod 1024), the upper half carrying on where the
+// lower one stops, and thread i is element i & 3 of eight neighbouring lanes.  v: zeros where the row has ended (n[it] false).
+template <int VPT>
+__device__ __forceinline__ float row_sum_1024(const float (&v)[VPT][4], const bool (&n)[VPT], float4* low, float* red) {
+  const int q = threadIdx.x & 255;
+  float s[4] = {0.f, 0.f, 0.f, 0.f};
+  auto add = [&]() {
+#pragma unroll
+    for (int it = 0; it < VPT; ++it)
+      if (n[it]) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) s[j] = fmaf(v[it][j], v[it][j], s[j]);
+      }
+  };
+  if (threadIdx.x < 256) {
+    add();
+    low[q] = make_float4(s[0], s[1], s[2], s[3]);
+  }
   __syncthreads();
-  return warp_sum((threadIdx.x & 31) < NT / 32 ? red[threadIdx.x & 31] : 0.f);
+  if (threadIdx.x >= 256) {
+    const float4 l = low[q];
+    s[0] = l.x; s[1] = l.y; s[2] = l.z; s[3] = l.w;
+    add();
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) s[j] += __shfl_xor_sync(0xffffffffu, s[j], o);
+    if ((q & 7) == 0) red[q >> 3] = (s[0] + s[2]) + (s[1] + s[3]);
+  }
+  __syncthreads();
+  return warp_sum(red[threadIdx.x & 31]);
 }
 
-template <typename AT, int NT, int VPT, int F>
-__global__ void __launch_bounds__(NT, 1) hy_row_op_few_kernel(RowOpArgs a) {
+template <typename AT, int VPT, int F>
+__global__ void __launch_bounds__(512, 1) hy_row_op_few_kernel(RowOpArgs a) {
   pdl_launch_dependents();
+  __shared__ float4 low[256];   // used once a sum, with two barriers between
   __shared__ float red[2][32];
   const long long t = blockIdx.x;
-  const int D = a.D;
+  const int D = a.D, c0 = (threadIdx.x >> 8) * VPT * 1024 + (threadIdx.x & 255) * 4;
   const bool branch = a.m1.f != nullptr || a.m1.h != nullptr, two = a.m2.f != nullptr || a.m2.h != nullptr, three = a.m3.f != nullptr || a.m3.h != nullptr;
   float bw[VPT][4], nw[VPT][4], x[VPT][4], v[VPT][4];
   int n1[VPT], n2[VPT], n3[VPT];
+  bool in[VPT];
 #pragma unroll
   for (int it = 0; it < VPT; ++it) {
-    const int c = (it * NT + threadIdx.x) * 4;
-    const bool in = c < D;
+    const int c = c0 + it * 1024;
+    in[it] = c < D;
 #pragma unroll
     for (int j = 0; j < 4; ++j) bw[it][j] = nw[it][j] = x[it][j] = v[it][j] = 0.f;
-    if (in && branch && !a.plain_add) hy_quad_f(a.bw + c, bw[it]);
-    if (in && a.nw != nullptr) {
+    if (in[it] && branch && !a.plain_add) hy_quad_f(a.bw + c, bw[it]);
+    if (in[it] && a.nw != nullptr) {
       if (a.nw_mode == 2) nw[it][0] = nw[it][1] = nw[it][2] = nw[it][3] = a.nw[0];
       else hy_quad_f(a.nw + c, nw[it]);
     }
-    n1[it] = in && branch ? lin_planes(a.m1, c) : 0;
-    n2[it] = in && two ? lin_planes(a.m2, c) : 0;
-    n3[it] = in && three ? lin_planes(a.m3, c) : 0;
+    n1[it] = in[it] && branch ? lin_planes(a.m1, c) : 0;
+    n2[it] = in[it] && two ? lin_planes(a.m2, c) : 0;
+    n3[it] = in[it] && three ? lin_planes(a.m3, c) : 0;
   }
   pdl_wait();
-  float ss = 0.f;
 #pragma unroll
   for (int it = 0; it < VPT; ++it) {
-    const int c = (it * NT + threadIdx.x) * 4;
-    if (c >= D) break;
+    const int c = c0 + it * 1024;
+    if (!in[it]) break;
     hy_quad_f(a.x + t * D + c, x[it]);
     if (branch) {
       float u[4];
@@ -394,29 +421,28 @@ __global__ void __launch_bounds__(NT, 1) hy_row_op_few_kernel(RowOpArgs a) {
         for (int j = 0; j < 4; ++j) v[it][j] += u[j];
       }
     }
-#pragma unroll
-    for (int j = 0; j < 4; ++j) ss += v[it][j] * v[it][j];
   }
-  const float inv = branch && !a.plain_add ? 1.0f / sqrtf(row_sum_once<NT>(ss, red[0]) / (float)D + a.eps) : 0.f;
-  float s2 = 0.f;
+  const float inv = branch && !a.plain_add ? 1.0f / sqrtf(row_sum_1024<VPT>(v, in, low, red[0]) / (float)D + a.eps) : 0.f;
 #pragma unroll
   for (int it = 0; it < VPT; ++it) {
-    const int c = (it * NT + threadIdx.x) * 4;
-    if (c >= D) break;
+    const int c = c0 + it * 1024;
+    if (!in[it]) break;
+    if (branch && a.plain_add) {
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      if (branch) x[it][j] += a.plain_add ? v[it][j] : v[it][j] * inv * (bw[it][j] + a.bw_one);
-      s2 += x[it][j] * x[it][j];
+      for (int j = 0; j < 4; ++j) x[it][j] += v[it][j];
+    } else if (branch) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) x[it][j] = fmaf(v[it][j] * inv, bw[it][j] + a.bw_one, x[it][j]);   // as hy_row_op_kernel's line comes out
     }
     if (branch) hy_quad_st(a.x + t * D + c, x[it]);
     if (a.xa != nullptr) hy_quad_st(reinterpret_cast<AT*>(a.xa) + t * D + c, x[it]);
   }
   if (a.nw == nullptr) return;
-  const float inv2 = 1.0f / sqrtf(row_sum_once<NT>(s2, red[1]) / (float)D + a.eps);
+  const float inv2 = 1.0f / sqrtf(row_sum_1024<VPT>(x, in, low, red[1]) / (float)D + a.eps);
 #pragma unroll
   for (int it = 0; it < VPT; ++it) {
-    const int c = (it * NT + threadIdx.x) * 4;
-    if (c >= D) break;
+    const int c = c0 + it * 1024;
+    if (!in[it]) break;
     float h[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) h[j] = x[it][j] * inv2 * (a.nw_mode == 0 ? 1.0f + nw[it][j] : nw[it][j]);

@@ -1,14 +1,15 @@
 """Latent attention in steps of few rows (a row a block: hy_latent_absorb_row_kernel, the read-out's early weights) against the same rows in a wider step, at
-sizes around what a thread fetches ahead (64 rows of keys' weights, 256 latent columns, 128 value channels) and at latent widths that take the older kernel."""
+sizes around what a thread fetches ahead (64 rows of keys' weights, 512 latent columns, 128 value channels) and at a latent width that takes the older kernel.  In
+float32 a row has the same bits in both: its sums do not hang on how many rows the step has."""
 import pytest
 import torch
 
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("dim,rank,vdim", [(64, 256, 128), (24, 48, 40), (72, 264, 136), (8, 16, 8), (130, 512, 64), (24, 44, 40)])
-@pytest.mark.parametrize("dtype,tol", [("float32", 1e-5), ("bfloat16", 2e-2)])   # fp32 sums in other orders; in bf16 every later rounding may fall the other way
-def test_few_rows_equal_many(built_lib, dim, rank, vdim, dtype, tol):
+@pytest.mark.parametrize("dim,rank,vdim", [(64, 256, 128), (24, 48, 40), (72, 264, 136), (8, 16, 8), (130, 512, 64), (24, 44, 40), (24, 45, 40)])
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+def test_few_rows_equal_many(built_lib, dim, rank, vdim, dtype):
   from xotorch_support_jetson_b200 import model_config, synth
   from xotorch_support_jetson_b200.models import model_cards
   from xotorch_support_jetson_b200.shard import Shard
@@ -39,4 +40,7 @@ def test_few_rows_equal_many(built_lib, dim, rank, vdim, dtype, tol):
   many = run([range(n)])
   few = run([range(0, 1), range(1, 4), range(4, 20)])
   assert torch.isfinite(few).all()
-  assert ((few - many).norm(dim=1) / many.norm(dim=1)).max() < tol
+  if dtype == "float32":
+    assert torch.equal(few, many)
+  # bf16 steps share their keys out by the step's rows: fp32 sums in another order, after which a rounding (2^-9) of any of the layer's activations may fall the other way
+  assert ((few - many).norm(dim=1) / many.norm(dim=1)).max() < 2 ** -7

@@ -1746,8 +1746,8 @@ static int hy_latent_mixer(xb_engine* e, const HyLayer& l, int T, const LinOut& 
   if (tiles && Q.h != nullptr && Q.bias == nullptr && Q.ld % 8 == 0 && l.off_q % 8 == 0)
     XB_TRY(hy_launch(e, hy_latent_absorb_mma_kernel, dim3((T + HY_HG_M - 1) / HY_HG_M, H, (R + HY_HG_N - 1) / HY_HG_N), dim3(128), 0, st, Q.h + l.off_q,
                      Q.ld, dr, (const bf16*)l.w_uk, hy->qa, H, T, n, R, r, m.tok_pos));
-  else if (mr == 1 && R % 8 == 0 && (size_t)(n + 3 + 8 * R) * sizeof(float) <= 48 * 1024 && (reinterpret_cast<uintptr_t>(l.w_uk) & 15) == 0)
-    XB_TRY(hy_launch(e, hy_latent_absorb_row_kernel, dim3(T, H), dim3(256), (size_t)(((n + 3) & ~3) + 8 * R) * sizeof(float), st, Q, l.off_q, dr,
+  else if (mr == 1 && R % 2 == 0 && R <= 512)
+    XB_TRY(hy_launch(e, hy_latent_absorb_row_kernel, dim3(T, H), dim3(R <= 256 ? 256 : 384), (size_t)(n > 64 ? n : 64) * sizeof(float), st, Q, l.off_q, dr,
                      (const bf16*)l.w_uk, hy->qa, H, n, R, r, m.tok_pos));
   else if (mr == 1)
     XB_TRY(hy_launch(e, hy_latent_absorb_kernel<1>, dim3(T, H), dim3(256), mm1, st, Q, l.off_q, dr, (const bf16*)l.w_uk, hy->qa, H, T, n, R, r, m.tok_pos));

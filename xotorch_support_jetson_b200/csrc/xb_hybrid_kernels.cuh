@@ -2412,7 +2412,7 @@ __global__ void __launch_bounds__(NT) hy_latent_down_kernel(LinOut P, int off_dk
 // Queries in the cache's space.  Q carries H heads of [K unrotated | dr rotated] (columns from qoff); per head
 //   qa[t, h, n]     = sum_k Q[t, h, k] * W[(h * K + k) * N + n]     n < N: the query folded into the latent space
 //   qa[t, h, N + i] = rot(rotated part)[i]                          i < dr
-// grid (ceil(T / ROWS), H), 256 threads over n; the rows' inputs sit in shared memory (ROWS * K floats).  One row a block and N a multiple of eight:
+// grid (ceil(T / ROWS), H), 256 threads over n; the rows' inputs sit in shared memory (ROWS * K floats).  One row a block and N even:
 // hy_latent_absorb_row_kernel.
 #define HY_MM_ROWS 8
 template <int ROWS>
@@ -2458,69 +2458,71 @@ __global__ void __launch_bounds__(256) hy_latent_absorb_kernel(LinOut Q, int qof
     for (int rr = 0; rr < nt; ++rr) qa[((long long)(t0 + rr) * H + h) * ld + n] = acc[rr];
   }
 }
-// The same for one row a block (steps of few rows), N a multiple of eight: a warp takes every eighth k, a lane eight neighbouring n.  All weights of K <= 64 are on
-// their way before the kernel before this one is done (the launch bound leaves them the registers: 32 a thread spilled without it); one column a thread, eight
-// k's at a time, took eight trips to memory behind the wait (8 tokens, 16 heads of 64 x 256: 12.8 -> 5.1 us cold).  grid (T, H), 256 threads; K + 8 N floats of shared memory.
-__global__ void __launch_bounds__(256, 2) hy_latent_absorb_row_kernel(LinOut Q, int qoff, int dr, const bf16* __restrict__ W, float* __restrict__ qa, int H, int K, int N,
+// The same for one row a block (steps of few rows), N even and at most 512: a thread owns two neighbouring n and adds over k in order, as the kernel above does, so
+// a row's numbers do not hang on how many rows the step has.  All weights of K <= 64 are on their way before the kernel before this one is done; one column a thread,
+// eight k's at a time, took eight trips to memory behind the wait.  The last 128 threads fetch the inputs and rotate: with the rotation between the weights' fetch
+// and their use the compiler spilled them (12.6 us).  128 registers (the bound of 512 threads) and 256 threads where N <= 256 leave room for two blocks an SM.
+// 8 tokens, 16 heads of 64 x 256, back to back 8.5 -> 5.2 us (the kernel above, this one); 64 x 512 10.5 -> 6.3; 16 tokens 7.4 -> 6.3.
+// grid (T, H), 128 threads and 128 (N <= 256) or 256 for the columns; max(K, 64) floats of shared memory.
+__global__ void __launch_bounds__(512, 1) hy_latent_absorb_row_kernel(LinOut Q, int qoff, int dr, const bf16* __restrict__ W, float* __restrict__ qa, int H, int K, int N,
                                                                       RotArgs r, const int* __restrict__ tok_pos) {
   pdl_launch_dependents();
-  extern __shared__ __align__(16) float xsm[];
-  float* part = xsm + ((K + 3) & ~3);
-  const int t = blockIdx.x, h = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  extern __shared__ __align__(16) float xsm[];   // the row's K inputs, room for PRE
+  constexpr int PRE = 64;
+  const int t = blockIdx.x, h = blockIdx.y, nw = blockDim.x - 128;
   const int qh = qoff + h * (K + dr), ld = N + dr;
-  const bf16* Wh = W + (long long)h * K * N;
-  constexpr int PRE = 8;
-  uint4 pre[PRE];
-#pragma unroll
-  for (int i = 0; i < PRE; ++i)
-    pre[i] = warp + 8 * i < K && lane * 8 < N ? *reinterpret_cast<const uint4*>(Wh + (long long)(warp + 8 * i) * N + lane * 8) : make_uint4(0u, 0u, 0u, 0u);
-  pdl_wait();
-  for (int k = threadIdx.x; k < K; k += 256) {
-    const int col[1] = {qh + k};
-    float v[1];
-    lin_at_cols<1, 8>(Q, t, col, v);
-    xsm[k] = v[0];
-  }
-  const int half = r.dims >> 1, per = dr - half;
   float* qd = qa + ((long long)t * H + h) * ld;
-  for (int i = 255 - threadIdx.x; i < per; i += 256) {   // by the threads that have no k where K is small
-    if (i < half) {
-      const int d0 = r.half ? i : 2 * i, d1 = r.half ? i + half : 2 * i + 1;
-      const int col[2] = {qh + K + d0, qh + K + d1};
-      float ab[2], cs, sn;
-      lin_at_cols<2, 8>(Q, t, col, ab);
-      hy_rot_cs(r, tok_pos[t], i, &cs, &sn);
-      qd[N + d0] = ab[0] * cs - ab[1] * sn;
-      qd[N + d1] = ab[1] * cs + ab[0] * sn;
-    } else {
-      qd[N + half + i] = lin_at(Q, t, qh + K + half + i);
+  if ((int)threadIdx.x >= nw) {
+    const int u = threadIdx.x - nw, half = r.dims >> 1, per = dr - half;
+    pdl_wait();
+    for (int k = u; k < K; k += 128) {
+      const int col[1] = {qh + k};
+      float v[1];
+      lin_at_cols<1, 8>(Q, t, col, v);
+      xsm[k] = v[0];
     }
-  }
-  __syncthreads();
-  for (int n = lane * 8; n < N; n += 256) {
-    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    auto add = [&](uint4 u, float x) {
-      const float2 a = bf2_to_f2(u.x), b = bf2_to_f2(u.y), c = bf2_to_f2(u.z), d = bf2_to_f2(u.w);
-      acc[0] = fmaf(x, a.x, acc[0]); acc[1] = fmaf(x, a.y, acc[1]); acc[2] = fmaf(x, b.x, acc[2]); acc[3] = fmaf(x, b.y, acc[3]);
-      acc[4] = fmaf(x, c.x, acc[4]); acc[5] = fmaf(x, c.y, acc[5]); acc[6] = fmaf(x, d.x, acc[6]); acc[7] = fmaf(x, d.y, acc[7]);
-    };
-    int k = warp;
-    if (n == lane * 8) {
-#pragma unroll
-      for (int i = 0; i < PRE; ++i, k += 8)
-        if (k < K) add(pre[i], xsm[k]);
+    __syncthreads();
+    for (int i = u; i < per; i += 128) {
+      if (i < half) {
+        const int d0 = r.half ? i : 2 * i, d1 = r.half ? i + half : 2 * i + 1;
+        const int col[2] = {qh + K + d0, qh + K + d1};
+        float ab[2], cs, sn;
+        lin_at_cols<2, 8>(Q, t, col, ab);
+        hy_rot_cs(r, tok_pos[t], i, &cs, &sn);
+        qd[N + d0] = ab[0] * cs - ab[1] * sn;
+        qd[N + d1] = ab[1] * cs + ab[0] * sn;
+      } else {
+        qd[N + half + i] = lin_at(Q, t, qh + K + half + i);
+      }
     }
-    for (; k < K; k += 8) add(*reinterpret_cast<const uint4*>(Wh + (long long)k * N + n), xsm[k]);
-    *reinterpret_cast<float4*>(part + warp * N + n) = make_float4(acc[0], acc[1], acc[2], acc[3]);
-    *reinterpret_cast<float4*>(part + warp * N + n + 4) = make_float4(acc[4], acc[5], acc[6], acc[7]);
+    return;
   }
-  __syncthreads();
-  for (int n = threadIdx.x; n < N; n += 256) {
-    float s = part[n];
+  const int n = threadIdx.x * 2;
+  const bf16* Wn = W + (long long)h * K * N + (n < N ? n : 0);
+  uint32_t pre[PRE];
 #pragma unroll
-    for (int w = 1; w < 8; ++w) s += part[w * N + n];
-    qd[n] = s;
+  for (int k = 0; k < PRE; ++k) pre[k] = *reinterpret_cast<const uint32_t*>(Wn + (long long)(k < K ? k : K - 1) * N);
+  pdl_wait();
+  __syncthreads();
+  if (n >= N) return;
+  float a0 = 0.f, a1 = 0.f;
+  auto add = [&](uint32_t u, float x) {
+    const float2 w = bf2_to_f2(u);
+    a0 = fmaf(x, w.x, a0);
+    a1 = fmaf(x, w.y, a1);
+  };
+#pragma unroll
+  for (int k = 0; k < PRE; k += 4) {
+    const float4 x = *reinterpret_cast<const float4*>(xsm + k);
+    if (k < K) add(pre[k], x.x);
+    if (k + 1 < K) add(pre[k + 1], x.y);
+    if (k + 2 < K) add(pre[k + 2], x.z);
+    if (k + 3 < K) add(pre[k + 3], x.w);
   }
+#pragma unroll 8
+  for (int k = PRE; k < K; ++k) add(*reinterpret_cast<const uint32_t*>(Wn + (long long)k * N), xsm[k]);
+  qd[n] = a0;      // (rows of N + dr floats: not on 8 bytes where dr is odd)
+  qd[n + 1] = a1;
 }
 // Per-head products with a weight that is stored head by head,
 // plain form (a latent read-out turned into the head's value): y[t, h * N + n] = sum_k x[t, h * K + k] * W[(h * N + n) * K + k]

@@ -41,3 +41,23 @@ def test_four_columns_equal_one(built_lib, monkeypatch, model, change, dtype, to
     st.close()
   assert torch.isfinite(outs[0]).all()
   assert ((outs[0] - outs[1]).norm() / outs[1].norm()).item() < tol
+
+
+@pytest.mark.parametrize("n", [65535, 65536])
+def test_logits_of_more_rows_than_a_grid_has(built_lib, n):
+  """A program may ask for the logits of any number of rows, the same one several times."""
+  from xotorch_support_jetson_b200 import model_config, synth
+  from xotorch_support_jetson_b200.models import model_cards
+  from xotorch_support_jetson_b200.shard import Shard
+  from xotorch_support_jetson_b200.stage import StageRuntime
+  hf = copy.deepcopy(model_cards["bibevik-tiny"]["hf_config"])
+  hf["vocab"], hf["layers"] = 64, hf["layers"][:1]
+  w = synth.random_bibevik_state(hf, seed=4)
+  cfg = model_config.hybrid_model_config(hf)
+  model_config.resolve_tensor_sizes(cfg, {k: tuple(v.shape) for k, v in w.items()})
+  st = StageRuntime(Shard("rows-test", 0, 0, 1), cfg, max_batch_tokens=64, max_seqs=1, max_tokens_per_seq=8, dtype="bfloat16", max_logit_rows=n)
+  st.load_state(w)
+  ids = torch.randint(0, hf["vocab"], (4,), generator=torch.Generator().manual_seed(1)).to("cuda", torch.int32)
+  got = st.forward([0], [4], [0], tokens=ids, want_rows=[i % 4 for i in range(n)]).clone()
+  assert torch.isfinite(got).all() and torch.equal(got, got[:4].repeat((n + 3) // 4, 1)[:n])
+  st.close()

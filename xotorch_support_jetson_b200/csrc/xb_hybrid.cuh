@@ -1809,7 +1809,7 @@ static int hy_run_head(xb_engine* e, int n_seqs, const BatchMeta& m, cudaStream_
     XB_TRY(hy_launch(e, hy_gather_rows_kernel<AT>, dim3(n), dim3(256), 0, st, (const float*)hy->hn, idx, reinterpret_cast<AT*>(hy->head_in), D));
   XB_TRY(hy_linear<AT>(e, in, D, hy->head, hy->t_head, nullptr, n, d.vocab, D, hy->head_raw, hy->cap_head, st, &y));
   const long long tot = (long long)n * d.vocab;
-  if (hy->use_quad && d.vocab % 4 == 0 && hy_planes4(y, 0) && hy_quad_ptr(e->logits))
+  if (hy->use_quad && n <= 65535 && d.vocab % 4 == 0 && hy_planes4(y, 0) && hy_quad_ptr(e->logits))   // a row a grid row, of which there are 65535
     return hy_launch(e, hy_logits_few_kernel, dim3((unsigned)((d.vocab / 4 + 255) / 256), n), dim3(256), 0, st, y, d.logit_softcap, e->logits, d.vocab);
   return hy_launch(e, hy_logits_kernel, dim3((unsigned)((tot + 255) / 256)), dim3(256), 0, st, y, d.logit_softcap, e->logits, n, d.vocab);
 }

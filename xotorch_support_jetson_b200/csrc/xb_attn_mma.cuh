@@ -687,7 +687,8 @@ __global__ void __launch_bounds__(192, 2) xb_attn_prefill_tc_kernel(
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(q_ready + 1);
   int* s_pages = reinterpret_cast<int*>(tmem_slot + 2);   // [XB_ATT_PG_CACHE] prefetched page ids
 
-  // A prompt's last tiles see the most keys: they start first, so that what ends last is short.  What waits for no kernel (metadata, page ids, barriers, TMEM) comes
+  // A prompt's last tiles see the most keys: they start first, so that what ends last is short.  (In a batch the sequences start from the last one, whatever their
+  // lengths.)  What waits for no kernel (metadata, page ids, barriers, TMEM) comes
   // ahead of the wait, which the warps that read q, k and v take themselves.  733 rows, 28 heads: 26 -> 23.4 us.
   const int tile = gridDim.x - 1 - blockIdx.x, kvh = blockIdx.y;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;

@@ -886,7 +886,7 @@ static int launch_resid_norm(xb_engine* e, const GemmPlan* gp, int T, const bf16
   const xb_model_desc& d = e->d;
   const size_t smem = (size_t)d.dim * sizeof(float);
   if (gp->args.mode == XB_GEMM_SKINNY) {
-    // decode-sized batches: one 1024-thread block per row
+    // decode-sized batches: one block per row
     if (d.dim % 4 == 0 && d.dim <= 1024 * 4 * 2) {
       // As many threads as a row has groups of four columns: the warps left out would add zeros.
 #define XB_RN_CASE(NT, VPT, F)                                                                                                                        \

@@ -499,7 +499,7 @@ static int xb_wide_run(const GemmPlan& p, cudaStream_t st, int pdl);
 // Depth of the shared-memory pipeline of the skinny (decode) Linear by token-column width.  Every stage is a 16 KB box
 // of weights plus the token tile; the stages a block can fill before the upstream grid is done are what keeps HBM
 // busy across the kernel boundary, while a block too large to share the SM with its neighbours in the stream loses
-// that overlap again.  Measured on the graph-replayed 8B step (ms per step; profiles/r02_decode_ab_stages.txt):
+// that overlap again.  Measured on the graph-replayed 8B step (ms per step):
 //   16 columns (bs=1):  5: 3.294  6: 3.249  7: 3.227  8: 3.280  9: 3.299  10: 3.335
 //   32 columns (bs=32): 5: 4.85   6: 4.67   7: 4.68   8: 4.70   9: 4.72   10: 4.76
 //   64 columns (bs=64): 4: 6.85   5: 6.60   6: 6.59   7: 6.59   8: 6.57

@@ -2607,14 +2607,14 @@ static int hy_run_body_t(xb_engine* e, int T, int n_seqs, int n_tiles, void* con
         if (rc != 0) return rc;
         XB_TRY(hy_linear<AT>(e, a2, c.ff, l.w_down, l.t_down, nullptr, T, D, c.ff, hy->m1, hy->cap_m, st, &dn));
       } else {
-      XB_TRY(hy_linear<AT>(e, a1, D, l.w_up, l.t_up, nullptr, T, c.ff, D, hy->P, hy->cap_P, st, &u));
-      const long long n = (long long)T * c.ff;
-      if (std::is_same<AT, bf16>::value && u.h != nullptr && u.bias == nullptr && c.ff % 8 == 0 && u.ld % 8 == 0)
-        XB_TRY(hy_launch(e, hy_relu2_vec_kernel, dim3((unsigned)((n / 8 + 255) / 256)), dim3(256), 0, st, u.h, u.ld, reinterpret_cast<bf16*>(hy->a1),
-                         (long long)c.ff, T, c.ff));
-      else
-        XB_TRY(hy_launch(e, hy_relu2_kernel<AT>, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, st, u, a1, (long long)c.ff, T, c.ff));
-      XB_TRY(hy_linear<AT>(e, a1, c.ff, l.w_down, l.t_down, nullptr, T, D, c.ff, hy->m1, hy->cap_m, st, &dn));
+        XB_TRY(hy_linear<AT>(e, a1, D, l.w_up, l.t_up, nullptr, T, c.ff, D, hy->P, hy->cap_P, st, &u));
+        const long long n = (long long)T * c.ff;
+        if (std::is_same<AT, bf16>::value && u.h != nullptr && u.bias == nullptr && c.ff % 8 == 0 && u.ld % 8 == 0)
+          XB_TRY(hy_launch(e, hy_relu2_vec_kernel, dim3((unsigned)((n / 8 + 255) / 256)), dim3(256), 0, st, u.h, u.ld, reinterpret_cast<bf16*>(hy->a1),
+                           (long long)c.ff, T, c.ff));
+        else
+          XB_TRY(hy_launch(e, hy_relu2_kernel<AT>, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, st, u, a1, (long long)c.ff, T, c.ff));
+        XB_TRY(hy_linear<AT>(e, a1, c.ff, l.w_down, l.t_down, nullptr, T, D, c.ff, hy->m1, hy->cap_m, st, &dn));
       }
       XB_TRY(hy_row_op<AT>(e, T, dn, 1.f, hy_none(), 0.f, l.norm2b, 1.f, has_side ? nullptr : next_norm, (has_side && !side_fused) ? (void*)a1 : nullptr, st));
     }

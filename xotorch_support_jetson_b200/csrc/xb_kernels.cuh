@@ -172,7 +172,7 @@ __global__ void __launch_bounds__(NT) xb_resid_norm_kernel(const float* __restri
   }
 }
 
-// Decode variant: one 1024-thread block per token row, 4 consecutive columns per thread (float4
+// Decode variant: one block of 512, 768 or 1024 threads per token row, 4 consecutive columns per thread (float4
 // reads of the split-K planes), row sum of squares by
 // shuffle + one shared-memory round.  Same arithmetic and rounding points as
 // xb_resid_norm_kernel<., 0>; planes are summed in plane order.  (An 8-block cluster per row with a
@@ -243,10 +243,12 @@ __global__ void __launch_bounds__(NT) xb_norm_row_kernel(const bf16* __restrict_
 }
 
 // F planes of a column and the residual go out together behind the wait, the norm's weights (which wait for no kernel) and the plane counts ahead of it:
-// one trip to L2 for a row, where planes four at a time, then the residual, then the weights took four or five.  From the exit of the Linear before to the
+// one trip to L2 for a row (a second one where a column has more than F planes: 7 of Qwen-2.5-7B's down Linear where F is 6), where planes four at a time, then the
+// residual, then the weights took four or five.  From the exit of the Linear before to the
 // start of the one behind, one row: 6.0 -> 4.1 us at 2048 columns, 6.7 -> 5.0 at 4096 (2.6 of it the two kernel boundaries).  (The bound of one block
-// an SM is what makes the compiler spend registers on loads in flight: without it F = 12 came out in 34 registers, two or three loads at a time.  Not more than
-// 48 K registers a block all the same: the next Linear's block has to find room beside it, or it starts when the norm is done.)
+// an SM is what makes the compiler spend registers on loads in flight: without it F = 12 came out in 34 registers, two or three loads at a time.  F is chosen
+// so that -Xptxas -v shows 79, 63, 47 and 48 registers, 40 to 48 K a block: the next Linear's block has to find room beside it, or it starts when the norm is
+// done; 1024 threads of 64 took the whole SM.)
 template <int NT, int VPT, int F>
 __global__ void __launch_bounds__(NT, 1) xb_resid_norm_row_kernel(const float* __restrict__ part, SplitInfo si,
                                                                long long split_stride, bf16* __restrict__ h,
@@ -587,6 +589,8 @@ __global__ void __launch_bounds__(256) xb_qkv_finalize_kernel(const float* __res
 // are separate bf16 ops in the reference.  Input = split-K partial planes of the fused gate/up
 // projection (decode path; the prefill GEMM does this in its epilogue, xb_gemm.cuh epi_wide_silu).
 // Fused gate/up columns are interleaved in 16-feature blocks; 4 consecutive features per thread.
+// The bound of two blocks an SM leaves the registers for four planes of both in flight (56 instead of 38): part of what took a token of llama-3.2-1b from 767 to 703 us,
+// and at 2 to 128 rows of 3B, 8B and Qwen-2.5-7B within 0.5 % or faster.
 __global__ void __launch_bounds__(256, 2) xb_silu_mul_kernel(const float* __restrict__ part, SplitInfo si, long long split_stride,
                                                           bf16* __restrict__ act, int T, int I) {
   pdl_launch_dependents();

@@ -226,7 +226,8 @@ __device__ __forceinline__ void wide_emit(const GemmArgs& g, int t, const WideQk
 
 // ---- the feed-forwards of hybrid models (ACT = 1): gate and up of the same 128 features are the two halves of a 256-column tile, so the activation leaves
 // from the epilogue in one piece and the matrix of gate and up rows is never written.  1800 rows x 2048 -> 2 x 8192, us: 111.5 with a kernel that read it,
-// 97.6 now (the products alone 91.2), experts 106.8 -> 95.6; 192 rows 26.9 -> 20.8.
+// 97.6 from the epilogue (the products alone 91.2), experts 106.8 -> 95.6; 192 rows 26.9 -> 20.8, all with approximate quotients; the exact ones below cost three
+// layers of bibevik-1b at 1500 rows 2 us of 1315.
 // Four warps finish a tile while the next one is multiplied; with the division's branches, one an element, they took longer than that (110.7 us).  Results have the
 // bits of hy_glu_vec_kernel and hy_moe_act_vec_kernel, so a row's do not hang on which of the two its step takes; the divisions are made without branches: 1 / d by one Newton step on the approximate reciprocal, which for every d from 1 to 2^126 is the correctly rounded one
 // (all 126 * 2^23 of them compared), and from it a / d = q + (a - d q) / d with q = a / d rounded (Markstein 1990), correctly rounded as well.  Sixteen
@@ -603,7 +604,6 @@ static int xb_wide_plan(GemmPlan* p, const bf16* x, long long ldx, const bf16* w
   GemmArgs& g = p->args;
   p->wide = vi;
   p->bn = v.bn;
-  g.a_tiles = (T + 127) / 128;
   g.b_tiles = (N + v.bn - 1) / v.bn;
   g.a_rows = T;
   g.b_rows = N;

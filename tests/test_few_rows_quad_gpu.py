@@ -1,6 +1,5 @@
-"""Gated feed-forwards, experts and logits of hybrid steps of few rows, four columns a thread, against the kernels that take one, on split-K planes (bf16) and
-plain matrices (float32), with vocabularies and widths that do and do not divide by four.  Per element they compute the same; the switch also
-changes the order in which these narrow models sum the squares of a row, which float32 shows at a few 2^-24 a layer and bf16 as roundings that fall the other way."""
+"""Gated feed-forwards, experts and logits of hybrid steps of few rows, four columns a thread, against the kernels that take one, bit for bit: on split-K planes
+(bf16; some columns with more of them than a round fetches) and plain matrices (float32), with vocabularies and widths that do and do not divide by four."""
 import copy
 
 import pytest
@@ -9,11 +8,12 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("model,change", [("bibevik-tiny", {}), ("bibevik-tiny", {"vocab": 386}), ("bibevik-tiny", {"ff": 66}), ("pufivik-tiny", {}), ("vusenex-tiny", {}),
-                                          ("rurutar-tiny", {}), ("sizolorn-tiny", {})])
-@pytest.mark.parametrize("dtype,tol", [("bfloat16", 2e-2), ("float32", 5e-6)])
+# rows of 1024 channels: narrower ones take, with the switch, another kernel for residual + norm as well
+@pytest.mark.parametrize("model,change", [("bibevik-tiny", {}), ("bibevik-tiny", {"vocab": 386}), ("bibevik-tiny", {"ff": 66}), ("bibevik-tiny", {"width": 4096}),
+                                          ("pufivik-tiny", {}), ("vusenex-tiny", {}), ("rurutar-tiny", {}), ("rurutar-tiny", {"width": 4096}), ("sizolorn-tiny", {})])
+@pytest.mark.parametrize("dtype", ["bfloat16", "float32"])
 @pytest.mark.parametrize("rows", [1, 5, 64])
-def test_four_columns_equal_one(built_lib, monkeypatch, model, change, dtype, tol, rows):
+def test_four_columns_equal_one(built_lib, monkeypatch, model, change, dtype, rows):
   import inspect
 
   from xotorch_support_jetson_b200 import model_config, synth
@@ -21,6 +21,7 @@ def test_four_columns_equal_one(built_lib, monkeypatch, model, change, dtype, to
   from xotorch_support_jetson_b200.shard import Shard
   from xotorch_support_jetson_b200.stage import StageRuntime
   hf = copy.deepcopy(model_cards[model]["hf_config"])
+  hf["width"] = change.get("width", 1024)   # 4096: 64 k-blocks over few tiles, a dozen planes and more a column
   if "vocab" in change:
     hf["vocab"] = change["vocab"]
   if "ff" in change:
@@ -40,7 +41,7 @@ def test_four_columns_equal_one(built_lib, monkeypatch, model, change, dtype, to
     outs.append(torch.stack([st.forward(list(range(rows)), [1] * rows, [s] * rows, tokens=ids[s].contiguous()).clone() for s in range(2)]).cpu())
     st.close()
   assert torch.isfinite(outs[0]).all()
-  assert ((outs[0] - outs[1]).norm() / outs[1].norm()).item() < tol
+  assert torch.equal(outs[0], outs[1])
 
 
 @pytest.mark.parametrize("n", [65535, 65536])

@@ -6,9 +6,10 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("D", [648, 2048, 2056, 3072, 3080, 4096, 4104, 8192])
+# (512, 8192): 32 split-K planes a column, where a round fetches 12; (3584, 18944): 7 where it fetches 6
+@pytest.mark.parametrize("D,I", [(648, 512), (2048, 512), (2056, 512), (3072, 512), (3080, 512), (4096, 512), (4104, 512), (8192, 512), (512, 8192), (2056, 16384), (3584, 18944)])
 @pytest.mark.parametrize("kind", ["interleaved", "half-split"])
-def test_token_step_against_prompt_and_cut(built_lib, D, kind):
+def test_token_step_against_prompt_and_cut(built_lib, D, I, kind):
   from oracle import torch_oracle as O
   from xotorch_support_jetson_b200 import models
   from xotorch_support_jetson_b200.shard import Shard
@@ -16,11 +17,11 @@ def test_token_step_against_prompt_and_cut(built_lib, D, kind):
   from xotorch_support_jetson_b200.synth import random_hf_state
   if kind == "interleaved":
     mid, hf = "llama-3.2-tiny", dict(models.model_cards["llama-3.2-tiny"]["hf_config"], hidden_size=D, num_attention_heads=8, num_key_value_heads=2, head_dim=64,
-                                     intermediate_size=512, num_hidden_layers=2)
+                                     intermediate_size=I, num_hidden_layers=2)
   else:   # with biases
     if D % 128:
       pytest.skip("heads of 128 fill the width")
-    mid, hf = "qwen-2.5-widths", models._qwen(D, D // 128, D // 128, 512, 2, vocab=1536, max_pos=4096)
+    mid, hf = "qwen-2.5-widths", models._qwen(D, D // 128, D // 128, I, 2, vocab=1536, max_pos=4096)
   cfg = O.model_config_from_hf(hf)
   state = random_hf_state(hf, seed=3, std=0.05, norm_jitter=0.1)
   n = 140

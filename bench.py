@@ -331,7 +331,7 @@ def run_b200(args):
   else:
     # DRAM bytes per launch of this kernel from the committed `ncu --set full` capture of the N=1 bs=32 step
     # (evidence from a profile run, not re-measured here; stages of an N>1 pipeline hold other matrices: null)
-    for name in ("r02_ncu_traffic.json", "r01_ncu_traffic.json"):
+    for name in ("llama_ncu_traffic.json",):
       prof = ROOT / "profiles" / name
       if prof.exists():
         try:

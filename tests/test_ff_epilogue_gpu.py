@@ -23,10 +23,9 @@ _FF = {
 }
 
 
-def _one_layer(name):
+def _one_layer(mid, at, ff):
   from xotorch_support_jetson_b200 import synth
   from xotorch_support_jetson_b200.models import model_cards
-  mid, at, ff = _FF[name]
   hf = copy.deepcopy(model_cards[mid]["hf_config"])
   hf["layers"] = [hf["layers"][at]]
   hf["layers"][0].pop("weights_of", None)
@@ -57,7 +56,7 @@ def _stream(hf, state, n, dtype):
 @pytest.mark.parametrize("n", [129, 256, 300])
 @pytest.mark.parametrize("gain", [1, 60])   # gates of a few units, and of up to some hundreds
 def test_epilogue_equals_kernel(built_lib, monkeypatch, name, n, gain):
-  _, hf, state = _one_layer(name)
+  _, hf, state = _one_layer(*_FF[name])
   for k in state:
     if k.startswith("l0.mlp.") and (k.endswith("gate") or k.endswith("up")):
       state[k] = state[k] * gain
@@ -72,7 +71,7 @@ def test_epilogue_equals_kernel(built_lib, monkeypatch, name, n, gain):
 
 @pytest.mark.parametrize("name", sorted(_FF))
 def test_epilogue_against_64_bits(built_lib, monkeypatch, name):
-  family, hf, state = _one_layer(name)
+  family, hf, state = _one_layer(*_FF[name])
   n = 140
   monkeypatch.setenv("XB_HY_ACT", "1")
   out, _ = _stream(hf, state, n, "bfloat16")
@@ -83,13 +82,23 @@ def test_epilogue_against_64_bits(built_lib, monkeypatch, name):
     ref = O.forward(hf, state, ids)[1][-1]
   elif family == "rurutar":
     ref = torch.as_tensor(O.forward(state, hf, ids, want_layers=True)[1][-1])
-  elif family == "pufivik":
-    ref = O.forward(hf, state, ids, return_layers=True)[1][-1]
   else:
     ref = O.forward(hf, state, ids, return_layers=True)[1][-1]
   rows = (out - torch.as_tensor(ref).double()).norm(dim=1) / torch.as_tensor(ref).double().norm(dim=1)
   # a chain of bf16 roundings (2^-9 each) from norm to norm: their spread is a few of them in every row; a router that ties sends single rows to another expert
   assert rows.quantile(0.9) < 0.02
+
+
+def test_rows_at_which_the_choice_flips(built_lib, monkeypatch):
+  """160 -> 2 x 2048 by the estimate: a kernel of its own up to 512 rows, the epilogue from 513 on."""
+  _, hf, state = _one_layer("rurutar-tiny", 0, {"kind": "dense", "ff": 2048})
+  for n in (512, 513):
+    monkeypatch.delenv("XB_HY_ACT", raising=False)
+    own, launches = _stream(hf, state, n, "bfloat16")
+    monkeypatch.setenv("XB_HY_ACT", "0")
+    kernel, more = _stream(hf, state, n, "bfloat16")
+    assert more - launches == n - 512
+    assert torch.equal(own, kernel)
 
 
 def test_layers_that_share_weights_keep_their_limits(built_lib, monkeypatch):
